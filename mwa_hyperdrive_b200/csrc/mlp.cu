@@ -8,11 +8,14 @@
 // correction to the centre input).  Training minimises the mean squared error
 // with Adam.
 //
-// Kernels: one tiled SGEMM (64x64 output tile per 256-thread CTA, 4x4 per
-// thread, K staged through shared memory 16 at a time) with transpose flags
-// and a fused bias + ReLU epilogue, a bias-gradient column reduction, the
-// ReLU backward mask, the MSE gradient and the Adam update.
+// Kernels: one tiled SGEMM body (64x64 output tile per 256-thread CTA, 4x4
+// per thread, K staged through shared memory 16 at a time, the next stage
+// read into registers meanwhile) with transpose flags and a fused epilogue
+// (bias, ReLU, the residual slice, or the ReLU backward mask), the MSE
+// gradient, every layer's weight and bias gradient in one launch split over
+// the batch, the sum of those splits and the Adam update.
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <random>
@@ -25,48 +28,87 @@ namespace mlp {
 
 constexpr int TM = 64, TN = 64, TK = 16;
 
-// C[M][N] (row-major, ldc) = op(A) op(B) (+ bias[N]) (relu), where
-// op(A)[m][k] = TA ? A[k][m] : A[m][k] (lda) and op(B)[k][n] = TB ? B[n][k] : B[k][n] (ldb).
-// beta: 0 overwrite, 1 accumulate.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int lda,
-                                                    const float* __restrict__ B, int ldb, float* __restrict__ C,
-                                                    int ldc, const float* __restrict__ bias, int relu, float beta) {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+// What a GEMM adds to or does with its sums.
+struct Epilogue {
+    const float* bias = nullptr;      // [N], added
+    const float* residual = nullptr;  // [M][residual_ld], added after the bias
+    int residual_ld = 0;
+    const float* mask = nullptr;      // [M][N]: 0 where mask <= 0 (ReLU backward)
+    bool relu = false;
+};
+
+// Four consecutive elements of a row of n from column j (zero past its end);
+// VEC: rows start 16-byte aligned and n is a multiple of 4.
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* __restrict__ row, int j, int n) {
+    if (VEC) return j < n ? __ldg(reinterpret_cast<const float4*>(row + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(j < n ? row[j] : 0.f, j + 1 < n ? row[j + 1] : 0.f, j + 2 < n ? row[j + 2] : 0.f,
+                       j + 3 < n ? row[j + 3] : 0.f);
+}
+
+struct Tiles {
+    alignas(16) float a[TK][TM + 4];
+    alignas(16) float b[TK][TN + 4];
+};
+
+// One 64 x 64 tile at (m0, n0) of C[M][N] = op(A) op(B) over k in [k0, k1)
+// (k0 a multiple of TK), op(A)[m][k] = TA ? A[k][m] : A[m][k], op(B)[k][n] =
+// TB ? B[n][k] : B[k][n]; the sums run over k in order.  colsum (TA only,
+// may be null): colsum[m] = sum_k A[k][m], by the tiles of column n0 = 0.
+template <bool TA, bool TB, bool VEC>
+__device__ __forceinline__ void gemm_tile(Tiles& t, int M, int N, int m0, int n0, int k0, int k1,
+                                          const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb,
+                                          float* __restrict__ C, int ldc, const Epilogue& ep,
+                                          float* __restrict__ colsum) {
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    // this thread's four elements of a stage: along m (n) at one k when the
+    // operand is stored that way round, else along k at one m (n)
+    const int ka = TA ? tid / 16 : (tid % 4) * 4, ma = TA ? (tid % 16) * 4 : tid / 4;
+    const int kb = TB ? (tid % 4) * 4 : tid / 16, nb = TB ? tid / 4 : (tid % 16) * 4;
+    float4 ra, rb;
+    auto fetch = [&](int k) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (TA)
+            ra = k + ka < k1 ? load4<VEC>(A + (size_t)(k + ka) * lda, m0 + ma, M) : zero;
+        else
+            ra = m0 + ma < M ? load4<VEC>(A + (size_t)(m0 + ma) * lda, k + ka, k1) : zero;
+        if (TB)
+            rb = n0 + nb < N ? load4<VEC>(B + (size_t)(n0 + nb) * ldb, k + kb, k1) : zero;
+        else
+            rb = k + kb < k1 ? load4<VEC>(B + (size_t)(k + kb) * ldb, n0 + nb, N) : zero;
+    };
     float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int i = threadIdx.x; i < TK * TM; i += 256) {
-            const int kk = i / TM, mm = i % TM;
-            const int m = m0 + mm, k = k0 + kk;
-            float v = 0.f;
-            if (m < M && k < K) v = TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-            As[kk][mm] = v;
+    float cs = 0.f;
+    fetch(k0);
+    for (int k = k0; k < k1; k += TK) {
+        __syncthreads();  // the previous stage has been read
+        if (TA) {
+            *reinterpret_cast<float4*>(&t.a[ka][ma]) = ra;
+        } else {
+            t.a[ka][ma] = ra.x, t.a[ka + 1][ma] = ra.y, t.a[ka + 2][ma] = ra.z, t.a[ka + 3][ma] = ra.w;
         }
-        for (int i = threadIdx.x; i < TK * TN; i += 256) {
-            const int kk = i / TN, nn = i % TN;
-            const int n = n0 + nn, k = k0 + kk;
-            float v = 0.f;
-            if (n < N && k < K) v = TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n];
-            Bs[kk][nn] = v;
+        if (TB) {
+            t.b[kb][nb] = rb.x, t.b[kb + 1][nb] = rb.y, t.b[kb + 2][nb] = rb.z, t.b[kb + 3][nb] = rb.w;
+        } else {
+            *reinterpret_cast<float4*>(&t.b[kb][nb]) = rb;
         }
         __syncthreads();
+        if (k + TK < k1) fetch(k + TK);
+        if (TA && colsum && n0 == 0 && tid < TM)
+#pragma unroll
+            for (int kk = 0; kk < TK; kk++) cs += t.a[kk][tid];
 #pragma unroll
         for (int kk = 0; kk < TK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+            const float4 av = *reinterpret_cast<const float4*>(&t.a[kk][ty * 4]);
+            const float4 bv = *reinterpret_cast<const float4*>(&t.b[kk][tx * 4]);
+            const float a[4] = {av.x, av.y, av.z, av.w}, b[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
     }
+    if (TA && colsum && n0 == 0 && tid < TM && m0 + tid < M) colsum[m0 + tid] = cs;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int m = m0 + ty * 4 + i;
@@ -76,28 +118,85 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
             const int n = n0 + tx * 4 + j;
             if (n >= N) continue;
             float v = acc[i][j];
-            if (bias) v += bias[n];
-            if (relu) v = fmaxf(v, 0.f);
-            float* c = C + (size_t)m * ldc + n;
-            *c = beta != 0.f ? *c + v : v;
+            if (ep.bias) v += ep.bias[n];
+            if (ep.residual) v += ep.residual[(size_t)m * ep.residual_ld + n];
+            if (ep.relu) v = fmaxf(v, 0.f);
+            if (ep.mask && ep.mask[(size_t)m * N + n] <= 0.f) v = 0.f;
+            C[(size_t)m * ldc + n] = v;
         }
     }
 }
 
-template <bool TA, bool TB>
-static cudaError_t sgemm(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                         const float* bias, bool relu, float beta, cudaStream_t s) {
+template <bool TB, bool VEC>
+__global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int lda,
+                                                    const float* __restrict__ B, int ldb, float* __restrict__ C,
+                                                    int ldc, const Epilogue ep) {
+    __shared__ Tiles t;
+    gemm_tile<false, TB, VEC>(t, M, N, blockIdx.y * TM, blockIdx.x * TN, 0, K, A, lda, B, ldb, C, ldc, ep, nullptr);
+}
+
+// Rows of both operands can be read as 16-byte vectors.
+static bool vec_ok(const float* A, int lda, const float* B, int ldb) {
+    return ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0 && lda % 4 == 0 && ldb % 4 == 0;
+}
+
+// C = A op(B) with the epilogue; the rows of op(B)'s storage and of A are
+// their leading dimensions long.
+template <bool TB>
+static cudaError_t sgemm(int M, int N, int K, const float* A, const float* B, float* C, const Epilogue& ep,
+                         cudaStream_t s) {
+    const int lda = K, ldb = TB ? K : N;
     dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-    sgemm_kernel<TA, TB><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, relu ? 1 : 0, beta);
+    if (vec_ok(A, lda, B, ldb))
+        sgemm_kernel<TB, true><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, N, ep);
+    else
+        sgemm_kernel<TB, false><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, N, ep);
     count_launches(1);
     return cudaGetLastError();
 }
 
-__global__ void add_residual_kernel(float* y, const float* x, int batch, int out_dim, int in_dim, int offset) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= batch * out_dim) return;
-    const int b = i / out_dim, j = i % out_dim;
-    y[i] += x[(size_t)b * in_dim + offset + j];
+// Weight and bias gradients of every layer in one launch: layer l's tiles of
+// dW_l = delta_{l+1}^T y_l ([out][in], over the batch) start at tile0; grid
+// (tiles of all layers, splits), split z sums rows [z rows, (z + 1) rows) of
+// the batch into part[z][parameter].  A layer's own 4 to 16 tiles would leave
+// most SMs idle over a batch of thousands (one launch per layer, no splits:
+// 1.1 ms each at a batch of 4096 with 256 hidden units).
+constexpr int MAXL = 8;  // layers per launch
+struct GradLayer {
+    const float *delta, *y;  // [batch][out], [batch][in]
+    int out, in, tile0, vec;
+    size_t w_off, b_off;
+};
+struct GradArgs {
+    GradLayer l[MAXL];
+    int nl, batch, rows;
+    float* part;
+    size_t nparams;
+};
+__global__ void __launch_bounds__(256) grad_kernel(const __grid_constant__ GradArgs G) {
+    __shared__ Tiles t;
+    int l = 0;
+    while (l + 1 < G.nl && (int)blockIdx.x >= G.l[l + 1].tile0) l++;
+    const GradLayer& L = G.l[l];
+    const int tile = blockIdx.x - L.tile0, ncol = (L.in + TN - 1) / TN;
+    const int m0 = tile / ncol * TM, n0 = tile % ncol * TN;
+    const int k0 = blockIdx.y * G.rows, k1 = min(G.batch, k0 + G.rows);
+    float* out = G.part + (size_t)blockIdx.y * G.nparams;
+    if (L.vec)
+        gemm_tile<true, false, true>(t, L.out, L.in, m0, n0, k0, k1, L.delta, L.out, L.y, L.in, out + L.w_off, L.in,
+                                     Epilogue{}, out + L.b_off);
+    else
+        gemm_tile<true, false, false>(t, L.out, L.in, m0, n0, k0, k1, L.delta, L.out, L.y, L.in, out + L.w_off, L.in,
+                                      Epilogue{}, out + L.b_off);
+}
+
+// g[i] = sum of the splits' parts, in order
+__global__ void grad_sum_kernel(const float* __restrict__ part, int splits, size_t n, float* __restrict__ g) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float v = 0.f;
+    for (int z = 0; z < splits; z++) v += part[z * n + i];
+    g[i] = v;
 }
 
 // d = 2 (y - t) / (batch * out_dim); loss partial sums per block
@@ -119,26 +218,6 @@ __global__ void mse_grad_kernel(const float* y, const float* t, float* d, int n,
     if (threadIdx.x == 0) atomicAdd(loss, red[0]);
 }
 
-__global__ void relu_backward_kernel(float* d, const float* act, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && act[i] <= 0.f) d[i] = 0.f;
-}
-
-// db[n] = sum_b d[b][n]
-__global__ void bias_grad_kernel(const float* d, float* db, int batch, int n) {
-    const int j = blockIdx.x;
-    float s = 0.f;
-    for (int b = threadIdx.x; b < batch; b += blockDim.x) s += d[(size_t)b * n + j];
-    __shared__ float red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[j] = red[0];
-}
-
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2,
                             float eps, float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,17 +236,26 @@ struct Net {
     float *d_params = nullptr, *d_grads = nullptr, *d_m = nullptr, *d_v = nullptr;
     size_t nparams = 0;
     std::vector<size_t> w_off, b_off;
-    // activations for training
+    // activations for training (acts[0] is unused: layer 0 reads the caller's
+    // input) and the gradient's parts per batch split
     std::vector<float*> acts, deltas;
+    float* d_part = nullptr;
     int cap_batch = 0;
     double* d_loss = nullptr;
     long long step = 0;
 
     int layers() const { return (int)dims.size() - 1; }
 
+    // Batch splits of the weight gradients: 256 rows each, at most 32 (a batch
+    // of 4096 fills the SMs twice over with 16; more parts cost more traffic
+    // than they save).
+    static int splits(int batch) { return std::min(32, (batch + 255) / 256); }
+
     void free_acts() {
         for (float* p : acts) cudaFree(p);
         for (float* p : deltas) cudaFree(p);
+        cudaFree(d_part);
+        d_part = nullptr;
         acts.clear();
         deltas.clear();
         cap_batch = 0;
@@ -176,16 +264,21 @@ struct Net {
     int ensure(int batch) {
         if (batch <= cap_batch) return HDC_OK;
         free_acts();
+        bool ok = cudaMalloc(&d_part, sizeof(float) * nparams * splits(batch)) == cudaSuccess;
         for (int l = 0; l <= layers(); l++) {
             float *a = nullptr, *d = nullptr;
-            if (cudaMalloc(&a, sizeof(float) * (size_t)batch * dims[l]) != cudaSuccess ||
-                cudaMalloc(&d, sizeof(float) * (size_t)batch * dims[l]) != cudaSuccess) {
-                cudaGetLastError();
-                set_error("mlp: activation allocation failed");
-                return HDC_ERR_ALLOC;
+            if (l > 0) {
+                ok = ok && cudaMalloc(&a, sizeof(float) * (size_t)batch * dims[l]) == cudaSuccess;
+                ok = ok && cudaMalloc(&d, sizeof(float) * (size_t)batch * dims[l]) == cudaSuccess;
             }
             acts.push_back(a);
             deltas.push_back(d);
+        }
+        if (!ok) {
+            free_acts();
+            cudaGetLastError();
+            set_error("mlp: activation allocation failed");
+            return HDC_ERR_ALLOC;
         }
         cap_batch = batch;
         return HDC_OK;
@@ -200,51 +293,61 @@ struct Net {
         cudaFree(d_loss);
     }
 
-    // forward into acts[0..L] (acts[0] = x copy), returns output pointer
-    int forward(const float* d_x, int batch, cudaStream_t s) {
+    // forward through acts[1..L]; the output into d_y (acts[L] when NULL)
+    int forward(const float* d_x, int batch, float* d_y, cudaStream_t s) {
         int rc = ensure(batch);
         if (rc) return rc;
-        HDC_CUDA_RET_INT(cudaMemcpyAsync(acts[0], d_x, sizeof(float) * (size_t)batch * dims[0],
-                                         cudaMemcpyDeviceToDevice, s));
         for (int l = 0; l < layers(); l++) {
             const bool last = l == layers() - 1;
-            HDC_CUDA_RET_INT((sgemm<false, true>(batch, dims[l + 1], dims[l], acts[l], dims[l], d_params + w_off[l],
-                                                 dims[l], acts[l + 1], dims[l + 1], d_params + b_off[l], !last, 0.f,
-                                                 s)));
-        }
-        if (residual_offset >= 0) {
-            const int n = batch * dims.back();
-            add_residual_kernel<<<(n + 255) / 256, 256, 0, s>>>(acts.back(), acts[0], batch, dims.back(), dims[0],
-                                                                residual_offset);
-            count_launches(1);
-            HDC_CUDA_RET_INT(cudaGetLastError());
+            Epilogue ep;
+            ep.bias = d_params + b_off[l];
+            ep.relu = !last;
+            if (last && residual_offset >= 0) {
+                ep.residual = d_x + residual_offset;
+                ep.residual_ld = dims[0];
+            }
+            HDC_CUDA_RET_INT((sgemm<true>(batch, dims[l + 1], dims[l], l == 0 ? d_x : acts[l], d_params + w_off[l],
+                                          last && d_y ? d_y : acts[l + 1], ep, s)));
         }
         return HDC_OK;
     }
 
-    // gradients of the mean squared error into d_grads; loss (sum of squares / n) to *loss
-    int backward(const float* d_target, int batch, double* h_loss, cudaStream_t s) {
+    // gradients of the mean squared error into d_grads after forward() of the
+    // same d_x; loss (sum of squares / n) to *loss
+    int backward(const float* d_x, const float* d_target, int batch, double* h_loss, cudaStream_t s) {
         const int L = layers();
         const int n = batch * dims[L];
         HDC_CUDA_RET_INT(cudaMemsetAsync(d_loss, 0, sizeof(double), s));
         mse_grad_kernel<<<(n + 255) / 256, 256, 0, s>>>(acts[L], d_target, deltas[L], n, 1.f / (float)n, d_loss);
         count_launches(1);
-        for (int l = L - 1; l >= 0; l--) {
-            // dW_l = delta_{l+1}^T y_l : [out][in];  db_l = colsum(delta_{l+1})
-            HDC_CUDA_RET_INT((sgemm<true, false>(dims[l + 1], dims[l], batch, deltas[l + 1], dims[l + 1], acts[l],
-                                                 dims[l], d_grads + w_off[l], dims[l], nullptr, false, 0.f, s)));
-            bias_grad_kernel<<<dims[l + 1], 256, 0, s>>>(deltas[l + 1], d_grads + b_off[l], batch, dims[l + 1]);
-            count_launches(1);
-            if (l > 0) {
-                // delta_l = (delta_{l+1} W_l) * relu'(y_l)
-                HDC_CUDA_RET_INT((sgemm<false, false>(batch, dims[l], dims[l + 1], deltas[l + 1], dims[l + 1],
-                                                      d_params + w_off[l], dims[l], deltas[l], dims[l], nullptr, false,
-                                                      0.f, s)));
-                const int nl = batch * dims[l];
-                relu_backward_kernel<<<(nl + 255) / 256, 256, 0, s>>>(deltas[l], acts[l], nl);
-                count_launches(1);
-            }
+        // delta_l = (delta_{l+1} W_l) * relu'(y_l)
+        for (int l = L - 1; l > 0; l--) {
+            Epilogue ep;
+            ep.mask = acts[l];
+            HDC_CUDA_RET_INT((sgemm<false>(batch, dims[l], dims[l + 1], deltas[l + 1], d_params + w_off[l], deltas[l],
+                                           ep, s)));
         }
+        const int ns = splits(batch);
+        for (int l0 = 0; l0 < L; l0 += MAXL) {
+            GradArgs G;
+            G.nl = std::min(MAXL, L - l0);
+            G.batch = batch;
+            G.rows = ((batch + ns - 1) / ns + TK - 1) / TK * TK;
+            G.part = d_part;
+            G.nparams = nparams;
+            int tiles = 0;
+            for (int i = 0; i < G.nl; i++) {
+                const int l = l0 + i;
+                const float* y = l == 0 ? d_x : acts[l];
+                G.l[i] = GradLayer{deltas[l + 1], y, dims[l + 1], dims[l], tiles, vec_ok(deltas[l + 1], dims[l + 1], y, dims[l]),
+                                   w_off[l], b_off[l]};
+                tiles += ((dims[l + 1] + TM - 1) / TM) * ((dims[l] + TN - 1) / TN);
+            }
+            grad_kernel<<<dim3(tiles, ns), 256, 0, s>>>(G);
+            count_launches(1);
+        }
+        grad_sum_kernel<<<(unsigned)((nparams + 255) / 256), 256, 0, s>>>(d_part, ns, nparams, d_grads);
+        count_launches(1);
         HDC_CUDA_RET_INT(cudaGetLastError());
         if (h_loss) {
             double l = 0.0;
@@ -336,10 +439,12 @@ extern "C" int hdc_mlp_set_params(HdcMlp* hm, const float* h_in) {
 extern "C" int hdc_mlp_forward(HdcMlp* hm, const float* d_x, int batch, float* d_y, hdcStream_t stream) {
     Net* n = reinterpret_cast<Net*>(hm);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = n->forward(d_x, batch, s);
-    if (rc) return rc;
-    HDC_CUDA_RET_INT(cudaMemcpyAsync(d_y, n->acts.back(), sizeof(float) * (size_t)batch * n->dims.back(),
-                                     cudaMemcpyDeviceToDevice, s));
+    // an output that overlaps the input is written once the input has been read
+    const size_t nx = (size_t)batch * n->dims.front(), ny = (size_t)batch * n->dims.back();
+    const bool overlap = d_y < d_x + nx && d_x < d_y + ny;
+    int rc = n->forward(d_x, batch, overlap ? nullptr : d_y, s);
+    if (rc || !overlap) return rc;
+    HDC_CUDA_RET_INT(cudaMemcpyAsync(d_y, n->acts.back(), sizeof(float) * ny, cudaMemcpyDeviceToDevice, s));
     return HDC_OK;
 }
 
@@ -347,9 +452,9 @@ extern "C" int hdc_mlp_gradients(HdcMlp* hm, const float* d_x, const float* d_ta
                                  double* h_loss, hdcStream_t stream) {
     Net* n = reinterpret_cast<Net*>(hm);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = n->forward(d_x, batch, s);
+    int rc = n->forward(d_x, batch, nullptr, s);
     if (rc) return rc;
-    rc = n->backward(d_target, batch, h_loss, s);
+    rc = n->backward(d_x, d_target, batch, h_loss, s);
     if (rc) return rc;
     if (h_grads) {
         HDC_CUDA_RET_INT(cudaMemcpyAsync(h_grads, n->d_grads, sizeof(float) * n->nparams, cudaMemcpyDeviceToHost, s));
@@ -362,9 +467,9 @@ extern "C" int hdc_mlp_train_step(HdcMlp* hm, const float* d_x, const float* d_t
                                   double* h_loss, hdcStream_t stream) {
     Net* n = reinterpret_cast<Net*>(hm);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = n->forward(d_x, batch, s);
+    int rc = n->forward(d_x, batch, nullptr, s);
     if (rc) return rc;
-    rc = n->backward(d_target, batch, h_loss, s);
+    rc = n->backward(d_x, d_target, batch, h_loss, s);
     if (rc) return rc;
     n->step++;
     const float b1 = 0.9f, b2 = 0.999f;
