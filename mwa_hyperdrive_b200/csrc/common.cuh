@@ -236,14 +236,40 @@ __device__ __forceinline__ void hadec_to_azel(double ha, double dec, double lat,
     el = atan2(z, r);
 }
 
-// FP64 phasor exp(2 pi i t) for a phase in turns: exact range reduction to
-// r = t - rint(t) in [-1/2, 1/2], then sincospi(2 r).
-__device__ __forceinline__ cplx phasor_turns(double t) {
-    double r = t - rint(t);
-    double s, c;
-    sincospi(2.0 * r, &s, &c);
-    return {c, s};
+constexpr double QMAGIC = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer held in the low word
+
+// FP64 phasor exp(2 pi i z / 4) for z in quarter-turns, |z| < 2^51: q =
+// rint(z) and r = z - q are exact; sin and cos of (pi/2) r on |r| <= 1/2 from
+// polynomials in r^2 (interpolated at Chebyshev nodes by
+// mwa_hyperdrive_b200/phasor_poly.py, within an ulp); the quadrant q mod 4
+// swaps and signs them.  18 FP64 operations, where sincospi takes about 40
+// and twice the integer ones.
+constexpr double QS0 = 1.57079632679489656e+00, QS1 = -6.45964097506244284e-01, QS2 = 7.96926262460435075e-02,
+                 QS3 = -4.68175413235088697e-03, QS4 = 1.60441150826272252e-04, QS5 = -3.59864367056375883e-06,
+                 QS6 = 5.63397775242345925e-08;
+constexpr double QC0 = -1.23370055013616975e+00, QC1 = 2.53669507901047864e-01, QC2 = -2.08634807633418309e-02,
+                 QC3 = 9.19260274564273204e-04, QC4 = -2.52020391586849619e-05, QC5 = 4.71068295306692582e-07,
+                 QC6 = -6.32999298457005379e-09;
+
+__device__ __forceinline__ cplx phasor_quarter_f64(double z) {
+    const double zq = __dadd_rn(z, QMAGIC);
+    const int q = __double2loint(zq);
+    const double r = __dsub_rn(z, __dsub_rn(zq, QMAGIC));
+    const double r2 = r * r;
+    const double ps = fma(fma(fma(fma(fma(fma(QS6, r2, QS5), r2, QS4), r2, QS3), r2, QS2), r2, QS1), r2, QS0) * r;
+    const double pc =
+        fma(fma(fma(fma(fma(fma(fma(QC6, r2, QC5), r2, QC4), r2, QC3), r2, QC2), r2, QC1), r2, QC0), r2, 1.0);
+    // as phasor_quarter_f32: odd q swaps sin and cos, bit 1 of q (q + 1) signs sin (cos)
+    const bool odd = q & 1;
+    const double a = odd ? pc : ps, b = odd ? ps : pc;
+    const uint32_t qs = (uint32_t)q << 30;
+    return {__hiloint2double(__double2hiint(b) ^ (int)((qs + 0x40000000u) & 0x80000000u), __double2loint(b)),
+            __hiloint2double(__double2hiint(a) ^ (int)(qs & 0x80000000u), __double2loint(a))};
 }
+
+// FP64 phasor exp(2 pi i t) for a phase in turns: exact range reduction to
+// r = t - rint(t) in [-1/2, 1/2] first, so any size of t is good.
+__device__ __forceinline__ cplx phasor_turns(double t) { return phasor_quarter_f64(4.0 * (t - rint(t))); }
 
 // FP32 phasor for the tensor-core predict and the chosen form's direct
 // kernels: sin and cos of 2 pi z for z in quarter-turns.  q = rint(z) and
@@ -251,7 +277,6 @@ __device__ __forceinline__ cplx phasor_turns(double t) {
 // least-squares polynomials in r^2 on |r| <= 1/2 (fitted by
 // mwa_hyperdrive_b200/phasor_poly.py, < 0.75 float32 ulp); the quadrant
 // q mod 4 swaps and signs them.
-constexpr double QMAGIC = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer held in the low word
 constexpr float PS0 = 1.570796371e+00f, PS1 = -6.459634900e-01f, PS2 = 7.968021929e-02f,
                 PS3 = -4.602163099e-03f;
 constexpr float PC0 = 1.000000000e+00f, PC1 = -1.233700514e+00f, PC2 = 2.536692023e-01f,

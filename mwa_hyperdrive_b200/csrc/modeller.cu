@@ -278,6 +278,7 @@ void TypeTables::release() {
     dfree(d_ccount);
     dfree(d_suv_tile);
     dfree(d_sdense);
+    dfree(d_sdense64);
     nc = 0;
 }
 
@@ -411,9 +412,19 @@ int Modeller::build_tables(const HdcSkyModel* sky) {
                         const double sgn = ((sc.n1 + sc.n2) & 3) < 2 ? 1.0 : -1.0;
                         dm[((size_t)k * SDN + sc.n1) * SDN + sc.n2] += sgn * sc.value;
                     }
-                std::vector<float> df(dm.begin(), dm.end());
-                HDC_CUDA_RET_INT(dalloc(&tt.d_sdense, df.size()));
-                HDC_CUDA_RET_INT(cudaMemcpy(tt.d_sdense, df.data(), sizeof(float) * df.size(), cudaMemcpyHostToDevice));
+                if (form == HDC_PREDICT_TENSOR) {
+                    std::vector<float> df(dm.begin(), dm.end());
+                    HDC_CUDA_RET_INT(dalloc(&tt.d_sdense, df.size()));
+                    HDC_CUDA_RET_INT(cudaMemcpy(tt.d_sdense, df.data(), sizeof(float) * df.size(),
+                                                cudaMemcpyHostToDevice));
+                }
+                // the form factored by tile: 1 / sqrt(2^n n!) of both axes folded in
+                double norm[SDN];
+                for (int q = 0; q < SDN; q++) norm[q] = 1.0 / std::sqrt(std::ldexp(std::tgamma(q + 1.0), q));
+                for (size_t i = 0; i < dm.size(); i++) dm[i] *= norm[(i / SDN) % SDN] * norm[i % SDN];
+                HDC_CUDA_RET_INT(dalloc(&tt.d_sdense64, dm.size()));
+                HDC_CUDA_RET_INT(cudaMemcpy(tt.d_sdense64, dm.data(), sizeof(double) * dm.size(),
+                                            cudaMemcpyHostToDevice));
             }
         }
     }
@@ -571,6 +582,7 @@ DirectParams Modeller::direct_params(int ty, void* vis) const {
     p.coeffs = t[ty].d_coeffs;
     p.coeff_start = t[ty].d_cstart;
     p.coeff_count = t[ty].d_ccount;
+    p.sdense64 = t[ty].d_sdense64;
     p.suv_bl = nullptr;
     p.suv_tile = t[ty].d_suv_tile;
     if (tile_beams()) {
@@ -584,6 +596,25 @@ DirectParams Modeller::direct_params(int ty, void* vis) const {
     p.vis = vis;
     p.err = d_err;
     return p;
+}
+
+// This timestep's baseline UVWs are differences of the tiles' (geometry()).
+void Modeller::set_tile_geometry(DirectParams& p, double lst) const {
+    const double ha = lst - pc.ra;
+    p.xyzs = d_xyzs;
+    // the centroid of the tiles whose positions are finite (others spoil only
+    // their own baselines)
+    p.xyz0 = XYZ{0.0, 0.0, 0.0};
+    for (const XYZ& x : xyzs) {
+        if (!std::isfinite(x.x + x.y + x.z)) continue;
+        p.xyz0.x += x.x / ntiles;
+        p.xyz0.y += x.y / ntiles;
+        p.xyz0.z += x.z / ntiles;
+    }
+    p.s_ha = std::sin(ha);
+    p.c_ha = std::cos(ha);
+    p.s_dec = std::sin(pc.dec);
+    p.c_dec = std::cos(pc.dec);
 }
 
 void Modeller::prof_begin(int cls, cudaStream_t s, EvPair& e) {
@@ -646,6 +677,7 @@ int Modeller::model_channels(double lst, void* d_vis, bool out64, int f0, int nf
             // direct kernel, in its FP32 form with a shared beam (FP64 with
             // per-tile beams)
             DirectParams p = direct_params(ty, vis);
+            set_tile_geometry(p, lst);
             p.nf = nfc;
             p.freqs = d_freqs + f0;
             p.flux = p.flux + (size_t)f0 * p.nc;

@@ -19,6 +19,7 @@ struct TypeTables {
     int* d_ccount = nullptr;
     double2* d_suv_tile = nullptr;  // [nc][ntiles]
     float* d_sdense = nullptr;      // [nc][SDN][SDN] signed dense coefficients, or NULL
+    double* d_sdense64 = nullptr;   // the same in FP64 with the basis functions' normalisation (direct form), or NULL
     JonesF64* d_B = nullptr;        // per-tile beams: [uniq tile][uniq freq][nc] at the current timestep
     JonesF32* d_B32 = nullptr;      // the same in FP32 (points in the tensor form: its producers' reads)
     void release();
@@ -102,6 +103,7 @@ struct Modeller {
     int geometry(double lst, cudaStream_t s);
     const JonesF64* weights(int ty) const;
     DirectParams direct_params(int ty, void* vis) const;
+    void set_tile_geometry(DirectParams& p, double lst) const;
     int model(double lst, void* d_vis, bool out64, UVW* h_uvws, cudaStream_t s);
     // the predict kernels of channels [f0, f0 + nfc) after geometry(); d_vis
     // is the whole [nf][nbl] visibility array.  Classes (types bit-set: 1

@@ -1,0 +1,357 @@
+// The native modeller's FP64 predict (HDC_PREDICT_DIRECT), factored by tile.
+//
+// A native modeller's baseline UVW is a tile difference (uvw_pq = uvw_p -
+// uvw_q), so the phasor of a term factors: exp(2 pi i t_pq) = A_p conj(A_q)
+// with A_p = exp(2 pi i (u_p l + v_p m + w_p (n - 1))), and an envelope's
+// coordinates are differences of per-tile ones.  A CTA takes a 32 x 32 block
+// of tile pairs of one channel (blocks on or above the diagonal) and, per
+// staged chunk of components, forms in shared memory the 64 tiles' phasors
+// (and Gaussian or shapelet coordinates); its 256 threads then take 2 x 2
+// pairs each, so one FP64 sincos serves 16 baselines and a pair costs a
+// complex product (4 operations) instead of a sincos.
+//
+// Shared beam (or none): W = B S B^H is Hermitian, so with W_xy = a + i b the
+// four correlations come from the sums of w_xx z, w_yy z, a z and b z (8
+// fused multiply-adds a term; XY = P + i Q and YX = P - i Q at the end).
+// Per-tile beams: M_p = A_p B_p S and N_q = A_q B_q are formed per tile, and
+// a term is M_p N_q^H (32 fused multiply-adds).
+//
+// Bound: the FP64 pipe (64 lanes per clock and SM; 0.64 busy over the points'
+// sweep and tables) and, level with it, shared-memory reads (96 bytes a lane
+// and component of the four pairs, 128 bytes a clock).  128 tiles x 384
+// channels x 1000 points: 13.2 ms with a thread per baseline, 4.3 with the
+// library's sincospi, 4.0 so; 1 x 2 pairs a thread 4.3, 4 x 2 at half the
+// warps 4.8.  Every value is FP64,
+// tile positions are taken from the array's centroid (so a tile's phase is no
+// larger than its baselines'), and sums run over the components in order.
+// The drop-in calls keep the per-baseline kernel (predict.cu): their UVWs
+// are the caller's and need not be tile differences.
+
+#include <type_traits>
+
+#include "predict.cuh"
+
+namespace hdc {
+namespace pairs {
+
+constexpr int TB = 32;     // tiles per block side
+constexpr int NTH = 256;   // 16 x 16 threads of 2 x 2 pairs
+constexpr int RI = 2;      // rows per thread, two columns (all 16 apart)
+
+// Tile's UVW from the array's centroid in wavelengths (ool = frequency / c).
+__device__ __forceinline__ void tile_uvw(const DirectParams& p, int tile, double ool, double& u, double& v, double& w) {
+    const XYZ a = p.xyzs[tile];
+    const double x = a.x - p.xyz0.x, y = a.y - p.xyz0.y, z = a.z - p.xyz0.z;
+    u = (p.s_ha * x + p.c_ha * y) * ool;
+    v = (-p.s_dec * p.c_ha * x + p.s_dec * p.s_ha * y + p.c_dec * z) * ool;
+    w = (p.c_dec * p.c_ha * x - p.c_dec * p.s_ha * y + p.s_dec * z) * ool;
+}
+
+// components per staged chunk: what fits 48 KB of static shared memory with
+// the per-tile tables
+template <int TYPE, bool TILE>
+struct Shape {
+    static constexpr int CH = TILE ? 8 : (TYPE == 0 ? 32 : 16);
+};
+
+// Linear interpolation between the tabulated basis values around position
+// pos (in table steps from the first entry), as sums over the dimensionless
+// Hermite polynomials: out[n] = H_n(x0) e0 (1 - frac) + H_n(x1) e1 frac with
+// x0, x1 the table's grid points and e = exp(-x^2 / 2); the factors
+// 1 / sqrt(2^n n!) are folded into the coefficients.  Evaluating the two
+// grid points (about 75 FP64 operations an axis) replaces twelve scattered
+// 16-byte loads, which cost a warp some 380 L1 cycles.
+__device__ __forceinline__ void hermite_interp(double pos, double (&out)[SDN]) {
+    const double fl = floor(pos);
+    const double frac = pos - fl;
+    // positions outside the table take its first or last interval, where the
+    // basis is zero
+    const double k = fmin(fmax(fl, 0.0), (double)(SBF_L - 2));
+    const double x0 = (k - SBF_C) * SBF_DX, x1 = (k + 1.0 - SBF_C) * SBF_DX;
+    const double s0 = exp(-0.5 * (x0 * x0)) * (1.0 - frac), s1 = exp(-0.5 * (x1 * x1)) * frac;
+    const double y0 = 2.0 * x0, y1 = 2.0 * x1;
+    double a0 = s0, a1 = s1, b0 = y0 * s0, b1 = y1 * s1;  // H_n s of two consecutive orders
+    out[0] = a0 + a1;
+    out[1] = b0 + b1;
+#pragma unroll
+    for (int n = 2; n < SDN; n++) {
+        const double c0 = fma(y0, b0, -2.0 * (n - 1) * a0), c1 = fma(y1, b1, -2.0 * (n - 1) * a1);
+        a0 = b0, a1 = b1, b0 = c0, b1 = c1;
+        out[n] = c0 + c1;
+    }
+}
+
+// The shapelet envelope of table coordinates (dx, dy) from the table's
+// centre with the component's signed dense coefficients cm [n1][n2].
+__device__ __forceinline__ cplx shapelet_env(const double* __restrict__ cm, double dx, double dy) {
+    double X[SDN], Y[SDN];
+    hermite_interp(dx + SBF_C, X);
+    hermite_interp(dy + SBF_C, Y);
+    cplx e = {0.0, 0.0};
+#pragma unroll
+    for (int n1 = 0; n1 < SDN; n1++) {
+        double tr = 0.0, ti = 0.0;
+#pragma unroll
+        for (int n2 = 0; n2 < SDN; n2++) {
+            if ((n1 + n2) & 1)
+                ti = fma(cm[n1 * SDN + n2], Y[n2], ti);
+            else
+                tr = fma(cm[n1 * SDN + n2], Y[n2], tr);
+        }
+        e.re = fma(X[n1], tr, e.re);
+        e.im = fma(X[n1], ti, e.im);
+    }
+    return e;
+}
+
+template <int TYPE, bool TILE, bool OUT64>
+__global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
+    constexpr int CH = Shape<TYPE, TILE>::CH;
+    __shared__ alignas(128) double4 s_lmn[2][CH];
+    __shared__ alignas(128) JonesF64 s_flux[2][CH];
+    __shared__ alignas(128) double4 s_gp[TYPE ? 2 : 1][TYPE ? CH : 1];
+    // shared beam: the phasors of the 32 row tiles, then the 32 column tiles;
+    // per-tile beams: M_p and N_q entries (xx, xy, yx, yy)
+    __shared__ alignas(16) double2 s_a[TILE ? 4 : 1][CH][2 * TB];
+    __shared__ alignas(16) double2 s_k[TYPE ? CH : 1][TYPE ? 2 * TB : 1];  // envelope coordinates
+    __shared__ alignas(16) double4 s_w[TILE ? 1 : CH];                    // xx, yy, Re xy, Im xy
+    __shared__ double s_dense[TYPE == 2 ? CH * SDN * SDN : 1];
+    __shared__ alignas(8) uint64_t bar[2];
+
+    const int tid = threadIdx.x, f = blockIdx.y;
+    const int nblk = (p.ntiles + TB - 1) / TB, noff = nblk * (nblk - 1) / 2;
+    // blocks off the diagonal first, then the cheaper diagonal ones
+    int pb, qb;
+    if ((int)blockIdx.x < noff)
+        baseline_to_tiles(blockIdx.x, nblk, pb, qb);
+    else
+        pb = qb = blockIdx.x - noff;
+
+    // this thread's tile of the chunk tables: its UVW in wavelengths and, for
+    // per-tile beams, its row of the beam table
+    const int slot = tid & (2 * TB - 1);
+    const int tile = slot < TB ? pb * TB + slot : qb * TB + slot - TB;
+    const double freq = p.freqs[f], ool = freq / VEL_C;
+    double u = 0.0, v = 0.0, w = 0.0;
+    const JonesF64* brow = nullptr;
+    if (tile < p.ntiles) {
+        tile_uvw(p, tile, ool, u, v, w);
+        if (TILE) brow = p.beam + (size_t)p.nc * ((size_t)p.n_uniq_freq * p.tile_map[tile] + p.freq_map[f]);
+    }
+
+    // a diagonal block's column tiles are its row tiles: formed once (per-tile
+    // beams need both M and N)
+    const bool same = !TILE && pb == qb;
+
+    // pairs of this thread: rows tr + 16 i, columns tc + 16 j.  want[h][j] is
+    // uniform over the CTA: false where no pair of that 16 x 16 quarter is a
+    // baseline.
+    const int tr = pb * TB + (tid >> 4), tc = qb * TB + (tid & 15);
+    bool want[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            want[i][j] = pb * TB + 16 * i < p.ntiles && qb * TB + 16 * j < p.ntiles && !(pb == qb && i > j);
+    const bool full = want[0][0] && want[0][1] && want[1][0] && want[1][1];
+
+    const int nchunks = (p.nc + CH - 1) / CH;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    auto issue = [&](int k) {
+        const int st = k & 1, c0 = k * CH, n = min(CH, p.nc - c0);
+        mbar_arrive_expect_tx(&bar[st], n * 32u + n * 64u + (TYPE ? n * 32u : 0u));
+        bulk_g2s(s_lmn[st], p.lmn + c0, n * 32u, &bar[st]);
+        bulk_g2s(s_flux[st], p.flux + (size_t)f * p.nc + c0, n * 64u, &bar[st]);
+        if (TYPE) bulk_g2s(s_gp[st], p.gp + c0, n * 32u, &bar[st]);
+    };
+    int issued = 0;  // chunks whose copies thread 0 has issued
+    if (tid == 0) {
+        fence_proxy_async_smem();
+        if (!p.stall) {
+            if (nchunks > 0) issue(0), issued = 1;
+            if (nchunks > 1) issue(1), issued = 2;
+        }
+    }
+    const uint64_t limit = p.wait_ns ? p.wait_ns : 2000000000ull;
+
+    // shared beam: sums of w_xx z, w_yy z, Re(w_xy) z, Im(w_xy) z; per-tile
+    // beams: the four correlations
+    cplx acc[RI][2][4];
+#pragma unroll
+    for (int i = 0; i < RI; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[i][j][e] = cplx{0.0, 0.0};
+
+    bool aborted = false;
+    for (int k = 0; k < nchunks; k++) {
+        const int st = k & 1;
+        const bool ok = mbar_wait_bounded(&bar[st], (k >> 1) & 1, p.err, limit);
+        const int c0 = k * CH, n = ok ? min(CH, p.nc - c0) : 0;
+
+        // ---- the chunk's per-tile tables ----
+        if (!same || slot < TB) {
+            for (int c = tid / (2 * TB); c < n; c += NTH / (2 * TB)) {
+                const double4 lmn = s_lmn[st][c];
+                const cplx a = phasor_quarter_f64(4.0 * (u * lmn.x + v * lmn.y + w * lmn.z));
+                if (!TILE) {
+                    const double2 x = make_double2(a.re, a.im);
+                    s_a[0][c][slot] = x;
+                    if (same) s_a[0][c][slot + TB] = x;
+                } else {
+                    J2 b = brow ? ldg_j(brow + c0 + c) : jzero();
+                    if (slot < TB) b = b * load_j(s_flux[st][c]);
+                    b = b * a;
+                    s_a[0][c][slot] = make_double2(b.a.re, b.a.im);
+                    s_a[TILE ? 1 : 0][c][slot] = make_double2(b.b.re, b.b.im);
+                    s_a[TILE ? 2 : 0][c][slot] = make_double2(b.c.re, b.c.im);
+                    s_a[TILE ? 3 : 0][c][slot] = make_double2(b.d.re, b.d.im);
+                }
+                if (TYPE) {
+                    const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
+                    double2 x;
+                    if (TYPE == 1) {
+                        x = make_double2(u * g.z + v * g.w, u * g.w - v * g.z);
+                    } else {
+                        double2 q = make_double2(0.0, 0.0);
+                        if (tile < p.ntiles) q = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + tile);
+                        const double su = q.x * ool, sv = q.y * ool;
+                        x = make_double2((su * g.z + sv * g.w) * g.x, (su * g.w - sv * g.z) * g.y);
+                    }
+                    s_k[TYPE ? c : 0][TYPE ? slot : 0] = x;
+                    if (same) s_k[TYPE ? c : 0][TYPE ? slot + TB : 0] = x;
+                }
+            }
+        }
+        if (!TILE && tid < n) {
+            const JonesF64 q = s_flux[st][tid];
+            s_w[TILE ? 0 : tid] = make_double4(q.j00_re, q.j11_re, q.j01_re, q.j01_im);
+        }
+        if (TYPE == 2)
+            for (int i = tid; i < n * SDN * SDN; i += NTH) s_dense[TYPE == 2 ? i : 0] = __ldg(p.sdense64 + (size_t)c0 * SDN * SDN + i);
+        if (__syncthreads_or(!ok)) {
+            // the sum is incomplete: leave the visibilities untouched
+            if (tid == 0) drain_two_stage(bar, k, issued);
+            aborted = true;
+            break;
+        }
+
+        // ---- the pairs ----
+        auto sweep = [&](auto all) {
+            for (int c = 0; c < n; c++) {
+#pragma unroll
+                for (int i = 0; i < RI; i++) {
+                    const int rp = (tid >> 4) + 16 * i;
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        if (!decltype(all)::value && !want[i][j]) continue;
+                        const int cq = TB + (tid & 15) + 16 * j;
+                        cplx env = {1.0, 0.0};
+                        if (TYPE) {
+                            const double2 kp = s_k[TYPE ? c : 0][TYPE ? rp : 0], kq = s_k[TYPE ? c : 0][TYPE ? cq : 0];
+                            const double dx = kp.x - kq.x, dy = kp.y - kq.y;
+                            if (TYPE == 1) {
+                                const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
+                                env.re = exp(g.x * (dx * dx) + g.y * (dy * dy));
+                            } else {
+                                env = shapelet_env(s_dense + (TYPE == 2 ? c * SDN * SDN : 0), dx, dy);
+                            }
+                        }
+                        cplx(&m)[4] = acc[i][j];
+                        if (!TILE) {
+                            const double2 ap = s_a[0][c][rp], aq = s_a[0][c][cq];
+                            cplx z = {fma(ap.x, aq.x, ap.y * aq.y), fma(ap.y, aq.x, -(ap.x * aq.y))};
+                            if (TYPE == 1) z = z * env.re;
+                            if (TYPE == 2) z = z * env;
+                            const double4 wv = s_w[TILE ? 0 : c];
+                            const double we[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                m[e].re = fma(we[e], z.re, m[e].re);
+                                m[e].im = fma(we[e], z.im, m[e].im);
+                            }
+                        } else {
+                            cplx M[4], N[4];
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const double2 a = s_a[TILE ? e : 0][c][rp], b = s_a[TILE ? e : 0][c][cq];
+                                M[e] = cplx{a.x, a.y};
+                                N[e] = cplx{b.x, b.y};
+                                if (TYPE == 1) M[e] = M[e] * env.re;
+                                if (TYPE == 2) M[e] = M[e] * env;
+                            }
+#pragma unroll
+                            for (int a = 0; a < 2; a++)
+#pragma unroll
+                                for (int b = 0; b < 2; b++)
+#pragma unroll
+                                    for (int y = 0; y < 2; y++) {
+                                        // M^{ay} conj(N^{by})
+                                        const cplx x = M[2 * a + y], q = N[2 * b + y];
+                                        cplx& o = m[2 * a + b];
+                                        o.re = fma(x.re, q.re, fma(x.im, q.im, o.re));
+                                        o.im = fma(x.im, q.re, fma(-x.re, q.im, o.im));
+                                    }
+                        }
+                    }
+                }
+            }
+        };
+        if (full)
+            sweep(std::true_type{});
+        else
+            sweep(std::false_type{});
+        __syncthreads();
+        if (tid == 0 && k + 2 < nchunks) {
+            fence_proxy_async_smem();
+            issue(k + 2);
+            issued = k + 3;
+        }
+    }
+
+    if (aborted) return;
+#pragma unroll
+    for (int i = 0; i < RI; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int tp = tr + 16 * i, tq = tc + 16 * j;
+            if (tp >= tq || tq >= p.ntiles) continue;
+            const cplx(&m)[4] = acc[i][j];
+            J2 r;
+            if (TILE)
+                r = J2{m[0], m[1], m[2], m[3]};
+            else
+                r = J2{m[0], cplx{m[2].re - m[3].im, m[2].im + m[3].re}, cplx{m[2].re + m[3].im, m[2].im - m[3].re}, m[1]};
+            add_vis<OUT64>(p.vis, (size_t)f * p.nbl + baseline_index(tp, tq, p.ntiles), r);
+        }
+}
+
+template <int TYPE, bool TILE>
+cudaError_t launch_t(bool out64, const DirectParams& p, cudaStream_t s) {
+    const int nblk = (p.ntiles + TB - 1) / TB;
+    const dim3 grid(nblk * (nblk + 1) / 2, p.nf);
+    if (out64)
+        pair_kernel<TYPE, TILE, true><<<grid, NTH, 0, s>>>(p);
+    else
+        pair_kernel<TYPE, TILE, false><<<grid, NTH, 0, s>>>(p);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+}  // namespace pairs
+
+cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s) {
+    if (ty == 0)
+        return tile_beam ? pairs::launch_t<0, true>(out64, p, s) : pairs::launch_t<0, false>(out64, p, s);
+    if (ty == 1)
+        return tile_beam ? pairs::launch_t<1, true>(out64, p, s) : pairs::launch_t<1, false>(out64, p, s);
+    return tile_beam ? pairs::launch_t<2, true>(out64, p, s) : pairs::launch_t<2, false>(out64, p, s);
+}
+
+}  // namespace hdc

@@ -40,6 +40,15 @@ struct DirectParams {
     const int* coeff_count;
     const ShapeletUV* suv_bl;  // [nbl][nc] m, or NULL
     const double2* suv_tile;   // [nc][ntiles] m, or NULL (then suv = tile1 - tile2)
+    // the native modeller's tiles, when the UVWs are their differences (the
+    // FP64 form factored by tile): geodetic positions and their centroid, and
+    // the phase centre's hour angle and declination; NULL otherwise
+    const XYZ* xyzs;
+    XYZ xyz0;
+    double s_ha, c_ha, s_dec, c_dec;
+    // the dense coefficients for that form: FP64, with the basis functions'
+    // normalisation folded in, or NULL
+    const double* sdense64;
     void* vis;                 // [nf][nbl] JonesF32 or JonesF64, accumulated
     int* err;
     // Limit of each bounded wait on the staged tables [ns] (0: the default
@@ -54,6 +63,36 @@ struct DirectParams {
 const char* kernel_error_string(int word);
 // Status code of a kernel error word for the native layer (HDC_OK for 0).
 int kernel_error_status(int word);
+
+// vis[o] += acc (JonesF64 or JonesF32 [channel][baseline] at element o).
+template <bool OUT64>
+__device__ __forceinline__ void add_vis(void* vis, size_t o, const J2& acc) {
+    if (OUT64) {
+        double2* q = reinterpret_cast<double2*>(reinterpret_cast<JonesF64*>(vis) + o);
+        const double2 a0 = q[0], b0 = q[1], c0 = q[2], d0 = q[3];
+        q[0] = make_double2(a0.x + acc.a.re, a0.y + acc.a.im);
+        q[1] = make_double2(b0.x + acc.b.re, b0.y + acc.b.im);
+        q[2] = make_double2(c0.x + acc.c.re, c0.y + acc.c.im);
+        q[3] = make_double2(d0.x + acc.d.re, d0.y + acc.d.im);
+    } else {
+        float4* q = reinterpret_cast<float4*>(reinterpret_cast<JonesF32*>(vis) + o);
+        float4 x = q[0], y = q[1];
+        x.x += (float)acc.a.re;
+        x.y += (float)acc.a.im;
+        x.z += (float)acc.b.re;
+        x.w += (float)acc.b.im;
+        y.x += (float)acc.c.re;
+        y.y += (float)acc.c.im;
+        y.z += (float)acc.d.re;
+        y.w += (float)acc.d.im;
+        q[0] = x;
+        q[1] = y;
+    }
+}
+
+// The FP64 predict of component type ty factored by tile (pairs.cu); p.xyzs
+// set, shapelets with p.sdense64.
+cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s);
 
 // Launch the direct kernel for component type ty (0 point, 1 Gaussian,
 // 2 shapelet).  tile_beam selects per-tile beam Jones; out64 an FP64 output;

@@ -1,0 +1,75 @@
+"""The predicts factored by tile (csrc/pairs.cu) at the edges of their 32 x 32
+blocks of tile pairs and of their staged chunks of components, against the
+CPU oracle."""
+
+import math
+
+import numpy as np
+import pytest
+
+from mwa_hyperdrive_b200 import srclist as sl
+from mwa_hyperdrive_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from mwa_hyperdrive_b200.model import SkyModeller  # noqa: E402
+
+PC = (0.2, math.radians(-27.0))
+LST = 0.25
+
+
+def components(kind, n, seed):
+    if kind == "points":
+        return synth.point_sky(n, PC, 10.0, seed, curved_q_sigma=0.2)
+    if kind == "gaussians":
+        return synth.gaussians_and_shapelets(n, 0, PC, seed)
+    return synth.gaussians_and_shapelets(0, n, PC, seed)
+
+
+def predict(sky, obs, form, beam, dtype):
+    kw = {}
+    if beam == "per_tile":
+        kw["dipole_gains"] = dipole_gains(obs.num_tiles)
+    m = SkyModeller(sky, obs.tile_xyzs, obs.freqs, obs.phase_centre, obs.latitude, form=form, beam=beam, **kw)
+    vis = torch.zeros((obs.freqs.size, obs.num_baselines, 8), dtype=dtype, device="cuda")
+    m.model_timestep_with(LST, vis)
+    m.close()
+    return vis.cpu().numpy()
+
+
+def dipole_gains(ntiles):
+    g = np.ones((ntiles, 2, 16))
+    for t in range(0, ntiles, 3):
+        g[t, t % 2, (t // 3) % 4] = 0.0
+    return g
+
+
+def expected(oracle, sky, obs, beam):
+    if beam == "per_tile":
+        uniq, tmap, ufreqs, fmap = oracle.unique_tile_beams(dipole_gains(obs.num_tiles), obs.freqs)
+        tables = [oracle.tile_beam_table(sky, ty, LST, obs.latitude, uniq, ufreqs)
+                  if np.any(sky.comp_type == ty) else None for ty in range(3)]
+        b = oracle.beam_struct(2, tables, tmap, fmap, ufreqs.size)
+    else:
+        b = oracle.beam_struct({"none": 0, "analytic": 1}[beam])
+    return oracle.model_timestep(sky, obs.tile_xyzs, obs.freqs, PC, LST, obs.latitude, beam=b, out_f64=True)[0]
+
+
+def observation(ntiles, seed):
+    return synth.Obs(synth.tiles_in_disk(ntiles, 750.0, seed), 167e6 + np.arange(3) * 1.28e6, PC, np.array([LST]))
+
+
+@pytest.mark.parametrize("beam", ["none", "analytic", "per_tile"])
+@pytest.mark.parametrize("kind", ["points", "gaussians", "shapelets"])
+@pytest.mark.parametrize("ntiles,n", [(2, 1), (16, 8), (17, 9), (33, 33), (64, 16), (65, 17)])
+def test_fp64(oracle, kind, beam, ntiles, n):
+    obs = observation(ntiles, ntiles)
+    sky = sl.SkyModelArrays.from_components(components(kind, n, 100 + n))
+    got = predict(sky, obs, "direct", beam, torch.float64)
+    ref = expected(oracle, sky, obs, beam)
+    rms = math.sqrt(np.mean(ref**2))
+    assert np.max(np.abs(got - ref)) < 1e-10 * rms  # the FP64 form's bar
