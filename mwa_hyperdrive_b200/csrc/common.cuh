@@ -298,6 +298,30 @@ __device__ __forceinline__ void phasor_quarter_f32(double z, float& sn, float& c
     cs = __uint_as_float(__float_as_uint(b) ^ ((qs + 0x40000000u) & 0x80000000u));
 }
 
+// Two FP32 numbers in one 64-bit register, multiplied and added in one
+// instruction (sm_100a's packed FP32 arithmetic, each half rounded to nearest).
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t dup2(float a) { return pack2(a, a); }
+__device__ __forceinline__ float2 unpack2(uint64_t a) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(a));
+    return d;
+}
+
 }  // namespace hdc
 
 // ---------------------------------------------------------------------------

@@ -272,6 +272,7 @@ void TypeTables::release() {
     dfree(d_S);
     dfree(d_W);
     dfree(d_gp);
+    dfree(d_gk);
     dfree(d_radec);
     dfree(d_coeffs);
     dfree(d_cstart);
@@ -379,6 +380,16 @@ int Modeller::build_tables(const HdcSkyModel* sky) {
         HDC_CUDA_RET_INT(cudaMemcpy(tt.d_gp, gp.data(), sizeof(double4) * nc, cudaMemcpyHostToDevice));
         HDC_CUDA_RET_INT(cudaMemcpy(tt.d_radec, radec.data(), sizeof(double2) * nc, cudaMemcpyHostToDevice));
         HDC_CUDA_RET_INT(cudaMemcpy(tt.d_S, S.data(), sizeof(JonesF64) * S.size(), cudaMemcpyHostToDevice));
+        if (ty == 1 && form == HDC_PREDICT_TENSOR) {
+            // gp.x, gp.y are -(pi/2)^2 / ln 2 times maj^2 and min^2 (natural exponent)
+            std::vector<double4> gk(nc);
+            for (int k = 0; k < nc; k++) {
+                const double sx = std::sqrt(-gp[k].x / LN_2), sy = std::sqrt(-gp[k].y / LN_2);
+                gk[k] = make_double4(gp[k].z * sx, gp[k].w * sx, gp[k].w * sy, -gp[k].z * sy);
+            }
+            HDC_CUDA_RET_INT(dalloc(&tt.d_gk, nc));
+            HDC_CUDA_RET_INT(cudaMemcpy(tt.d_gk, gk.data(), sizeof(double4) * nc, cudaMemcpyHostToDevice));
+        }
         FluxComp* d_fc = nullptr;
         HDC_CUDA_RET_INT(dalloc(&d_fc, nc));
         HDC_CUDA_RET_INT(cudaMemcpy(d_fc, fc.data(), sizeof(FluxComp) * nc, cudaMemcpyHostToDevice));
@@ -575,6 +586,7 @@ DirectParams Modeller::direct_params(int ty, void* vis) const {
     p.lmn = t[ty].d_lmn;
     p.flux = weights(ty);
     p.gp = t[ty].d_gp;
+    p.gk = t[ty].d_gk;
     p.sbf = d_sbf;
     p.sbf32 = form == HDC_PREDICT_TENSOR ? device_shapelet_basis_f32() : nullptr;
     p.sbfp = form == HDC_PREDICT_TENSOR ? device_shapelet_basis_pairs() : nullptr;

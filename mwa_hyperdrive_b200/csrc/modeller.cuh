@@ -13,6 +13,7 @@ struct TypeTables {
     JonesF64* d_S = nullptr;     // [nf][nc] instrumental flux
     JonesF64* d_W = nullptr;     // [nf][nc] B S B^H (beam set)
     double4* d_gp = nullptr;     // [nc]
+    double4* d_gk = nullptr;     // [nc] Gaussians, tensor form (DirectParams::gk)
     double2* d_radec = nullptr;  // [nc]
     ShapeletCoeff* d_coeffs = nullptr;
     int* d_cstart = nullptr;

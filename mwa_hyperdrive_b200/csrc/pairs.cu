@@ -27,6 +27,7 @@
 // The drop-in calls keep the per-baseline kernel (predict.cu): their UVWs
 // are the caller's and need not be tile differences.
 
+#include <atomic>
 #include <type_traits>
 
 #include "predict.cuh"
@@ -45,6 +46,13 @@ __device__ __forceinline__ void tile_uvw(const DirectParams& p, int tile, double
     u = (p.s_ha * x + p.c_ha * y) * ool;
     v = (-p.s_dec * p.c_ha * x + p.s_dec * p.s_ha * y + p.c_dec * z) * ool;
     w = (p.c_dec * p.c_ha * x - p.c_dec * p.s_ha * y + p.s_dec * z) * ool;
+}
+
+// 2^-x of x >= 0 (results below the smallest normal number become 0)
+__device__ __forceinline__ float exp2_neg(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-x));
+    return r;
 }
 
 // components per staged chunk: what fits 48 KB of static shared memory with
@@ -352,6 +360,250 @@ cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams&
     if (ty == 1)
         return tile_beam ? pairs::launch_t<1, true>(out64, p, s) : pairs::launch_t<1, false>(out64, p, s);
     return tile_beam ? pairs::launch_t<2, true>(out64, p, s) : pairs::launch_t<2, false>(out64, p, s);
+}
+
+// ---------------------------------------------------------------------------
+// The chosen (tensor) form's Gaussians with a shared beam, factored by tile
+// as above: FP32 phasors per tile after the FP64 phase and its exact range
+// reduction; the envelope's base-2 exponent -|K_p - K_q|^2 from FP64 per-tile
+// coordinates K held as two FP32 numbers (a multiple of 2^-8, whose
+// differences and squares are exact where the envelope is not zero, and the
+// rest), rounded once per axis; products and sums over SUM chunks in FP32,
+// those sums in FP64 (kept in shared memory between, so that a thread's
+// registers hold only the FP32 ones).  Products are packed in pairs
+// (fma.rn.f32x2: two FP32 operations an issue slot).
+//
+// Bound: shared-memory reads (128 bytes a clock and SM, whether or not lanes
+// share an address: 28 bytes a lane and term here) and the issue slots, about
+// 24 warp instructions a term (a thread per baseline, with the phasor per
+// baseline and unpacked: 64).  500 Gaussians, 128 tiles x 384 channels: 2.75
+// ms -> 2.08 ms; with an FP64 exponent per pair and packed phasors stored
+// ready 2.39 ms (40 bytes a lane and term); 4 x 2 pairs at half the warps
+// 2.38 ms.
+// ---------------------------------------------------------------------------
+namespace pairs {
+
+constexpr int FCHUNK = 16;  // components per staged chunk
+constexpr int SUM = 2;      // chunks summed in FP32
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// An FP64 coordinate's upper part: x rounded to a multiple of 2^-8 (|x| < 2^14, else to FP32)
+__device__ __forceinline__ float coarse(double x) {
+    const float f = (float)x;
+    constexpr float M = 49152.f;
+    return fabsf(f) < 16384.f ? __fsub_rn(__fadd_rn(f, M), M) : f;
+}
+
+struct FastSmem {
+    double4 lmn[2][FCHUNK];
+    JonesF64 flux[2][FCHUNK];
+    double4 gp[2][FCHUNK];     // K = (u gp.x + v gp.y, u gp.z + v gp.w): the exponent is -|K_p - K_q|^2
+    float2 a[FCHUNK][2 * TB];  // phasors of the row tiles, then the column tiles
+    float4 k[FCHUNK][2 * TB];  // envelope coordinates (hx, hy, lx, ly), negated for column tiles
+    float4 w[FCHUNK];          // xx, yy, Re xy, Im xy
+    double2 sum[2 * RI][4][NTH];  // [pair][sum][thread]
+    uint64_t bar[2];
+};
+
+template <bool OUT64>
+__global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    FastSmem& S = *reinterpret_cast<FastSmem*>(smem_raw);
+    const int tid = threadIdx.x, f = blockIdx.y;
+    const int nblk = (p.ntiles + TB - 1) / TB, noff = nblk * (nblk - 1) / 2;
+    int pb, qb;
+    if ((int)blockIdx.x < noff)
+        baseline_to_tiles(blockIdx.x, nblk, pb, qb);
+    else
+        pb = qb = blockIdx.x - noff;
+
+    const int slot = tid & (2 * TB - 1);
+    const int tile = slot < TB ? pb * TB + slot : qb * TB + slot - TB;
+    const double freq = p.freqs[f], ool = freq / VEL_C;
+    double u = 0.0, v = 0.0, w = 0.0;  // wavelengths
+    if (tile < p.ntiles) tile_uvw(p, tile, ool, u, v, w);
+
+    const bool same = pb == qb;  // the column tiles are the row tiles
+    const int tr = pb * TB + (tid >> 4), tc = qb * TB + (tid & 15);
+    const int rp = tid >> 4, cq = TB + (tid & 15);
+    // warps whose pairs are all past the array have nothing to sum
+    const bool any = __any_sync(0xffffffffu, tr < p.ntiles && tc < p.ntiles);
+
+    const int nchunks = (p.nc + FCHUNK - 1) / FCHUNK;
+    if (tid == 0) {
+        mbar_init(&S.bar[0], 1);
+        mbar_init(&S.bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    auto issue = [&](int k) {
+        const int st = k & 1, c0 = k * FCHUNK, n = min(FCHUNK, p.nc - c0);
+        mbar_arrive_expect_tx(&S.bar[st], n * 128u);
+        bulk_g2s(S.lmn[st], p.lmn + c0, n * 32u, &S.bar[st]);
+        bulk_g2s(S.flux[st], p.flux + (size_t)f * p.nc + c0, n * 64u, &S.bar[st]);
+        bulk_g2s(S.gp[st], p.gk + c0, n * 32u, &S.bar[st]);
+    };
+    int issued = 0;  // chunks whose copies thread 0 has issued
+    if (tid == 0) {
+        fence_proxy_async_smem();
+        if (!p.stall) {
+            if (nchunks > 0) issue(0), issued = 1;
+            if (nchunks > 1) issue(1), issued = 2;
+        }
+    }
+    const uint64_t limit = p.wait_ns ? p.wait_ns : 2000000000ull;
+
+    uint64_t acc[2 * RI][4];  // [pair] (re, im) of the sums of w_xx z, w_yy z, Re(w_xy) z, Im(w_xy) z
+#pragma unroll
+    for (int i = 0; i < 2 * RI; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[i][e] = 0;
+
+    const uint64_t two = dup2(2.f);
+    bool aborted = false;
+    for (int k = 0; k < nchunks; k++) {
+        const int st = k & 1;
+        const bool ok = mbar_wait_bounded(&S.bar[st], (k >> 1) & 1, p.err, limit);
+        const int n = ok ? min(FCHUNK, p.nc - k * FCHUNK) : 0;
+        if (tid < n) {
+            const JonesF64 q = S.flux[st][tid];
+            S.w[tid] = make_float4((float)q.j00_re, (float)q.j11_re, (float)q.j01_re, (float)q.j01_im);
+        }
+        if (!same || slot < TB) {
+            for (int c = tid / (2 * TB); c < n; c += NTH / (2 * TB)) {
+                const double4 lmn = S.lmn[st][c], sc = S.gp[st][c];
+                float sn, cs;
+                phasor_quarter_f32(4.0 * (u * lmn.x + v * lmn.y + w * lmn.z), sn, cs);
+                const double2 xx = make_double2(u * sc.x + v * sc.y, u * sc.z + v * sc.w);
+                const float hx = coarse(xx.x), hy = coarse(xx.y);
+                const float4 x = make_float4(hx, hy, (float)(xx.x - (double)hx), (float)(xx.y - (double)hy));
+                const float4 nx = make_float4(-x.x, -x.y, -x.z, -x.w);
+                S.a[c][slot] = make_float2(cs, sn);
+                S.k[c][slot] = slot < TB ? x : nx;
+                if (same) {
+                    S.a[c][slot + TB] = make_float2(cs, sn);
+                    S.k[c][slot + TB] = nx;
+                }
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            // the sum is incomplete: leave the visibilities untouched
+            if (tid == 0) drain_two_stage(S.bar, k, issued);
+            aborted = true;
+            break;
+        }
+
+        // in stages over the thread's four pairs, so that their chains (loads,
+        // exponent, exponential) overlap; a pair that is no baseline (past the
+        // array, or below the diagonal in a quarter on it) is summed like the
+        // others and not stored
+        auto sweep = [&](auto diag) {
+            constexpr bool DIAG = decltype(diag)::value;  // the lower left quarter holds no baseline
+            for (int c = 0; c < n; c++) {
+                const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(S.k[c]);
+                const ulonglong2 kq[2] = {kr[cq], kr[cq + 16]};
+                float e[2 * RI];
+#pragma unroll
+                for (int i = 0; i < RI; i++) {
+                    const ulonglong2 kp = kr[rp + 16 * i];
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        if (DIAG && i > j) continue;
+                        // dh^2 + dl (2 dh + dl): dh exact, one rounding
+                        const uint64_t dh = add2(kp.x, kq[j].x), dl = add2(kp.y, kq[j].y);
+                        const float2 q = unpack2(fma2(dh, dh, mul2(dl, fma2(two, dh, dl))));
+                        e[2 * i + j] = q.x + q.y;
+                    }
+                }
+                const float4 wv = S.w[c];
+                const uint64_t w[4] = {dup2(wv.x), dup2(wv.y), dup2(wv.z), dup2(wv.w)};
+                uint64_t qx[2], qy[2];
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const float2 aq = S.a[c][cq + 16 * j];
+                    qx[j] = dup2(aq.x);
+                    qy[j] = dup2(aq.y);
+                }
+#pragma unroll
+                for (int i = 0; i < RI; i++) {
+                    const float2 ap = S.a[c][rp + 16 * i];
+                    const uint64_t px = pack2(ap.x, ap.y), py = pack2(ap.y, -ap.x);
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        if (DIAG && i > j) continue;
+                        uint64_t(&m)[4] = acc[2 * i + j];
+                        const uint64_t z = mul2(fma2(py, qy[j], mul2(px, qx[j])), dup2(exp2_neg(e[2 * i + j])));
+#pragma unroll
+                        for (int x = 0; x < 4; x++) m[x] = fma2(w[x], z, m[x]);
+                    }
+                }
+            }
+        };
+        if (any && same)
+            sweep(std::true_type{});
+        else if (any)
+            sweep(std::false_type{});
+        if (k % SUM == SUM - 1 || k == nchunks - 1) {
+            const bool first = k < SUM;
+#pragma unroll
+            for (int i = 0; i < 2 * RI; i++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float2 a = unpack2(acc[i][e]);
+                    double2 s = first ? make_double2(0.0, 0.0) : S.sum[i][e][tid];
+                    s.x += (double)a.x;
+                    s.y += (double)a.y;
+                    S.sum[i][e][tid] = s;
+                    acc[i][e] = 0;
+                }
+        }
+        __syncthreads();
+        if (tid == 0 && k + 2 < nchunks) {
+            fence_proxy_async_smem();
+            issue(k + 2);
+            issued = k + 3;
+        }
+    }
+
+    if (aborted) return;
+#pragma unroll
+    for (int i = 0; i < 2 * RI; i++) {
+        const int tp = tr + 16 * (i >> 1), tq = tc + 16 * (i & 1);
+        if (tp >= tq || tq >= p.ntiles) continue;
+        const double2 xx = S.sum[i][0][tid], yy = S.sum[i][1][tid], a = S.sum[i][2][tid], b = S.sum[i][3][tid];
+        add_vis<OUT64>(p.vis, (size_t)f * p.nbl + baseline_index(tp, tq, p.ntiles),
+                       J2{{xx.x, xx.y}, {a.x - b.y, a.y + b.x}, {a.x + b.y, a.y - b.x}, {yy.x, yy.y}});
+    }
+}
+
+template <bool OUT64>
+cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
+    // the opt-in above 48 KB of dynamic shared memory, once per device
+    static std::atomic<bool> attr[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!attr[dev].load(std::memory_order_relaxed)) {
+        e = cudaFuncSetAttribute(fast_gauss_kernel<OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(FastSmem));
+        if (e != cudaSuccess) return e;
+        attr[dev].store(true, std::memory_order_relaxed);
+    }
+    const int nblk = (p.ntiles + TB - 1) / TB;
+    fast_gauss_kernel<OUT64><<<dim3(nblk * (nblk + 1) / 2, p.nf), NTH, sizeof(FastSmem), s>>>(p);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+}  // namespace pairs
+
+cudaError_t launch_fast_gauss(bool out64, const DirectParams& p, cudaStream_t s) {
+    return out64 ? pairs::launch_fast_gauss<true>(p, s) : pairs::launch_fast_gauss<false>(p, s);
 }
 
 }  // namespace hdc

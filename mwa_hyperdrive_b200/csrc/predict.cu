@@ -899,7 +899,7 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
     // the FP32 form needs per-tile shapelet UVs and the FP32 basis table, and
     // with per-tile beams a unique-tile count it can stage (not the points,
     // whose chosen form is the tensor kernel)
-    fast = fast && (ty != 2 || (p.suv_tile && !p.suv_bl && p.sbf32)) &&
+    fast = fast && p.xyzs && (ty != 2 || (p.suv_tile && !p.suv_bl && p.sbf32)) &&
            (!tile_beam || (ty != 0 && p.n_uniq_tile > 0 && p.n_uniq_tile <= FT_MAX_NU && !p.unflagged_map));
     if (fast && ty == 2 && p.sdense && !p.sbfp) return cudaErrorInvalidValue;
     // UVWs that are tile differences: the FP64 form factored by tile (128
@@ -908,6 +908,7 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
     // or more keep the per-baseline kernel, which reads the basis table per
     // coefficient.
     if (!fast && p.xyzs && (ty != 2 || p.sdense64)) return launch_pairs(ty, tile_beam, out64, p, s);
+    if (fast && ty == 1 && !tile_beam) return launch_fast_gauss(out64, p, s);
     if (ty == 0) return launch_t<0>(tile_beam, out64, fast, p, s);
     if (ty == 1) return launch_t<1>(tile_beam, out64, fast, p, s);
     return launch_t<2>(tile_beam, out64, fast, p, s);

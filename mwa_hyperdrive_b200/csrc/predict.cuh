@@ -19,6 +19,8 @@ struct DirectParams {
     const double4* lmn;   // [nc] (l, m, n - 1, 0), dimensionless (turn units)
     const JonesF64* flux; // [nf][nc]: B S B^H when the beam is shared (or none), S when per tile
     const double4* gp;    // [nc] Gaussian: (C maj^2, C min^2, sin pa, cos pa); shapelet: (maj K, -min K, sin pa, cos pa)
+    const double4* gk;    // [nc] Gaussians of the chosen form: rows of the 2 x 2 matrix that takes (u, v) to the
+                          // coordinates whose squared length is the envelope's base-2 exponent, or NULL
     // per-tile beam, reference layout [uniq_tile][uniq_freq][nc]
     const JonesF64* beam;
     const int* tile_map;
@@ -93,6 +95,8 @@ __device__ __forceinline__ void add_vis(void* vis, size_t o, const J2& acc) {
 // The FP64 predict of component type ty factored by tile (pairs.cu); p.xyzs
 // set, shapelets with p.sdense64.
 cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s);
+// The chosen form's Gaussians with a shared beam, factored by tile; p.xyzs set.
+cudaError_t launch_fast_gauss(bool out64, const DirectParams& p, cudaStream_t s);
 
 // Launch the direct kernel for component type ty (0 point, 1 Gaussian,
 // 2 shapelet).  tile_beam selects per-tile beam Jones; out64 an FP64 output;

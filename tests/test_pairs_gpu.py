@@ -73,3 +73,15 @@ def test_fp64(oracle, kind, beam, ntiles, n):
     ref = expected(oracle, sky, obs, beam)
     rms = math.sqrt(np.mean(ref**2))
     assert np.max(np.abs(got - ref)) < 1e-10 * rms  # the FP64 form's bar
+
+
+@pytest.mark.parametrize("kind", ["gaussians"])
+@pytest.mark.parametrize("ntiles,n", [(2, 1), (17, 15), (33, 33), (64, 64), (65, 17)])
+def test_chosen_form(oracle, kind, ntiles, n):
+    obs = observation(ntiles, ntiles)
+    sky = sl.SkyModelArrays.from_components(components(kind, n, 200 + n))
+    for dtype in (torch.float64, torch.float32):
+        got = predict(sky, obs, "tensor", "analytic", dtype)
+        ref = expected(oracle, sky, obs, "analytic")
+        # the chosen form's bar
+        assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
