@@ -350,8 +350,9 @@ const char* take_word_sync(int* w, const char* who);
 // Shapelet basis table on the current device (SBF_N x SBF_L doubles).
 const double* device_shapelet_basis();
 const float* device_shapelet_basis_f32();
-// FP32 (value, next - value) pairs of the table's orders 0 .. SDN_TABLE - 1,
-// position-major: [SBF_L][SDN_TABLE / 2] float4 (one record per position).
+// FP32 values v and differences d = next - v of the table's orders 0 ..
+// SDN_TABLE - 1, position-major: [SBF_L][SDN_TABLE / 2] float4 (v, v', d, d')
+// of two orders (one record per position).
 constexpr int SDN_TABLE = 6;
 const float4* device_shapelet_basis_pairs();
 void host_shapelet_basis(double* out);

@@ -12,6 +12,7 @@
 // reference does (model/cpu.rs:341-348, gpu/model.cu:171).
 
 #include <atomic>
+#include <climits>
 #include <cstdio>
 #include <vector>
 
@@ -93,127 +94,112 @@ __device__ __forceinline__ void shapelet_envelope_f32(const DirectParams& p, int
 }
 
 // The chosen form's dense shapelet envelope (every order below SDN): the
-// basis is interpolated once per order along each axis (one 8-byte gather of
-// a (value, next - value) pair each), then contracted with the component's
-// signed dense coefficient matrix C (shared memory):
+// basis is interpolated once per order along each axis and contracted with
+// the component's signed dense coefficient matrix C (shared memory):
 //     env = sum_{n1,n2} C[n1][n2] X[n1] Y[n2],  even n1 + n2 -> re, odd -> im.
-__device__ __forceinline__ void shapelet_dense_at(const DirectParams& p, const float* __restrict__ cm, double x_pos,
-                                                  double y_pos, float& er, float& ei) {
-    const double fx = floor(x_pos), fy = floor(y_pos);
-    const int xi = fx > 0.0 ? (int)fmin(fx, (double)(SBF_L - 2)) : 0;
-    const int yi = fy > 0.0 ? (int)fmin(fy, (double)(SBF_L - 2)) : 0;
-    const float xfrac = (float)(x_pos - fx), yfrac = (float)(y_pos - fy);
-    // one 48-byte record per position holds all orders' pairs
-    float X[SDN], Y[SDN];
-#pragma unroll
-    for (int h = 0; h < SDN / 2; h++) {
-        const float4 a = __ldg(p.sbfp + (size_t)xi * (SDN / 2) + h);
-        const float4 b = __ldg(p.sbfp + (size_t)yi * (SDN / 2) + h);
-        X[2 * h] = fmaf(a.y, xfrac, a.x);
-        X[2 * h + 1] = fmaf(a.w, xfrac, a.z);
-        Y[2 * h] = fmaf(b.y, yfrac, b.x);
-        Y[2 * h + 1] = fmaf(b.w, yfrac, b.z);
-    }
-    float re = 0.f, im = 0.f;
-#pragma unroll
-    for (int n1 = 0; n1 < SDN; n1++) {
-        float tr = 0.f, ti = 0.f;
-#pragma unroll
-        for (int n2 = 0; n2 < SDN; n2++) {
-            if ((n1 + n2) & 1)
-                ti = fmaf(cm[n1 * SDN + n2], Y[n2], ti);
-            else
-                tr = fmaf(cm[n1 * SDN + n2], Y[n2], tr);
-        }
-        re = fmaf(X[n1], tr, re);
-        im = fmaf(X[n1], ti, im);
-    }
-    er = re;
-    ei = im;
+// One 48-byte record of the basis table holds, for a position's interval, the
+// six orders' (value, next - value) as three float4 (v0, v1, d0, d1).
+struct ShapeRec {
+    int k;  // table interval from the centre
+    ulonglong2 r[SDN / 2];
+};
+// Records of the intervals within SWIN of the table's centre, staged in
+// shared memory by the shapelet kernel with a shared beam (win), because a
+// warp's scattered 16-byte loads cost about 32 cycles from L1 and a third of
+// that from shared memory; others come from the table.
+constexpr int SWIN = 320;
+
+// Position dx (table steps from the centre) -> its interval k (clamped to the
+// table, whose end intervals are zero) and the fraction within it, exactly as
+// a position counted from the table's start up to FP64 rounding.
+__device__ __forceinline__ float shape_pos(double scale, double ool, int& k) {
+    // rint(dx - 1/2): the floor, or at a tie the interval below with fraction
+    // 1, which interpolates to the same value
+    const double t = fma(scale, ool, -0.5) + QMAGIC;
+    const double fl = t - QMAGIC;
+    const int lo = __double2loint(t), hi = __double2hiint(t);
+    // |dx| < 2^31: the low word is the integer
+    const bool small = (unsigned)(hi - 0x4337ffff) <= 1u;
+    constexpr int C = (int)SBF_C;
+    k = small ? min(max(lo, -C), SBF_L - 2 - C) : (scale < 0.0 ? -C : SBF_L - 2 - C);
+    return (float)fma(scale, ool, -fl);
 }
 
-__device__ __forceinline__ void shapelet_envelope_dense(const DirectParams& p, const float* __restrict__ cm,
-                                                        double4 g, double su, double sv, float& er, float& ei) {
-    const double x = su * g.z + sv * g.w;
-    const double y = su * g.w - sv * g.z;
-    shapelet_dense_at(p, cm, x * g.x + SBF_C, y * g.y + SBF_C, er, ei);
+template <bool WIN>
+__device__ __forceinline__ void shape_load(const DirectParams& p, const float4* win, ShapeRec& rec, int k) {
+    rec.k = k;
+    const float4* q;
+    if (WIN && (unsigned)(k + SWIN) < 2u * SWIN) {
+        q = win + (k + SWIN) * (SDN / 2);
+#pragma unroll
+        for (int h = 0; h < SDN / 2; h++) rec.r[h] = *reinterpret_cast<const ulonglong2*>(q + h);
+    } else {
+        q = p.sbfp + (size_t)(k + (int)SBF_C) * (SDN / 2);
+#pragma unroll
+        for (int h = 0; h < SDN / 2; h++) rec.r[h] = __ldg(reinterpret_cast<const ulonglong2*>(q + h));
+    }
 }
 
-// shapelet_dense_at for N channels of one component at once: the basis of
-// each channel is interpolated as there, and each row of the coefficient
-// matrix is read from shared memory once (three 8-byte loads) for all N
-// channels; same arithmetic order per channel
-template <int N>
-__device__ __forceinline__ void shapelet_dense_multi(const DirectParams& p, const float* __restrict__ cm,
-                                                     const double (&x_pos)[N], const double (&y_pos)[N],
-                                                     float (&er)[N], float (&ei)[N]) {
-    float X[N][SDN], Y[N][SDN];
-    int xi[N], yi[N];
-    float xfrac[N], yfrac[N];
+// The envelopes of N channels (ool = frequency / c) at sx, sy table steps per
+// wavelength^-1.  A thread's channels usually share a table interval (their
+// positions differ by the channels' relative frequency spacing): a channel
+// whose interval equals the previous one's takes its record instead of
+// loading it again.  Each row of the coefficients is read once for all N
+// channels.
+template <int N, bool WIN>
+__device__ __forceinline__ void shapelet_dense(const DirectParams& p, const float4* win, const float* __restrict__ cm,
+                                               double sx, double sy, const double (&ool)[N], float (&er)[N],
+                                               float (&ei)[N]) {
+    float2 X[N][SDN / 2];
+    uint64_t Y[N][SDN / 2];
+    ShapeRec rec;
+    rec.k = INT_MIN;
 #pragma unroll
     for (int i = 0; i < N; i++) {
-        const double fx = floor(x_pos[i]), fy = floor(y_pos[i]);
-        xi[i] = fx > 0.0 ? (int)fmin(fx, (double)(SBF_L - 2)) : 0;
-        yi[i] = fy > 0.0 ? (int)fmin(fy, (double)(SBF_L - 2)) : 0;
-        xfrac[i] = (float)(x_pos[i] - fx);
-        yfrac[i] = (float)(y_pos[i] - fy);
-        er[i] = 0.f, ei[i] = 0.f;
+        int k;
+        const uint64_t f = dup2(shape_pos(sx, ool[i], k));
+        if (k != rec.k) shape_load<WIN>(p, win, rec, k);
+#pragma unroll
+        for (int h = 0; h < SDN / 2; h++) X[i][h] = unpack2(fma2(rec.r[h].y, f, rec.r[h].x));
     }
-    // A thread's channels usually share a table interval (their positions
-    // differ by the channels' relative frequency spacing): a channel whose
-    // interval equals the previous channel's takes its records instead of
-    // gathering them again, so only lanes with a new interval load.
+    rec.k = INT_MIN;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        int k;
+        const uint64_t f = dup2(shape_pos(sy, ool[i], k));
+        if (k != rec.k) shape_load<WIN>(p, win, rec, k);
+#pragma unroll
+        for (int h = 0; h < SDN / 2; h++) Y[i][h] = fma2(rec.r[h].y, f, rec.r[h].x);
+    }
+    // rows of even n1: (re, im) += X[n1] (C[n1][0], C[n1][1]) (Y0, Y1) + ..;
+    // of odd n1 the two parts change places
+    const ulonglong2* row = reinterpret_cast<const ulonglong2*>(cm);  // two rows: three 16-byte loads
+    uint64_t even[N], odd[N];
 #pragma unroll
     for (int h = 0; h < SDN / 2; h++) {
-        float4 a, b;
+        const ulonglong2 c0 = row[3 * h], c1 = row[3 * h + 1], c2 = row[3 * h + 2];
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            if (i == 0 || xi[i] != xi[i - 1]) a = __ldg(p.sbfp + (size_t)xi[i] * (SDN / 2) + h);
-            if (i == 0 || yi[i] != yi[i - 1]) b = __ldg(p.sbfp + (size_t)yi[i] * (SDN / 2) + h);
-            X[i][2 * h] = fmaf(a.y, xfrac[i], a.x);
-            X[i][2 * h + 1] = fmaf(a.w, xfrac[i], a.z);
-            Y[i][2 * h] = fmaf(b.y, yfrac[i], b.x);
-            Y[i][2 * h + 1] = fmaf(b.w, yfrac[i], b.z);
+            const uint64_t te = fma2(c1.x, Y[i][2], fma2(c0.y, Y[i][1], mul2(c0.x, Y[i][0])));
+            const uint64_t to = fma2(c2.y, Y[i][2], fma2(c2.x, Y[i][1], mul2(c1.y, Y[i][0])));
+            const uint64_t xe = dup2(X[i][h].x), xo = dup2(X[i][h].y);
+            even[i] = h ? fma2(xe, te, even[i]) : mul2(xe, te);
+            odd[i] = h ? fma2(xo, to, odd[i]) : mul2(xo, to);
         }
     }
-    const float2* row = reinterpret_cast<const float2*>(cm);
 #pragma unroll
-    for (int n1 = 0; n1 < SDN; n1++) {
-        float c[SDN];
-#pragma unroll
-        for (int h = 0; h < SDN / 2; h++) {
-            const float2 v = row[n1 * (SDN / 2) + h];
-            c[2 * h] = v.x, c[2 * h + 1] = v.y;
-        }
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            float tr = 0.f, ti = 0.f;
-#pragma unroll
-            for (int n2 = 0; n2 < SDN; n2++) {
-                if ((n1 + n2) & 1)
-                    ti = fmaf(c[n2], Y[i][n2], ti);
-                else
-                    tr = fmaf(c[n2], Y[i][n2], tr);
-            }
-            er[i] = fmaf(X[i][n1], tr, er[i]);
-            ei[i] = fmaf(X[i][n1], ti, ei[i]);
-        }
+    for (int i = 0; i < N; i++) {
+        const float2 e = unpack2(even[i]), o = unpack2(odd[i]);
+        er[i] = e.x + o.y;
+        ei[i] = e.y + o.x;
     }
 }
 
-// FAST (the chosen form's Gaussians and shapelets, shared beam only): the
-// phasor from the FP32 quarter-turn polynomials after exact FP64 range
-// reduction, envelopes in FP32 (arguments and table positions in FP64),
-// each component's term W ph env in FP32
-// (W staged once per chunk as FP32), summed in FP32 within a 64-component
-// chunk and in FP64 across chunks.  Error ~1e-7 of the visibility.
-template <int TYPE, bool TILE_BEAM, bool OUT64, bool FAST>
+template <int TYPE, bool TILE_BEAM, bool OUT64>
 __global__ void __launch_bounds__(DT) direct_kernel(const DirectParams p) {
     __shared__ alignas(128) double4 s_lmn[2][CH];
     __shared__ alignas(128) JonesF64 s_flux[2][CH];
     __shared__ alignas(128) double4 s_gp[2][CH];
-    __shared__ alignas(16) float s_wf[FAST ? CH * 8 : 1];
-    __shared__ alignas(16) float s_dense[(FAST && TYPE == 2) ? CH * SDN * SDN : 1];
     __shared__ alignas(8) uint64_t bar[2];
 
     const int f = blockIdx.y;
@@ -288,52 +274,7 @@ __global__ void __launch_bounds__(DT) direct_kernel(const DirectParams p) {
         }
         const int c0 = k * CH;
         const int n = min(CH, p.nc - c0);
-        if (FAST) {
-            const double* src = reinterpret_cast<const double*>(s_flux[st]);
-            for (int i = threadIdx.x; i < n * 8; i += DT) s_wf[i] = (float)src[i];
-            if (TYPE == 2 && p.sdense)
-                for (int i = threadIdx.x; i < n * SDN * SDN; i += DT)
-                    s_dense[i] = __ldg(p.sdense + (size_t)c0 * SDN * SDN + i);
-            __syncthreads();
-        }
-        if (FAST && active) {
-            float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int c = 0; c < n; c++) {
-                const double4 lmn = s_lmn[st][c];
-                float sn, cs;
-                phasor_quarter_f32(4.0 * (u * lmn.x + v * lmn.y + w * lmn.z), sn, cs);
-                float er = 1.f, ei = 0.f;
-                if (TYPE == 1) {
-                    // the exponent in FP64 (an FP32 exponent's absolute error,
-                    // ~1e-7 of its size, would become the envelope's relative
-                    // error); exp of its FP32 head, first order in the tail
-                    const double4 g = s_gp[st][c];
-                    const double kx = u * g.z + v * g.w;
-                    const double ky = u * g.w - v * g.z;
-                    const double ex = g.x * (kx * kx) + g.y * (ky * ky);
-                    const float exh = (float)ex;
-                    er = expf(exh) * (1.f + (float)(ex - (double)exh));
-                } else if (TYPE == 2) {
-                    const double4 g = s_gp[st][c];
-                    const double2 ta = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + t1);
-                    const double2 tb = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + t2);
-                    if (p.sdense)
-                        shapelet_envelope_dense(p, s_dense + c * SDN * SDN, g, (ta.x - tb.x) * ool,
-                                                (ta.y - tb.y) * ool, er, ei);
-                    else
-                        shapelet_envelope_f32(p, c0 + c, g, (ta.x - tb.x) * ool, (ta.y - tb.y) * ool, er, ei);
-                }
-                // ph * env
-                const float zr = cs * er - sn * ei, zi = fmaf(cs, ei, sn * er);
-                const float* wv = s_wf + c * 8;
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    a[2 * e] += fmaf(wv[2 * e], zr, -wv[2 * e + 1] * zi);
-                    a[2 * e + 1] += fmaf(wv[2 * e], zi, wv[2 * e + 1] * zr);
-                }
-            }
-            acc = acc + J2{{a[0], a[1]}, {a[2], a[3]}, {a[4], a[5]}, {a[6], a[7]}};
-        } else if (active) {
+        if (active) {
             for (int c = 0; c < n; c++) {
                 const double4 lmn = s_lmn[st][c];
                 J2 wj = load_j(s_flux[st][c]);
@@ -403,21 +344,24 @@ __global__ void __launch_bounds__(DT) direct_kernel(const DirectParams p) {
     }
 }
 
+// Shapelet component c's UV [m] of a tile (zero for other types).
+template <int TYPE>
+__device__ __forceinline__ double2 shape_uv(const DirectParams& p, int c, int tile) {
+    return TYPE == 2 ? __ldg(p.suv_tile + (size_t)c * p.ntiles + tile) : make_double2(0.0, 0.0);
+}
+
 // The channel-independent FP64 work of one Gaussian or shapelet term of the
-// chosen form at baseline (um, vm, wm) [m] (tiles t1, t2): the phase in
-// metres, the Gaussian exponent in metres^2 (base 2) or the shapelet
-// coordinates, and the dense shapelet envelopes of the FCH channels (cm:
-// the component's dense coefficient matrix in shared memory, or NULL).
-template <int TYPE, int FCH>
+// chosen form at baseline (um, vm, wm) [m] (its tiles' shapelet UVs ta, tb):
+// the phase in metres, the Gaussian exponent in metres^2 (base 2), or the shapelet
+// coordinates (in metres; dense: in table steps per wavelength^-1).
+template <int TYPE>
 struct FastTerm {
     double tm, exm, su, sv;
-    float der[FCH], dei[FCH];
 };
 
-template <int TYPE, int FCH>
-__device__ __forceinline__ void fast_term(const DirectParams& p, double4 lmn, double4 g, double um, double vm, double wm,
-                                          int cglob, int t1, int t2, const double (&ool)[FCH], const float* cm,
-                                          FastTerm<TYPE, FCH>& f) {
+template <int TYPE>
+__device__ __forceinline__ void fast_term(double4 lmn, double4 g, double um, double vm, double wm, double2 ta, double2 tb,
+                                          bool dense, FastTerm<TYPE>& f) {
     f.tm = um * lmn.x + vm * lmn.y + wm * lmn.z;
     f.exm = f.su = f.sv = 0.0;
     if (TYPE == 1) {
@@ -429,100 +373,90 @@ __device__ __forceinline__ void fast_term(const DirectParams& p, double4 lmn, do
         const double ky = um * g.w - vm * g.z;
         f.exm = (g.x * (kx * kx) + g.y * (ky * ky)) * 1.4426950408889634074;
     } else {
-        const double2 ta = __ldg(p.suv_tile + (size_t)cglob * p.ntiles + t1);
-        const double2 tb = __ldg(p.suv_tile + (size_t)cglob * p.ntiles + t2);
         f.su = ta.x - tb.x;
         f.sv = ta.y - tb.y;
-        if (cm) {
-            const double xm = f.su * g.z + f.sv * g.w;
-            const double ym = f.su * g.w - f.sv * g.z;
-            double xp[FCH], yp[FCH];
-#pragma unroll
-            for (int i = 0; i < FCH; i++) {
-                xp[i] = xm * (ool[i] * g.x) + SBF_C;
-                yp[i] = ym * (ool[i] * g.y) + SBF_C;
-            }
-            shapelet_dense_multi<FCH>(p, cm, xp, yp, f.der, f.dei);
+        if (dense) {
+            const double x = (f.su * g.z + f.sv * g.w) * g.x, y = (f.su * g.w - f.sv * g.z) * g.y;
+            f.su = x;
+            f.sv = y;
         }
     }
 }
 
-// z = envelope x phasor of channel i of a FastTerm (ool_i = its frequency / c).
-template <int TYPE, int FCH>
-__device__ __forceinline__ void fast_z(const DirectParams& p, const FastTerm<TYPE, FCH>& f, int i, double ool_i,
-                                       int cglob, double4 g, bool dense, float& zr, float& zi) {
-    float sn, cs;
-    phasor_quarter_f32(4.0 * ool_i * f.tm, sn, cs);
+// The envelopes of a FastTerm's N channels (ool = frequency / c): a
+// Gaussian's is real; dense shapelets with coefficients cm and win (WIN) the
+// staged records.
+template <int TYPE, int N, bool WIN>
+__device__ __forceinline__ void fast_envelopes(const DirectParams& p, const FastTerm<TYPE>& f, const double (&ool)[N],
+                                               int cglob, double4 g, bool dense, const float* cm, const float4* win,
+                                               float (&er)[N], float (&ei)[N]) {
     if (TYPE == 1) {
         // exponent in FP64, exp2 in FP32: rounding the exponent to FP32 moves
-        // the envelope by ln2 |x| 6e-8 2^-|x| <= 2.2e-8 of the component's flux;
-        // a Gaussian's envelope is real
-        const float er = exp2f((float)(f.exm * (ool_i * ool_i)));
-        zr = cs * er;
-        zi = sn * er;
-    } else {
-        float er, ei;
-        if (dense) {
-            er = f.der[i];
-            ei = f.dei[i];
-        } else {
-            shapelet_envelope_f32(p, cglob, g, f.su * ool_i, f.sv * ool_i, er, ei);
+        // the envelope by ln2 |x| 6e-8 2^-|x| <= 2.2e-8 of the component's flux
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            er[i] = exp2f((float)(f.exm * (ool[i] * ool[i])));
+            ei[i] = 0.f;
         }
-        zr = cs * er - sn * ei;
-        zi = fmaf(cs, ei, sn * er);
+    } else if (dense) {
+        shapelet_dense<N, WIN>(p, win, cm, f.su, f.sv, ool, er, ei);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) shapelet_envelope_f32(p, cglob, g, f.su * ool[i], f.sv * ool[i], er[i], ei[i]);
     }
 }
 
-// The chosen form's Gaussians and shapelets with FCH channels per thread: a
-// CTA covers 256 baselines of FCH consecutive channels, so each component's
-// FP64 work that does not depend on the channel -- the phase in metres, the
-// Gaussian exponent in metres^2, the shapelet coordinates, their shared-
-// memory and table-position loads -- is done once for all FCH channels and
-// only scaled per channel (lambda^-1 for the phase and positions, lambda^-2
-// for the exponent).  The arithmetic per channel is that of the FAST
-// direct_kernel above, except that the accumulation uses W's Hermitian
-// symmetry (a shared beam).  Channels per thread, CTAs per SM and components
-// per staged chunk by type, chosen by timing: Gaussians (1) 4 channels, 2 CTAs
-// per SM, 64 components; shapelets (2) the same but 32 components, to keep
-// the static shared memory under 48 KB with the per-channel basis
-// coordinates (4 channels beat 2 once a thread's channels share the gathered
-// basis-table records: 10.2 against 11.5 ms per mixed step).
+// z = envelope x phasor of one channel.
 template <int TYPE>
-struct FastShape {
-    static constexpr int FCH = 4;
-    static constexpr int MIN_CTAS = 2;
-    static constexpr int CHUNK = 64;
-};
-template <>
-struct FastShape<2> {
-    static constexpr int FCH = 4;
-    static constexpr int MIN_CTAS = 2;
-    static constexpr int CHUNK = 32;
+__device__ __forceinline__ void fast_z(const FastTerm<TYPE>& f, double ool, float er, float ei, float& zr, float& zi) {
+    float sn, cs;
+    phasor_quarter_f32(4.0 * ool * f.tm, sn, cs);
+    zr = TYPE == 1 ? cs * er : cs * er - sn * ei;
+    zi = TYPE == 1 ? sn * er : fmaf(cs, ei, sn * er);
+}
+
+// The chosen form's shapelets with a beam shared by all tiles (or none): a
+// thread takes one baseline and SFCH consecutive channels, so each
+// component's FP64 work that does not depend on the channel (the phase in
+// metres, the coordinates, their loads) is done once, and the basis records
+// gathered for one channel serve its neighbours.  W = B S B^H is Hermitian:
+// with W_xy = a + i b the sums of w_xx z, w_yy z, a z and b z (four packed
+// fused multiply-adds) give the correlations as XY = P + i Q, YX = P - i Q.
+// Sums over a chunk of components are FP32; the FP64 sums over chunks live in
+// shared memory, which keeps the registers to the FP32 ones.
+// Bound: latency at 16 warps an SM (issue slots about half busy, shared-memory
+// reads above half: the scattered records and the coefficient rows).  100
+// shapelets, 128 tiles x 384 channels: 2.55 ms with all gathers from L1 and
+// the FP64 sums in registers, 1.84 ms so (per-channel coefficient reads 2.32;
+// those in registers at 128 threads 2.65; two channels a thread 5 to 7).
+constexpr int SFCH = 4;
+constexpr int SNT = 256;  // threads (baselines) per CTA
+constexpr int SCH = 16;   // components per staged chunk
+constexpr int SSUM = 2;   // chunks summed in FP32
+struct ShapeSmem {
+    double4 lmn[2][SCH];
+    JonesF64 flux[2][SFCH][SCH];
+    double4 gp[2][SCH];
+    float4 w[SFCH][SCH];  // xx, yy, Re xy, Im xy
+    float dense[SCH * SDN * SDN];
+    float4 win[2 * SWIN * (SDN / 2)];
+    double2 sum[SFCH][4][SNT];
+    uint64_t bar[3];
 };
 
-template <int TYPE, bool OUT64>
-__global__ void __launch_bounds__(DT, FastShape<TYPE>::MIN_CTAS) fast_kernel(const DirectParams p) {
-    constexpr int FCH = FastShape<TYPE>::FCH;
-    constexpr int CH = FastShape<TYPE>::CHUNK;  // components per staged chunk
-    __shared__ alignas(128) double4 s_lmn[2][CH];
-    __shared__ alignas(128) JonesF64 s_flux[2][FCH][CH];
-    __shared__ alignas(128) double4 s_gp[2][CH];
-    // W of each channel as (XX, YY, Re XY, Im XY): this kernel runs with a
-    // beam shared by all tiles (or none), where W = B S B^H is Hermitian
-    // (XX and YY real, YX = conj XY)
-    __shared__ alignas(16) float s_wf[FCH][CH * 4];
-    __shared__ alignas(16) float s_dense[TYPE == 2 ? CH * SDN * SDN : 1];
-    __shared__ alignas(8) uint64_t bar[2];
-
-    const int f0 = blockIdx.y * FCH;
-    const int bl = blockIdx.x * DT + threadIdx.x;
+template <bool DENSE, bool OUT64>
+__global__ void __launch_bounds__(SNT, 2) fast_shapelet_kernel(const DirectParams p) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    ShapeSmem& S = *reinterpret_cast<ShapeSmem*>(smem_raw);
+    const int f0 = blockIdx.y * SFCH;
+    const int bl = blockIdx.x * SNT + threadIdx.x;
     const bool active = bl < p.nbl;
     int t1 = 0, t2 = 1;
     if (active) baseline_to_tiles(bl, p.ntiles, t1, t2);
-    int fr[FCH];
-    double ool[FCH];
+    int fr[SFCH];
+    double ool[SFCH];
 #pragma unroll
-    for (int i = 0; i < FCH; i++) {
+    for (int i = 0; i < SFCH; i++) {
         fr[i] = min(f0 + i, p.nf - 1);  // a missing last channel repeats the previous one and is not stored
         ool[i] = p.freqs[fr[i]] / VEL_C;
     }
@@ -532,91 +466,100 @@ __global__ void __launch_bounds__(DT, FastShape<TYPE>::MIN_CTAS) fast_kernel(con
         um = q.u, vm = q.v, wm = q.w;
     }
 
-    const int nchunks = (p.nc + CH - 1) / CH;
+    const int nchunks = (p.nc + SCH - 1) / SCH;
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < 3; i++) mbar_init(&S.bar[i], 1);
         fence_barrier_init();
     }
     __syncthreads();
 
     auto issue = [&](int k) {
         const int st = k & 1;
-        const int c0 = k * CH;
-        const int n = min(CH, p.nc - c0);
-        const uint32_t bytes = n * 32u + FCH * n * 64u + n * 32u;
-        mbar_arrive_expect_tx(&bar[st], bytes);
-        bulk_g2s(s_lmn[st], p.lmn + c0, n * 32u, &bar[st]);
+        const int c0 = k * SCH;
+        const int n = min(SCH, p.nc - c0);
+        mbar_arrive_expect_tx(&S.bar[st], n * 32u + SFCH * n * 64u + n * 32u);
+        bulk_g2s(S.lmn[st], p.lmn + c0, n * 32u, &S.bar[st]);
 #pragma unroll
-        for (int i = 0; i < FCH; i++) bulk_g2s(s_flux[st][i], p.flux + (size_t)fr[i] * p.nc + c0, n * 64u, &bar[st]);
-        bulk_g2s(s_gp[st], p.gp + c0, n * 32u, &bar[st]);
+        for (int i = 0; i < SFCH; i++) bulk_g2s(S.flux[st][i], p.flux + (size_t)fr[i] * p.nc + c0, n * 64u, &S.bar[st]);
+        bulk_g2s(S.gp[st], p.gp + c0, n * 32u, &S.bar[st]);
     };
     int issued = 0;  // chunks whose copies thread 0 has issued
     if (threadIdx.x == 0) {
         fence_proxy_async_smem();
         if (!p.stall) {
+            if (DENSE) {
+                mbar_arrive_expect_tx(&S.bar[2], sizeof(S.win));
+                bulk_g2s(S.win, p.sbfp + (size_t)((int)SBF_C - SWIN) * (SDN / 2), sizeof(S.win), &S.bar[2]);
+            }
             if (nchunks > 0) issue(0), issued = 1;
             if (nchunks > 1) issue(1), issued = 2;
         }
     }
     const uint64_t limit = p.wait_ns ? p.wait_ns : 2000000000ull;
+    const bool win_ok = !DENSE || mbar_wait_bounded(&S.bar[2], 0, p.err, limit);
 
-    J2 acc[FCH];
+    uint64_t acc[SFCH][4];
 #pragma unroll
-    for (int i = 0; i < FCH; i++) acc[i] = jzero();
+    for (int i = 0; i < SFCH; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[i][e] = 0;
     bool aborted = false;
     for (int k = 0; k < nchunks; k++) {
         const int st = k & 1;
-        const bool ok = mbar_wait_bounded(&bar[st], (k >> 1) & 1, p.err, limit);
+        const bool ok = win_ok && mbar_wait_bounded(&S.bar[st], (k >> 1) & 1, p.err, limit);
+        const int c0 = k * SCH;
+        const int n = ok ? min(SCH, p.nc - c0) : 0;
+        for (int e = threadIdx.x; e < SFCH * SCH; e += SNT) {
+            const int i = e / SCH, c = e % SCH;
+            if (c >= n) continue;
+            const JonesF64 q = S.flux[st][i][c];
+            S.w[i][c] = make_float4((float)q.j00_re, (float)q.j11_re, (float)q.j01_re, (float)q.j01_im);
+        }
+        if (DENSE)
+            for (int e = threadIdx.x; e < n * SDN * SDN; e += SNT) S.dense[e] = __ldg(p.sdense + (size_t)c0 * SDN * SDN + e);
         if (__syncthreads_or(!ok)) {
             // the sum is incomplete: leave the visibilities untouched
-            if (threadIdx.x == 0) drain_two_stage(bar, k, issued);
+            if (threadIdx.x == 0) {
+                drain_two_stage(S.bar, k, issued);
+                if (DENSE && issued > 0) mbar_wait_bounded(&S.bar[2], 0, nullptr);
+            }
             aborted = true;
             break;
         }
-        const int c0 = k * CH;
-        const int n = min(CH, p.nc - c0);
-#pragma unroll
-        for (int i = 0; i < FCH; i++) {
-            const double* src = reinterpret_cast<const double*>(s_flux[st][i]);
-            for (int e = threadIdx.x; e < n * 4; e += DT) {
-                const int q = e & 3;  // XX re (0), YY re (6), XY re (2), XY im (3) of the component's 8
-                s_wf[i][e] = (float)src[(e >> 2) * 8 + (q == 0 ? 0 : (q == 1 ? 6 : q))];
-            }
-        }
-        if (TYPE == 2 && p.sdense)
-            for (int e = threadIdx.x; e < n * SDN * SDN; e += DT) s_dense[e] = __ldg(p.sdense + (size_t)c0 * SDN * SDN + e);
-        __syncthreads();
         if (active) {
-            float a[FCH][8];
-#pragma unroll
-            for (int i = 0; i < FCH; i++)
-#pragma unroll
-                for (int e = 0; e < 8; e++) a[i][e] = 0.f;
             for (int c = 0; c < n; c++) {
-                const double4 g = s_gp[st][c];
-                FastTerm<TYPE, FCH> term;
-                fast_term<TYPE, FCH>(p, s_lmn[st][c], g, um, vm, wm, c0 + c, t1, t2, ool,
-                                     TYPE == 2 && p.sdense ? s_dense + c * SDN * SDN : nullptr, term);
+                const double4 g = S.gp[st][c];
+                FastTerm<2> term;
+                fast_term<2>(S.lmn[st][c], g, um, vm, wm, shape_uv<2>(p, c0 + c, t1), shape_uv<2>(p, c0 + c, t2), DENSE,
+                             term);
+                float er[SFCH], ei[SFCH];
+                fast_envelopes<2, SFCH, DENSE>(p, term, ool, c0 + c, g, DENSE, S.dense + c * SDN * SDN, S.win, er, ei);
 #pragma unroll
-                for (int i = 0; i < FCH; i++) {
+                for (int i = 0; i < SFCH; i++) {
                     float zr, zi;
-                    fast_z<TYPE, FCH>(p, term, i, ool[i], c0 + c, g, p.sdense != nullptr, zr, zi);
-                    // a += W z with W Hermitian: 12 fused multiply-adds
-                    const float4 wv = *reinterpret_cast<const float4*>(s_wf[i] + c * 4);
-                    a[i][0] = fmaf(wv.x, zr, a[i][0]);
-                    a[i][1] = fmaf(wv.x, zi, a[i][1]);
-                    a[i][2] = fmaf(-wv.w, zi, fmaf(wv.z, zr, a[i][2]));
-                    a[i][3] = fmaf(wv.w, zr, fmaf(wv.z, zi, a[i][3]));
-                    a[i][4] = fmaf(wv.w, zi, fmaf(wv.z, zr, a[i][4]));
-                    a[i][5] = fmaf(-wv.w, zr, fmaf(wv.z, zi, a[i][5]));
-                    a[i][6] = fmaf(wv.y, zr, a[i][6]);
-                    a[i][7] = fmaf(wv.y, zi, a[i][7]);
+                    fast_z<2>(term, ool[i], er[i], ei[i], zr, zi);
+                    const uint64_t z = pack2(zr, zi);
+                    const float4 wv = S.w[i][c];
+                    acc[i][0] = fma2(dup2(wv.x), z, acc[i][0]);
+                    acc[i][1] = fma2(dup2(wv.y), z, acc[i][1]);
+                    acc[i][2] = fma2(dup2(wv.z), z, acc[i][2]);
+                    acc[i][3] = fma2(dup2(wv.w), z, acc[i][3]);
                 }
             }
+            if (k % SSUM == SSUM - 1 || k == nchunks - 1) {
+                const bool first = k < SSUM;
 #pragma unroll
-            for (int i = 0; i < FCH; i++)
-                acc[i] = acc[i] + J2{{a[i][0], a[i][1]}, {a[i][2], a[i][3]}, {a[i][4], a[i][5]}, {a[i][6], a[i][7]}};
+                for (int i = 0; i < SFCH; i++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float2 a = unpack2(acc[i][e]);
+                        double2 s = first ? make_double2(0.0, 0.0) : S.sum[i][e][threadIdx.x];
+                        s.x += (double)a.x;
+                        s.y += (double)a.y;
+                        S.sum[i][e][threadIdx.x] = s;
+                        acc[i][e] = 0;
+                    }
+            }
         }
         __syncthreads();
         if (threadIdx.x == 0 && k + 2 < nchunks) {
@@ -628,10 +571,32 @@ __global__ void __launch_bounds__(DT, FastShape<TYPE>::MIN_CTAS) fast_kernel(con
 
     if (!active || aborted) return;
 #pragma unroll
-    for (int i = 0; i < FCH; i++) {
+    for (int i = 0; i < SFCH; i++) {
         if (f0 + i >= p.nf) break;
-        add_vis<OUT64>(p.vis, (size_t)(f0 + i) * p.nbl + bl, acc[i]);
+        const double2 xx = S.sum[i][0][threadIdx.x], yy = S.sum[i][1][threadIdx.x];
+        const double2 a = S.sum[i][2][threadIdx.x], b = S.sum[i][3][threadIdx.x];
+        add_vis<OUT64>(p.vis, (size_t)(f0 + i) * p.nbl + bl,
+                       J2{{xx.x, xx.y}, {a.x - b.y, a.y + b.x}, {a.x + b.y, a.y - b.x}, {yy.x, yy.y}});
     }
+}
+
+template <bool DENSE, bool OUT64>
+static cudaError_t launch_fast_shapelet(const DirectParams& p, cudaStream_t s) {
+    // the opt-in above 48 KB of dynamic shared memory, once per device
+    static std::atomic<bool> attr[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!attr[dev].load(std::memory_order_relaxed)) {
+        e = cudaFuncSetAttribute(fast_shapelet_kernel<DENSE, OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(ShapeSmem));
+        if (e != cudaSuccess) return e;
+        attr[dev].store(true, std::memory_order_relaxed);
+    }
+    const dim3 grid((p.nbl + SNT - 1) / SNT, (p.nf + SFCH - 1) / SFCH);
+    fast_shapelet_kernel<DENSE, OUT64><<<grid, SNT, sizeof(ShapeSmem), s>>>(p);
+    return cudaGetLastError();
 }
 
 // The chosen form's Gaussians and shapelets with a beam per tile: each
@@ -770,13 +735,17 @@ __global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) 
         if (active) {
             for (int c = 0; c < n; c++) {
                 const double4 g = s_gp[st][c];
-                FastTerm<TYPE, FCH> term;
-                fast_term<TYPE, FCH>(p, s_lmn[st][c], g, um, vm, wm, c0 + c, t1, t2, ool,
-                                     TYPE == 2 && p.sdense ? s_dense + c * SDN * SDN : nullptr, term);
+                const bool dense = TYPE == 2 && p.sdense;
+                FastTerm<TYPE> term;
+                fast_term<TYPE>(s_lmn[st][c], g, um, vm, wm, shape_uv<TYPE>(p, c0 + c, t1), shape_uv<TYPE>(p, c0 + c, t2),
+                                dense, term);
+                float er[FCH], ei[FCH];
+                fast_envelopes<TYPE, FCH, false>(p, term, ool, c0 + c, g, dense, s_dense + (TYPE == 2 ? c * SDN * SDN : 0),
+                                                 nullptr, er, ei);
 #pragma unroll
                 for (int i = 0; i < FCH; i++) {
                     float zr, zi;
-                    fast_z<TYPE, FCH>(p, term, i, ool[i], c0 + c, g, p.sdense != nullptr, zr, zi);
+                    fast_z<TYPE>(term, ool[i], er[i], ei[i], zr, zi);
                     const float4* rg = s_gh + ((size_t)(i * CH + c) * nu + u1) * 6;
                     const double2* rh = reinterpret_cast<const double2*>(s_gh + ((size_t)(i * CH + c) * nu + u2) * 6 + 2);
                     const float4 g0 = rg[0], g1 = rg[1];
@@ -842,26 +811,18 @@ static cudaError_t launch_t(bool tile_beam, bool out64, bool fast, const DirectP
         if (e != cudaSuccess) return e;
     } else if (tile_beam) {
         if (out64)
-            direct_kernel<TYPE, true, true, false><<<grid, DT, 0, s>>>(p);
+            direct_kernel<TYPE, true, true><<<grid, DT, 0, s>>>(p);
         else
-            direct_kernel<TYPE, true, false, false><<<grid, DT, 0, s>>>(p);
-    } else if (fast && TYPE != 0) {
-        constexpr int FCH = FastShape<TYPE == 0 ? 1 : TYPE>::FCH;
-        const dim3 fgrid((p.nbl + DT - 1) / DT, (p.nf + FCH - 1) / FCH);
-        if (out64)
-            fast_kernel<TYPE == 0 ? 1 : TYPE, true><<<fgrid, DT, 0, s>>>(p);
-        else
-            fast_kernel<TYPE == 0 ? 1 : TYPE, false><<<fgrid, DT, 0, s>>>(p);
-    } else if (fast) {
-        if (out64)
-            direct_kernel<TYPE, false, true, true><<<grid, DT, 0, s>>>(p);
-        else
-            direct_kernel<TYPE, false, false, true><<<grid, DT, 0, s>>>(p);
+            direct_kernel<TYPE, true, false><<<grid, DT, 0, s>>>(p);
+    } else if (fast && TYPE == 2) {
+        const cudaError_t e = p.sdense ? (out64 ? launch_fast_shapelet<true, true>(p, s) : launch_fast_shapelet<true, false>(p, s))
+                                       : (out64 ? launch_fast_shapelet<false, true>(p, s) : launch_fast_shapelet<false, false>(p, s));
+        if (e != cudaSuccess) return e;
     } else {
         if (out64)
-            direct_kernel<TYPE, false, true, false><<<grid, DT, 0, s>>>(p);
+            direct_kernel<TYPE, false, true><<<grid, DT, 0, s>>>(p);
         else
-            direct_kernel<TYPE, false, false, false><<<grid, DT, 0, s>>>(p);
+            direct_kernel<TYPE, false, false><<<grid, DT, 0, s>>>(p);
     }
     count_launches(1);
     return cudaGetLastError();

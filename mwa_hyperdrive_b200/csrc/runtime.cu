@@ -232,15 +232,16 @@ const float4* device_shapelet_basis_pairs() {
     if (!g_sbfp[d]) {
         std::vector<double> h((size_t)SBF_N * SBF_L);
         host_shapelet_basis(h.data());
-        // position-major: the SDN orders' (value, next - value) pairs at one
-        // position are one 48-byte record (three float4)
+        // position-major: the orders' values and differences at one position
+        // are one 48-byte record, (v, v', d, d') of two orders per float4
         std::vector<float> hp((size_t)SBF_L * 2 * SDN_TABLE);
         for (int i = 0; i < SBF_L; i++)
             for (int n = 0; n < SDN_TABLE; n++) {
                 const size_t k = (size_t)n * SBF_L + i;
                 const double nxt = i + 1 < SBF_L ? h[k + 1] : h[k];
-                hp[((size_t)i * SDN_TABLE + n) * 2] = (float)h[k];
-                hp[((size_t)i * SDN_TABLE + n) * 2 + 1] = (float)(nxt - h[k]);
+                float* rec = &hp[((size_t)i * SDN_TABLE + (n & ~1)) * 2];
+                rec[n & 1] = (float)h[k];
+                rec[2 + (n & 1)] = (float)(nxt - h[k]);
             }
         if (cudaMalloc(&g_sbfp[d], hp.size() * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();

@@ -1,6 +1,6 @@
-"""The predicts factored by tile (csrc/pairs.cu) at the edges of their 32 x 32
-blocks of tile pairs and of their staged chunks of components, against the
-CPU oracle."""
+"""The predicts factored by tile (csrc/pairs.cu) and the shapelet kernel of the
+chosen form (csrc/predict.cu) at the edges of their 32 x 32 blocks of tile
+pairs and of their staged chunks of components, against the CPU oracle."""
 
 import math
 
@@ -75,7 +75,7 @@ def test_fp64(oracle, kind, beam, ntiles, n):
     assert np.max(np.abs(got - ref)) < 1e-10 * rms  # the FP64 form's bar
 
 
-@pytest.mark.parametrize("kind", ["gaussians"])
+@pytest.mark.parametrize("kind", ["gaussians", "shapelets"])
 @pytest.mark.parametrize("ntiles,n", [(2, 1), (17, 15), (33, 33), (64, 64), (65, 17)])
 def test_chosen_form(oracle, kind, ntiles, n):
     obs = observation(ntiles, ntiles)
@@ -85,3 +85,21 @@ def test_chosen_form(oracle, kind, ntiles, n):
         ref = expected(oracle, sky, obs, "analytic")
         # the chosen form's bar
         assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
+
+
+def test_chosen_form_shapelets_beyond_the_staged_window(oracle):
+    """Sources of a degree on long baselines: positions far from the basis
+    table's centre, and past its ends."""
+    obs = synth.Obs(synth.tiles_in_disk(20, 3000.0, 5), 180e6 + np.arange(5) * 80e3, PC, np.array([LST]))
+    rng = np.random.default_rng(6)
+    comps = []
+    for k, maj in enumerate(np.radians([0.02, 0.2, 1.0, 4.0])):
+        co = [sl.ShapeletCoeff(int(rng.integers(0, 6)), int(rng.integers(0, 6)), float(rng.normal())) for _ in range(8)]
+        comps.append(sl.SourceComponent(PC[0] + 0.01 * k, PC[1], sl.Shapelet(maj, 0.7 * maj, 0.3 * k, co),
+                                        sl.PowerLaw(-0.7, sl.FluxDensity(150e6, 1.0 + k))))
+    sky = sl.SkyModelArrays.from_components(comps)
+    ref = expected(oracle, sky, obs, "none")
+    got = predict(sky, obs, "tensor", "none", torch.float64)
+    assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
+    got = predict(sky, obs, "direct", "none", torch.float64)
+    assert np.linalg.norm(got - ref) < 1e-10 * np.linalg.norm(ref)
