@@ -670,10 +670,9 @@ int hdc_peel_timeblock_batched(JonesF32 *d_resid_tfb, const float *d_weights_tfb
                                const RADec *h_source_positions, IonoConsts *h_iono_consts, const HdcPeelParams *params,
                                hdcStream_t stream);
 
-/* The accumulation-sweep launch shape the batched peel's autotuner chose for
- * the last new problem shape (low-resolution bins and sources per CTA;
- * sources 0: the variant staging 16 baselines' residual in shared memory for
- * every source) and its measured time. */
+/* The accumulation sweep's launch shape for the last new problem shape
+ * (threads of a CTA along the low-resolution bins and along the sources; a
+ * thread takes several of both) and the measured time of its first sweep. */
 int hdc_peel_batched_tuning(int *block_bins, int *block_sources, float *ms);
 
 /* ---- Visibility preparation before DI calibration ---------------------- */

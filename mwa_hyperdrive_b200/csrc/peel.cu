@@ -98,7 +98,7 @@ __global__ void average_kernel(const JonesF32* hi, const float* w, JonesF32* lo,
 struct IonoDev {
     double alpha, beta, gain;
     int stop;
-    int pad;
+    int pad;  // blocks of the current iteration that have finished (iono_traces_kernel)
 };
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -165,20 +165,14 @@ __global__ void __launch_bounds__(PT) iono_partials_kernel(const JonesF32* resid
                        partials + (size_t)blockIdx.y * gridDim.x * 7);
 }
 
-// The same for a batch of sources: grid (ceil(nbl/PT), nf, nsrc); source s
-// reads resid/model/model_rot at s * nf * nbl, weights shared, uvws at
-// s * nbl, state st[s], partials [nsrc][nf][nblk][7].
-__global__ void __launch_bounds__(PT) iono_partials_batched_kernel(const JonesF32* resid, const float* weights,
-                                                                   const JonesF32* model, JonesF32* model_rot,
-                                                                   const IonoDev* st, const UVW* uvws,
-                                                                   const double* lambdas, int nbl, int nf,
-                                                                   double* partials) {
-    const int src = blockIdx.z;
-    if (st[src].stop) return;
-    const size_t off = (size_t)src * nf * nbl;
-    iono_partials_body(resid + off, weights, model + off, model_rot + off, st + src, uvws + (size_t)src * nbl,
-                       lambdas, nbl, blockIdx.y, blockIdx.x, gridDim.x,
-                       partials + ((size_t)src * nf + blockIdx.y) * gridDim.x * 7);
+// The constants' update from the seven sums (peel.cu:327-432).
+__device__ __forceinline__ void iono_step(const double* t, IonoDev* st, double convergence) {
+    const double a_uu = t[0], a_uv = t[1], a_vv = t[2], A_u = t[3], A_v = t[4], s_vm = t[5], s_mm = t[6];
+    const double denom = TAU * (a_uu * a_vv - a_uv * a_uv);
+    st->alpha += convergence * (A_u * a_vv - A_v * a_uv) / denom;
+    st->beta += convergence * (A_v * a_uu - A_u * a_uv) / denom;
+    st->gain *= 1. + convergence * (s_vm / s_mm - 1);
+    if (st->gain < 0.0) st->stop = 1;  // peel.cu:711
 }
 
 // Channel reduction with the lambda scaling and the constants update
@@ -212,12 +206,7 @@ __device__ __forceinline__ void iono_update_body(const double* partials, int nbl
             t[k] = 0.0;
             for (int w = 0; w < (int)(blockDim.x / 32); w++) t[k] += red[w][k];
         }
-        const double a_uu = t[0], a_uv = t[1], a_vv = t[2], A_u = t[3], A_v = t[4], s_vm = t[5], s_mm = t[6];
-        const double denom = TAU * (a_uu * a_vv - a_uv * a_uv);
-        st->alpha += convergence * (A_u * a_vv - A_v * a_uv) / denom;
-        st->beta += convergence * (A_v * a_uu - A_u * a_uv) / denom;
-        st->gain *= 1. + convergence * (s_vm / s_mm - 1);
-        if (st->gain < 0.0) st->stop = 1;  // peel.cu:711
+        iono_step(t, st, convergence);
     }
 }
 
@@ -225,14 +214,6 @@ __global__ void iono_update_kernel(const double* partials, int nblk, const doubl
                                    double convergence) {
     if (st->stop) return;
     iono_update_body(partials, nblk, lambdas, nf, st, convergence);
-}
-
-// grid (nsrc): source s updates st[s] from partials [s][nf][nblk][7].
-__global__ void iono_update_batched_kernel(const double* partials, int nblk, const double* lambdas, int nf,
-                                           IonoDev* st, double convergence) {
-    const int src = blockIdx.x;
-    if (st[src].stop) return;
-    iono_update_body(partials + (size_t)src * nf * nblk * 7, nblk, lambdas, nf, st + src, convergence);
 }
 
 __global__ void subtract_iono_kernel(JonesF32* resid, const JonesF32* model, IonoConsts c, IonoConsts old,
@@ -320,34 +301,118 @@ const char* iono_loop_on(const JonesF32* d_resid, const float* d_w, const JonesF
 }
 
 
-// iono_loop for a batch of sources on one stream, every source starting
-// from its own constants in `consts` and writing the fitted ones back; one
-// host read at the end.  Buffers: resid/model/model_rot [nsrc][nf][nbl],
-// uvws [nsrc][nbl]; scratch holds partials [nsrc][nf][nblk][7] then the
-// per-source IonoDev states.
-size_t iono_batched_scratch_bytes(int nsrc, int nbl, int nf) {
-    const int nblk = (nbl + PT - 1) / PT;
-    return sizeof(double) * ((size_t)nsrc * nf * nblk * 7 + 4) + sizeof(IonoDev) * (size_t)nsrc;
+// One iteration of the fits of a batch of sources from traces (XX + YY; the
+// fit reads nothing else): grid (ceil(nbl / PT), nsrc).  A thread takes one
+// baseline and all channels, so u and v leave the channel sums and the block
+// reduces 7 numbers once instead of once a channel; the source's last block to
+// finish adds the blocks' partials in order and updates its constants.
+// Bound: load latency over the short channel loop, then FP64 arithmetic
+// (about 36 operations a baseline and channel).  30 sources x 24 channels x
+// 8128 baselines: 185 us and a 32 us update kernel an iteration on Jones
+// matrices, a reduction per channel; 41 us so.
+__global__ void __launch_bounds__(PT) iono_traces_kernel(const float2* __restrict__ resid, const float* __restrict__ weights,
+                                                         const float2* __restrict__ model, IonoDev* states,
+                                                         const UVW* __restrict__ uvws, const double* __restrict__ lambdas,
+                                                         int nbl, int nf, double* partials, double convergence) {
+    const int src = blockIdx.y, nblk = gridDim.x;
+    IonoDev* st = states + src;
+    if (st->stop) return;
+    __shared__ double red[PT / 32][7];
+    __shared__ bool last;
+    const int bl = blockIdx.x * PT + threadIdx.x;
+    double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    if (bl < nbl) {
+        const UVW q = uvws[(size_t)src * nbl + bl];
+        const double turn = -4.0 * (q.u * st->alpha + q.v * st->beta), gain = st->gain;
+        double mm2 = 0.0, mr1 = 0.0;  // sums of w mm lambda^2 and w mr lambda
+        const float2 *rs = resid + (size_t)src * nf * nbl + bl, *ms = model + (size_t)src * nf * nbl + bl;
+        // four channels' loads in flight at a time
+        for (int f0 = 0; f0 < nf; f0 += 4) {
+            float2 r[4], m[4];
+            float w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const size_t i = (size_t)min(f0 + j, nf - 1) * nbl;
+                r[j] = rs[i];
+                m[j] = ms[i];
+                w[j] = f0 + j < nf ? __ldg(weights + i + bl) : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (f0 + j >= nf) break;
+                const double lam = __ldg(lambdas + f0 + j);
+                const cplx mi = cplx{(double)m[j].x, (double)m[j].y} * (phasor_quarter_f64(turn * lam) * gain);
+                const double wm = (double)w[j] * mi.re, mm = wm * mi.re;
+                mm2 = fma(mm, lam * lam, mm2);
+                mr1 = fma(wm * ((double)r[j].y - mi.im), lam, mr1);
+                v[5] = fma(wm, (double)r[j].x, v[5]);
+                v[6] += mm;
+            }
+        }
+        v[0] = mm2 * q.u * q.u;
+        v[1] = mm2 * q.u * q.v;
+        v[2] = mm2 * q.v * q.v;
+        v[3] = -mr1 * q.u;
+        v[4] = -mr1 * q.v;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        const double s = warp_sum(v[k]);
+        if (lane == 0) red[warp][k] = s;
+    }
+    __syncthreads();
+    double* part = partials + (size_t)src * nblk * 7;
+    if (threadIdx.x < 7) {
+        double s = 0.0;
+        for (int w = 0; w < PT / 32; w++) s += red[w][threadIdx.x];
+        part[(size_t)blockIdx.x * 7 + threadIdx.x] = s;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(&st->pad, 1) == nblk - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x < 7) {
+        double s = 0.0;
+        for (int b = 0; b < nblk; b++) s += __ldcg(part + (size_t)b * 7 + threadIdx.x);
+        red[0][threadIdx.x] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        iono_step(red[0], st, convergence);
+        st->pad = 0;
+    }
 }
 
-const char* iono_loop_batched_on(const JonesF32* d_resid, const float* d_w, const JonesF32* d_model,
-                                 JonesF32* d_model_rot, void* d_scratch, IonoConsts* consts, int nsrc, int nbl, int nf,
-                                 int niter, const UVW* d_uvws, const double* d_lambdas, double convergence,
-                                 cudaStream_t s) {
+// iono_loop for a batch of sources on one stream from their traces, every
+// source starting from its own constants in `consts` and writing the fitted
+// ones back; one host read at the end.  resid and model [nsrc][nf][nbl], uvws
+// [nsrc][nbl]; scratch holds partials [nsrc][nblk][7] then the per-source
+// IonoDev states.
+size_t iono_batched_scratch_bytes(int nsrc, int nbl) {
+    const int nblk = (nbl + PT - 1) / PT;
+    return sizeof(double) * ((size_t)nsrc * nblk * 7 + 4) + sizeof(IonoDev) * (size_t)nsrc;
+}
+
+const char* iono_loop_traces_on(const float2* d_resid, const float* d_w, const float2* d_model, void* d_scratch,
+                                IonoConsts* consts, int nsrc, int nbl, int nf, int niter, const UVW* d_uvws,
+                                const double* d_lambdas, double convergence, cudaStream_t s) {
     if (nbl <= 0 || nf <= 0 || nsrc <= 0) return NULL;
     const int nblk = (nbl + PT - 1) / PT;
     double* partials = reinterpret_cast<double*>(d_scratch);
-    const size_t part_doubles = (size_t)nsrc * nf * nblk * 7;
+    const size_t part_doubles = (size_t)nsrc * nblk * 7;
     IonoDev* st = reinterpret_cast<IonoDev*>(partials + ((part_doubles + 3) & ~(size_t)3));
     std::vector<IonoDev> h(nsrc);
     for (int i = 0; i < nsrc; i++) h[i] = IonoDev{consts[i].alpha, consts[i].beta, consts[i].gain, 0, 0};
     HDC_CUDA_RET_STR(cudaMemcpyAsync(st, h.data(), sizeof(IonoDev) * nsrc, cudaMemcpyHostToDevice, s));
-    const dim3 g(nblk, nf, nsrc);
     for (int it = 0; it < niter; it++) {
-        iono_partials_batched_kernel<<<g, PT, 0, s>>>(d_resid, d_w, d_model, d_model_rot, st, d_uvws, d_lambdas, nbl,
-                                                      nf, partials);
-        iono_update_batched_kernel<<<nsrc, PT, 0, s>>>(partials, nblk, d_lambdas, nf, st, convergence);
-        count_launches(2);
+        iono_traces_kernel<<<dim3(nblk, nsrc), PT, 0, s>>>(d_resid, d_w, d_model, st, d_uvws, d_lambdas, nbl, nf,
+                                                           partials, convergence);
+        count_launches(1);
     }
     HDC_CUDA_RET_STR(cudaGetLastError());
     HDC_CUDA_RET_STR(cudaMemcpyAsync(h.data(), st, sizeof(IonoDev) * nsrc, cudaMemcpyDeviceToHost, s));

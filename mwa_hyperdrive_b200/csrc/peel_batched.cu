@@ -25,7 +25,13 @@
 // Every phase on a baseline is a difference of per-tile phases (uvw_pq =
 // uvw_p - uvw_q), so the rotation and ionospheric phasors come from per-tile
 // tables [source][timestep][channel][tile] -- 128 phasors where a baseline
-// loop would evaluate 8128 -- and a baseline takes tab[p] conj(tab[q]).
+// loop would evaluate 8128 -- and a baseline takes tab[p] conj(tab[q]).  Both
+// sweeps take 32 x 32 blocks of tile pairs (2 x 2 a thread, on or above the
+// diagonal) with the block's 64 rows of the tables in shared memory.
+// The fit reads only the traces (XX + YY) of D_s and Mr_s, so the accumulate
+// sweep forms only those, from the residual's weighted traces (one complex
+// number a sample instead of four), and the fit's low-resolution arrays are
+// a quarter as large.
 // With one source this is the reference's sequence exactly (up to rounding:
 // FP32 products and sums with FP32 phasors after an exact FP64 range
 // reduction, as against its f32 intermediates); with several,
@@ -33,17 +39,12 @@
 // fitted in the same pass do not see each other's updates until the next
 // pass.  The source models M_s (high resolution, source frame) are predicted
 // once per timeblock by the modeller and reused by every pass.
-//
-// The accumulate sweep's CTA shape (low-resolution bins x sources per CTA;
-// sources in a CTA share the residual loads through L1) is chosen by timing
-// the candidates on the first call for a problem shape (the sweep only
-// writes its low-resolution outputs, so trial runs have no side effects).
 
-#include <chrono>
+#include <algorithm>
 #include <cmath>
-#include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -53,30 +54,31 @@ namespace hdc {
 cudaError_t k_xyzs_to_uvws(const XYZ* xyzs, const double* lmsts, UVW* uvws, RADec pc, int ntiles, int nbl, int nt,
                            cudaStream_t s);
 cudaError_t k_weights_average(const float* w, float* lo, int nt, int nbl, int nf, int favg, cudaStream_t s);
-size_t iono_batched_scratch_bytes(int nsrc, int nbl, int nf);
-const char* iono_loop_batched_on(const JonesF32* d_resid, const float* d_w, const JonesF32* d_model,
-                                 JonesF32* d_model_rot, void* d_scratch, IonoConsts* consts, int nsrc, int nbl, int nf,
-                                 int niter, const UVW* d_uvws, const double* d_lambdas, double convergence,
-                                 cudaStream_t s);
+size_t iono_batched_scratch_bytes(int nsrc, int nbl);
+const char* iono_loop_traces_on(const float2* d_resid, const float* d_w, const float2* d_model, void* d_scratch,
+                                IonoConsts* consts, int nsrc, int nbl, int nf, int niter, const UVW* d_uvws,
+                                const double* d_lambdas, double convergence, cudaStream_t s);
 
 namespace pb {
 
 struct SweepArgs {
-    const JonesF32* resid;  // [nt][nf][nbl], phase-centre frame
+    JonesF32* resid;        // [nt][nf][nbl], phase-centre frame
     const float* w;         // [nt][nf][nbl]
+    float2* wtr;            // [nt][nf][nbl]: w (XX + YY) of the residual
     const JonesF32* models; // [nsrc][nt][nf][nbl], source frames (general sources)
-    const JonesF32* ptab;   // [nsrc][nt][nf]: point-at-centre sources' models, or null
+    const float4* ptab;     // [nsrc][nt][nf]: point-at-centre sources' models (xx, yy, Re xy, Im xy; Hermitian), or null
     // per-tile phasors [nsrc][nt][nf][ntiles]; a baseline's factor is
     // tab[p] conj(tab[q]) for its tiles p, q (the phases are differences of
-    // per-tile phases, since uvw_pq = uvw_p - uvw_q)
-    const float2* rot;      // exp(-2 pi i (w_src,p - w_pc,p) / lambda): to the source frame
-    const float2* io_old;   // exp(-2 pi i (alpha u_p + beta v_p) lambda) of the old constants
-    const float2* ap_old;   // conj(rot) io_old (apply sweep)
-    const float2* ap_new;   // conj(rot) io_new (apply sweep)
+    // per-tile phases, since uvw_pq = uvw_p - uvw_q).  Two phasors a record,
+    // (re, re', im, im'), so that both products go through packed arithmetic:
+    float4* acc;            // exp(-2 pi i (w_src,p - w_pc,p) / lambda) (rotation to the source frame) and
+                            // exp(-2 pi i (alpha u_p + beta v_p) lambda) of the old constants
+    float4* app;            // conj(rotation) x the ionospheric phasor of the old and of the new constants
     const IonoConsts* old;  // [nsrc]
     const IonoConsts* neu;  // [nsrc] (apply sweep)
-    JonesF32* d_lo;         // [nsrc][nlo][nbl]
-    JonesF32* m_lo;         // [nsrc][nlo][nbl]
+    float4* gains;          // [nsrc] (apply sweep): old gain, minus the new one, 1 where no constant changed
+    float2* d_lo;           // [nsrc][nlo][nbl] traces of D
+    float2* m_lo;           // [nsrc][nlo][nbl] traces of Mr
     int nt, nf, nbl, ntiles, nsrc, favg;
 };
 
@@ -113,33 +115,113 @@ __global__ void tile_uvw_kernel(const XYZ* __restrict__ xyz, const double* __res
                  c_dec * c_ha * a.x - c_dec * s_ha * a.y + s_dec * a.z};
 }
 
-// rot[s][t][f][p] = exp(-2 pi i (w_s,p - w_pc,p) / lambda_f)
-__global__ void rot_table_kernel(const UVW* __restrict__ tuvw, const double* __restrict__ inv_lam, int ns, int nt,
-                                 int nf, int ntiles, float2* __restrict__ rot) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)ns * nt * nf * ntiles) return;
-    const int p = (int)(i % ntiles), f = (int)((i / ntiles) % nf), t = (int)((i / ((size_t)ntiles * nf)) % nt);
-    const int src = (int)(i / ((size_t)ntiles * nf * nt));
-    const double dw = tuvw[((size_t)src * nt + t) * ntiles + p].w - tuvw[((size_t)ns * nt + t) * ntiles + p].w;
-    rot[i] = phase_f(-TAU * dw * inv_lam[f]);
+// The ionospheric phasor of a tile, exactly 1 when alpha = beta = 0 (as
+// add_model skips it).
+__device__ __forceinline__ float2 iono_phasor(const IonoConsts& c, const UVW& q, double lam) {
+    if (c.alpha == 0.0 && c.beta == 0.0) return make_float2(1.f, 0.f);
+    return phase_f(-TAU * (q.u * c.alpha + q.v * c.beta) * lam);
 }
 
-// out[s][t][f][p] = [conj(rot) x] exp(-2 pi i (alpha u_s,p + beta v_s,p) lambda_f),
-// the ionospheric phase exactly 1 when alpha = beta = 0 (as add_model skips it)
-__global__ void iono_table_kernel(const UVW* __restrict__ tuvw, const double* __restrict__ lam,
-                                  const IonoConsts* __restrict__ k, const float2* __restrict__ rot, int ns, int nt,
-                                  int nf, int ntiles, float2* __restrict__ out) {
+// acc[s][t][f][p]: the rotation and the old constants' ionospheric phasor
+// (lam: lambda, then 1 / lambda)
+__global__ void acc_table_kernel(const UVW* __restrict__ tuvw, const double* __restrict__ lam,
+                                 const IonoConsts* __restrict__ k, int ns, int nt, int nf, int ntiles,
+                                 float4* __restrict__ acc) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)ns * nt * nf * ntiles) return;
     const int p = (int)(i % ntiles), f = (int)((i / ntiles) % nf), t = (int)((i / ((size_t)ntiles * nf)) % nt);
     const int src = (int)(i / ((size_t)ntiles * nf * nt));
-    const IonoConsts c = k[src];
-    float2 v = make_float2(1.f, 0.f);
-    if (c.alpha != 0.0 || c.beta != 0.0) {
-        const UVW q = tuvw[((size_t)src * nt + t) * ntiles + p];
-        v = phase_f(-TAU * (q.u * c.alpha + q.v * c.beta) * lam[f]);
+    const UVW q = tuvw[((size_t)src * nt + t) * ntiles + p];
+    const double dw = q.w - tuvw[((size_t)ns * nt + t) * ntiles + p].w;
+    const float2 r = phase_f(-TAU * dw * lam[nf + f]), io = iono_phasor(k[src], q, lam[f]);
+    acc[i] = make_float4(r.x, io.x, r.y, io.y);
+}
+
+// app[s][t][f][p] for the fitted constants; acc takes their phasor for the
+// next pass.
+__global__ void app_table_kernel(const UVW* __restrict__ tuvw, const double* __restrict__ lam,
+                                 const IonoConsts* __restrict__ old, const IonoConsts* __restrict__ k, int ns, int nt,
+                                 int nf, int ntiles, float4* __restrict__ acc, float4* __restrict__ app,
+                                 float4* __restrict__ gains) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (size_t)ns) {
+        const IonoConsts a = old[i], b = k[i];
+        const bool same = a.alpha == b.alpha && a.beta == b.beta && a.gain == b.gain;
+        gains[i] = make_float4((float)a.gain, -(float)b.gain, same ? 1.f : 0.f, 0.f);
     }
-    out[i] = rot ? cmulcf(v, rot[i]) : v;
+    if (i >= (size_t)ns * nt * nf * ntiles) return;
+    const int p = (int)(i % ntiles), f = (int)((i / ntiles) % nf), t = (int)((i / ((size_t)ntiles * nf)) % nt);
+    const int src = (int)(i / ((size_t)ntiles * nf * nt));
+    const float4 a = acc[i];
+    const float2 rot = make_float2(a.x, a.z);
+    const float2 io = iono_phasor(k[src], tuvw[((size_t)src * nt + t) * ntiles + p], lam[f]);
+    const float2 o = cmulcf(make_float2(a.y, a.w), rot), n = cmulcf(io, rot);
+    app[i] = make_float4(o.x, n.x, o.y, n.y);
+    acc[i] = make_float4(a.x, io.x, a.z, io.y);
+}
+
+// w (XX + YY) of every residual sample
+__global__ void trace_kernel(const JonesF32* __restrict__ resid, const float* __restrict__ w, size_t n,
+                             float2* __restrict__ wtr) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 a = reinterpret_cast<const float4*>(resid + i)[0], b = reinterpret_cast<const float4*>(resid + i)[1];
+    const float wt = w[i];
+    wtr[i] = make_float2(wt * (a.x + b.z), wt * (a.y + b.w));
+}
+
+// A sweep's block of tile pairs: rows 32 pb .., columns 32 qb .. (blocks on
+// or above the diagonal); 256 threads of 2 x 2 pairs, rows and columns 16
+// apart.
+constexpr int TB = 32, NTH = 256;
+struct PairBlock {
+    int pb, qb, rp, cq;  // this thread's first row and column slot (columns after the TB rows)
+    int bl[4];           // baselines of the pairs (row 0 col 0, row 0 col 1, ..), -1 where none
+};
+__device__ __forceinline__ PairBlock pair_block(int blk, int ntiles) {
+    PairBlock B;
+    const int nblk = (ntiles + TB - 1) / TB, noff = nblk * (nblk - 1) / 2;
+    if (blk < noff)
+        baseline_to_tiles(blk, nblk, B.pb, B.qb);
+    else
+        B.pb = B.qb = blk - noff;
+    B.rp = threadIdx.x >> 4;
+    B.cq = TB + (threadIdx.x & 15);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int p = B.pb * TB + B.rp + 16 * (i >> 1), q = B.qb * TB + B.cq - TB + 16 * (i & 1);
+        B.bl[i] = p < q && q < ntiles ? baseline_index(p, q, ntiles) : -1;
+    }
+    return B;
+}
+int pair_blocks(int ntiles) {
+    const int nblk = (ntiles + TB - 1) / TB;
+    return nblk * (nblk + 1) / 2;
+}
+// Start copying the record of a block's slot (row tiles, then column tiles)
+// from a table row into shared memory; zero past the array.
+__device__ __forceinline__ void copy_record(float4* dst, const float4* __restrict__ row, const PairBlock& B, int slot,
+                                            int ntiles) {
+    const int tile = slot < TB ? B.pb * TB + slot : B.qb * TB + slot - TB;
+    const int bytes = tile < ntiles ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(row + (bytes ? tile : 0)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_16(float4* dst, const float4* __restrict__ src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the newest group of this thread's copies have landed
+__device__ __forceinline__ void copy_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// Both phasors of a pair from its tiles' records: (re, re') and (im, im') of
+// a_p conj(a_q)
+__device__ __forceinline__ void pair_phasors(const float4& p, const float4& q, uint64_t& re, uint64_t& im) {
+    const uint64_t px = pack2(p.x, p.y), py = pack2(p.z, p.w), nx = pack2(-p.x, -p.y);
+    const uint64_t qx = pack2(q.x, q.y), qy = pack2(q.z, q.w);
+    re = fma2(py, qy, mul2(px, qx));
+    im = fma2(nx, qy, mul2(py, qx));
 }
 
 // a Jones matrix as four complex FP32 numbers
@@ -152,263 +234,320 @@ __device__ __forceinline__ JF load_jf(const JonesF32& j) {
     return JF{{make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)}};
 }
 
-__device__ __forceinline__ JonesF32 to_f32(const J2& v) {
-    return JonesF32{(float)v.a.re, (float)v.a.im, (float)v.b.re, (float)v.b.im,
-                    (float)v.c.re, (float)v.c.im, (float)v.d.re, (float)v.d.im};
-}
-
-// blockDim (BX, SY): x = low-resolution bins, y = sources of this CTA's chunk
-// Grid: one dimension, source groups fastest -- the CTAs of all source
-// groups of a bin block run close together, so each residual tile comes
-// from DRAM once and from L2 for the other sources.  Products are formed and
-// summed in FP32 (the data are FP32; a bin sums nt x favg = 128 samples,
-// ~1e-7 relative rounding), at 64 registers so that 4 CTAs share an SM.
-template <int BX, int SY>
-__global__ void __launch_bounds__(BX* SY, 4) accumulate_kernel(const SweepArgs A) {
-    const int nlo = A.nf / A.favg;
-    const int ngrp = (A.nsrc + SY - 1) / SY;
-    const int bin = (int)(blockIdx.x / ngrp) * BX + threadIdx.x;
-    const int src = (int)(blockIdx.x % ngrp) * SY + threadIdx.y;
-    if (bin >= nlo * A.nbl || src >= A.nsrc) return;
-    const int bl = bin % A.nbl, flo = bin / A.nbl;
-    int tp, tq;
-    baseline_to_tiles(bl, A.ntiles, tp, tq);
-    const float g = (float)A.old[src].gain;
-    const size_t nvis = (size_t)A.nt * A.nf * A.nbl;
-    const JonesF32* M = A.ptab ? nullptr : A.models + (size_t)src * nvis;
-    float2 sd[4] = {}, sm[4] = {};
-    float sw = 0.f;
-    for (int t = 0; t < A.nt; t++) {
-        for (int fc = flo * A.favg; fc < flo * A.favg + A.favg; fc++) {
-            const size_t i = ((size_t)t * A.nf + fc) * A.nbl + bl;
-            const float wt = A.w[i];
-            const size_t tb = (((size_t)src * A.nt + t) * A.nf + fc) * A.ntiles;
-            const float2 rot = cmulcf(A.rot[tb + tp], A.rot[tb + tq]);
-            const float2 io1 = cmulcf(A.io_old[tb + tp], A.io_old[tb + tq]);
-            const float2 io = make_float2(io1.x * g, io1.y * g);
-            const JF mj = load_jf(A.ptab ? A.ptab[((size_t)src * A.nt + t) * A.nf + fc] : M[i]);
-            const JF r = load_jf(A.resid[i]);
+// The accumulate sweep: traces of D_s and Mr_s of G sources (from blockIdx.z
+// G) at the block's pairs and one low-resolution channel.  The tables of
+// NSAMP samples are copied while the previous ones are used; a sample and
+// source cost a pair two packed products for the two phasors and seven
+// multiply-adds.  Products are formed and summed in FP32 (the data are FP32; a
+// bin sums nt x favg samples, ~1e-7 relative rounding).
+// Bound: issue slots (about 60 % busy at 16 warps an SM, the residual's loads
+// read one sample ahead).  30 sources, 8 timesteps x 384 channels x 8128
+// baselines: 3.5 ms with all four correlations and a thread per baseline and
+// source, 1.16 ms so.
+constexpr int NSAMP = 4;
+template <bool POINTS, int G>
+__global__ void __launch_bounds__(NTH, 2) accumulate_kernel(const SweepArgs A) {
+    __shared__ alignas(16) float4 s_tab[2][NSAMP][G][2 * TB];
+    const PairBlock B = pair_block(blockIdx.x, A.ntiles);
+    const int flo = blockIdx.y, nlo = A.nf / A.favg, s0 = blockIdx.z * G;
+    const int ng = min(G, A.nsrc - s0), nsamp = A.nt * A.favg;
+    const size_t nvis = (size_t)A.nt * A.nf * A.nbl, ntf = (size_t)A.nt * A.nf;
+    // samples in order: timestep, then channel of the group; tf = t nf + f
+    struct Walk {
+        int c, tf;
+    };
+    auto step = [&](Walk& x) {
+        x.tf++;
+        if (++x.c == A.favg) x.c = 0, x.tf += A.nf - A.favg;
+    };
+    const int slot = threadIdx.x & (2 * TB - 1), r0 = threadIdx.x / (2 * TB);
+    // this thread's copies: slot's records of the samples (and, G > 1, the
+    // source) that its quarter of the CTA takes
+    constexpr int NQ = NTH / (2 * TB), KSTEP = G == 1 ? NQ : 1;
+    static_assert(G == 1 || G == NQ, "a quarter of the CTA per source, or per sample");
+    const int js = G == 1 ? 0 : r0;
+    const float4* tab0 = A.acc + (size_t)(s0 + min(js, ng - 1)) * ntf * A.ntiles;
+    Walk ws = {0, flo * A.favg};
+    if (G == 1)
+        for (int e = 0; e < r0; e++) step(ws);
+    auto stage = [&](int k0, int buf) {
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const float2 m = cmulf(mj.v[e], io);
-                const float2 d = cmulf(r.v[e], rot);
-                sd[e].x = fmaf(d.x + m.x, wt, sd[e].x);
-                sd[e].y = fmaf(d.y + m.y, wt, sd[e].y);
-                sm[e].x = fmaf(m.x, wt, sm[e].x);
-                sm[e].y = fmaf(m.y, wt, sm[e].y);
+        for (int k = G == 1 ? r0 : 0; k < NSAMP; k += KSTEP) {
+            if (js < ng && k0 + k < nsamp) {
+                copy_record(&s_tab[buf][k][js][slot], tab0 + (size_t)ws.tf * A.ntiles, B, slot, A.ntiles);
+#pragma unroll
+                for (int e = 0; e < KSTEP; e++) step(ws);
             }
-            sw += wt;
         }
-    }
-    const double ws = sw;
-    const double acc_d[8] = {sd[0].x, sd[0].y, sd[1].x, sd[1].y, sd[2].x, sd[2].y, sd[3].x, sd[3].y};
-    const double acc_m[8] = {sm[0].x, sm[0].y, sm[1].x, sm[1].y, sm[2].x, sm[2].y, sm[3].x, sm[3].y};
-    const double inv = 1.0 / (ws > 0.0 ? ws : 1.0);
-    const size_t o = ((size_t)src * nlo + flo) * A.nbl + bl;
-    A.d_lo[o] = JonesF32{(float)(acc_d[0] * inv), (float)(acc_d[1] * inv), (float)(acc_d[2] * inv),
-                         (float)(acc_d[3] * inv), (float)(acc_d[4] * inv), (float)(acc_d[5] * inv),
-                         (float)(acc_d[6] * inv), (float)(acc_d[7] * inv)};
-    A.m_lo[o] = JonesF32{(float)(acc_m[0] * inv), (float)(acc_m[1] * inv), (float)(acc_m[2] * inv),
-                         (float)(acc_m[3] * inv), (float)(acc_m[4] * inv), (float)(acc_m[5] * inv),
-                         (float)(acc_m[6] * inv), (float)(acc_m[7] * inv)};
-}
-
-// one thread per high-resolution visibility; all sources' updates, summed in
-// FP32 and added to the residual once:
-//   R += sum_s M_s conj(rot_s) (g_old io_old - g_new io_new)
-// with conj(rot) io per baseline = ap[p] conj(ap[q]) from the per-tile tables
-__global__ void __launch_bounds__(256) apply_kernel(JonesF32* resid, const SweepArgs A) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t nvis = (size_t)A.nt * A.nf * A.nbl;
-    if (i >= nvis) return;
-    const int bl = (int)(i % A.nbl);
-    const int f = (int)((i / A.nbl) % A.nf);
-    const int t = (int)(i / ((size_t)A.nbl * A.nf));
-    int tp, tq;
-    baseline_to_tiles(bl, A.ntiles, tp, tq);
-    float2 dl[4] = {};
-#pragma unroll 4  // several sources' table loads in flight
-    for (int s = 0; s < A.nsrc; s++) {
-        const IonoConsts ko = A.old[s], kn = A.neu[s];
-        if (ko.alpha == kn.alpha && ko.beta == kn.beta && ko.gain == kn.gain) continue;
-        const size_t tb = (((size_t)s * A.nt + t) * A.nf + f) * A.ntiles;
-        const float2 po = cmulcf(A.ap_old[tb + tp], A.ap_old[tb + tq]);
-        const float2 pn = cmulcf(A.ap_new[tb + tp], A.ap_new[tb + tq]);
-        const float go = (float)ko.gain, gn = (float)kn.gain;
-        const float2 bd = make_float2(fmaf(go, po.x, -gn * pn.x), fmaf(go, po.y, -gn * pn.y));
-        const JF m = load_jf(A.ptab ? A.ptab[((size_t)s * A.nt + t) * A.nf + f] : A.models[(size_t)s * nvis + i]);
+        copy_commit();
+    };
+    float2 nr[4];
+    float nw[4];
+    Walk wf = {0, flo * A.favg};
+    auto fetch = [&](int k) {
+        const size_t row = (size_t)wf.tf * A.nbl;
+        const float2* pr = A.wtr + row;
+        const float* pw = A.w + row;
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float2 c = cmulf(m.v[e], bd);
-            dl[e].x += c.x, dl[e].y += c.y;
+        for (int i = 0; i < 4; i++) {
+            const bool has = k < nsamp && B.bl[i] >= 0;
+            nr[i] = has ? __ldg(pr + B.bl[i]) : make_float2(0.f, 0.f);
+            nw[i] = has ? __ldg(pw + B.bl[i]) : 0.f;
+        }
+        step(wf);
+    };
+    stage(0, 0);
+    fetch(0);
+    float g[G];
+#pragma unroll
+    for (int j = 0; j < G; j++) g[j] = j < ng ? (float)A.old[s0 + j].gain : 0.f;
+    float2 sd[4][G], sm[4][G];
+    float sw[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < G; j++) sd[i][j] = sm[i][j] = make_float2(0.f, 0.f);
+    Walk wk = {0, flo * A.favg};
+    for (int k0 = 0; k0 < nsamp; k0 += NSAMP) {
+        const int n = min(NSAMP, nsamp - k0), buf = (k0 / NSAMP) & 1;
+        stage(k0 + NSAMP, buf ^ 1);
+        copy_wait_one();
+        __syncthreads();
+        for (int k = 0; k < n; k++) {
+            const size_t tf = wk.tf, row = tf * A.nbl;
+            step(wk);
+            float2 r[4];
+            float w[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) r[i] = nr[i], w[i] = nw[i], sw[i] += w[i];
+            fetch(k0 + k + 1);  // the next sample's, in flight during this one
+#pragma unroll
+            for (int j = 0; j < G; j++) {
+                if (j >= ng) break;
+                float gm = g[j];
+                if (POINTS) {
+                    const float2 m = __ldg(reinterpret_cast<const float2*>(A.ptab + (size_t)(s0 + j) * ntf + tf));
+                    gm *= m.x + m.y;
+                }
+                const float4(&tab)[2 * TB] = s_tab[buf][k][j];
+                const float4 p[2] = {tab[B.rp], tab[B.rp + 16]}, q[2] = {tab[B.cq], tab[B.cq + 16]};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    uint64_t re2, im2;
+                    pair_phasors(p[i >> 1], q[i & 1], re2, im2);
+                    const float2 re = unpack2(re2), im = unpack2(im2);  // rotation, ionosphere
+                    sd[i][j].x = fmaf(r[i].x, re.x, fmaf(-r[i].y, im.x, sd[i][j].x));
+                    sd[i][j].y = fmaf(r[i].x, im.x, fmaf(r[i].y, re.x, sd[i][j].y));
+                    const float c = w[i] * gm;
+                    if (POINTS) {
+                        sm[i][j].x = fmaf(c, re.y, sm[i][j].x);
+                        sm[i][j].y = fmaf(c, im.y, sm[i][j].y);
+                    } else if (B.bl[i] >= 0) {
+                        const float4* mp = reinterpret_cast<const float4*>(A.models + (size_t)(s0 + j) * nvis + row + B.bl[i]);
+                        const float4 m0 = __ldg(mp), m1 = __ldg(mp + 1);
+                        const float2 cm = make_float2(c * (m0.x + m1.z), c * (m0.y + m1.w));
+                        sm[i][j].x = fmaf(cm.x, re.y, fmaf(-cm.y, im.y, sm[i][j].x));
+                        sm[i][j].y = fmaf(cm.x, im.y, fmaf(cm.y, re.y, sm[i][j].y));
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (B.bl[i] < 0) continue;
+        const double inv = 1.0 / (sw[i] > 0.f ? (double)sw[i] : 1.0);
+#pragma unroll
+        for (int j = 0; j < G; j++) {
+            if (j >= ng) break;
+            const size_t o = ((size_t)(s0 + j) * nlo + flo) * A.nbl + B.bl[i];
+            A.d_lo[o] = make_float2((float)((sd[i][j].x + sm[i][j].x) * inv), (float)((sd[i][j].y + sm[i][j].y) * inv));
+            A.m_lo[o] = make_float2((float)(sm[i][j].x * inv), (float)(sm[i][j].y * inv));
         }
     }
-    float4* p = reinterpret_cast<float4*>(resid + i);
-    const float4 a = p[0], b = p[1];
-    p[0] = make_float4(a.x + dl[0].x, a.y + dl[0].y, a.z + dl[1].x, a.w + dl[1].y);
-    p[1] = make_float4(b.x + dl[2].x, b.y + dl[2].y, b.z + dl[3].x, b.w + dl[3].y);
 }
 
-// ptab[(src * nt + t) * nf + f] = W[f][src] as FP32 (W = B S B^H of the
-// combined point-source modeller at timestep t)
+// The apply sweep: all sources' updates at the block's pairs of TFS
+// consecutive (timestep, channel) rows, summed in FP32 and added to the
+// residual once:
+//   R += sum_s M_s conj(rot_s) (g_old io_old - g_new io_new)
+// and, where a further sub-batch follows (next), its weighted trace.  A point
+// source's M is Hermitian: with M_xy = a + i b the sums of m_xx z, m_yy z, a z
+// and b z give XY = P + i Q, YX = P - i Q.  The tables of SCHUNK sources are
+// copied while the previous ones are used, across rows.
+// Bound: issue slots and, below them, the residual's two passes over memory
+// (0.3 ms).  The same problem: 2.97 ms with a thread per baseline, 1.18 ms so.
+constexpr int SCHUNK = 16, TFS = 8;
+template <bool POINTS>
+__global__ void __launch_bounds__(NTH, 2) apply_kernel(const SweepArgs A, bool next) {
+    __shared__ alignas(16) float4 s_tab[2][SCHUNK][2 * TB];
+    __shared__ alignas(16) float4 s_m[2][SCHUNK], s_g[2][SCHUNK];
+    const int nblk = (A.ntiles + TB - 1) / TB, nblocks = nblk * (nblk + 1) / 2;
+    const PairBlock B = pair_block(blockIdx.x % nblocks, A.ntiles);
+    const size_t ntf = (size_t)A.nt * A.nf, tf0 = (size_t)(blockIdx.x / nblocks) * TFS;
+    const int rows = (int)min((size_t)TFS, ntf - tf0), nch = (A.nsrc + SCHUNK - 1) / SCHUNK, steps = rows * nch;
+    const int slot = threadIdx.x & (2 * TB - 1), r0 = threadIdx.x / (2 * TB);
+    auto stage = [&](int st, int buf) {
+        if (st < steps) {
+            const int s0 = (st % nch) * SCHUNK;
+            const float4* row = A.app + ((size_t)s0 * ntf + tf0 + st / nch) * A.ntiles;
+            const int n = min(SCHUNK, A.nsrc - s0);
+            for (int j = r0; j < n; j += NTH / (2 * TB))
+                copy_record(&s_tab[buf][j][slot], row + (size_t)j * ntf * A.ntiles, B, slot, A.ntiles);
+            const int j = threadIdx.x % SCHUNK;
+            if (threadIdx.x < SCHUNK && j < n)
+                copy_16(&s_g[buf][j], A.gains + s0 + j);
+            else if (POINTS && threadIdx.x < 2 * SCHUNK && j < n)
+                copy_16(&s_m[buf][j], A.ptab + (size_t)(s0 + j) * ntf + tf0 + st / nch);
+        }
+        copy_commit();
+    };
+    stage(0, 0);
+    uint64_t acc[4][4];
+    float4 ra[4], rb[4];
+    for (int st = 0; st < steps; st++) {
+        const int chunk = st % nch, s0 = chunk * SCHUNK, n = min(SCHUNK, A.nsrc - s0);
+        const size_t tf = tf0 + st / nch, row = tf * A.nbl;
+        if (chunk == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[i][e] = 0;
+                // the row's residual, in flight while its sources are summed
+                const float4* r = reinterpret_cast<const float4*>(A.resid + row + max(B.bl[i], 0));
+                ra[i] = r[0];
+                rb[i] = r[1];
+            }
+        }
+        stage(st + 1, (st + 1) & 1);
+        copy_wait_one();
+        __syncthreads();
+        for (int j = 0; j < n; j++) {
+            const float4 gn = s_g[st & 1][j];
+            if (gn.z != 0.f) continue;  // its constants did not change
+            const float4(&tab)[2 * TB] = s_tab[st & 1][j];
+            const float4 p[2] = {tab[B.rp], tab[B.rp + 16]}, q[2] = {tab[B.cq], tab[B.cq + 16]};
+            const uint64_t gg = pack2(gn.x, gn.y);
+            uint64_t wm[4];
+            if (POINTS) {
+                const float4 m = s_m[st & 1][j];
+                wm[0] = dup2(m.x), wm[1] = dup2(m.y), wm[2] = dup2(m.z), wm[3] = dup2(m.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                uint64_t re2, im2;
+                pair_phasors(p[i >> 1], q[i & 1], re2, im2);
+                const float2 re = unpack2(mul2(re2, gg)), im = unpack2(mul2(im2, gg));
+                const float2 z = make_float2(re.x + re.y, im.x + im.y);
+                if (POINTS) {
+                    const uint64_t z2 = pack2(z.x, z.y);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[i][e] = fma2(wm[e], z2, acc[i][e]);
+                } else if (B.bl[i] >= 0) {
+                    const JF m = load_jf(A.models[(size_t)(s0 + j) * ntf * A.nbl + row + B.bl[i]]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float2 c = cmulf(m.v[e], z), o = unpack2(acc[i][e]);
+                        acc[i][e] = pack2(o.x + c.x, o.y + c.y);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (chunk != nch - 1) continue;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (B.bl[i] < 0) continue;
+            const float2 c0 = unpack2(acc[i][0]), c1 = unpack2(acc[i][1]), c2 = unpack2(acc[i][2]), c3 = unpack2(acc[i][3]);
+            // general sources keep the four correlations in their order
+            const float2 xx = c0, yy = POINTS ? c1 : c3;
+            const float2 xy = POINTS ? make_float2(c2.x - c3.y, c2.y + c3.x) : c1;
+            const float2 yx = POINTS ? make_float2(c2.x + c3.y, c2.y - c3.x) : c2;
+            const float4 a = ra[i], b = rb[i];
+            const float4 na = make_float4(a.x + xx.x, a.y + xx.y, a.z + xy.x, a.w + xy.y);
+            const float4 nb = make_float4(b.x + yx.x, b.y + yx.y, b.z + yy.x, b.w + yy.y);
+            float4* r = reinterpret_cast<float4*>(A.resid + row + B.bl[i]);
+            r[0] = na;
+            r[1] = nb;
+            if (next) {
+                const float wt = __ldg(A.w + row + B.bl[i]);
+                A.wtr[row + B.bl[i]] = make_float2(wt * (na.x + nb.z), wt * (na.y + nb.w));
+            }
+        }
+    }
+}
+
+// ptab[(src * nt + t) * nf + f] = W[f][src] as FP32 (xx, yy, Re xy, Im xy; W =
+// B S B^H of the combined point-source modeller at timestep t, Hermitian)
 __global__ void point_table_kernel(const JonesF64* __restrict__ W, int ns, int nf, int nt, int t,
-                                   JonesF32* __restrict__ ptab) {
+                                   float4* __restrict__ ptab) {
     const int src = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
     if (src >= ns) return;
     const JonesF64 w = W[(size_t)f * ns + src];
-    ptab[((size_t)src * nt + t) * nf + f] = JonesF32{(float)w.j00_re, (float)w.j00_im, (float)w.j01_re, (float)w.j01_im,
-                                                     (float)w.j10_re, (float)w.j10_im, (float)w.j11_re, (float)w.j11_im};
+    ptab[((size_t)src * nt + t) * nf + f] =
+        make_float4((float)w.j00_re, (float)w.j11_re, (float)w.j01_re, (float)w.j01_im);
 }
-
-// The same sums with the residual staged in shared memory: a CTA takes SB
-// consecutive baselines of one low-resolution channel, loads their
-// nt x favg samples of residual and weight once (coalesced), and its 256
-// threads (SB baselines x 256 / SB source lanes) then run every source of the
-// pass over them, so the residual crosses L2 once per pass instead of once per
-// source.  Shared memory: samples x SB x 36 bytes.
-constexpr int SB = 16;
-__global__ void __launch_bounds__(256) accumulate_staged_kernel(const SweepArgs A) {
-    extern __shared__ float4 st_smem[];
-    const int nlo = A.nf / A.favg, ns_samp = A.nt * A.favg;
-    const int nbb = (A.nbl + SB - 1) / SB;
-    const int flo = (int)(blockIdx.x / nbb), bl0 = (int)(blockIdx.x % nbb) * SB;
-    float4* R = st_smem;                                          // [sample][SB][2]
-    float* W = reinterpret_cast<float*>(st_smem + (size_t)ns_samp * SB * 2);  // [sample][SB]
-    for (int i = threadIdx.x; i < ns_samp * SB * 2; i += blockDim.x) {
-        const int h = i & 1, b = (i >> 1) % SB, k = (i >> 1) / SB;
-        const int t = k / A.favg, fc = flo * A.favg + k % A.favg, bl = bl0 + b;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (bl < A.nbl) v = reinterpret_cast<const float4*>(A.resid + ((size_t)t * A.nf + fc) * A.nbl + bl)[h];
-        R[i] = v;
-    }
-    for (int i = threadIdx.x; i < ns_samp * SB; i += blockDim.x) {
-        const int b = i % SB, k = i / SB;
-        const int t = k / A.favg, fc = flo * A.favg + k % A.favg, bl = bl0 + b;
-        W[i] = bl < A.nbl ? A.w[((size_t)t * A.nf + fc) * A.nbl + bl] : 0.f;
-    }
-    __syncthreads();
-    const int b = threadIdx.x % SB, lanes = blockDim.x / SB;
-    const int bl = bl0 + b;
-    if (bl >= A.nbl) return;
-    int tp, tq;
-    baseline_to_tiles(bl, A.ntiles, tp, tq);
-    const size_t nvis = (size_t)A.nt * A.nf * A.nbl;
-    for (int src = threadIdx.x / SB; src < A.nsrc; src += lanes) {
-        const float g = (float)A.old[src].gain;
-        const JonesF32* M = A.ptab ? nullptr : A.models + (size_t)src * nvis;
-        float2 sd[4] = {}, sm[4] = {};
-        float sw = 0.f;
-        for (int k = 0; k < ns_samp; k++) {
-            const int t = k / A.favg, fc = flo * A.favg + k % A.favg;
-            const float wt = W[k * SB + b];
-            const size_t tb = (((size_t)src * A.nt + t) * A.nf + fc) * A.ntiles;
-            const float2 rot = cmulcf(A.rot[tb + tp], A.rot[tb + tq]);
-            const float2 io1 = cmulcf(A.io_old[tb + tp], A.io_old[tb + tq]);
-            const float2 io = make_float2(io1.x * g, io1.y * g);
-            const JF mj = load_jf(A.ptab ? A.ptab[((size_t)src * A.nt + t) * A.nf + fc]
-                                         : M[((size_t)t * A.nf + fc) * A.nbl + bl]);
-            const float4 r0 = R[(k * SB + b) * 2], r1 = R[(k * SB + b) * 2 + 1];
-            const JF r = {{make_float2(r0.x, r0.y), make_float2(r0.z, r0.w), make_float2(r1.x, r1.y),
-                           make_float2(r1.z, r1.w)}};
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const float2 m = cmulf(mj.v[e], io);
-                const float2 d = cmulf(r.v[e], rot);
-                sd[e].x = fmaf(d.x + m.x, wt, sd[e].x);
-                sd[e].y = fmaf(d.y + m.y, wt, sd[e].y);
-                sm[e].x = fmaf(m.x, wt, sm[e].x);
-                sm[e].y = fmaf(m.y, wt, sm[e].y);
-            }
-            sw += wt;
-        }
-        const double inv = 1.0 / ((double)sw > 0.0 ? (double)sw : 1.0);
-        const size_t o = ((size_t)src * nlo + flo) * A.nbl + bl;
-        A.d_lo[o] = JonesF32{(float)(sd[0].x * inv), (float)(sd[0].y * inv), (float)(sd[1].x * inv),
-                             (float)(sd[1].y * inv), (float)(sd[2].x * inv), (float)(sd[2].y * inv),
-                             (float)(sd[3].x * inv), (float)(sd[3].y * inv)};
-        A.m_lo[o] = JonesF32{(float)(sm[0].x * inv), (float)(sm[0].y * inv), (float)(sm[1].x * inv),
-                             (float)(sm[1].y * inv), (float)(sm[2].x * inv), (float)(sm[2].y * inv),
-                             (float)(sm[3].x * inv), (float)(sm[3].y * inv)};
-    }
-}
-
-size_t staged_smem_bytes(const SweepArgs& A) { return (size_t)A.nt * A.favg * SB * 36; }
-
-void launch_staged(const SweepArgs& A, cudaStream_t s) {
-    const unsigned grid = (unsigned)((A.nf / A.favg) * ((A.nbl + SB - 1) / SB));
-    accumulate_staged_kernel<<<grid, 256, staged_smem_bytes(A), s>>>(A);
-    count_launches(1);
-}
-
-struct Variant {
-    int bx, sy;
-    void (*launch)(const SweepArgs&, cudaStream_t);
-};
-
-template <int BX, int SY>
-void launch_acc(const SweepArgs& A, cudaStream_t s) {
-    const int nbins = (A.nf / A.favg) * A.nbl;
-    const unsigned grid = (unsigned)((nbins + BX - 1) / BX) * (unsigned)((A.nsrc + SY - 1) / SY);
-    accumulate_kernel<BX, SY><<<grid, dim3(BX, SY), 0, s>>>(A);
-    count_launches(1);
-}
-
-// the last variant (bins 0 in the report: one CTA per SB baselines, every
-// source) stages the residual; it runs only when its shared memory fits
-const Variant kVariants[] = {{256, 1, launch_acc<256, 1>},
-                             {128, 2, launch_acc<128, 2>},
-                             {64, 4, launch_acc<64, 4>},
-                             {32, 8, launch_acc<32, 8>},
-                             {SB, 0, launch_staged}};
-constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-constexpr size_t kStagedSmemMax = 200 * 1024;
 
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int, int>, int> g_tuned;  // (nt, nf, nbl, nsrc, favg) -> variant
+std::set<std::tuple<int, int, int, int, int>> g_seen;  // shapes (nt, nf, nbl, nsrc, favg) timed
 struct Tuning {
     int bx = 0, sy = 0;
     float ms = 0.f;
 } g_last;
 
-// the fastest accumulate variant for this shape (timed once, then cached)
-int choose_variant(const SweepArgs& A, cudaStream_t s) {
-    const auto key = std::make_tuple(A.nt, A.nf, A.nbl, A.nsrc, A.favg);
+template <bool POINTS, int G>
+void launch_acc(const SweepArgs& A, cudaStream_t s) {
+    const dim3 grid(pair_blocks(A.ntiles), A.nf / A.favg, (A.nsrc + G - 1) / G);
+    accumulate_kernel<POINTS, G><<<grid, NTH, 0, s>>>(A);
+    count_launches(1);
+}
+
+// The accumulate sweep: GRP sources a thread share its residual loads where
+// that leaves two CTAs for every SM, else one.  The first sweep of a problem
+// shape is timed (hdc_peel_batched_tuning reports it).
+constexpr int GRP = 4;
+cudaError_t accumulate(const SweepArgs& A, cudaStream_t s) {
+    const long long ctas = (long long)pair_blocks(A.ntiles) * (A.nf / A.favg) * ((A.nsrc + GRP - 1) / GRP);
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const bool group = ctas >= 2 * nsm;
+    bool timed;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) return it->second;
+        timed = g_seen.insert(std::make_tuple(A.nt, A.nf, A.nbl, A.nsrc, A.favg)).second;
     }
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    int best = 0;
-    float best_ms = 1e30f;
-    const size_t st_smem = staged_smem_bytes(A);
-    const bool staged_ok =
-        st_smem <= kStagedSmemMax &&
-        cudaFuncSetAttribute(accumulate_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st_smem) ==
-            cudaSuccess;
-    cudaGetLastError();
-    for (int v = 0; v < kNumVariants; v++) {
-        if (kVariants[v].sy == 0 && !staged_ok) continue;
-        kVariants[v].launch(A, s);  // warm
+    cudaEvent_t a = nullptr, b = nullptr;
+    if (timed) {
+        cudaEventCreate(&a);
+        cudaEventCreate(&b);
         cudaEventRecord(a, s);
-        kVariants[v].launch(A, s);
-        cudaEventRecord(b, s);
-        cudaEventSynchronize(b);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, a, b);
-        if (cudaGetLastError() == cudaSuccess && ms < best_ms) {
-            best_ms = ms;
-            best = v;
-        }
     }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[key] = best;
-    g_last = Tuning{kVariants[best].bx, kVariants[best].sy, best_ms};
-    return best;
+    if (A.ptab)
+        group ? launch_acc<true, GRP>(A, s) : launch_acc<true, 1>(A, s);
+    else
+        group ? launch_acc<false, GRP>(A, s) : launch_acc<false, 1>(A, s);
+    cudaError_t e = cudaGetLastError();
+    if (timed) {
+        float ms = 0.f;
+        cudaEventRecord(b, s);
+        if (e == cudaSuccess) e = cudaEventSynchronize(b);
+        if (e == cudaSuccess) cudaEventElapsedTime(&ms, a, b);
+        cudaEventDestroy(a);
+        cudaEventDestroy(b);
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        g_last = Tuning{NTH, 1, ms};
+    }
+    return e;
+}
+
+void apply(const SweepArgs& A, bool next, cudaStream_t s) {
+    const unsigned grid = (unsigned)((size_t)pair_blocks(A.ntiles) * (((size_t)A.nt * A.nf + TFS - 1) / TFS));
+    if (A.ptab)
+        apply_kernel<true><<<grid, NTH, 0, s>>>(A, next);
+    else
+        apply_kernel<false><<<grid, NTH, 0, s>>>(A, next);
+    count_launches(1);
 }
 
 // call-scoped device buffers from the library's stream-ordered pool: freed
@@ -495,15 +634,15 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     }
     size_t free_b = 0, total_b = 0;
     PB_CK(cudaMemGetInfo(&free_b, &total_b));
-    const size_t need = points ? sizeof(JonesF32) * (size_t)ns * nt * nf : sizeof(JonesF32) * nvis * (size_t)ns;
+    const size_t need = points ? sizeof(float4) * (size_t)ns * nt * nf : sizeof(JonesF32) * nvis * (size_t)ns;
     if (need + (size_t)(1u << 30) > free_b) {
         set_error("hdc_peel_timeblock_batched: the %d source models need %zu MB of device memory, %zu MB free", ns,
                   need >> 20, free_b >> 20);
         return HDC_ERR_ALLOC;
     }
-    pb::DevBuf b_tuvw, b_radec, b_rot, b_io, b_apo, b_apn;
-    pb::DevBuf b_lam, b_lam_lo, b_lmst, b_avg_lmst, b_xyz, b_uv_src, b_uv_lo, b_models, b_dlo, b_mlo, b_mlo_rot,
-        b_wlo, b_scr, b_old, b_new;
+    pb::DevBuf b_tuvw, b_radec, b_acc, b_app, b_wtr;
+    pb::DevBuf b_lam, b_lam_lo, b_lmst, b_avg_lmst, b_xyz, b_uv_src, b_uv_lo, b_models, b_dlo, b_mlo, b_wlo, b_scr,
+        b_old, b_new, b_gains;
     PB_CK(b_lam.alloc(sizeof(double) * 2 * nf, s));  // lambda, then 1 / lambda
     PB_CK(b_lam_lo.alloc(sizeof(double) * nlo, s));
     PB_CK(b_lmst.alloc(sizeof(double) * nt, s));
@@ -513,39 +652,44 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     const size_t ntab = (size_t)ns * nt * nf * num_tiles;  // per-tile phasor tables
     PB_CK(b_tuvw.alloc(sizeof(UVW) * (size_t)(ns + 1) * nt * num_tiles, s));
     PB_CK(b_radec.alloc(sizeof(double2) * (ns + 1), s));
-    PB_CK(b_rot.alloc(sizeof(float2) * ntab, s));
-    PB_CK(b_io.alloc(sizeof(float2) * ntab, s));
-    PB_CK(b_apo.alloc(sizeof(float2) * ntab, s));
-    PB_CK(b_apn.alloc(sizeof(float2) * ntab, s));
+    PB_CK(b_acc.alloc(sizeof(float4) * ntab, s));
+    // one sub-batch's apply table at a time
+    const int batch = params->batch_size > 0 ? std::min(params->batch_size, ns) : ns;
+    PB_CK(b_app.alloc(sizeof(float4) * (size_t)batch * nt * nf * num_tiles, s));
+    PB_CK(b_wtr.alloc(sizeof(float2) * nvis, s));
     PB_CK(b_uv_lo.alloc(sizeof(UVW) * (size_t)ns * nbl, s));
     PB_CK(points ? b_models.alloc(need, s) : b_models.alloc_plain(need));
-    PB_CK(b_dlo.alloc(sizeof(JonesF32) * (size_t)ns * nlo * nbl, s));
-    PB_CK(b_mlo.alloc(sizeof(JonesF32) * (size_t)ns * nlo * nbl, s));
-    PB_CK(b_mlo_rot.alloc(sizeof(JonesF32) * (size_t)ns * nlo * nbl, s));
+    PB_CK(b_dlo.alloc(sizeof(float2) * (size_t)batch * nlo * nbl, s));
+    PB_CK(b_mlo.alloc(sizeof(float2) * (size_t)batch * nlo * nbl, s));
     PB_CK(b_wlo.alloc(sizeof(float) * (size_t)nlo * nbl, s));
-    PB_CK(b_scr.alloc(iono_batched_scratch_bytes(ns, nbl, nlo), s));
+    PB_CK(b_scr.alloc(iono_batched_scratch_bytes(batch, nbl), s));
     PB_CK(b_old.alloc(sizeof(IonoConsts) * ns, s));
     PB_CK(b_new.alloc(sizeof(IonoConsts) * ns, s));
+    PB_CK(b_gains.alloc(sizeof(float4) * batch, s));
     PB_CK(cudaMemcpyAsync(b_lam.p, lam.data(), sizeof(double) * 2 * nf, cudaMemcpyHostToDevice, s));
     PB_CK(cudaMemcpyAsync(b_lam_lo.p, lam_lo.data(), sizeof(double) * nlo, cudaMemcpyHostToDevice, s));
     PB_CK(cudaMemcpyAsync(b_lmst.p, h_lmsts, sizeof(double) * nt, cudaMemcpyHostToDevice, s));
     PB_CK(cudaMemcpyAsync(b_avg_lmst.p, &average_lmst, sizeof(double), cudaMemcpyHostToDevice, s));
     PB_CK(cudaMemcpyAsync(b_xyz.p, xyz_t.data(), sizeof(XYZ) * xyz_t.size(), cudaMemcpyHostToDevice, s));
     PB_CK(k_weights_average(d_weights_tfb, b_wlo.as<float>(), nt, nbl, nf, favg, s));
-    // per-tile UVWs in every source's frame and the phase centre's, and the
-    // rotation phasors to each source (fixed for the timeblock)
+    // per-tile UVWs in every source's frame and the phase centre's, the
+    // rotation phasors to each source (fixed for the timeblock) with the given
+    // constants' ionospheric ones, and the residual's weighted traces
     std::vector<double2> radec(ns + 1);
     for (int i = 0; i < ns; i++) radec[i] = make_double2(h_source_positions[i].ra, h_source_positions[i].dec);
     radec[ns] = make_double2(phase_centre.ra, phase_centre.dec);
     PB_CK(cudaMemcpyAsync(b_radec.p, radec.data(), sizeof(double2) * (ns + 1), cudaMemcpyHostToDevice, s));
+    PB_CK(cudaMemcpyAsync(b_old.p, h_iono_consts, sizeof(IonoConsts) * ns, cudaMemcpyHostToDevice, s));
     {
         const int n = (ns + 1) * nt * num_tiles;
         pb::tile_uvw_kernel<<<(n + 255) / 256, 256, 0, s>>>(b_xyz.as<XYZ>(), b_lmst.as<double>(),
                                                             b_radec.as<double2>(), ns + 1, nt, num_tiles,
                                                             b_tuvw.as<UVW>());
-        pb::rot_table_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, s>>>(
-            b_tuvw.as<UVW>(), b_lam.as<double>() + nf, ns, nt, nf, num_tiles, b_rot.as<float2>());
-        count_launches(2);
+        pb::acc_table_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, s>>>(
+            b_tuvw.as<UVW>(), b_lam.as<double>(), b_old.as<IonoConsts>(), ns, nt, nf, num_tiles, b_acc.as<float4>());
+        pb::trace_kernel<<<(unsigned)((nvis + 255) / 256), 256, 0, s>>>(d_resid_tfb, d_weights_tfb, nvis,
+                                                                       b_wtr.as<float2>());
+        count_launches(3);
         PB_CK(cudaGetLastError());
     }
     PB_CK(cudaMemsetAsync(b_models.p, 0, need, s));
@@ -585,7 +729,7 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
             rc = m->geometry(h_lmsts[t], s);
             if (rc) return rc;
             pb::point_table_kernel<<<dim3((ns + 127) / 128, nf), 128, 0, s>>>(m->weights(0), ns, nf, nt, t,
-                                                                              b_models.as<JonesF32>());
+                                                                              b_models.as<float4>());
             count_launches(1);
             PB_CK(cudaGetLastError());
         }
@@ -611,16 +755,16 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     pb::SweepArgs A;
     A.resid = d_resid_tfb;
     A.w = d_weights_tfb;
+    A.wtr = b_wtr.as<float2>();
     A.models = points ? nullptr : b_models.as<JonesF32>();
-    A.ptab = points ? b_models.as<JonesF32>() : nullptr;
-    A.rot = b_rot.as<float2>();
-    A.io_old = b_io.as<float2>();
-    A.ap_old = b_apo.as<float2>();
-    A.ap_new = b_apn.as<float2>();
+    A.ptab = points ? b_models.as<float4>() : nullptr;
+    A.acc = b_acc.as<float4>();
+    A.app = b_app.as<float4>();
     A.old = b_old.as<IonoConsts>();
     A.neu = b_new.as<IonoConsts>();
-    A.d_lo = b_dlo.as<JonesF32>();
-    A.m_lo = b_mlo.as<JonesF32>();
+    A.gains = b_gains.as<float4>();
+    A.d_lo = b_dlo.as<float2>();
+    A.m_lo = b_mlo.as<float2>();
     A.nt = nt;
     A.nf = nf;
     A.nbl = nbl;
@@ -631,37 +775,24 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     // sources in sub-batches of `batch` in list order: within a sub-batch the
     // fits share the residual (Jacobi); each sub-batch sees the residual the
     // earlier ones left (the reference's Gauss-Seidel order between them)
-    const int batch = params->batch_size > 0 ? std::min(params->batch_size, ns) : ns;
     for (int pass = 0; pass < params->num_passes; pass++) {
         for (int b0 = 0; b0 < ns; b0 += batch) {
             const int nb = std::min(batch, ns - b0);
-            const size_t tab0 = (size_t)b0 * nt * nf * num_tiles, ntab_b = (size_t)nb * nt * nf * num_tiles;
+            const size_t ntab_b = (size_t)nb * nt * nf * num_tiles;
             pb::SweepArgs B = A;
             B.nsrc = nb;
             B.models = A.models ? A.models + (size_t)b0 * nvis : nullptr;
             B.ptab = A.ptab ? A.ptab + (size_t)b0 * nt * nf : nullptr;
-            B.rot = A.rot + tab0;
-            B.io_old = A.io_old + tab0;
-            B.ap_old = A.ap_old + tab0;
-            B.ap_new = A.ap_new + tab0;
+            B.acc = A.acc + (size_t)b0 * nt * nf * num_tiles;
             B.old = A.old + b0;
             B.neu = A.neu + b0;
-            const UVW* tuvw_b = b_tuvw.as<UVW>() + (size_t)b0 * nt * num_tiles;
             PB_CK(cudaMemcpyAsync(b_old.as<IonoConsts>() + b0, h_iono_consts + b0, sizeof(IonoConsts) * nb,
                                   cudaMemcpyHostToDevice, s));
-            const unsigned tgrid = (unsigned)((ntab_b + 255) / 256);
-            pb::iono_table_kernel<<<tgrid, 256, 0, s>>>(tuvw_b, b_lam.as<double>(), B.old, nullptr, nb, nt, nf,
-                                                        num_tiles, b_io.as<float2>() + tab0);
-            count_launches(1);
-            PB_CK(cudaGetLastError());
-            const int v = pb::choose_variant(B, s);
-            pb::kVariants[v].launch(B, s);
-            PB_CK(cudaGetLastError());
+            PB_CK(pb::accumulate(B, s));
             for (int i = 0; i < nb; i++) fit[i] = IonoConsts{0.0, 0.0, 1.0};
-            const char* err = iono_loop_batched_on(b_dlo.as<JonesF32>(), b_wlo.as<float>(), b_mlo.as<JonesF32>(),
-                                                   b_mlo_rot.as<JonesF32>(), b_scr.p, fit.data(), nb, nbl, nlo,
-                                                   params->num_loops, b_uv_lo.as<UVW>() + (size_t)b0 * nbl,
-                                                   b_lam_lo.as<double>(), params->convergence, s);
+            const char* err = iono_loop_traces_on(B.d_lo, b_wlo.as<float>(), B.m_lo, b_scr.p, fit.data(), nb, nbl, nlo,
+                                                  params->num_loops, b_uv_lo.as<UVW>() + (size_t)b0 * nbl,
+                                                  b_lam_lo.as<double>(), params->convergence, s);
             if (err) {
                 set_error("hdc_peel_timeblock_batched: %s", err);
                 return HDC_ERR_CUDA;
@@ -675,14 +806,13 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
             }
             PB_CK(cudaMemcpyAsync(b_new.as<IonoConsts>() + b0, next.data() + b0, sizeof(IonoConsts) * nb,
                                   cudaMemcpyHostToDevice, s));
-            pb::iono_table_kernel<<<tgrid, 256, 0, s>>>(tuvw_b, b_lam.as<double>(), B.old, B.rot, nb, nt, nf,
-                                                        num_tiles, b_apo.as<float2>() + tab0);
-            pb::iono_table_kernel<<<tgrid, 256, 0, s>>>(tuvw_b, b_lam.as<double>(), B.neu, B.rot, nb, nt, nf,
-                                                        num_tiles, b_apn.as<float2>() + tab0);
-            count_launches(2);
-            PB_CK(cudaGetLastError());
-            pb::apply_kernel<<<(unsigned)((nvis + 255) / 256), 256, 0, s>>>(d_resid_tfb, B);
+            // app from tuvw rows of this sub-batch's sources
+            pb::app_table_kernel<<<(unsigned)((ntab_b + 255) / 256), 256, 0, s>>>(
+                b_tuvw.as<UVW>() + (size_t)b0 * nt * num_tiles, b_lam.as<double>(), B.old, B.neu, nb, nt, nf,
+                num_tiles, B.acc, B.app, B.gains);
             count_launches(1);
+            PB_CK(cudaGetLastError());
+            pb::apply(B, pass + 1 < params->num_passes || b0 + batch < ns, s);
             PB_CK(cudaGetLastError());
             PB_CK(cudaStreamSynchronize(s));  // `next` is read by the copy above
             for (int i = 0; i < nb; i++) h_iono_consts[b0 + i] = next[b0 + i];

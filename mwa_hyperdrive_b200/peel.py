@@ -94,9 +94,9 @@ def peel_gpu(d_resid_tfb, d_weights_tfb, freqs, tile_xyzs, lmsts, average_lmst, 
 
 
 def batched_tuning():
-    """(bins per CTA, sources per CTA, ms) the batched peel's autotuner chose
-    for the last new problem shape; (16, 0) is the variant that stages the
-    residual of 16 baselines in shared memory for every source."""
+    """(threads along the bins, along the sources, ms) of the batched peel's
+    accumulation sweep for the last new problem shape: its CTAs' shape and the
+    time of its first sweep."""
     bx, sy, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_float()
     _lib.check(_lib.lib().hdc_peel_batched_tuning(ctypes.byref(bx), ctypes.byref(sy), ctypes.byref(ms)),
                "hdc_peel_batched_tuning")
