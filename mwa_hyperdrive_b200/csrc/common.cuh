@@ -267,9 +267,12 @@ __device__ __forceinline__ cplx phasor_quarter_f64(double z) {
             __hiloint2double(__double2hiint(a) ^ (int)(qs & 0x80000000u), __double2loint(a))};
 }
 
-// FP64 phasor exp(2 pi i t) for a phase in turns: exact range reduction to
-// r = t - rint(t) in [-1/2, 1/2] first, so any size of t is good.
-__device__ __forceinline__ cplx phasor_turns(double t) { return phasor_quarter_f64(4.0 * (t - rint(t))); }
+// FP64 phasor exp(2 pi i t) for a phase of any size in turns: whole turns go
+// first (beyond 2^51 turns t is a whole number and what the rounding leaves is
+// one too).
+__device__ __forceinline__ cplx phasor_turns(double t) {
+    return phasor_quarter_f64(4.0 * __dsub_rn(t, __dsub_rn(__dadd_rn(t, QMAGIC), QMAGIC)));
+}
 
 // FP32 phasor for the tensor-core predict and the chosen form's direct
 // kernels: sin and cos of 2 pi z for z in quarter-turns.  q = rint(z) and

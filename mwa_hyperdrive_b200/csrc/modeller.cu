@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "modeller.cuh"
+#include "peel.cuh"
 #include "predict.cuh"
 
 namespace hdc {
@@ -84,13 +85,8 @@ struct FluxComp {
     double freq, i, q, u, v, si, cq;
 };
 
-__global__ void flux_kernel(const FluxComp* comps, int nc, const double* freqs, int nf, JonesF64* S) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f = blockIdx.y;
-    if (c >= nc) return;
-    const FluxComp k = comps[c];
-    if (k.flux_type == 0) return;
-    const double nu = freqs[f];
+// a (curved) power law's instrumental flux at nu
+__device__ __forceinline__ JonesF64 power_law_flux(const FluxComp& k, double nu) {
     const double ratio = pow(nu / k.freq, k.si);
     double i = k.i * ratio, q = k.q * ratio, u = k.u * ratio, v = k.v * ratio;
     if (k.flux_type == 2) {
@@ -101,7 +97,15 @@ __global__ void flux_kernel(const FluxComp* comps, int nc, const double* freqs, 
         u *= curved;
         v *= curved;
     }
-    S[(size_t)f * nc + c] = JonesF64{i - q, 0.0, u, -v, u, v, i + q, 0.0};
+    return JonesF64{i - q, 0.0, u, -v, u, v, i + q, 0.0};
+}
+
+__global__ void flux_kernel(const FluxComp* comps, int nc, const double* freqs, int nf, JonesF64* S) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = blockIdx.y;
+    if (c >= nc) return;
+    const FluxComp k = comps[c];
+    if (k.flux_type != 0) S[(size_t)f * nc + c] = power_law_flux(k, freqs[f]);
 }
 
 // Baseline UVWs (m) as tile-UVW differences at one hour angle / declination.
@@ -215,6 +219,27 @@ __global__ void beam_weight_kernel(const double2* radec, int nc, const double* f
     const J2 b = analytic_beam(az, el, freqs[f]);
     const J2 s = load_j(S[(size_t)f * nc + c]);
     W[(size_t)f * nc + c] = store_j((b * s) * herm(b));
+}
+
+// The models of point sources at their own positions (peel_point_table):
+// thread per (source, channel) of a timestep.  list: the list fluxes'
+// instrumental Jones [channel][source], NULL when every source is a power law.
+__global__ void point_model_kernel(const FluxComp* comps, const JonesF64* list, const double2* radec, int ns,
+                                   const double* freqs, int nf, double lst, int t, int nt, double lat, int beam_kind,
+                                   float4* out) {
+    const int src = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = blockIdx.y;
+    if (src >= ns) return;
+    const FluxComp k = comps[src];
+    J2 w = load_j(k.flux_type ? power_law_flux(k, freqs[f]) : list[(size_t)f * ns + src]);
+    if (beam_kind == HDC_BEAM_ANALYTIC_DIPOLE) {
+        const double2 rd = radec[src];
+        double az, el;
+        hadec_to_azel(lst - rd.x, rd.y, lat, az, el);
+        const J2 b = analytic_beam(az, el, freqs[f]);
+        w = (b * w) * herm(b);
+    }
+    out[((size_t)src * nt + t) * nf + f] = make_float4((float)w.a.re, (float)w.d.re, (float)w.b.re, (float)w.b.im);
 }
 
 // FP32 copy of a per-tile beam table (n Jones matrices).
@@ -1003,6 +1028,66 @@ extern "C" int hdc_source_brightness_fee(const HdcSkyModel* sky, const int* h_co
                                   phase_centre, HDC_BEAM_FEE, beam, source_dist_cutoff_rad, min_elevation_rad,
                                   h_brightness);
 }
+
+namespace hdc {
+bool peel_point_sources(const HdcSkyModel* h_sources, const RADec* h_positions, int num_sources, int beam_kind) {
+    if (beam_kind != HDC_BEAM_NONE && beam_kind != HDC_BEAM_ANALYTIC_DIPOLE) return false;
+    for (int i = 0; i < num_sources; i++) {
+        const HdcSkyModel& m = h_sources[i];
+        if (m.num_components != 1 || m.comp_type[0] != HDC_POINT || std::fabs(m.ra[0] - h_positions[i].ra) >= 1e-12 ||
+            std::fabs(m.dec[0] - h_positions[i].dec) >= 1e-12 || m.flux_type[0] < 0 || m.flux_type[0] > 2 ||
+            m.fd_count[0] < 1)
+            return false;
+    }
+    return true;
+}
+
+int peel_point_table(const HdcSkyModel* h_sources, int num_sources, const double* h_freqs, int num_freqs,
+                     const double* h_lmsts, int num_timesteps, double latitude, int beam_kind, float4* d_table,
+                     cudaStream_t s) {
+    const int ns = num_sources, nf = num_freqs, nt = num_timesteps;
+    std::vector<FluxComp> fc(ns);
+    std::vector<double2> radec(ns);
+    std::vector<JonesF64> list;
+    for (int i = 0; i < ns; i++) {
+        const HdcSkyModel* m = h_sources + i;
+        const int ft = m->flux_type[0];
+        FluxComp f = {};
+        f.flux_type = ft;
+        radec[i] = make_double2(m->ra[0], m->dec[0]);
+        if (ft == HDC_FLUX_LIST) {
+            list.resize((size_t)nf * ns);
+            for (int k = 0; k < nf; k++) list[(size_t)k * ns + i] = inst_stokes(estimate_list(m, 0, h_freqs[k]));
+        } else {
+            const Stokes r = fd_entry(m, m->fd_start[0]);
+            f.freq = r.freq, f.i = r.i, f.q = r.q, f.u = r.u, f.v = r.v;
+            f.si = m->si[0];
+            f.cq = ft == HDC_FLUX_CURVED_POWER_LAW ? m->q[0] : 0.0;
+        }
+        fc[i] = f;
+    }
+    DevBuf b_fc, b_radec, b_list, b_freqs;
+    HDC_CUDA_RET_INT(b_fc.alloc(sizeof(FluxComp) * ns, s));
+    HDC_CUDA_RET_INT(b_radec.alloc(sizeof(double2) * ns, s));
+    HDC_CUDA_RET_INT(b_freqs.alloc(sizeof(double) * nf, s));
+    HDC_CUDA_RET_INT(cudaMemcpyAsync(b_fc.p, fc.data(), sizeof(FluxComp) * ns, cudaMemcpyHostToDevice, s));
+    HDC_CUDA_RET_INT(cudaMemcpyAsync(b_radec.p, radec.data(), sizeof(double2) * ns, cudaMemcpyHostToDevice, s));
+    HDC_CUDA_RET_INT(cudaMemcpyAsync(b_freqs.p, h_freqs, sizeof(double) * nf, cudaMemcpyHostToDevice, s));
+    if (!list.empty()) {
+        HDC_CUDA_RET_INT(b_list.alloc(sizeof(JonesF64) * list.size(), s));
+        HDC_CUDA_RET_INT(cudaMemcpyAsync(b_list.p, list.data(), sizeof(JonesF64) * list.size(), cudaMemcpyHostToDevice, s));
+    }
+    const int threads = ns >= 128 ? 128 : 32;
+    for (int t = 0; t < nt; t++) {
+        point_model_kernel<<<dim3((ns + threads - 1) / threads, nf), threads, 0, s>>>(
+            b_fc.as<FluxComp>(), b_list.as<JonesF64>(), b_radec.as<double2>(), ns, b_freqs.as<double>(), nf, h_lmsts[t],
+            t, nt, latitude, beam_kind, d_table);
+        count_launches(1);
+    }
+    HDC_CUDA_RET_INT(cudaGetLastError());
+    return HDC_OK;
+}
+}  // namespace hdc
 
 extern "C" int hdc_modeller_new(const HdcSkyModel* sky, int pols, const XYZ* h_xyzs, int num_tiles,
                                 const double* h_freqs, int num_freqs, RADec phase_centre, double array_latitude_rad,

@@ -14,7 +14,7 @@
 
 #include <vector>
 
-#include "common.cuh"
+#include "peel.cuh"
 
 namespace hdc {
 
@@ -56,20 +56,37 @@ __device__ __forceinline__ JonesF32 jf32_mul_c32(const JonesF32& a, cplx r) {
                     __fadd_rn(__fmul_rn(a.j11_re, y), __fmul_rn(a.j11_im, x))};
 }
 
-__global__ void rotate_kernel(JonesF32* vis, int nt, int nbl, int nf, const UVW* from, const UVW* to,
-                              const double* lambdas) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = (size_t)nt * nf * nbl;
-    if (i >= n) return;
-    const int bl = (int)(i % nbl);
-    const int f = (int)((i / nbl) % nf);
-    const int t = (int)(i / ((size_t)nbl * nf));
-    const double arg = -TAU * (to[(size_t)t * nbl + bl].w - from[(size_t)t * nbl + bl].w);
-    double s, c;
-    sincos(arg / lambdas[f], &s, &c);
-    JonesF32 j = vis[i];
-    jf32_mul_f64(j, cplx{c, s});
-    vis[i] = j;
+// A thread takes ROT_F channels of one (timestep, baseline): its UVWs and
+// indices serve them all.  blockIdx.x = baseline block, fastest, then channel
+// group, then timestep.
+constexpr int ROT_F = 4;
+struct VisThread {
+    int bl, f0, t;
+};
+__device__ __forceinline__ VisThread vis_thread(int nbl, int nf) {
+    const unsigned nbb = (nbl + PT - 1) / PT, nfg = (nf + ROT_F - 1) / ROT_F;
+    return VisThread{(int)(blockIdx.x % nbb) * PT + (int)threadIdx.x, (int)((blockIdx.x / nbb) % nfg) * ROT_F,
+                     (int)(blockIdx.x / (nbb * nfg))};
+}
+static unsigned vis_grid(int nt, int nf, int nbl) {
+    return (unsigned)((size_t)((nbl + PT - 1) / PT) * ((nf + ROT_F - 1) / ROT_F) * nt);
+}
+
+__global__ void __launch_bounds__(PT) rotate_kernel(JonesF32* vis, int nt, int nbl, int nf, const UVW* from,
+                                                    const UVW* to, const double* lambdas) {
+    const VisThread x = vis_thread(nbl, nf);
+    if (x.bl >= nbl) return;
+    const size_t r = (size_t)x.t * nbl + x.bl;
+    const double dw = to[r].w - from[r].w;
+#pragma unroll
+    for (int k = 0; k < ROT_F; k++) {
+        const int f = x.f0 + k;
+        if (f >= nf) break;
+        const size_t i = ((size_t)x.t * nf + f) * nbl + x.bl;
+        JonesF32 j = vis[i];
+        jf32_mul_f64(j, phasor_turns(-dw / __ldg(lambdas + f)));
+        vis[i] = j;
+    }
 }
 
 __global__ void average_kernel(const JonesF32* hi, const float* w, JonesF32* lo, int nt, int nbl, int nf, int favg) {
@@ -91,15 +108,6 @@ __global__ void average_kernel(const JonesF32* hi, const float* w, JonesF32* lo,
                                           (float)(sum.b.im / d),  (float)(sum.c.re / d), (float)(sum.c.im / d),
                                           (float)(sum.d.re / d),  (float)(sum.d.im / d)};
 }
-
-// Device state of one iono_loop call, kept at the end of the caller's
-// d_iono_fits scratch: the constants, a stop flag and per-(channel, CTA)
-// partial sums.
-struct IonoDev {
-    double alpha, beta, gain;
-    int stop;
-    int pad;  // blocks of the current iteration that have finished (iono_traces_kernel)
-};
 
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -268,7 +276,7 @@ __global__ void add_model_kernel(JonesF32* resid, const JonesF32* model, IonoCon
 
 static unsigned grid1(size_t n) { return (unsigned)((n + PT - 1) / PT); }
 
-// Host-side body of iono_loop on a stream; also used by the native peel.
+// Host-side body of iono_loop on a stream.
 const char* iono_loop_on(const JonesF32* d_resid, const float* d_w, const JonesF32* d_model, JonesF32* d_model_rot,
                          JonesF64* d_fits, IonoConsts* consts, int nbl, int nf, int niter, const UVW* d_uvws,
                          const double* d_lambdas, double convergence, cudaStream_t s) {
@@ -302,14 +310,17 @@ const char* iono_loop_on(const JonesF32* d_resid, const float* d_w, const JonesF
 
 
 // One iteration of the fits of a batch of sources from traces (XX + YY; the
-// fit reads nothing else): grid (ceil(nbl / PT), nsrc).  A thread takes one
-// baseline and all channels, so u and v leave the channel sums and the block
-// reduces 7 numbers once instead of once a channel; the source's last block to
-// finish adds the blocks' partials in order and updates its constants.
+// fit reads nothing else): grid (ceil(nbl / IONO_BL), nsrc).  A thread takes one
+// baseline and every fourth channel, so u and v leave the channel sums and the
+// block reduces 7 numbers once instead of once a channel; the source's last
+// block to finish adds the blocks' partials and updates its
+// constants.
 // Bound: load latency over the short channel loop, then FP64 arithmetic
 // (about 36 operations a baseline and channel).  30 sources x 24 channels x
 // 8128 baselines: 185 us and a 32 us update kernel an iteration on Jones
-// matrices, a reduction per channel; 41 us so.
+// matrices, a reduction per channel; 41 us so.  One source x 12 channels:
+// 27 -> 9 us.
+constexpr int IONO_BL = 64, IONO_CH = PT / IONO_BL;
 __global__ void __launch_bounds__(PT) iono_traces_kernel(const float2* __restrict__ resid, const float* __restrict__ weights,
                                                          const float2* __restrict__ model, IonoDev* states,
                                                          const UVW* __restrict__ uvws, const double* __restrict__ lambdas,
@@ -319,28 +330,28 @@ __global__ void __launch_bounds__(PT) iono_traces_kernel(const float2* __restric
     if (st->stop) return;
     __shared__ double red[PT / 32][7];
     __shared__ bool last;
-    const int bl = blockIdx.x * PT + threadIdx.x;
+    const int bl = blockIdx.x * IONO_BL + threadIdx.x % IONO_BL;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     if (bl < nbl) {
         const UVW q = uvws[(size_t)src * nbl + bl];
         const double turn = -4.0 * (q.u * st->alpha + q.v * st->beta), gain = st->gain;
         double mm2 = 0.0, mr1 = 0.0;  // sums of w mm lambda^2 and w mr lambda
         const float2 *rs = resid + (size_t)src * nf * nbl + bl, *ms = model + (size_t)src * nf * nbl + bl;
-        // four channels' loads in flight at a time
-        for (int f0 = 0; f0 < nf; f0 += 4) {
-            float2 r[4], m[4];
-            float w[4];
+        // two channels' loads in flight at a time
+        for (int f0 = threadIdx.x / IONO_BL; f0 < nf; f0 += 2 * IONO_CH) {
+            float2 r[2], m[2];
+            float w[2];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const size_t i = (size_t)min(f0 + j, nf - 1) * nbl;
+            for (int j = 0; j < 2; j++) {
+                const size_t i = (size_t)min(f0 + j * IONO_CH, nf - 1) * nbl;
                 r[j] = rs[i];
                 m[j] = ms[i];
-                w[j] = f0 + j < nf ? __ldg(weights + i + bl) : 0.f;
+                w[j] = __ldg(weights + i + bl);
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (f0 + j >= nf) break;
-                const double lam = __ldg(lambdas + f0 + j);
+            for (int j = 0; j < 2; j++) {
+                if (f0 + j * IONO_CH >= nf) break;
+                const double lam = __ldg(lambdas + f0 + j * IONO_CH);
                 const cplx mi = cplx{(double)m[j].x, (double)m[j].y} * (phasor_quarter_f64(turn * lam) * gain);
                 const double wm = (double)w[j] * mi.re, mm = wm * mi.re;
                 mm2 = fma(mm, lam * lam, mm2);
@@ -376,10 +387,12 @@ __global__ void __launch_bounds__(PT) iono_traces_kernel(const float2* __restric
     }
     __syncthreads();
     if (!last) return;
-    if (threadIdx.x < 7) {
+    // warp k adds sum k's partials
+    if (warp < 7) {
         double s = 0.0;
-        for (int b = 0; b < nblk; b++) s += __ldcg(part + (size_t)b * 7 + threadIdx.x);
-        red[0][threadIdx.x] = s;
+        for (int b = lane; b < nblk; b += 32) s += __ldcg(part + (size_t)b * 7 + warp);
+        s = warp_sum(s);
+        if (lane == 0) red[0][warp] = s;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -388,37 +401,191 @@ __global__ void __launch_bounds__(PT) iono_traces_kernel(const float2* __restric
     }
 }
 
-// iono_loop for a batch of sources on one stream from their traces, every
-// source starting from its own constants in `consts` and writing the fitted
-// ones back; one host read at the end.  resid and model [nsrc][nf][nbl], uvws
-// [nsrc][nbl]; scratch holds partials [nsrc][nblk][7] then the per-source
-// IonoDev states.
-size_t iono_batched_scratch_bytes(int nsrc, int nbl) {
-    const int nblk = (nbl + PT - 1) / PT;
-    return sizeof(double) * ((size_t)nsrc * nblk * 7 + 4) + sizeof(IonoDev) * (size_t)nsrc;
+size_t iono_partials_bytes(int nsrc, int nbl) {
+    return sizeof(double) * (size_t)nsrc * ((nbl + IONO_BL - 1) / IONO_BL) * 7;
 }
 
-const char* iono_loop_traces_on(const float2* d_resid, const float* d_w, const float2* d_model, void* d_scratch,
-                                IonoConsts* consts, int nsrc, int nbl, int nf, int niter, const UVW* d_uvws,
-                                const double* d_lambdas, double convergence, cudaStream_t s) {
-    if (nbl <= 0 || nf <= 0 || nsrc <= 0) return NULL;
-    const int nblk = (nbl + PT - 1) / PT;
-    double* partials = reinterpret_cast<double*>(d_scratch);
-    const size_t part_doubles = (size_t)nsrc * nblk * 7;
-    IonoDev* st = reinterpret_cast<IonoDev*>(partials + ((part_doubles + 3) & ~(size_t)3));
-    std::vector<IonoDev> h(nsrc);
-    for (int i = 0; i < nsrc; i++) h[i] = IonoDev{consts[i].alpha, consts[i].beta, consts[i].gain, 0, 0};
-    HDC_CUDA_RET_STR(cudaMemcpyAsync(st, h.data(), sizeof(IonoDev) * nsrc, cudaMemcpyHostToDevice, s));
-    for (int it = 0; it < niter; it++) {
-        iono_traces_kernel<<<dim3(nblk, nsrc), PT, 0, s>>>(d_resid, d_w, d_model, st, d_uvws, d_lambdas, nbl, nf,
-                                                           partials, convergence);
-        count_launches(1);
+__global__ void iono_init_kernel(IonoDev* st, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) st[i] = IonoDev{0.0, 0.0, 1.0, 0, 0};
+}
+
+cudaError_t iono_states_init(IonoDev* states, int nsrc, cudaStream_t s) {
+    iono_init_kernel<<<grid1(nsrc), PT, 0, s>>>(states, nsrc);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+// The fitted constants, or the old ones where the reference's rule reverts
+// them (gpu.rs:541-627); the states are ready for the next fit.
+__global__ void iono_result_kernel(IonoDev* st, const IonoConsts* old, IonoConsts* neu, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const IonoConsts o = old[i];
+    const IonoConsts c = {o.alpha + st[i].alpha, o.beta + st[i].beta, o.gain * st[i].gain};
+    const bool revert = fabs(c.alpha) > 1e-3 || fabs(c.beta) > 1e-3 || c.gain < 0.0 || c.gain > 1.5;
+    neu[i] = revert ? o : c;
+    st[i] = IonoDev{0.0, 0.0, 1.0, 0, 0};
+}
+
+cudaError_t iono_fit(const float2* d_resid, const float* d_w, const float2* d_model, double* d_partials,
+                     IonoDev* d_states, const IonoConsts* d_old, IonoConsts* d_neu, int nsrc, int nbl, int nf, int niter,
+                     const UVW* d_uvws, const double* d_lambdas, double convergence, cudaStream_t s) {
+    if (nbl <= 0 || nf <= 0 || nsrc <= 0) return cudaSuccess;
+    const dim3 grid((nbl + IONO_BL - 1) / IONO_BL, nsrc);
+    for (int it = 0; it < niter; it++)
+        iono_traces_kernel<<<grid, PT, 0, s>>>(d_resid, d_w, d_model, d_states, d_uvws, d_lambdas, nbl, nf, d_partials,
+                                               convergence);
+    iono_result_kernel<<<grid1(nsrc), PT, 0, s>>>(d_states, d_old, d_neu, nsrc);
+    count_launches(niter + 1);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// The source-by-source loop's two passes over the residual.  They take the
+// reference's steps in its order and roundings (rotate to FP32, add_model's
+// FP32 product and sum, FP64 averages; rotate, then subtract_iono in FP64)
+// without storing what lies between: rotate, two add_models, two averages,
+// the copy of the residual and the clears were twelve passes over it.
+// ---------------------------------------------------------------------------
+// add_model's factor: the ionospheric phasor (exactly 1 when alpha = beta = 0)
+// times the gain, as FP32
+__device__ __forceinline__ float2 iono_factor(const IonoConsts& c, const UVW& q, double lam) {
+    cplx r = {1.0, 0.0};
+    if (!(c.alpha == 0.0 && c.beta == 0.0)) r = phasor_turns(-(q.u * c.alpha + q.v * c.beta) * lam);
+    return make_float2((float)(r.re * c.gain), (float)(r.im * c.gain));
+}
+// x y in FP32, each product rounded (JonesF32 * C64 of gpu/common.cuh)
+__device__ __forceinline__ float2 mul_rn(float2 x, float2 y) {
+    return make_float2(__fsub_rn(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y)),
+                       __fadd_rn(__fmul_rn(x.x, y.y), __fmul_rn(x.y, y.x)));
+}
+__device__ __forceinline__ float2 rotated(float re, float im, cplx r) {
+    const cplx v = cplx{(double)re, (double)im} * r;
+    return make_float2((float)v.re, (float)v.im);
+}
+
+// Weighted means of the traces (XX + YY, which is all that the fit reads) of
+// the rotated residual with the source added back and of the source alone:
+// 64 bins a CTA, each bin's samples split over 4 threads.
+// Bound: the residual's and weights' one pass over memory, then FP64
+// arithmetic (two phasors a sample).  4 timesteps x 192 channels x 8128
+// baselines: 68 us for what took 680 us in seven launches.
+template <bool POINT>
+__global__ void __launch_bounds__(PT) seq_accumulate_kernel(const SeqArgs A, float2* __restrict__ d_lo,
+                                                            float2* __restrict__ m_lo) {
+    constexpr int BINS = 64, SPLIT = PT / BINS;
+    __shared__ double part[SPLIT - 1][5][BINS];
+    const int lane = threadIdx.x % BINS, g = threadIdx.x / BINS;
+    const int nlo = A.nf / A.favg;
+    const size_t bin = (size_t)blockIdx.x * BINS + lane;
+    const bool active = bin < (size_t)nlo * A.nbl;
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // data re, im, model re, im, weight
+    if (active) {
+        const int bl = (int)(bin % A.nbl), flo = (int)(bin / A.nbl);
+        const IonoConsts c = *A.old;
+        UVW to;
+        double dw = 0.0;
+        int tcur = -1;
+        for (int k = g; k < A.nt * A.favg; k += SPLIT) {
+            const int t = k / A.favg, f = flo * A.favg + k - t * A.favg;
+            if (t != tcur) {
+                to = A.to[(size_t)t * A.nbl + bl];
+                dw = to.w - A.from[(size_t)t * A.nbl + bl].w;
+                tcur = t;
+            }
+            const size_t tf = (size_t)t * A.nf + f, i = tf * A.nbl + bl;
+            const float4 ra = __ldg(reinterpret_cast<const float4*>(A.resid + i));
+            const float4 rb = __ldg(reinterpret_cast<const float4*>(A.resid + i) + 1);
+            const double wt = (double)__ldg(A.w + i), lam = __ldg(A.lam + f);
+            float2 mx, my;
+            if (POINT) {
+                const float4 m = __ldg(A.point + tf);
+                mx = make_float2(m.x, 0.f), my = make_float2(m.y, 0.f);
+            } else {
+                const float4 ma = __ldg(reinterpret_cast<const float4*>(A.model + i));
+                const float4 mb = __ldg(reinterpret_cast<const float4*>(A.model + i) + 1);
+                mx = make_float2(ma.x, ma.y), my = make_float2(mb.z, mb.w);
+            }
+            const float2 io = iono_factor(c, to, lam);
+            const cplx rot = phasor_turns(-dw / lam);
+            mx = mul_rn(mx, io), my = mul_rn(my, io);
+            const float2 rx = rotated(ra.x, ra.y, rot), ry = rotated(rb.z, rb.w, rot);
+            v[0] = fma(wt, (double)__fadd_rn(rx.x, mx.x) + (double)__fadd_rn(ry.x, my.x), v[0]);
+            v[1] = fma(wt, (double)__fadd_rn(rx.y, mx.y) + (double)__fadd_rn(ry.y, my.y), v[1]);
+            v[2] = fma(wt, (double)mx.x + (double)my.x, v[2]);
+            v[3] = fma(wt, (double)mx.y + (double)my.y, v[3]);
+            v[4] += wt;
+        }
     }
-    HDC_CUDA_RET_STR(cudaGetLastError());
-    HDC_CUDA_RET_STR(cudaMemcpyAsync(h.data(), st, sizeof(IonoDev) * nsrc, cudaMemcpyDeviceToHost, s));
-    HDC_CUDA_RET_STR(cudaStreamSynchronize(s));
-    for (int i = 0; i < nsrc; i++) consts[i] = IonoConsts{h[i].alpha, h[i].beta, h[i].gain};
-    return NULL;
+    if (g > 0)
+#pragma unroll
+        for (int k = 0; k < 5; k++) part[g - 1][k][lane] = v[k];
+    __syncthreads();
+    if (g > 0 || !active) return;
+#pragma unroll
+    for (int q = 0; q < SPLIT - 1; q++)
+#pragma unroll
+        for (int k = 0; k < 5; k++) v[k] += part[q][k][lane];
+    const double d = v[4] > 0.0 ? v[4] : 1.0;
+    d_lo[bin] = make_float2((float)(v[0] / d), (float)(v[1] / d));
+    m_lo[bin] = make_float2((float)(v[2] / d), (float)(v[3] / d));
+}
+
+// The residual into the source's frame with the source re-subtracted:
+// rotate, + M iono(old) - M iono(new).
+// Bound: FP64 arithmetic (three phasors and three complex products a
+// visibility) and, level with it, the residual's two passes over memory (the
+// same problem: 127 us; rotate and subtract_iono were 119 + 168 us).
+template <bool POINT>
+__global__ void __launch_bounds__(PT) seq_update_kernel(const SeqArgs A) {
+    const VisThread x = vis_thread(A.nbl, A.nf);
+    if (x.bl >= A.nbl) return;
+    const UVW q = A.to[(size_t)x.t * A.nbl + x.bl];
+    const double dw = q.w - A.from[(size_t)x.t * A.nbl + x.bl].w;
+    const IonoConsts old = *A.old, c = *A.neu;
+    const double po = -(q.u * old.alpha + q.v * old.beta), pn = -(q.u * c.alpha + q.v * c.beta);
+#pragma unroll
+    for (int k = 0; k < ROT_F; k++) {
+        const int f = x.f0 + k;
+        if (f >= A.nf) break;
+        const size_t tf = (size_t)x.t * A.nf + f, i = tf * A.nbl + x.bl;
+        const double lam = __ldg(A.lam + f);
+        JonesF32 j = A.resid[i];
+        jf32_mul_f64(j, phasor_turns(-dw / lam));
+        J2 m;
+        if (POINT) {
+            const float4 p = __ldg(A.point + tf);
+            m = J2{{(double)p.x, 0.0}, {(double)p.z, (double)p.w}, {(double)p.z, -(double)p.w}, {(double)p.y, 0.0}};
+        } else {
+            m = load_j32(A.model[i]);
+        }
+        J2 r = load_j32(j);
+        r = r + m * (phasor_turns(po * lam) * old.gain);
+        r = r - m * (phasor_turns(pn * lam) * c.gain);
+        A.resid[i] = JonesF32{(float)r.a.re, (float)r.a.im, (float)r.b.re, (float)r.b.im,
+                              (float)r.c.re, (float)r.c.im, (float)r.d.re, (float)r.d.im};
+    }
+}
+
+cudaError_t seq_accumulate(const SeqArgs& A, float2* d_lo, float2* m_lo, cudaStream_t s) {
+    const unsigned grid = (unsigned)(((size_t)(A.nf / A.favg) * A.nbl + 63) / 64);
+    if (A.model)
+        seq_accumulate_kernel<false><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
+    else
+        seq_accumulate_kernel<true><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t seq_update(const SeqArgs& A, cudaStream_t s) {
+    const unsigned grid = vis_grid(A.nt, A.nf, A.nbl);
+    if (A.model)
+        seq_update_kernel<false><<<grid, PT, 0, s>>>(A);
+    else
+        seq_update_kernel<true><<<grid, PT, 0, s>>>(A);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 // Stream-aware launchers (the drop-in entry points below use stream 0).
@@ -433,36 +600,8 @@ cudaError_t k_xyzs_to_uvws(const XYZ* xyzs, const double* lmsts, UVW* uvws, RADe
 
 cudaError_t k_rotate(JonesF32* vis, int nt, int nbl, int nf, const UVW* from, const UVW* to, const double* lambdas,
                      cudaStream_t s) {
-    const size_t n = (size_t)nt * nf * nbl;
-    if (n == 0) return cudaSuccess;
-    rotate_kernel<<<grid1(n), PT, 0, s>>>(vis, nt, nbl, nf, from, to, lambdas);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t k_average(const JonesF32* hi, const float* w, JonesF32* lo, int nt, int nbl, int nf, int favg,
-                      cudaStream_t s) {
-    const size_t n = (size_t)(nf / favg) * nbl;
-    if (n == 0) return cudaSuccess;
-    average_kernel<<<grid1(n), PT, 0, s>>>(hi, w, lo, nt, nbl, nf, favg);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t k_subtract_iono(JonesF32* resid, const JonesF32* model, IonoConsts c, IonoConsts old, const UVW* uvws,
-                            const double* lambdas, int nt, int nbl, int nf, cudaStream_t s) {
-    const size_t n = (size_t)nt * nf * nbl;
-    if (n == 0) return cudaSuccess;
-    subtract_iono_kernel<<<grid1(n), PT, 0, s>>>(resid, model, c, old, uvws, lambdas, nt, nbl, nf);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t k_add_model(JonesF32* resid, const JonesF32* model, IonoConsts c, const double* lambdas, const UVW* uvws,
-                        int nt, int nf, int nbl, cudaStream_t s) {
-    const size_t n = (size_t)nt * nf * nbl;
-    if (n == 0) return cudaSuccess;
-    add_model_kernel<<<grid1(n), PT, 0, s>>>(resid, model, c, lambdas, uvws, nt, nf, nbl);
+    if ((size_t)nt * nf * nbl == 0) return cudaSuccess;
+    rotate_kernel<<<vis_grid(nt, nf, nbl), PT, 0, s>>>(vis, nt, nbl, nf, from, to, lambdas);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -505,11 +644,7 @@ extern "C" const char* xyzs_to_uvws(const XYZ* d_xyzs, const double* d_lmsts, UV
 
 extern "C" const char* rotate(JonesF32* vis_fb, const int num_timesteps, const int num_baselines, const int num_freqs,
                               const UVW* uvws_from, const UVW* uvws_to, const double* lambdas) {
-    const size_t n = (size_t)num_timesteps * num_freqs * num_baselines;
-    if (n == 0) return NULL;
-    rotate_kernel<<<grid1(n), PT>>>(vis_fb, num_timesteps, num_baselines, num_freqs, uvws_from, uvws_to, lambdas);
-    count_launches(1);
-    HDC_CUDA_RET_STR(cudaGetLastError());
+    HDC_CUDA_RET_STR(k_rotate(vis_fb, num_timesteps, num_baselines, num_freqs, uvws_from, uvws_to, lambdas, 0));
     return NULL;
 }
 

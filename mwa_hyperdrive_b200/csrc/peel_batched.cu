@@ -48,17 +48,9 @@
 #include <tuple>
 #include <vector>
 
-#include "modeller.cuh"
+#include "peel.cuh"
 
 namespace hdc {
-cudaError_t k_xyzs_to_uvws(const XYZ* xyzs, const double* lmsts, UVW* uvws, RADec pc, int ntiles, int nbl, int nt,
-                           cudaStream_t s);
-cudaError_t k_weights_average(const float* w, float* lo, int nt, int nbl, int nf, int favg, cudaStream_t s);
-size_t iono_batched_scratch_bytes(int nsrc, int nbl);
-const char* iono_loop_traces_on(const float2* d_resid, const float* d_w, const float2* d_model, void* d_scratch,
-                                IonoConsts* consts, int nsrc, int nbl, int nf, int niter, const UVW* d_uvws,
-                                const double* d_lambdas, double convergence, cudaStream_t s);
-
 namespace pb {
 
 struct SweepArgs {
@@ -75,7 +67,6 @@ struct SweepArgs {
                             // exp(-2 pi i (alpha u_p + beta v_p) lambda) of the old constants
     float4* app;            // conj(rotation) x the ionospheric phasor of the old and of the new constants
     const IonoConsts* old;  // [nsrc]
-    const IonoConsts* neu;  // [nsrc] (apply sweep)
     float4* gains;          // [nsrc] (apply sweep): old gain, minus the new one, 1 where no constant changed
     float2* d_lo;           // [nsrc][nlo][nbl] traces of D
     float2* m_lo;           // [nsrc][nlo][nbl] traces of Mr
@@ -478,17 +469,6 @@ __global__ void __launch_bounds__(NTH, 2) apply_kernel(const SweepArgs A, bool n
     }
 }
 
-// ptab[(src * nt + t) * nf + f] = W[f][src] as FP32 (xx, yy, Re xy, Im xy; W =
-// B S B^H of the combined point-source modeller at timestep t, Hermitian)
-__global__ void point_table_kernel(const JonesF64* __restrict__ W, int ns, int nf, int nt, int t,
-                                   float4* __restrict__ ptab) {
-    const int src = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
-    if (src >= ns) return;
-    const JonesF64 w = W[(size_t)f * ns + src];
-    ptab[((size_t)src * nt + t) * nf + f] =
-        make_float4((float)w.j00_re, (float)w.j11_re, (float)w.j01_re, (float)w.j01_im);
-}
-
 std::mutex g_tune_mu;
 std::set<std::tuple<int, int, int, int, int>> g_seen;  // shapes (nt, nf, nbl, nsrc, favg) timed
 struct Tuning {
@@ -550,28 +530,6 @@ void apply(const SweepArgs& A, bool next, cudaStream_t s) {
     count_launches(1);
 }
 
-// call-scoped device buffers from the library's stream-ordered pool: freed
-// blocks stay mapped, so later calls reuse them without new mappings
-struct DevBuf {
-    void* p = nullptr;
-    cudaStream_t s = nullptr;
-    bool pooled = false;
-    cudaError_t alloc(size_t bytes, cudaStream_t st) {
-        s = st;
-        pooled = true;
-        return pool_malloc_async(&p, bytes, st);
-    }
-    // large one-off buffers stay outside the pool, which keeps what it holds
-    cudaError_t alloc_plain(size_t bytes) { return cudaMalloc(&p, bytes); }
-    ~DevBuf() {
-        if (p) pooled ? cudaFreeAsync(p, s) : cudaFree(p);
-    }
-    template <class T>
-    T* as() {
-        return reinterpret_cast<T*>(p);
-    }
-};
-
 }  // namespace pb
 }  // namespace hdc
 
@@ -626,12 +584,7 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     // the models need ns x nvis JonesF32 of device memory
     // (with a beam shared by all tiles, or none: per-tile beams make a
     // point's model depend on the baseline)
-    bool points = params->beam_kind == HDC_BEAM_NONE || params->beam_kind == HDC_BEAM_ANALYTIC_DIPOLE;
-    for (int i = 0; i < ns && points; i++) {
-        const HdcSkyModel& m = h_sources[i];
-        points = m.num_components == 1 && m.comp_type[0] == 0 && std::fabs(m.ra[0] - h_source_positions[i].ra) < 1e-12 &&
-                 std::fabs(m.dec[0] - h_source_positions[i].dec) < 1e-12;
-    }
+    const bool points = peel_point_sources(h_sources, h_source_positions, ns, params->beam_kind);
     size_t free_b = 0, total_b = 0;
     PB_CK(cudaMemGetInfo(&free_b, &total_b));
     const size_t need = points ? sizeof(float4) * (size_t)ns * nt * nf : sizeof(JonesF32) * nvis * (size_t)ns;
@@ -640,9 +593,9 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
                   need >> 20, free_b >> 20);
         return HDC_ERR_ALLOC;
     }
-    pb::DevBuf b_tuvw, b_radec, b_acc, b_app, b_wtr;
-    pb::DevBuf b_lam, b_lam_lo, b_lmst, b_avg_lmst, b_xyz, b_uv_src, b_uv_lo, b_models, b_dlo, b_mlo, b_wlo, b_scr,
-        b_old, b_new, b_gains;
+    DevBuf b_tuvw, b_radec, b_acc, b_app, b_wtr;
+    DevBuf b_lam, b_lam_lo, b_lmst, b_avg_lmst, b_xyz, b_uv_src, b_uv_lo, b_models, b_dlo, b_mlo, b_wlo, b_part,
+        b_st, b_consts, b_gains;
     PB_CK(b_lam.alloc(sizeof(double) * 2 * nf, s));  // lambda, then 1 / lambda
     PB_CK(b_lam_lo.alloc(sizeof(double) * nlo, s));
     PB_CK(b_lmst.alloc(sizeof(double) * nt, s));
@@ -662,9 +615,9 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     PB_CK(b_dlo.alloc(sizeof(float2) * (size_t)batch * nlo * nbl, s));
     PB_CK(b_mlo.alloc(sizeof(float2) * (size_t)batch * nlo * nbl, s));
     PB_CK(b_wlo.alloc(sizeof(float) * (size_t)nlo * nbl, s));
-    PB_CK(b_scr.alloc(iono_batched_scratch_bytes(batch, nbl), s));
-    PB_CK(b_old.alloc(sizeof(IonoConsts) * ns, s));
-    PB_CK(b_new.alloc(sizeof(IonoConsts) * ns, s));
+    PB_CK(b_part.alloc(iono_partials_bytes(batch, nbl), s));
+    PB_CK(b_st.alloc(sizeof(IonoDev) * batch, s));
+    PB_CK(b_consts.alloc(sizeof(IonoConsts) * 2 * ns, s));  // a pass's old and new constants, then the other way round
     PB_CK(b_gains.alloc(sizeof(float4) * batch, s));
     PB_CK(cudaMemcpyAsync(b_lam.p, lam.data(), sizeof(double) * 2 * nf, cudaMemcpyHostToDevice, s));
     PB_CK(cudaMemcpyAsync(b_lam_lo.p, lam_lo.data(), sizeof(double) * nlo, cudaMemcpyHostToDevice, s));
@@ -679,20 +632,20 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     for (int i = 0; i < ns; i++) radec[i] = make_double2(h_source_positions[i].ra, h_source_positions[i].dec);
     radec[ns] = make_double2(phase_centre.ra, phase_centre.dec);
     PB_CK(cudaMemcpyAsync(b_radec.p, radec.data(), sizeof(double2) * (ns + 1), cudaMemcpyHostToDevice, s));
-    PB_CK(cudaMemcpyAsync(b_old.p, h_iono_consts, sizeof(IonoConsts) * ns, cudaMemcpyHostToDevice, s));
+    PB_CK(cudaMemcpyAsync(b_consts.p, h_iono_consts, sizeof(IonoConsts) * ns, cudaMemcpyHostToDevice, s));
+    PB_CK(iono_states_init(b_st.as<IonoDev>(), batch, s));
     {
         const int n = (ns + 1) * nt * num_tiles;
         pb::tile_uvw_kernel<<<(n + 255) / 256, 256, 0, s>>>(b_xyz.as<XYZ>(), b_lmst.as<double>(),
                                                             b_radec.as<double2>(), ns + 1, nt, num_tiles,
                                                             b_tuvw.as<UVW>());
         pb::acc_table_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, s>>>(
-            b_tuvw.as<UVW>(), b_lam.as<double>(), b_old.as<IonoConsts>(), ns, nt, nf, num_tiles, b_acc.as<float4>());
+            b_tuvw.as<UVW>(), b_lam.as<double>(), b_consts.as<IonoConsts>(), ns, nt, nf, num_tiles, b_acc.as<float4>());
         pb::trace_kernel<<<(unsigned)((nvis + 255) / 256), 256, 0, s>>>(d_resid_tfb, d_weights_tfb, nvis,
                                                                        b_wtr.as<float2>());
         count_launches(3);
         PB_CK(cudaGetLastError());
     }
-    PB_CK(cudaMemsetAsync(b_models.p, 0, need, s));
     // per source: UVWs in its frame and its high-resolution model (once per
     // timeblock)
     for (int i = 0; i < ns; i++) {
@@ -703,40 +656,11 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
                              h_source_positions[i], num_tiles, nbl, 1, s));
     }
     if (points) {
-        // A single point at its own position has, on every baseline, the model
-        // B S B^H (phase 1).  One modeller over all the sources' components
-        // (two tiles: the weights do not depend on the baselines or the phase
-        // centre) gives B S B^H per (channel, source) after each timestep's
-        // geometry; the table kernel stores it as [source][timestep][channel].
-        std::vector<int> ctype(ns, HDC_POINT), ftype(ns), fstart(ns), fcount(ns), zero(ns, 0);
-        std::vector<double> ra(ns), dec(ns), nil(ns, 0.0), si(ns), q(ns), fds;
-        for (int i = 0; i < ns; i++) {
-            const HdcSkyModel& m = h_sources[i];
-            ra[i] = m.ra[0], dec[i] = m.dec[0], ftype[i] = m.flux_type[0], si[i] = m.si[0], q[i] = m.q[0];
-            fstart[i] = (int)(fds.size() / 5);
-            fcount[i] = m.fd_count[0];
-            fds.insert(fds.end(), m.fds + 5 * (size_t)m.fd_start[0], m.fds + 5 * (size_t)(m.fd_start[0] + m.fd_count[0]));
-        }
-        const HdcSkyModel all = {ns,          ctype.data(), ra.data(),     dec.data(),   nil.data(), nil.data(),
-                                 nil.data(),  ftype.data(), si.data(),     q.data(),     fstart.data(), fcount.data(),
-                                 fds.data(),  zero.data(),  zero.data(),   zero.data(),  zero.data(), nil.data()};
-        HdcModeller* hm = nullptr;
-        int rc = hdc_modeller_new(&all, 0, h_tile_xyzs, 2, h_freqs, num_freqs, phase_centre,
-                                  params->array_latitude_rad, params->beam_kind, HDC_PREDICT_DIRECT, &hm);
+        const int rc = peel_point_table(h_sources, ns, h_freqs, nf, h_lmsts, nt, params->array_latitude_rad,
+                                        params->beam_kind, b_models.as<float4>(), s);
         if (rc) return rc;
-        std::unique_ptr<Modeller> m(reinterpret_cast<Modeller*>(hm));
-        for (int t = 0; t < nt; t++) {
-            rc = m->geometry(h_lmsts[t], s);
-            if (rc) return rc;
-            pb::point_table_kernel<<<dim3((ns + 127) / 128, nf), 128, 0, s>>>(m->weights(0), ns, nf, nt, t,
-                                                                              b_models.as<float4>());
-            count_launches(1);
-            PB_CK(cudaGetLastError());
-        }
-        // the modeller's tables are freed when it goes out of scope: let the
-        // table kernels finish reading them first
-        PB_CK(cudaStreamSynchronize(s));
     } else {
+        PB_CK(cudaMemsetAsync(b_models.p, 0, need, s));
         for (int i = 0; i < ns; i++) {
             HdcModeller* hm = nullptr;
             int rc = peel_modeller_new(&h_sources[i], h_tile_xyzs, num_tiles, h_freqs, num_freqs,
@@ -760,8 +684,6 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     A.ptab = points ? b_models.as<float4>() : nullptr;
     A.acc = b_acc.as<float4>();
     A.app = b_app.as<float4>();
-    A.old = b_old.as<IonoConsts>();
-    A.neu = b_new.as<IonoConsts>();
     A.gains = b_gains.as<float4>();
     A.d_lo = b_dlo.as<float2>();
     A.m_lo = b_mlo.as<float2>();
@@ -771,11 +693,13 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     A.ntiles = num_tiles;
     A.nsrc = ns;
     A.favg = favg;
-    std::vector<IonoConsts> fit(ns), next(ns);
     // sources in sub-batches of `batch` in list order: within a sub-batch the
     // fits share the residual (Jacobi); each sub-batch sees the residual the
     // earlier ones left (the reference's Gauss-Seidel order between them)
+    const IonoConsts* result = b_consts.as<IonoConsts>();
     for (int pass = 0; pass < params->num_passes; pass++) {
+        const IonoConsts* old = b_consts.as<IonoConsts>() + (pass & 1) * ns;
+        IonoConsts* neu = b_consts.as<IonoConsts>() + ((pass + 1) & 1) * ns;
         for (int b0 = 0; b0 < ns; b0 += batch) {
             const int nb = std::min(batch, ns - b0);
             const size_t ntab_b = (size_t)nb * nt * nf * num_tiles;
@@ -784,40 +708,23 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
             B.models = A.models ? A.models + (size_t)b0 * nvis : nullptr;
             B.ptab = A.ptab ? A.ptab + (size_t)b0 * nt * nf : nullptr;
             B.acc = A.acc + (size_t)b0 * nt * nf * num_tiles;
-            B.old = A.old + b0;
-            B.neu = A.neu + b0;
-            PB_CK(cudaMemcpyAsync(b_old.as<IonoConsts>() + b0, h_iono_consts + b0, sizeof(IonoConsts) * nb,
-                                  cudaMemcpyHostToDevice, s));
+            B.old = old + b0;
             PB_CK(pb::accumulate(B, s));
-            for (int i = 0; i < nb; i++) fit[i] = IonoConsts{0.0, 0.0, 1.0};
-            const char* err = iono_loop_traces_on(B.d_lo, b_wlo.as<float>(), B.m_lo, b_scr.p, fit.data(), nb, nbl, nlo,
-                                                  params->num_loops, b_uv_lo.as<UVW>() + (size_t)b0 * nbl,
-                                                  b_lam_lo.as<double>(), params->convergence, s);
-            if (err) {
-                set_error("hdc_peel_timeblock_batched: %s", err);
-                return HDC_ERR_CUDA;
-            }
-            for (int i = 0; i < nb; i++) {
-                const IonoConsts old = h_iono_consts[b0 + i];
-                IonoConsts c = {old.alpha + fit[i].alpha, old.beta + fit[i].beta, old.gain * fit[i].gain};
-                // the reference's revert rule (gpu.rs:541-627)
-                if (std::fabs(c.alpha) > 1e-3 || std::fabs(c.beta) > 1e-3 || c.gain < 0.0 || c.gain > 1.5) c = old;
-                next[b0 + i] = c;
-            }
-            PB_CK(cudaMemcpyAsync(b_new.as<IonoConsts>() + b0, next.data() + b0, sizeof(IonoConsts) * nb,
-                                  cudaMemcpyHostToDevice, s));
+            PB_CK(iono_fit(B.d_lo, b_wlo.as<float>(), B.m_lo, b_part.as<double>(), b_st.as<IonoDev>(), old + b0,
+                           neu + b0, nb, nbl, nlo, params->num_loops, b_uv_lo.as<UVW>() + (size_t)b0 * nbl,
+                           b_lam_lo.as<double>(), params->convergence, s));
             // app from tuvw rows of this sub-batch's sources
             pb::app_table_kernel<<<(unsigned)((ntab_b + 255) / 256), 256, 0, s>>>(
-                b_tuvw.as<UVW>() + (size_t)b0 * nt * num_tiles, b_lam.as<double>(), B.old, B.neu, nb, nt, nf,
+                b_tuvw.as<UVW>() + (size_t)b0 * nt * num_tiles, b_lam.as<double>(), old + b0, neu + b0, nb, nt, nf,
                 num_tiles, B.acc, B.app, B.gains);
             count_launches(1);
             PB_CK(cudaGetLastError());
             pb::apply(B, pass + 1 < params->num_passes || b0 + batch < ns, s);
             PB_CK(cudaGetLastError());
-            PB_CK(cudaStreamSynchronize(s));  // `next` is read by the copy above
-            for (int i = 0; i < nb; i++) h_iono_consts[b0 + i] = next[b0 + i];
         }
+        result = neu;
     }
+    PB_CK(cudaMemcpyAsync(h_iono_consts, result, sizeof(IonoConsts) * ns, cudaMemcpyDeviceToHost, s));
     PB_CK(cudaStreamSynchronize(s));
     return HDC_OK;
 }

@@ -104,3 +104,45 @@ def test_pass(ntiles, nsrc, nt, favg):
         r = d.cpu().numpy().astype(np.float64)
         r = r[..., 0::2] + 1j * r[..., 1::2]
         assert np.max(np.abs(r - want_r)) < 1e-6 * 6.0 * nsrc
+
+
+@pytest.mark.parametrize("halves", [1, 2])
+@pytest.mark.parametrize("ntiles,nsrc,nt,favg", [(12, 1, 1, 3), (33, 3, 2, 5)])
+def test_source_by_source(ntiles, nsrc, nt, favg, halves):
+    """The source-by-source loop (FP64 steps, the reference's roundings) on the
+    point table and on materialised models: one source is one pass in float64;
+    several agree with batched sub-batches of one."""
+    rng = np.random.default_rng(ntiles)
+    xyzs = synth.tiles_in_disk(ntiles, 750.0, ntiles)
+    freqs = 170e6 + np.arange(2 * favg) * 640e3
+    lsts = 0.12 + np.arange(nt) * 6e-4
+    nbl = ntiles * (ntiles - 1) // 2
+    i_ref = rng.uniform(2.0, 6.0, nsrc)
+    pos = [(PC[0] + math.radians(rng.uniform(-3, 3)), PC[1] + math.radians(rng.uniform(-3, 3))) for _ in range(nsrc)]
+    resid = rng.normal(0.0, 0.3, (nt, freqs.size, nbl, 8)).astype(np.float32)
+    weights = rng.uniform(0.1, 8.0, (nt, freqs.size, nbl)).astype(np.float32)
+    skies = [sl.SkyModelArrays.from_components(
+        [sl.SourceComponent(*pos[k], sl.Point(), sl.PowerLaw(-0.8, sl.FluxDensity(150e6, i_ref[k] / halves)))
+         for _ in range(halves)]) for k in range(nsrc)]
+    out = {}
+    for batched in (False, True):
+        d = torch.from_numpy(resid.copy()).cuda()
+        got = P.peel_timeblock(d, torch.from_numpy(weights).cuda(), freqs, xyzs, lsts, float(lsts.mean()), PC, skies,
+                               pos, [P.IonoConsts()] * nsrc, 2, 6, 1.0, favg, synth.MWA_LAT_RAD, batched=batched,
+                               batch_size=1)
+        out[batched] = np.array([[c.alpha, c.beta, c.gain] for c in got]), d.cpu().numpy()
+    a, b = out[False], out[True]
+    assert np.max(np.abs(a[0][:, :2] - b[0][:, :2])) < 1e-5 * np.max(np.abs(a[0][:, :2])) + 1e-11
+    assert np.max(np.abs(a[0][:, 2] - b[0][:, 2])) < 1e-5
+    assert np.max(np.abs(a[1] - b[1])) < 2e-6 * 6.0 * nsrc
+    if nsrc == 1:
+        d = torch.from_numpy(resid.copy()).cuda()
+        got = P.peel_timeblock(d, torch.from_numpy(weights).cuda(), freqs, xyzs, lsts, float(lsts.mean()), PC, skies,
+                               pos, [P.IonoConsts()], 1, 6, 1.0, favg, synth.MWA_LAT_RAD)
+        want, want_r = one_pass(resid, weights, freqs, xyzs, lsts, float(lsts.mean()),
+                                [(*pos[0], i_ref[0] * (freqs / 150e6) ** -0.8)], favg, 6)
+        assert abs(got[0].alpha - want[0, 0]) < 1e-6 * np.max(np.abs(want[0, :2]))
+        assert abs(got[0].gain - want[0, 2]) < 1e-6
+        r = d.cpu().numpy().astype(np.float64)
+        r = r[..., 0::2] + 1j * r[..., 1::2]
+        assert np.max(np.abs(r - want_r)) < 1e-6 * 6.0
