@@ -112,7 +112,15 @@ __device__ __forceinline__ cplx shapelet_env(const double* __restrict__ cm, doub
     return e;
 }
 
-template <int TYPE, bool TILE, bool OUT64>
+// FAST (Gaussians): the envelope's exponential in FP32 of the FP64 base-2
+// exponent (gp holds DirectParams::gk), as the chosen form takes it: rounding
+// the exponent moves the envelope by ln2 |x| 6e-8 2^-|x| <= 2.2e-8 of the
+// component's flux.  Only the chosen form with per-tile beams comes here, all
+// else in FP64 (error's p99.9 3.4e-7 with FP32 phasors and left operands,
+// 2.6e-7 so).  128 tiles x 192 channels x 250 Gaussians, 17 unique tiles: 2.37
+// ms with a thread per baseline (phasors and records of 17 tiles gathered from
+// shared memory per term), 1.95 so, the FP64 pipe 0.61 busy.
+template <int TYPE, bool TILE, bool OUT64, bool FAST>
 __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
     constexpr int CH = Shape<TYPE, TILE>::CH;
     __shared__ alignas(128) double4 s_lmn[2][CH];
@@ -225,7 +233,8 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
                     const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
                     double2 x;
                     if (TYPE == 1) {
-                        x = make_double2(u * g.z + v * g.w, u * g.w - v * g.z);
+                        x = FAST ? make_double2(u * g.x + v * g.y, u * g.z + v * g.w)
+                                 : make_double2(u * g.z + v * g.w, u * g.w - v * g.z);
                     } else {
                         double2 q = make_double2(0.0, 0.0);
                         if (tile < p.ntiles) q = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + tile);
@@ -264,7 +273,9 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
                         if (TYPE) {
                             const double2 kp = s_k[TYPE ? c : 0][TYPE ? rp : 0], kq = s_k[TYPE ? c : 0][TYPE ? cq : 0];
                             const double dx = kp.x - kq.x, dy = kp.y - kq.y;
-                            if (TYPE == 1) {
+                            if (TYPE == 1 && FAST) {
+                                env.re = (double)exp2_neg((float)fma(dx, dx, dy * dy));
+                            } else if (TYPE == 1) {
                                 const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
                                 env.re = exp(g.x * (dx * dx) + g.y * (dy * dy));
                             } else {
@@ -340,14 +351,14 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
         }
 }
 
-template <int TYPE, bool TILE>
+template <int TYPE, bool TILE, bool FAST = false>
 cudaError_t launch_t(bool out64, const DirectParams& p, cudaStream_t s) {
     const int nblk = (p.ntiles + TB - 1) / TB;
     const dim3 grid(nblk * (nblk + 1) / 2, p.nf);
     if (out64)
-        pair_kernel<TYPE, TILE, true><<<grid, NTH, 0, s>>>(p);
+        pair_kernel<TYPE, TILE, true, FAST><<<grid, NTH, 0, s>>>(p);
     else
-        pair_kernel<TYPE, TILE, false><<<grid, NTH, 0, s>>>(p);
+        pair_kernel<TYPE, TILE, false, FAST><<<grid, NTH, 0, s>>>(p);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -602,7 +613,12 @@ cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
 
 }  // namespace pairs
 
-cudaError_t launch_fast_gauss(bool out64, const DirectParams& p, cudaStream_t s) {
+cudaError_t launch_fast_gauss(bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s) {
+    if (tile_beam) {
+        DirectParams q = p;
+        q.gp = p.gk;
+        return pairs::launch_t<1, true, true>(out64, q, s);
+    }
     return out64 ? pairs::launch_fast_gauss<true>(p, s) : pairs::launch_fast_gauss<false>(p, s);
 }
 

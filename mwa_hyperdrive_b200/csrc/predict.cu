@@ -344,61 +344,38 @@ __global__ void __launch_bounds__(DT) direct_kernel(const DirectParams p) {
     }
 }
 
-// Shapelet component c's UV [m] of a tile (zero for other types).
-template <int TYPE>
+// Shapelet component c's UV [m] of a tile.
 __device__ __forceinline__ double2 shape_uv(const DirectParams& p, int c, int tile) {
-    return TYPE == 2 ? __ldg(p.suv_tile + (size_t)c * p.ntiles + tile) : make_double2(0.0, 0.0);
+    return __ldg(p.suv_tile + (size_t)c * p.ntiles + tile);
 }
 
-// The channel-independent FP64 work of one Gaussian or shapelet term of the
-// chosen form at baseline (um, vm, wm) [m] (its tiles' shapelet UVs ta, tb):
-// the phase in metres, the Gaussian exponent in metres^2 (base 2), or the shapelet
-// coordinates (in metres; dense: in table steps per wavelength^-1).
-template <int TYPE>
+// The channel-independent FP64 work of one shapelet term of the chosen form
+// at baseline (um, vm, wm) [m] (its tiles' shapelet UVs ta, tb): the phase in
+// metres and the shapelet coordinates (in metres; dense: in table steps per
+// wavelength^-1).
 struct FastTerm {
-    double tm, exm, su, sv;
+    double tm, su, sv;
 };
 
-template <int TYPE>
 __device__ __forceinline__ void fast_term(double4 lmn, double4 g, double um, double vm, double wm, double2 ta, double2 tb,
-                                          bool dense, FastTerm<TYPE>& f) {
+                                          bool dense, FastTerm& f) {
     f.tm = um * lmn.x + vm * lmn.y + wm * lmn.z;
-    f.exm = f.su = f.sv = 0.0;
-    if (TYPE == 1) {
-        // the exponent in FP64 (an FP32 exponent's absolute error, ~1e-7 of
-        // its size, would become the envelope's relative error), in base 2
-        // (exp(x) = 2^(x log2 e)): the per-channel exp2f costs fewer
-        // instructions than expf (measured)
-        const double kx = um * g.z + vm * g.w;
-        const double ky = um * g.w - vm * g.z;
-        f.exm = (g.x * (kx * kx) + g.y * (ky * ky)) * 1.4426950408889634074;
-    } else {
-        f.su = ta.x - tb.x;
-        f.sv = ta.y - tb.y;
-        if (dense) {
-            const double x = (f.su * g.z + f.sv * g.w) * g.x, y = (f.su * g.w - f.sv * g.z) * g.y;
-            f.su = x;
-            f.sv = y;
-        }
+    f.su = ta.x - tb.x;
+    f.sv = ta.y - tb.y;
+    if (dense) {
+        const double x = (f.su * g.z + f.sv * g.w) * g.x, y = (f.su * g.w - f.sv * g.z) * g.y;
+        f.su = x;
+        f.sv = y;
     }
 }
 
-// The envelopes of a FastTerm's N channels (ool = frequency / c): a
-// Gaussian's is real; dense shapelets with coefficients cm and win (WIN) the
-// staged records.
-template <int TYPE, int N, bool WIN>
-__device__ __forceinline__ void fast_envelopes(const DirectParams& p, const FastTerm<TYPE>& f, const double (&ool)[N],
+// The envelopes of a FastTerm's N channels (ool = frequency / c); dense: the
+// coefficients cm and (WIN) the staged records win.
+template <int N, bool WIN>
+__device__ __forceinline__ void fast_envelopes(const DirectParams& p, const FastTerm& f, const double (&ool)[N],
                                                int cglob, double4 g, bool dense, const float* cm, const float4* win,
                                                float (&er)[N], float (&ei)[N]) {
-    if (TYPE == 1) {
-        // exponent in FP64, exp2 in FP32: rounding the exponent to FP32 moves
-        // the envelope by ln2 |x| 6e-8 2^-|x| <= 2.2e-8 of the component's flux
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            er[i] = exp2f((float)(f.exm * (ool[i] * ool[i])));
-            ei[i] = 0.f;
-        }
-    } else if (dense) {
+    if (dense) {
         shapelet_dense<N, WIN>(p, win, cm, f.su, f.sv, ool, er, ei);
     } else {
 #pragma unroll
@@ -407,12 +384,11 @@ __device__ __forceinline__ void fast_envelopes(const DirectParams& p, const Fast
 }
 
 // z = envelope x phasor of one channel.
-template <int TYPE>
-__device__ __forceinline__ void fast_z(const FastTerm<TYPE>& f, double ool, float er, float ei, float& zr, float& zi) {
+__device__ __forceinline__ void fast_z(const FastTerm& f, double ool, float er, float ei, float& zr, float& zi) {
     float sn, cs;
     phasor_quarter_f32(4.0 * ool * f.tm, sn, cs);
-    zr = TYPE == 1 ? cs * er : cs * er - sn * ei;
-    zi = TYPE == 1 ? sn * er : fmaf(cs, ei, sn * er);
+    zr = cs * er - sn * ei;
+    zi = fmaf(cs, ei, sn * er);
 }
 
 // The chosen form's shapelets with a beam shared by all tiles (or none): a
@@ -529,15 +505,15 @@ __global__ void __launch_bounds__(SNT, 2) fast_shapelet_kernel(const DirectParam
         if (active) {
             for (int c = 0; c < n; c++) {
                 const double4 g = S.gp[st][c];
-                FastTerm<2> term;
-                fast_term<2>(S.lmn[st][c], g, um, vm, wm, shape_uv<2>(p, c0 + c, t1), shape_uv<2>(p, c0 + c, t2), DENSE,
+                FastTerm term;
+                fast_term(S.lmn[st][c], g, um, vm, wm, shape_uv(p, c0 + c, t1), shape_uv(p, c0 + c, t2), DENSE,
                              term);
                 float er[SFCH], ei[SFCH];
-                fast_envelopes<2, SFCH, DENSE>(p, term, ool, c0 + c, g, DENSE, S.dense + c * SDN * SDN, S.win, er, ei);
+                fast_envelopes<SFCH, DENSE>(p, term, ool, c0 + c, g, DENSE, S.dense + c * SDN * SDN, S.win, er, ei);
 #pragma unroll
                 for (int i = 0; i < SFCH; i++) {
                     float zr, zi;
-                    fast_z<2>(term, ool[i], er[i], ei[i], zr, zi);
+                    fast_z(term, ool[i], er[i], ei[i], zr, zi);
                     const uint64_t z = pack2(zr, zi);
                     const float4 wv = S.w[i][c];
                     acc[i][0] = fma2(dup2(wv.x), z, acc[i][0]);
@@ -599,52 +575,40 @@ static cudaError_t launch_fast_shapelet(const DirectParams& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// The chosen form's Gaussians and shapelets with a beam per tile: each
-// thread takes one baseline (p, q) and FastTileShape::FCH consecutive channels, as
-// fast_kernel does.  Per staged chunk of components the CTA forms in shared
-// memory G = B_u S (FP32) and H = B_u (FP64) for every unique tile u and each
-// of its channels (B the tile's beam Jones at the channel's beam frequency,
-// S the component's instrumental flux), laid out [channel][component][unique
-// tile] so that a warp's threads, which share tile p and mostly share the
-// unique beam of tile q, read the same or neighbouring records.  A
-// visibility term is then z G_p H_q^H = B_p (z S) B_q^H: the phasor and
-// envelope z in FP32 exactly as fast_kernel computes them, z G_p in FP32,
-// and its product with H_q^H accumulated in FP64 (32 fused multiply-adds).
-// Measured on the tests' skies (p99.9 of the error, Gaussians / shapelets):
-// this form 3.4e-7 / 5.3e-7; FP32 two-product sums added into FP64
-// accumulators 4.2e-7 / 5.9e-7 (7 % faster Gaussians); everything in FP32,
+// The chosen form's shapelets with a beam per tile: each thread takes one
+// baseline (p, q) and FT_FCH consecutive channels, as fast_shapelet_kernel
+// does.  Per staged chunk of components the CTA forms in shared memory
+// G = B_u S (FP32) and H = B_u (FP64) for every unique tile u and each of its
+// channels (B the tile's beam Jones at the channel's beam frequency, S the
+// component's instrumental flux), laid out [channel][component][unique tile]
+// so that a warp's threads, which share tile p and mostly share the unique
+// beam of tile q, read the same or neighbouring records.  A visibility term
+// is then z G_p H_q^H = B_p (z S) B_q^H: the phasor and envelope z in FP32
+// exactly as fast_shapelet_kernel computes them, z G_p in FP32, and its
+// product with H_q^H accumulated in FP64 (32 fused multiply-adds).
+// Measured on the tests' skies (p99.9 of the error): this form 5.3e-7; FP32
+// two-product sums added into FP64 accumulators 5.9e-7; everything in FP32,
 // chunk sums included, 1.0-1.15e-6, over the 1e-6 bar.
-// Channels per thread and components per staged chunk by type, chosen by
-// timing on 17 unique tiles (one timestep, 128 tiles, 384 channels):
-// Gaussians (1) 2 x 16 (4 x 8: 9.4 -> 10.8 ms, 156 registers); shapelets (2)
-// 4 x 8, whose channels then share more gathered basis records (2 x 16: 5.4
-// ms, 4 x 8: 4.6 ms, bit-identical).  Both stage 32 (channel, component)
-// records per unique tile, so the shared memory does not depend on the type.
-template <int TYPE>
-struct FastTileShape {
-    static constexpr int FCH = 2;
-    static constexpr int CH = 16;
-};
-template <>
-struct FastTileShape<2> {
-    static constexpr int FCH = 4;
-    static constexpr int CH = 8;
-};
-constexpr int FT_RECS = 32;    // FCH x CH of every type
+// Four channels share the gathered basis records: 2 channels x 16 components
+// a chunk 5.4 ms, 4 x 8 4.6 ms, bit-identical (17 unique tiles, one timestep,
+// 128 tiles, 384 channels).  The tile-factored FP64 form (pairs.cu), which
+// evaluates the basis per pair and channel, takes 1.80 ms where this one takes
+// 1.07 (50 shapelets, 128 tiles, 192 channels).
+constexpr int FT_FCH = 4;      // channels per thread
+constexpr int FT_CH = 8;       // components per staged chunk
+constexpr int FT_RECS = FT_FCH * FT_CH;
 constexpr int FT_MAX_NU = 32;  // unique tiles (more: the FP64 per-tile kernel)
-static_assert(FastTileShape<1>::FCH * FastTileShape<1>::CH == FT_RECS, "per-tile records");
-static_assert(FastTileShape<2>::FCH * FastTileShape<2>::CH == FT_RECS, "per-tile records");
 
 inline size_t fast_tile_smem_bytes(int nu) { return (size_t)FT_RECS * nu * 6 * sizeof(float4); }
 
-template <int TYPE, bool OUT64>
+template <bool OUT64>
 __global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) {
-    constexpr int FCH = FastTileShape<TYPE>::FCH;
-    constexpr int CH = FastTileShape<TYPE>::CH;
+    constexpr int FCH = FT_FCH;
+    constexpr int CH = FT_CH;
     __shared__ alignas(128) double4 s_lmn[2][CH];
     __shared__ alignas(128) JonesF64 s_flux[2][FCH][CH];
     __shared__ alignas(128) double4 s_gp[2][CH];
-    __shared__ alignas(16) float s_dense[TYPE == 2 ? CH * SDN * SDN : 1];
+    __shared__ alignas(16) float s_dense[CH * SDN * SDN];
     __shared__ alignas(8) uint64_t bar[2];
     // [FCH][CH][nu] records of 96 bytes: G (2 float4: a, b | c, d), then H
     // (4 double2: a, b, c, d)
@@ -729,23 +693,21 @@ __global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) 
             r[2] = make_double2(b.c.re, b.c.im);
             r[3] = make_double2(b.d.re, b.d.im);
         }
-        if (TYPE == 2 && p.sdense)
+        if (p.sdense)
             for (int e = threadIdx.x; e < n * SDN * SDN; e += DT) s_dense[e] = __ldg(p.sdense + (size_t)c0 * SDN * SDN + e);
         __syncthreads();
         if (active) {
             for (int c = 0; c < n; c++) {
                 const double4 g = s_gp[st][c];
-                const bool dense = TYPE == 2 && p.sdense;
-                FastTerm<TYPE> term;
-                fast_term<TYPE>(s_lmn[st][c], g, um, vm, wm, shape_uv<TYPE>(p, c0 + c, t1), shape_uv<TYPE>(p, c0 + c, t2),
-                                dense, term);
+                const bool dense = p.sdense;
+                FastTerm term;
+                fast_term(s_lmn[st][c], g, um, vm, wm, shape_uv(p, c0 + c, t1), shape_uv(p, c0 + c, t2), dense, term);
                 float er[FCH], ei[FCH];
-                fast_envelopes<TYPE, FCH, false>(p, term, ool, c0 + c, g, dense, s_dense + (TYPE == 2 ? c * SDN * SDN : 0),
-                                                 nullptr, er, ei);
+                fast_envelopes<FCH, false>(p, term, ool, c0 + c, g, dense, s_dense + c * SDN * SDN, nullptr, er, ei);
 #pragma unroll
                 for (int i = 0; i < FCH; i++) {
                     float zr, zi;
-                    fast_z<TYPE>(term, ool[i], er[i], ei[i], zr, zi);
+                    fast_z(term, ool[i], er[i], ei[i], zr, zi);
                     const float4* rg = s_gh + ((size_t)(i * CH + c) * nu + u1) * 6;
                     const double2* rh = reinterpret_cast<const double2*>(s_gh + ((size_t)(i * CH + c) * nu + u2) * 6 + 2);
                     const float4 g0 = rg[0], g1 = rg[1];
@@ -782,7 +744,7 @@ __global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) 
     }
 }
 
-template <int TYPE, bool OUT64>
+template <bool OUT64>
 static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
     const size_t smem = fast_tile_smem_bytes(p.n_uniq_tile);
     // the opt-in above 48 KB of dynamic shared memory, once per device
@@ -792,22 +754,21 @@ static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr[dev].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(fast_tile_kernel<TYPE, OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(fast_tile_kernel<OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)fast_tile_smem_bytes(FT_MAX_NU));
         if (e != cudaSuccess) return e;
         attr[dev].store(true, std::memory_order_relaxed);
     }
-    const dim3 grid((p.nbl + DT - 1) / DT, (p.nf + FastTileShape<TYPE>::FCH - 1) / FastTileShape<TYPE>::FCH);
-    fast_tile_kernel<TYPE, OUT64><<<grid, DT, smem, s>>>(p);
+    const dim3 grid((p.nbl + DT - 1) / DT, (p.nf + FT_FCH - 1) / FT_FCH);
+    fast_tile_kernel<OUT64><<<grid, DT, smem, s>>>(p);
     return cudaSuccess;
 }
 
 template <int TYPE>
 static cudaError_t launch_t(bool tile_beam, bool out64, bool fast, const DirectParams& p, cudaStream_t s) {
     dim3 grid((p.nbl + DT - 1) / DT, p.nf);
-    if (tile_beam && fast && TYPE != 0) {
-        const cudaError_t e = out64 ? launch_fast_tile<TYPE == 0 ? 1 : TYPE, true>(p, s)
-                                    : launch_fast_tile<TYPE == 0 ? 1 : TYPE, false>(p, s);
+    if (tile_beam && fast && TYPE == 2) {
+        const cudaError_t e = out64 ? launch_fast_tile<true>(p, s) : launch_fast_tile<false>(p, s);
         if (e != cudaSuccess) return e;
     } else if (tile_beam) {
         if (out64)
@@ -858,8 +819,9 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
         }
     }
     // the FP32 form needs per-tile shapelet UVs and the FP32 basis table, and
-    // with per-tile beams a unique-tile count it can stage (not the points,
-    // whose chosen form is the tensor kernel)
+    // with per-tile beams a unique-tile count its shapelets can stage, past
+    // which the Gaussians stay in FP64 with them (not the points, whose chosen
+    // form is the tensor kernel)
     fast = fast && p.xyzs && (ty != 2 || (p.suv_tile && !p.suv_bl && p.sbf32)) &&
            (!tile_beam || (ty != 0 && p.n_uniq_tile > 0 && p.n_uniq_tile <= FT_MAX_NU && !p.unflagged_map));
     if (fast && ty == 2 && p.sdense && !p.sbfp) return cudaErrorInvalidValue;
@@ -869,7 +831,7 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
     // or more keep the per-baseline kernel, which reads the basis table per
     // coefficient.
     if (!fast && p.xyzs && (ty != 2 || p.sdense64)) return launch_pairs(ty, tile_beam, out64, p, s);
-    if (fast && ty == 1 && !tile_beam) return launch_fast_gauss(out64, p, s);
+    if (fast && ty == 1) return launch_fast_gauss(tile_beam, out64, p, s);
     if (ty == 0) return launch_t<0>(tile_beam, out64, fast, p, s);
     if (ty == 1) return launch_t<1>(tile_beam, out64, fast, p, s);
     return launch_t<2>(tile_beam, out64, fast, p, s);

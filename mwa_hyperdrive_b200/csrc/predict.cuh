@@ -95,8 +95,9 @@ __device__ __forceinline__ void add_vis(void* vis, size_t o, const J2& acc) {
 // The FP64 predict of component type ty factored by tile (pairs.cu); p.xyzs
 // set, shapelets with p.sdense64.
 cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s);
-// The chosen form's Gaussians with a shared beam, factored by tile; p.xyzs set.
-cudaError_t launch_fast_gauss(bool out64, const DirectParams& p, cudaStream_t s);
+// The chosen form's Gaussians factored by tile (a shared beam in FP32, a beam
+// per tile with FP64 products); p.xyzs and p.gk set.
+cudaError_t launch_fast_gauss(bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s);
 
 // Launch the direct kernel for component type ty (0 point, 1 Gaussian,
 // 2 shapelet).  tile_beam selects per-tile beam Jones; out64 an FP64 output;

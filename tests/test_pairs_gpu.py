@@ -87,6 +87,18 @@ def test_chosen_form(oracle, kind, ntiles, n):
         assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("kind", ["gaussians", "shapelets"])
+@pytest.mark.parametrize("ntiles,n", [(2, 1), (16, 8), (17, 9), (33, 33), (65, 17)])
+def test_chosen_form_per_tile(oracle, kind, ntiles, n):
+    obs = observation(ntiles, ntiles)
+    sky = sl.SkyModelArrays.from_components(components(kind, n, 300 + n))
+    ref = expected(oracle, sky, obs, "per_tile")
+    for dtype in (torch.float64, torch.float32):
+        got = predict(sky, obs, "tensor", "per_tile", dtype)
+        # the chosen form's bar
+        assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
+
+
 def test_chosen_form_shapelets_beyond_the_staged_window(oracle):
     """Sources of a degree on long baselines: positions far from the basis
     table's centre, and past its ends."""
