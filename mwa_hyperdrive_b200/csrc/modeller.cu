@@ -242,15 +242,22 @@ __global__ void point_model_kernel(const FluxComp* comps, const JonesF64* list, 
     out[((size_t)src * nt + t) * nf + f] = make_float4((float)w.a.re, (float)w.d.re, (float)w.b.re, (float)w.b.im);
 }
 
-// FP32 copy of a per-tile beam table (n Jones matrices).
-__global__ void jones_to_f32_kernel(const JonesF64* __restrict__ in, size_t n, JonesF32* __restrict__ out) {
+// The FP32 rows of a per-tile beam table (TensorBeam::beam32): n table rows of
+// nc components, a row of the output padded to ncp with zeros.
+__global__ void beam_rows_f32_kernel(const JonesF64* __restrict__ in, size_t n, int nc, int ncp, float4* __restrict__ out) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double4* a = reinterpret_cast<const double4*>(in + i);
-    const double4 x = a[0], y = a[1];
-    float4* o = reinterpret_cast<float4*>(out + i);
-    o[0] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
-    o[1] = make_float4((float)y.x, (float)y.y, (float)y.z, (float)y.w);
+    if (i >= n * ncp) return;
+    const size_t row = i / ncp;
+    const int c = (int)(i - row * ncp);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    if (c < nc) {
+        const double4* a = reinterpret_cast<const double4*>(in + row * nc + c);
+        const double4 p = a[0], q = a[1];
+        x = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
+        y = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+    }
+    out[row * 2 * ncp + c] = x;
+    out[(row * 2 + 1) * ncp + c] = y;
 }
 
 // Per-tile beams B [uniq tile][uniq freq][nc] of one component type at this
@@ -475,7 +482,7 @@ int Modeller::alloc_tile_beam_tables() {
         if (t[ty].nc == 0) continue;
         HDC_CUDA_RET_INT(dalloc(&t[ty].d_B, (size_t)tb.n_uniq_tile * tb.n_uniq_freq * t[ty].nc));
         if (ty == 0 && form == HDC_PREDICT_TENSOR)
-            HDC_CUDA_RET_INT(dalloc(&t[ty].d_B32, (size_t)tb.n_uniq_tile * tb.n_uniq_freq * t[ty].nc));
+            HDC_CUDA_RET_INT(dalloc(&t[ty].d_B32, (size_t)tb.n_uniq_tile * tb.n_uniq_freq * 2 * beam32_row(t[ty].nc)));
     }
     return HDC_OK;
 }
@@ -577,8 +584,9 @@ int Modeller::geometry(double lst, cudaStream_t s) {
         }
         // the points' table in FP32 for the tensor form's producers
         if (t[0].d_B32) {
-            const size_t n = (size_t)tb.n_uniq_tile * tb.n_uniq_freq * t[0].nc;
-            jones_to_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(t[0].d_B, n, t[0].d_B32);
+            const size_t n = (size_t)tb.n_uniq_tile * tb.n_uniq_freq;
+            const int ncp = (int)beam32_row(t[0].nc);
+            beam_rows_f32_kernel<<<(unsigned)((n * ncp + 255) / 256), 256, 0, s>>>(t[0].d_B, n, t[0].nc, ncp, t[0].d_B32);
             count_launches(1);
             HDC_CUDA_RET_INT(cudaGetLastError());
         }
@@ -701,13 +709,15 @@ int Modeller::model_channels(double lst, void* d_vis, bool out64, int f0, int nf
         if (ty == 0 && form == HDC_PREDICT_TENSOR) {
             // the workspace holds planes for all nf channels; a chunk of nfc
             // channels uses its start (chunks of one call run in order on s)
-            void* ws = tensor_workspace(out64);
+            size_t ws_bytes = 0;
+            void* ws = tensor_workspace(out64, ws_bytes);
             if (!ws) return HDC_ERR_ALLOC;
             TensorBeam tbm = {t[0].d_B, t[0].d_B32, tb.d_tile_map, tb.d_freq_map + f0, tb.n_uniq_tile,
                               tb.n_uniq_freq};
             const int rc = launch_tensor_points(nfc, nbl, ntiles, t[0].nc, d_freqs + f0, d_xyzs, lst - pc.ra, pc.dec,
                                                 t[0].d_lmn, weights(0) + (size_t)f0 * t[0].nc,
-                                                tile_beams() ? &tbm : nullptr, vis, out64, ws, d_err, s, tensor_sync());
+                                                tile_beams() ? &tbm : nullptr, vis, out64, ws, ws_bytes, d_err, s,
+                                                tensor_sync());
             if (rc) return rc;
         } else {
             // the chosen (tensor) form keeps Gaussians and shapelets in the
@@ -1378,14 +1388,15 @@ int Modeller::model_host_points_last(double lst, JonesF32* h_vis, UVW* h_uvws, c
     rc = model_channels(lst, d_host_model, false, 0, nf, pipe_s[1], 2 | 4, false);
     if (rc) return rc;
     HDC_CUDA_RET_INT(cudaStreamWaitEvent(pipe_s[1], up, 0));
-    void* ws = tensor_workspace(false);
+    size_t ws_bytes = 0;
+    void* ws = tensor_workspace(false, ws_bytes);
     if (!ws) return HDC_ERR_ALLOC;
     PointsLastCtx ctx{this, h_vis, pipe_ev[3]};
     const TensorChunkOut out{d_host_model, points_last_chunk_done, &ctx};
     EvPair e{};
     prof_begin(0, pipe_s[1], e);
     rc = launch_tensor_points(nf, nbl, ntiles, t[0].nc, d_freqs, d_xyzs, lst - pc.ra, pc.dec, t[0].d_lmn, weights(0),
-                              nullptr, d_host_vis, false, ws, d_err, pipe_s[1], tensor_sync(), &out);
+                              nullptr, d_host_vis, false, ws, ws_bytes, d_err, pipe_s[1], tensor_sync(), &out);
     if (rc) return rc;
     prof_end(pipe_s[1], e);
     if (h_uvws)

@@ -22,7 +22,7 @@ struct TypeTables {
     float* d_sdense = nullptr;      // [nc][SDN][SDN] signed dense coefficients, or NULL
     double* d_sdense64 = nullptr;   // the same in FP64 with the basis functions' normalisation (direct form), or NULL
     JonesF64* d_B = nullptr;        // per-tile beams: [uniq tile][uniq freq][nc] at the current timestep
-    JonesF32* d_B32 = nullptr;      // the same in FP32 (points in the tensor form: its producers' reads)
+    float4* d_B32 = nullptr;        // its rows in FP32 (points in the tensor form: TensorBeam::beam32)
     void release();
 };
 
@@ -132,7 +132,7 @@ struct Modeller {
     int model_uvws(double lst, const UVW* d_uvws_ext, JonesF32* d_vis, cudaStream_t s);
     int autos(double lst, JonesF32* d_vis, cudaStream_t s);
     int tensor_setup();
-    void* tensor_workspace(bool out64);
+    void* tensor_workspace(bool out64, size_t& bytes);
     TensorSync* tensor_sync();  // the tensor predict's second stream (NULL: none)
     void tensor_release();
     ~Modeller();

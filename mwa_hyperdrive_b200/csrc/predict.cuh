@@ -109,9 +109,12 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
 // [n_uniq_freq][nc] (the reference's layout), the unique row of every tile
 // (any unflagged-tile map already applied) and the unique column of every
 // channel of the launch.
+// components of a TensorBeam::beam32 row (pairs are read in one aligned load)
+__host__ __device__ inline size_t beam32_row(int nc) { return ((size_t)nc + 1) & ~(size_t)1; }
 struct TensorBeam {
     const JonesF64* beam;
-    const JonesF32* beam32;  // the same table in FP32 (the producers' reads), or NULL
+    const float4* beam32;  // its rows in FP32 (the producers' reads), or NULL: [unique tile][unique
+                           // frequency][row X, Y][beam32_row(nc)], a row entry as re, im of its two columns
     const int* tile_map;
     const int* freq_map;
     int n_uniq_tile;
@@ -131,10 +134,12 @@ void tensor_sync_free(TensorSync& t);
 
 // The tensor-core point predict of one timestep (csrc/tensor.cu): d_W is
 // B S B^H [nf][nc] with a beam shared by all tiles (beam NULL), or S [nf][nc]
-// with per-tile beams.  ws: tensor_workspace_bytes(nf, nbl, ntiles, nc,
-// per-tile beams, out64, sync != NULL) bytes; sync NULL runs every kernel
-// on s in turn.
-size_t tensor_workspace_bytes(int nf, int nbl, int ntiles, int nc, bool tile_beam, bool out64, bool two_tables);
+// with per-tile beams.  ws: ws_bytes >= tensor_workspace_bytes(nf, nbl,
+// ntiles, nc, unique tiles of per-tile beams or 0, out64, sync != NULL, least)
+// bytes; least takes per-tile beams' table of one channel at a time.  sync
+// NULL runs every kernel on s in turn.
+size_t tensor_workspace_bytes(int nf, int nbl, int ntiles, int nc, int n_uniq_tile, bool out64, bool two_tables,
+                              bool least);
 // Per-chunk output of the table form (shared beam, nc <= tensor_single_pass()
 // components, JonesF32 output): after the Gram products of channels
 // [f0, f0 + nch) the chunk's visibilities become vis + model + planes (model:
@@ -148,7 +153,7 @@ struct TensorChunkOut {
 int tensor_single_pass();
 int launch_tensor_points(int nf, int nbl, int ntiles, int nc, const double* d_freqs, const XYZ* d_xyzs, double ha,
                          double dec, const double4* d_lmn, const JonesF64* d_W, const TensorBeam* beam, void* d_vis,
-                         bool out64, void* ws, int* d_err, cudaStream_t s, TensorSync* sync,
+                         bool out64, void* ws, size_t ws_bytes, int* d_err, cudaStream_t s, TensorSync* sync,
                          const TensorChunkOut* chunk_out = nullptr);
 
 struct AutosParams {

@@ -23,7 +23,9 @@
 //     M^a_{p,(c,y)} = A_pc (B_pc S_c)^{ay},   N^b_{q,(c,y)} = A_qc B_qc^{by},
 // a Gram product over K = 2 x components (y the second index of S); again
 // XX, YY and XY suffice (S Hermitian: V^YX_pq = conj(V^XY_qp)).  Both
-// operands carry the beam, so they are formed in the Gram CTA itself.
+// operands carry the beam and would make a table of a row per tile and
+// polarisation; the Gram CTA forms them from a smaller one, the phasors A of
+// each tile and the factors B S of each unique tile.
 //
 // With X the left and Y the right operand, in real form
 //     Re V = Xr Yr^T + Xi Yi^T,   Im V = Xi Yr^T + Xr (-Yi)^T.
@@ -61,8 +63,8 @@
 // 1).  MODE 2: a copy warp brings each stage's A planes from the table
 // (one bulk copy, prefetched into L2 eight stages ahead) and sixteen
 // producer warps form Y = A conj(W) sx from the table's phasors and weights
-// and write its byte planes.  MODE 1: the sixteen producer warps compute
-// the phasors, beams, X and Y and write all planes.  Planes are in the
+// and write its byte planes.  MODE 1: the sixteen producer warps form X
+// and Y from the table and write all planes.  Planes are in the
 // K-major no-swizzle core-matrix layout (one warp store = one 128-byte core
 // matrix).  One thread issues the MMAs of a stage (plane pairs x {Xr, Xi},
 // N = 128 = [Re | Im] of the 64 columns) into 4 TMEM accumulators (one per
@@ -72,6 +74,13 @@
 // of p < q as XY, of p > q as YX = conj); a coalesced pass then adds the four
 // planes into the visibilities, so every Jones matrix is read and written
 // once.
+//
+// MODE 1 is bound by shared memory's data path (the producers' loads and
+// stores and, level with them, the tensor core's operand reads: 20 products of
+// 8 KB a stage); tensor cores 0.46 busy.  One timestep of 2000 points, 17
+// unique tiles, 128 tiles x 192 channels: 2.95 ms with the phasors (FP64
+// phases) and B S formed by each of a channel's six jobs for each row, 1.73 so,
+// 0.2 of it the table; the table in chunks that stay in L2 (96 MB) 1.98.
 //
 // Every mbarrier wait is bounded by the global timer; on a timeout the CTA
 // records KERR_TIMEOUT, waits (bounded) for its issued MMAs and copies and
@@ -132,24 +141,24 @@ struct Cfg<2> {
 constexpr int PL_BYTES = 2 * 3 * XT_BYTES;
 constexpr int PH_ROW = KC * 8;
 constexpr int PH_BYTES = NH * PH_ROW;
+// MODE 1 table of one (channel, stage of 16 components): the FP32 phasors
+// (cos, sin) of the tiles and of one row of zeros (the tiles past the array),
+// in the producer warps' order [8 tiles][component half][tile][pair of
+// components], so that a warp reads 512 contiguous bytes; then the left
+// factors B S sx of each unique tile: row a (X, Y), component (by halves, of
+// each the even ones first: 64 bytes of a tile a read), column y, as re, im.
+constexpr int PH1_GROUP = 8 * 16 * 8;
+constexpr int G1_ROW = 16 * 16;
+__host__ __device__ inline size_t ph1_bytes(int ntiles) { return (size_t)(ntiles + 8) / 8 * PH1_GROUP; }
 template <int MODE>
 struct Lay {
     static constexpr int Y_OFF = 2 * Cfg<MODE>::XDIG * XT_BYTES;                     // X: [re, im][digits]
     static constexpr int STAGE_BYTES = Y_OFF + 3 * Cfg<MODE>::YDIG * YT_BYTES;       // Y: [im, re, -im][digits]
     static constexpr int SMEM_BYTES = Cfg<MODE>::NSTAGE * STAGE_BYTES + 1024;
-    static constexpr int CRING = Cfg<MODE>::NSTAGE + 2;  // component ring: warps may be NSTAGE stages apart
 };
 static_assert(Lay<2>::SMEM_BYTES <= 220 * 1024, "MODE 2 stages exceed shared memory");
 static_assert(Lay<2>::STAGE_BYTES % 16 == 0 && PH_ROW % 16 == 0, "bulk copies need 16-byte alignment");
 constexpr int PF_STAGES = 8;  // MODE 2: table blocks are prefetched into L2 this many stages ahead
-
-// MODE 1 component data of one stage, staged in shared memory (structure
-// of arrays so that 16-byte loads of consecutive components are
-// conflict-free)
-struct CompStage1 {
-    double l[16], m[16], n[16];  // turn units (n - 1 in n)
-    float4 s[16][2];             // S (xx, xy | yx, yy as re, im) of this channel
-};
 
 struct Params {
     int nf, nbl, ntiles, nc, c0, cn;
@@ -161,7 +170,7 @@ struct Params {
     // MODE 1: beam [uniq tile][uniq freq][nc], unique row of each tile and
     // column of each channel, and per channel bounds of |B| and |S| entries
     const JonesF64* beam;
-    const JonesF32* beam32;  // MODE 1: the beam table in FP32, or NULL (then read from beam)
+    const float4* beam32;  // MODE 1: the beam rows in FP32, or NULL (then read from beam)
     const int* tile_map;
     const int* freq_map;
     int n_uniq_freq;
@@ -170,9 +179,10 @@ struct Params {
     const double* maxs;
     void* planes;          // [4][nf][nbl] float2 (or double2 with OUT64)
     int* err;
-    // MODE 2: channels f0 + blockIdx.y; the table of channel f0 + i at
-    // table + i * tab_chan, its stage k at + k * tab_block (row-block planes
-    // first, the column-block phasors from tab_ph_off)
+    // channels f0 + blockIdx.y; the table of channel f0 + i at table + i *
+    // tab_chan, its stage k at + k * tab_block (MODE 2: row-block planes
+    // first, the column-block phasors from tab_ph_off; MODE 1: phasors first,
+    // the left factors from tab_ph_off)
     int f0;
     const unsigned char* table;
     size_t tab_chan, tab_block, tab_ph_off;
@@ -295,22 +305,39 @@ __device__ __forceinline__ void tile_uvw(const Params& P, int tile, double oq, d
     }
 }
 
-// the beam table row of a tile (its unique tile at unique frequency column
-// fm: unique tile x unique frequencies + fm), looked up once per thread; -1
-// past the array
-__device__ __forceinline__ int beam_base(const Params& P, int tile, int fm) {
-    if (tile >= P.ntiles) return -1;
-    return __ldg(P.tile_map + tile) * P.n_uniq_freq + fm;
+// MODE 1 operand scales of channel f from its bounds, |M| <= 2 max|B| max|S|
+// and |N| <= max|B|; false when the bounds are zero (the products are zero)
+__device__ __forceinline__ bool mode1_scales(const Params& P, int f, float& sx, float& sy) {
+    const double bmax = P.maxb[P.by_channel ? f : P.freq_map[f]];
+    const double bound = 2.0 * bmax * P.maxs[f];
+    const bool any = bound > 0.0;
+    sx = any ? (float)(FULL31 / bound) : 0.f;
+    sy = any ? (float)(FULL31 / bmax) : 0.f;
+    return any;
 }
 
-// one row of a beam Jones (two complex numbers, FP32): component c of the
-// pass in beam table row `base`
-__device__ __forceinline__ float4 beam_row(const Params& P, int base, int c, int row) {
-    if (base < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
-    if (P.beam32) return __ldg(reinterpret_cast<const float4*>(P.beam32 + (size_t)base * P.nc + P.c0 + c) + row);
+// 32 bytes in one load (the address a multiple of 32)
+__device__ __forceinline__ void ldg32(const void* a, float4& x, float4& y) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
+                 : "l"(a));
+}
+
+// one row of the beam Jones (two complex numbers, FP32) of components c and
+// c + 1 of the pass (c even) in beam table row `base`
+__device__ __forceinline__ void beam_rows(const Params& P, int base, int c, int row, float4& b0, float4& b1) {
+    c = c < P.cn ? c : 0;
+    if (P.beam32) {
+        ldg32(P.beam32 + ((size_t)base * 2 + row) * beam32_row(P.nc) + P.c0 + c, b0, b1);
+        return;
+    }
     const double2* b = reinterpret_cast<const double2*>(P.beam + (size_t)base * P.nc + P.c0 + c) + 2 * row;
     const double2 e0 = __ldg(b), e1 = __ldg(b + 1);
-    return make_float4((float)e0.x, (float)e0.y, (float)e1.x, (float)e1.y);
+    b0 = b1 = make_float4((float)e0.x, (float)e0.y, (float)e1.x, (float)e1.y);
+    if (c + 1 < P.cn) {
+        const double2 f0 = __ldg(b + 4), f1 = __ldg(b + 5);
+        b1 = make_float4((float)f0.x, (float)f0.y, (float)f1.x, (float)f1.y);
+    }
 }
 
 template <int MODE, bool OUT64>
@@ -318,17 +345,12 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
     using C = Cfg<MODE>;
     using L = Lay<MODE>;
     constexpr int NSTAGE = C::NSTAGE;
-    constexpr int CRING = L::CRING;
     constexpr int NTHR = C::THREADS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ alignas(8) uint64_t full_bar[NSTAGE], empty_bar[NSTAGE], done_bar;
     __shared__ alignas(8) uint64_t copy_bar[NSTAGE];  // MODE 2: the stage's A planes have landed
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
-    // MODE 1: the ring of component data
-    __shared__ __align__(16) CompStage1 comp_s[MODE == 1 ? CRING : 1];
-    __shared__ alignas(8) uint64_t comp_bar[MODE == 1 ? CRING : 1];
-
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int f = P.f0 + blockIdx.y;  // channel (planes, W, frequency)
     const uint32_t job = P.jobs[blockIdx.x];
@@ -346,8 +368,6 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
             mbar_init(&full_bar[s], NPW);  // one arrival per producer warp
             mbar_init(&empty_bar[s], 1);
         }
-        if (MODE == 1)
-            for (int s = 0; s < CRING; s++) mbar_init(&comp_bar[s], 1);  // the stashing warp arrives once
         if (MODE == 2)
             for (int s = 0; s < NSTAGE; s++) mbar_init(&copy_bar[s], 1);  // the copy thread's expect_tx
         mbar_init(&done_bar, 1);
@@ -355,19 +375,18 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
         fence_barrier_init();
     }
     __syncthreads();
-    double bound, bmax = 1.0;
-    if (MODE == 2) {
-        bound = reinterpret_cast<const double*>(P.table + (size_t)blockIdx.y * P.tab_chan + P.tab_bound_off)[pol];
-    } else {
-        bmax = P.maxb[P.by_channel ? f : P.freq_map[f]];
-        bound = 2.0 * bmax * P.maxs[f];
-    }
     const int n = P.ntiles;
     // A polarisation whose weights are all exactly zero (e.g. XY of a
     // Stokes-I sky) contributes exactly zero: its baselines get zeros.
-    const bool zero = !(bound > 0.0);
-    const float sx = zero ? 0.f : (float)(FULL31 / bound);
-    const float sy = MODE == 2 ? SY0 : (zero ? 0.f : (float)(FULL31 / bmax));
+    bool zero;
+    float sx, sy = SY0;
+    if (MODE == 2) {
+        const double bound = reinterpret_cast<const double*>(P.table + (size_t)blockIdx.y * P.tab_chan + P.tab_bound_off)[pol];
+        zero = !(bound > 0.0);
+        sx = zero ? 0.f : (float)(FULL31 / bound);
+    } else {
+        zero = !mode1_scales(P, f, sx, sy);
+    }
     const double inv = zero ? 0.0 : 1.0 / ((double)sx * (double)sy);
     const int nchunks = zero ? 0 : (P.cn + C::CPS - 1) / C::CPS;
 
@@ -381,8 +400,6 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    const double freq = P.freqs[f];
-    const int fm = MODE == 1 ? __ldg(P.freq_map + f) : 0;
 
     if (zero) {
         // nothing to multiply
@@ -472,23 +489,31 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
         // warp = 8 tile rows x 16 K bytes of a stage; lane = (row rl, quad of
         // 4 K bytes), and every thread also takes the row 64 tiles down, so a
         // warp's store of one byte plane is one whole 128-byte core matrix.
-        // Its Y row is column r0 of the column block: one of its two X rows
-        // when the column block lies inside the row block, else a third tile.
+        // Its Y row is column r0 of the column block.
         const int g = warp & 7;             // rows 8g .. 8g + 7 (and + 64)
         const int kq = warp >> 3;           // K bytes [kq * 16, kq * 16 + 16) of a stage
         const int rl = lane >> 2, quad = lane & 3;
         const int r0 = 8 * g + rl;          // rows r0 and r0 + 64 of the block
-        const int ry = cb - 2 * rb;         // the X row that is the Y tile (0 or 1), else separate
-        const bool ysep = ry != 0 && ry != 1;
         const int prow[2] = {NT * rb + r0, NT * rb + r0 + 64};
         const int qcol = NH * cb + r0;
-        // the three tiles' beam row blocks (MODE 1), looked up once
-        const int bbase[3] = {MODE == 1 ? beam_base(P, prow[0], fm) : -1, MODE == 1 ? beam_base(P, prow[1], fm) : -1,
-                              MODE == 1 ? beam_base(P, qcol, fm) : -1};
+        // K bytes 4 quad .. 4 quad + 3 of this warp's 16 = components c0l,
+        // c0l + 1 (stage-local) x y in {X, Y}: the thread's table rows there
+        // (tiles past the array take the row of zero phasors)
+        const int c0l = kq * 8 + quad * 2;
+        const unsigned char* tch = P.table + (size_t)blockIdx.y * P.tab_chan;
+        const unsigned char* ph = tch + kq * (PH1_GROUP / 2) + quad * 16;
+        const unsigned char* gf = tch + P.tab_ph_off + arow * G1_ROW + kq * 128 + quad * 16;
+        auto ph_off = [&](int tile) {
+            const int t = min(tile, n);
+            return (uint32_t)((t >> 3) * PH1_GROUP + (t & 7) * 64);
+        };
+        const uint32_t po[3] = {ph_off(prow[0]), ph_off(prow[1]), ph_off(qcol)};
+        const uint32_t go[2] = {prow[0] < n ? (uint32_t)__ldg(P.tile_map + prow[0]) * (2 * G1_ROW) : 0u,
+                                prow[1] < n ? (uint32_t)__ldg(P.tile_map + prow[1]) * (2 * G1_ROW) : 0u};
+        const int bq = (qcol < n ? __ldg(P.tile_map + qcol) * P.n_uniq_freq : 0) + __ldg(P.freq_map + f);
         // The upper 64 rows of the block pair with no column of it when they
         // lie beyond the array, or in an XX / YY block whose columns all lie
-        // below them: their X planes stay zero and are not produced.  (Then
-        // the Y tile is never one of them: ry != 1.)
+        // below them: their X planes stay zero and are not produced.
         const bool skip_hi = NT * rb + 64 >= n || (pol < 2 && NT * rb + 64 >= NH * cb + NH - 1);
         if (skip_hi) {
             for (int st = 0; st < NSTAGE; st++)
@@ -497,95 +522,49 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                     for (int i = tid; i < XT_BYTES / 32; i += NPT) z[i] = make_uint4(0u, 0u, 0u, 0u);
                 }
         }
-        const double oq = 4.0 * freq / VEL_C;
-        double u[3], v[3], w[3];  // quarter-turns per unit l, m, n - 1 of the two X rows and the Y tile
-        tile_uvw(P, prow[0], oq, u[0], v[0], w[0]);
-        tile_uvw(P, prow[1], oq, u[1], v[1], w[1]);
-        tile_uvw(P, qcol, oq, u[2], v[2], w[2]);
-        const double4* lmn = P.lmn + P.c0;
-        const JonesF64* Wf = P.W + (size_t)f * P.nc + P.c0;
-        // the first CPS threads fetch a stage's component data (zeros past the end)
-        auto fetch = [&](int k, double2& a, double2& b) {
-            const int c = k * C::CPS + tid;
-            if (c < P.cn) {
-                a = __ldg(reinterpret_cast<const double2*>(lmn + c));
-                b = __ldg(reinterpret_cast<const double2*>(lmn + c) + 1);
-            } else {
-                a = b = make_double2(0.0, 0.0);
-            }
-        };
-        // S is read at stash time
-        auto stash = [&](int k, int buf, const double2& a, const double2& b) {
-            CompStage1& cs = comp_s[buf];
-            cs.l[tid] = a.x;
-            cs.m[tid] = a.y;
-            cs.n[tid] = b.x;
-            const int c = k * C::CPS + tid;
-            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-            if (c < P.cn) {
-                const double2* sp = reinterpret_cast<const double2*>(Wf + c);
-                const double2 xx = __ldg(sp), xy = __ldg(sp + 1), yx = __ldg(sp + 2), yy = __ldg(sp + 3);
-                s0 = make_float4((float)xx.x, (float)xx.y, (float)xy.x, (float)xy.y);
-                s1 = make_float4((float)yx.x, (float)yx.y, (float)yy.x, (float)yy.y);
-            }
-            cs.s[tid][0] = s0;
-            cs.s[tid][1] = s1;
-        };
-        // Software pipeline: iteration k writes the byte planes of stage k
-        // from registers and computes the values of stage k + 1 in the same
-        // straight-line block.  Component data goes through a ring of CRING
-        // slots, stashed two stages ahead by the first CPS threads.  Stages
-        // past the end read zeros (their values are never written out).
-        // compute and write_planes take SKIP (skip_hi) as a compile-time
-        // constant, so the two rows' work stays one straight-line block
-        auto compute = [&](auto skip_c, int k, int (&xr)[2][4], int (&xi)[2][4], int (&yr)[4], int (&yi)[4],
-                           int (&yn)[4]) {
+        // A stage's operands: the phasors of the two X rows and the Y row at
+        // two components, the X rows' left factors and the Y row's beam row.
+        // They are loaded a stage ahead, while the stage before is written.
+        float4 pa[3], gx[2][2], bb[2];
+        auto load = [&](auto skip_c, int k) {
             constexpr bool SKIP = decltype(skip_c)::value;
-            const CompStage1& cs_ = comp_s[k % CRING];
-            {
-                // K bytes 4 quad .. 4 quad + 3 of this warp's 16 = components
-                // c0l, c0l + 1 (stage-local) x y in {X, Y}
-                const int c0l = kq * 8 + quad * 2;
-                const int cg = k * C::CPS + c0l;  // component of the pass
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const int c = cg + j < P.cn ? cg + j : 0;  // past the end: bounded values, zero S
-                    const double cl = cs_.l[c0l + j], cm = cs_.m[c0l + j], cn = cs_.n[c0l + j];
-                    const float4 s0 = cs_.s[c0l + j][0], s1 = cs_.s[c0l + j][1];
-                    float snq = 0.f, csq = 0.f;
+            for (int s2 = 0; s2 < 3; s2++)
+                if (!(SKIP && s2 == 1)) pa[s2] = __ldg(reinterpret_cast<const float4*>(ph + po[s2]));
 #pragma unroll
-                    for (int s2 = 0; s2 < 2; s2++) {
-                        if (SKIP && s2 == 1) continue;
-                        float sn, cs;
-                        phasor_quarter_f32(u[s2] * cl + v[s2] * cm + w[s2] * cn, sn, cs);
-                        if (s2 == ry) snq = sn, csq = cs;
-                        // (B S)^{a y} = B^{aX} S^{Xy} + B^{aY} S^{Yy}, then times A
-                        const float4 b = beam_row(P, bbase[s2], c, arow);  // (B^{aX}, B^{aY}) as re, im
+            for (int s2 = 0; s2 < 2; s2++) {
+                if (SKIP && s2 == 1) continue;
+                gx[s2][0] = __ldg(reinterpret_cast<const float4*>(gf + go[s2]));
+                gx[s2][1] = __ldg(reinterpret_cast<const float4*>(gf + go[s2] + 64));
+            }
+            beam_rows(P, bq, k * C::CPS + c0l, brow, bb[0], bb[1]);  // past the end: times a zero phasor
+            ph += P.tab_block;
+            gf += P.tab_block;
+        };
+        auto compute = [&](auto skip_c, int (&xr)[2][4], int (&xi)[2][4], int (&yr)[4], int (&yi)[4], int (&yn)[4]) {
+            constexpr bool SKIP = decltype(skip_c)::value;
 #pragma unroll
-                        for (int y = 0; y < 2; y++) {
-                            // S^{Xy}: s0 (y = 0: xx, y = 1: xy); S^{Yy}: s1 (yx, yy)
-                            const float sxr = y ? s0.z : s0.x, sxi = y ? s0.w : s0.y;
-                            const float syr = y ? s1.z : s1.x, syi = y ? s1.w : s1.y;
-                            const float tr = b.x * sxr - b.y * sxi + b.z * syr - b.w * syi;
-                            const float ti = b.x * sxi + b.y * sxr + b.z * syi + b.w * syr;
-                            const float Xr = fmaf(tr, cs, -ti * sn) * sx;
-                            const float Xi = fmaf(tr, sn, ti * cs) * sx;
-                            xr[s2][2 * j + y] = __float2int_rn(Xr) + 0x808080;
-                            xi[s2][2 * j + y] = __float2int_rn(Xi) + 0x808080;
-                        }
-                    }
-                    if (ysep) phasor_quarter_f32(u[2] * cl + v[2] * cm + w[2] * cn, snq, csq);
-                    const float4 bq = beam_row(P, bbase[2], c, brow);
+            for (int j = 0; j < 2; j++) {
+#pragma unroll
+                for (int s2 = 0; s2 < 2; s2++) {
+                    if (SKIP && s2 == 1) continue;
+                    const float cs = j ? pa[s2].z : pa[s2].x, sn = j ? pa[s2].w : pa[s2].y;
+                    const float4 t = gx[s2][j];  // B S sx: (y = X, y = Y) as re, im
 #pragma unroll
                     for (int y = 0; y < 2; y++) {
-                        const float br = y ? bq.z : bq.x, bi = y ? bq.w : bq.y;
-                        const float Yr = fmaf(br, csq, -bi * snq) * sy;
-                        const float Yi = fmaf(br, snq, bi * csq) * sy;
-                        const int ir = __float2int_rn(Yr), ii = __float2int_rn(Yi);
-                        yr[2 * j + y] = ir + 0x808080;
-                        yi[2 * j + y] = ii + 0x808080;
-                        yn[2 * j + y] = -ii + 0x808080;
+                        const float tr = y ? t.z : t.x, ti = y ? t.w : t.y;
+                        xr[s2][2 * j + y] = __float2int_rn(fmaf(tr, cs, -ti * sn)) + 0x808080;
+                        xi[s2][2 * j + y] = __float2int_rn(fmaf(tr, sn, ti * cs)) + 0x808080;
                     }
+                }
+                const float cs = (j ? pa[2].z : pa[2].x) * sy, sn = (j ? pa[2].w : pa[2].y) * sy;
+#pragma unroll
+                for (int y = 0; y < 2; y++) {
+                    const float br = y ? bb[j].z : bb[j].x, bi = y ? bb[j].w : bb[j].y;
+                    const int ir = __float2int_rn(fmaf(br, cs, -bi * sn)), ii = __float2int_rn(fmaf(br, sn, bi * cs));
+                    yr[2 * j + y] = ir + 0x808080;
+                    yi[2 * j + y] = ii + 0x808080;
+                    yn[2 * j + y] = -ii + 0x808080;
                 }
             }
         };
@@ -619,58 +598,33 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                         b < 3 ? pl[b] ^ 0x80808080u : pl[b];
             }
         };
-        if (tid < C::CPS) {
-            double2 a, b;
-            fetch(0, a, b);
-            stash(0, 0, a, b);
-            fetch(1, a, b);
-            stash(1, 1, a, b);
-        }
-        producers_sync_or(false);
         auto producer_loop = [&](auto skip_c) {
-        int xr[2][4], xi[2][4], yr[4], yi[4], yn[4];
-        compute(skip_c, 0, xr, xi, yr, yi, yn);
-        // The producer warps run decoupled: each warp arrives on a stage's
-        // full barrier once its planes are written, waits for the tensor
-        // core only on the buffer it is about to overwrite, and for the
-        // component data only on the ring slot it is about to read.  Any
-        // timeout sets abort_s; the others leave at their next stage or their
-        // own bounded wait.
-        for (int k = 0; k < nchunks; k++) {
-            const int st = k % NSTAGE;
-            double2 na, nb;  // stage k + 2's component data, in flight during this stage
-            const bool pre = tid < C::CPS;
-            if (pre) fetch(k + 2, na, nb);
-            if (k >= NSTAGE &&
-                !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st], ((k / NSTAGE) - 1) & 1, P.err))) {
-                abort_s = 1;
-                break;
+            int xr[2][4], xi[2][4], yr[4], yi[4], yn[4];
+            load(skip_c, 0);
+            // The producer warps run decoupled: each warp arrives on a stage's
+            // full barrier once its planes are written and waits for the
+            // tensor core only on the buffer it is about to overwrite.  Any
+            // timeout sets abort_s; the others leave at their next stage or
+            // their own bounded wait.
+            for (int k = 0; k < nchunks; k++) {
+                const int st = k % NSTAGE;
+                compute(skip_c, xr, xi, yr, yi, yn);
+                if (k + 1 < nchunks) load(skip_c, k + 1);
+                if (k >= NSTAGE &&
+                    !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st], ((k / NSTAGE) - 1) & 1, P.err))) {
+                    abort_s = 1;
+                    break;
+                }
+                write_planes(skip_c, st, xr, xi, yr, yi, yn);
+                fence_proxy_async_smem();  // make the generic-proxy stores visible to the tensor core
+                __syncwarp();              // the lanes' stores and fences before the warp's one arrival
+                if (lane == 0) mbar_arrive(&full_bar[st]);
+                if (abort_s != 0) break;
             }
-            int nxr[2][4], nxi[2][4], nyr[4], nyi[4], nyn[4];
-            write_planes(skip_c, st, xr, xi, yr, yi, yn);
-            // stage k + 1's component data: stages 0 and 1 were published by
-            // the barrier above, later ones by warp 0 in its iteration k - 1
-            if (k + 1 >= 2 && !__all_sync(0xffffffffu, mbar_wait_bounded(&comp_bar[(k + 1) % CRING],
-                                                                           ((k - 1) / CRING) & 1, P.err))) {
-                abort_s = 1;
-                break;
-            }
-            compute(skip_c, k + 1, nxr, nxi, nyr, nyi, nyn);
-            fence_proxy_async_smem();  // make the generic-proxy stores visible to the tensor core
-            if (pre) stash(k + 2, (k + 2) % CRING, na, nb);
-            __syncwarp();  // the lanes' stores and fences before the warp's one arrival
-            if (lane == 0) {
-                mbar_arrive(&full_bar[st]);
-                if (pre) mbar_arrive(&comp_bar[(k + 2) % CRING]);
-            }
-            if (abort_s != 0) break;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                xr[0][j] = nxr[0][j], xr[1][j] = nxr[1][j], xi[0][j] = nxi[0][j], xi[1][j] = nxi[1][j];
-                yr[j] = nyr[j], yi[j] = nyi[j], yn[j] = nyn[j];
-            }
-        }
         };
+        // the zeroed upper planes before any warp's first arrival
+        if (skip_hi) fence_proxy_async_smem();
+        producers_sync_or(false);
         if (skip_hi)
             producer_loop(std::true_type{});
         else
@@ -681,8 +635,14 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
         if (lane == 0) {
             const uint32_t sbase = smem_u32(smem);
             const uint32_t id = idesc_s8();
+            // MODE 1: the channel's first job brings the table's stages into L2
+            // PF_STAGES ahead of the producers of all its jobs
+            const unsigned char* tch = P.table + (size_t)blockIdx.y * P.tab_chan;
+            const bool pre = MODE == 1 && blockIdx.x == 0;
+            for (int k = 0; pre && k < nchunks && k < PF_STAGES; k++) prefetch_l2(tch + (size_t)k * P.tab_block, P.tab_block);
             for (int k = 0; k < nchunks; k++) {
                 const int st = k % NSTAGE;
+                if (pre && k + PF_STAGES < nchunks) prefetch_l2(tch + (size_t)(k + PF_STAGES) * P.tab_block, P.tab_block);
                 bool ok = MODE == 2 ? mbar_wait_sleep(&full_bar[st], (k / NSTAGE) & 1, P.err)
                                     : mbar_wait_bounded(&full_bar[st], (k / NSTAGE) & 1, P.err);
                 // MODE 2: the A planes came by bulk copy (complete before
@@ -952,6 +912,80 @@ __global__ void __launch_bounds__(TT) phasor_table_kernel(const __grid_constant_
     }
 }
 
+// MODE 1 table of one pass: grid (groups of T1_STAGES stages, groups of 64
+// tiles then of 32 unique tiles, channels of the chunk), 256 threads.  A
+// thread takes two tiles and two components of each stage of its group (the
+// same FP64 phase and FP32 polynomials as MODE 2's), or one row of B S sx of
+// one component and four unique tiles, formed in FP64 and rounded once.  A
+// warp's stores are 512 contiguous bytes.
+constexpr int T1_STAGES = 16;
+constexpr int T1_TILES = 64, T1_UNIQ = 32;
+__global__ void __launch_bounds__(256) tile_beam_table_kernel(const __grid_constant__ Params P, int n_uniq_tile) {
+    const int f = P.f0 + blockIdx.z, t = threadIdx.x, lane = t & 31;
+    const int nstg = (P.cn + Cfg<1>::CPS - 1) / Cfg<1>::CPS;
+    const int k0 = blockIdx.x * T1_STAGES, k1 = min(k0 + T1_STAGES, nstg);
+    const int ntg = (P.ntiles + T1_TILES) / T1_TILES;  // the tiles and the row of zeros
+    unsigned char* blk = const_cast<unsigned char*>(P.table) + (size_t)blockIdx.z * P.tab_chan + (size_t)k0 * P.tab_block;
+    if ((int)blockIdx.y < ntg) {
+        const int kq = (t >> 5) & 1, c0l = kq * 8 + (lane & 3) * 2;
+        const int tile0 = blockIdx.y * T1_TILES + (t >> 6) * 8 + (lane >> 2);
+        const double oq = 4.0 * P.freqs[f] / VEL_C;
+        double u[2], v[2], w[2];
+        tile_uvw(P, tile0, oq, u[0], v[0], w[0]);
+        tile_uvw(P, tile0 + 32, oq, u[1], v[1], w[1]);
+        unsigned char* dst = blk + (size_t)(tile0 >> 3) * PH1_GROUP + kq * (PH1_GROUP / 2) + lane * 16;
+        for (int k = k0; k < k1; k++, dst += P.tab_block) {
+            float ph[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int c = k * Cfg<1>::CPS + c0l + j;
+                const double2* q = reinterpret_cast<const double2*>(P.lmn + P.c0 + (c < P.cn ? c : 0));
+                const double2 a = __ldg(q);
+                const double nn = __ldg(reinterpret_cast<const double*>(q + 1));
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    float sn, cs;
+                    phasor_quarter_f32(u[i] * a.x + v[i] * a.y + w[i] * nn, sn, cs);
+                    const bool live = c < P.cn && tile0 + 32 * i < P.ntiles;
+                    ph[i][2 * j] = live ? cs : 0.f;
+                    ph[i][2 * j + 1] = live ? sn : 0.f;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if (tile0 + 32 * i <= P.ntiles)
+                    *reinterpret_cast<float4*>(dst + i * (4 * PH1_GROUP)) =
+                        make_float4(ph[i][0], ph[i][1], ph[i][2], ph[i][3]);
+        }
+        return;
+    }
+    const int u0 = (blockIdx.y - ntg) * T1_UNIQ + (t >> 5), cl = lane & 15, a = lane >> 4;
+    const int u1 = min(((int)blockIdx.y - ntg + 1) * T1_UNIQ, n_uniq_tile);
+    float sx, sy;
+    mode1_scales(P, f, sx, sy);
+    const JonesF64* B = P.beam + (size_t)P.freq_map[f] * P.nc + P.c0;
+    const JonesF64* S = P.W + (size_t)f * P.nc + P.c0;
+    const size_t ustride = (size_t)P.n_uniq_freq * P.nc;
+    unsigned char* dst = blk + P.tab_ph_off + a * G1_ROW + (cl >> 3) * 128 + (cl & 1) * 64 + ((cl >> 1) & 3) * 16;
+    for (int k = k0; k < k1; k++, dst += P.tab_block) {
+        const int c = k * Cfg<1>::CPS + cl;
+        const bool live = c < P.cn;
+        const double2* sp = reinterpret_cast<const double2*>(S + (live ? c : 0));
+        const double2 x0 = __ldg(sp), x1 = __ldg(sp + 1), y0 = __ldg(sp + 2), y1 = __ldg(sp + 3);
+        for (int u = u0; u < u1; u += 8) {
+            const double2* b = reinterpret_cast<const double2*>(B + u * ustride + (live ? c : 0)) + 2 * a;
+            const double2 b0 = __ldg(b), b1 = __ldg(b + 1);
+            // (B S)^{a y} = B^{aX} S^{Xy} + B^{aY} S^{Yy}
+            float4 o;
+            o.x = (float)((b0.x * x0.x - b0.y * x0.y + b1.x * y0.x - b1.y * y0.y) * sx);
+            o.y = (float)((b0.x * x0.y + b0.y * x0.x + b1.x * y0.y + b1.y * y0.x) * sx);
+            o.z = (float)((b0.x * x1.x - b0.y * x1.y + b1.x * y1.x - b1.y * y1.y) * sx);
+            o.w = (float)((b0.x * x1.y + b0.y * x1.x + b1.x * y1.y + b1.y * y1.x) * sx);
+            *reinterpret_cast<float4*>(dst + (size_t)u * (2 * G1_ROW)) = live ? o : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
 // vis [nf][nbl] += the four planes (one thread per visibility, coalesced)
 template <bool OUT64>
 __global__ void combine_kernel(const void* planes, void* vis, size_t n) {
@@ -1061,8 +1095,8 @@ int build_jobs(int ntiles, uint32_t* jobs) {
 }
 
 // The MODE 2 table of a pass: bytes per (channel, stage) and per channel,
-// and the channels of one chunk: as many as fit in TABLE_CAP, rounded down
-// to a multiple that fills whole waves of the SMs with jobs.
+// and the channels of one chunk: as many as fit in TABLE_CAP (of both modes),
+// rounded down to a multiple that fills whole waves of the SMs with jobs.
 constexpr size_t TABLE_CAP = (size_t)1 << 30;
 
 struct TableShape {
@@ -1088,15 +1122,49 @@ static TableShape table_shape(int nf, int ntiles, int cn, int njobs) {
     return t;
 }
 
+// The MODE 1 table of a pass: its bytes per (channel, stage) and per channel.
+static TableShape table1_shape(int ntiles, int n_uniq_tile, int cn) {
+    TableShape t = {};
+    t.nstg = (cn + Cfg<1>::CPS - 1) / Cfg<1>::CPS;
+    t.block = ph1_bytes(ntiles) + (size_t)n_uniq_tile * 2 * G1_ROW;
+    t.chan = (size_t)t.nstg * t.block;
+    return t;
+}
+
+// Channels of one MODE 1 chunk whose table may take `bytes`
+static int table1_chunk(const TableShape& t, int nf, int njobs, size_t bytes) {
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaGetLastError();
+    const int fit = (int)std::min<size_t>(nf, std::max<size_t>(1, bytes / t.chan));
+    if (fit == nf) return nf;
+    // of the upper half of what fits, the count that fills the last wave best
+    int best = fit;
+    double eff = 0.0;
+    for (int c = fit; c >= std::max(1, fit / 2); c--) {
+        const long jobs = (long)c * njobs, waves = (jobs + sms - 1) / sms;
+        const double e = (double)jobs / (double)(waves * sms);
+        if (e > eff + 1e-9) best = c, eff = e;
+    }
+    return best;
+}
+
 }  // namespace tc
 
 // Bytes of device workspace the tensor predict needs for nf channels of
-// nc components: the four planes, the MODE 1 per-channel bounds and, with
-// a shared beam, the MODE 2 table of one chunk of channels.
-size_t tensor_workspace_bytes(int nf, int nbl, int ntiles, int nc, bool tile_beam, bool out64, bool two_tables) {
+// nc components: the four planes, the MODE 1 bounds and the table of one
+// chunk of channels (n_uniq_tile: MODE 1, 0 with a shared beam).  least: MODE
+// 1's smallest, one channel a chunk.
+size_t tensor_workspace_bytes(int nf, int nbl, int ntiles, int nc, int n_uniq_tile, bool out64, bool two_tables,
+                              bool least) {
     const size_t planes = (size_t)4 * nf * nbl * (out64 ? 16 : 8);
     size_t bytes = ((planes + 255) & ~(size_t)255) + ((2 * sizeof(double) * (size_t)nf + 255) & ~(size_t)255);
-    if (!tile_beam && nc > 0 && nf > 0) {
+    if (n_uniq_tile > 0 && nc > 0 && nf > 0) {
+        const tc::TableShape t = tc::table1_shape(ntiles, n_uniq_tile, std::min(nc, tc::Cfg<1>::KPASS));
+        std::vector<uint32_t> jobs(tc::MAXJOBS);
+        const int c = least ? 1 : tc::table1_chunk(t, nf, tc::build_jobs(ntiles, jobs.data()), tc::TABLE_CAP);
+        bytes += (two_tables && c < nf && !least ? 2 : 1) * (size_t)c * t.chan;
+    } else if (nc > 0 && nf > 0) {
         std::vector<uint32_t> jobs(tc::MAXJOBS);
         const int nj = tc::build_jobs(ntiles, jobs.data());
         const tc::TableShape t = tc::table_shape(nf, ntiles, std::min(nc, tc::Cfg<2>::KPASS), nj);
@@ -1109,6 +1177,7 @@ struct TensorState {
     bool configured = false;
     void* ws = nullptr;
     size_t ws_bytes = 0;
+    bool ws_short = false;  // ws is the least the predict does with
     TensorSync sync;
     bool sync_ok = false, sync_failed = false;
 };
@@ -1170,9 +1239,9 @@ int Modeller::tensor_setup() {
 // [nc] (turns), W [nf][nc] (B S B^H of a beam shared by all tiles, or S with
 // per-tile beams in `beam`), tile XYZs, hour angle and declination of the
 // phase centre; accumulates into vis [nf][nbl] (JonesF32, or JonesF64 with
-// out64).  ws: tensor_workspace_bytes(nf, nbl, ntiles, nc, per-tile beams,
-// out64, sync != NULL) bytes of device memory.  With sync, the tables of a
-// shared beam alternate between two buffers and are written on sync->ts,
+// out64).  ws: ws_bytes of device memory, at least tensor_workspace_bytes(nf,
+// nbl, ntiles, nc, unique tiles, out64, sync != NULL, least).  With sync, the
+// tables alternate between two buffers and are written on sync->ts,
 // each chunk's Gram kernel (on s) waiting for its table and each table for
 // the Gram kernel that last read its buffer, so that writing the next
 // chunk's table overlaps the current Gram kernel.
@@ -1180,7 +1249,7 @@ int tensor_single_pass() { return tc::Cfg<2>::KPASS; }
 
 int launch_tensor_points(int nf, int nbl, int ntiles, int nc, const double* d_freqs, const XYZ* d_xyzs, double ha,
                          double dec, const double4* d_lmn, const JonesF64* d_W, const TensorBeam* beam, void* d_vis,
-                         bool out64, void* ws, int* d_err, cudaStream_t s, TensorSync* sync,
+                         bool out64, void* ws, size_t ws_bytes, int* d_err, cudaStream_t s, TensorSync* sync,
                          const TensorChunkOut* chunk_out) {
     if (nc == 0 || nf == 0) return HDC_OK;
     if (chunk_out && (out64 || (beam && beam->beam) || nc > tc::Cfg<2>::KPASS)) {
@@ -1241,13 +1310,44 @@ int launch_tensor_points(int nf, int nbl, int ntiles, int nc, const double* d_fr
                 c0, P.cn, bounds, bounds + nf);
             count_launches(1);
             HDC_CUDA_RET_INT(cudaGetLastError());
-            const dim3 grid(P.njobs, nf);
-            if (out64)
-                tc::gram_i8_kernel<1, true><<<grid, tc::Cfg<1>::THREADS, tc::Lay<1>::SMEM_BYTES, s>>>(P);
-            else
-                tc::gram_i8_kernel<1, false><<<grid, tc::Cfg<1>::THREADS, tc::Lay<1>::SMEM_BYTES, s>>>(P);
-            count_launches(1);
-            HDC_CUDA_RET_INT(cudaGetLastError());
+            // the table of a chunk of channels, then their Gram products, as
+            // with a shared beam; what the workspace holds sets the chunk
+            const tc::TableShape t = tc::table1_shape(ntiles, beam->n_uniq_tile, P.cn);
+            P.tab_block = t.block;
+            P.tab_chan = t.chan;
+            P.tab_ph_off = tc::ph1_bytes(ntiles);
+            const size_t room = ws_bytes - (size_t)(table0 - static_cast<const unsigned char*>(ws));
+            int chunk = tc::table1_chunk(t, nf, P.njobs, std::min(room, tc::TABLE_CAP));
+            const bool two = sync != nullptr && chunk < nf && 2 * (size_t)chunk * t.chan <= room;
+            const int ny = (ntiles + tc::T1_TILES) / tc::T1_TILES + (beam->n_uniq_tile + tc::T1_UNIQ - 1) / tc::T1_UNIQ;
+            if (two) {
+                HDC_CUDA_RET_INT(cudaEventRecord(sync->start, s));
+                HDC_CUDA_RET_INT(cudaStreamWaitEvent(sync->ts, sync->start, 0));
+            }
+            for (int f0 = 0, i = 0; f0 < nf; f0 += chunk, i++) {
+                const int nch = std::min(chunk, nf - f0), b = two ? (i & 1) : 0;
+                cudaStream_t tsx = two ? sync->ts : s;
+                P.f0 = f0;
+                P.table = table0 + (size_t)b * chunk * t.chan;
+                if (two && i >= 2) HDC_CUDA_RET_INT(cudaStreamWaitEvent(sync->ts, sync->gram_done[b], 0));
+                tc::tile_beam_table_kernel<<<dim3((t.nstg + tc::T1_STAGES - 1) / tc::T1_STAGES, ny, nch), 256, 0, tsx>>>(
+                    P, beam->n_uniq_tile);
+                count_launches(1);
+                HDC_CUDA_RET_INT(cudaGetLastError());
+                if (two) {
+                    HDC_CUDA_RET_INT(cudaEventRecord(sync->table_done[b], sync->ts));
+                    HDC_CUDA_RET_INT(cudaStreamWaitEvent(s, sync->table_done[b], 0));
+                }
+                const dim3 grid(P.njobs, nch);
+                if (out64)
+                    tc::gram_i8_kernel<1, true><<<grid, tc::Cfg<1>::THREADS, tc::Lay<1>::SMEM_BYTES, s>>>(P);
+                else
+                    tc::gram_i8_kernel<1, false><<<grid, tc::Cfg<1>::THREADS, tc::Lay<1>::SMEM_BYTES, s>>>(P);
+                count_launches(1);
+                HDC_CUDA_RET_INT(cudaGetLastError());
+                if (two) HDC_CUDA_RET_INT(cudaEventRecord(sync->gram_done[b], s));
+            }
+            P.f0 = 0;
         } else {
             // the table of a chunk of channels, then their Gram products;
             // with sync the tables alternate between two buffers on the
@@ -1317,19 +1417,34 @@ int launch_tensor_points(int nf, int nbl, int ntiles, int nc, const double* d_fr
 }
 
 // The modeller's workspace for the tensor predict of up to nf channels.
-void* Modeller::tensor_workspace(bool out64) {
-    const size_t need = tensor_workspace_bytes(nf, nbl, ntiles, t[0].nc, tile_beams(), out64, tensor_sync() != nullptr);
+void* Modeller::tensor_workspace(bool out64, size_t& bytes) {
+    const int nu = tile_beams() ? tb.n_uniq_tile : 0;
+    size_t need = tensor_workspace_bytes(nf, nbl, ntiles, t[0].nc, nu, out64, tensor_sync() != nullptr, false);
+    const size_t least = tensor_workspace_bytes(nf, nbl, ntiles, t[0].nc, nu, out64, tensor_sync() != nullptr, true);
     if (tc->ws_bytes < need) {
+        // short of memory, per-tile beams do with the table of one channel
+        if (tc->ws_bytes >= least && tc->ws_short) {
+            bytes = tc->ws_bytes;
+            return tc->ws;
+        }
         if (tc->ws) cudaFree(tc->ws);
         tc->ws = nullptr;
         tc->ws_bytes = 0;
+        tc->ws_short = false;
         if (cudaMalloc(&tc->ws, need) != cudaSuccess) {
             cudaGetLastError();
-            set_error("tensor predict workspace of %zu bytes: allocation failed", need);
-            return nullptr;
+            tc->ws_short = true;
+            need = least;
+            if (cudaMalloc(&tc->ws, need) != cudaSuccess) {
+                cudaGetLastError();
+                tc->ws = nullptr;
+                set_error("tensor predict workspace of %zu bytes: allocation failed", need);
+                return nullptr;
+            }
         }
         tc->ws_bytes = need;
     }
+    bytes = tc->ws_bytes;
     return tc->ws;
 }
 

@@ -87,8 +87,8 @@ def test_chosen_form(oracle, kind, ntiles, n):
         assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
 
 
-@pytest.mark.parametrize("kind", ["gaussians", "shapelets"])
-@pytest.mark.parametrize("ntiles,n", [(2, 1), (16, 8), (17, 9), (33, 33), (65, 17)])
+@pytest.mark.parametrize("kind", ["points", "gaussians", "shapelets"])
+@pytest.mark.parametrize("ntiles,n", [(2, 1), (16, 8), (17, 9), (33, 33), (65, 17), (130, 16)])
 def test_chosen_form_per_tile(oracle, kind, ntiles, n):
     obs = observation(ntiles, ntiles)
     sky = sl.SkyModelArrays.from_components(components(kind, n, 300 + n))
@@ -97,6 +97,22 @@ def test_chosen_form_per_tile(oracle, kind, ntiles, n):
         got = predict(sky, obs, "tensor", "per_tile", dtype)
         # the chosen form's bar
         assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
+
+
+def test_points_per_tile_in_chunks_of_channels():
+    """More components than a pass takes and a table that exceeds its cap, so
+    that channels go through it in turn, against the FP64 form."""
+    ntiles, nf = 80, 45
+    obs = synth.Obs(synth.tiles_in_disk(ntiles, 750.0, 3), 167e6 + np.arange(nf) * 40e3, PC, np.array([LST]))
+    sky = sl.SkyModelArrays.from_components(components("points", 8011, 7))
+    gains = np.random.default_rng(8).uniform(0.5, 1.0, (ntiles, 2, 16))
+    vis = {}
+    for form in ("direct", "tensor"):
+        m = SkyModeller(sky, obs.tile_xyzs, obs.freqs, PC, obs.latitude, form=form, beam="per_tile", dipole_gains=gains)
+        vis[form] = torch.zeros((nf, obs.num_baselines, 8), dtype=torch.float64, device="cuda")
+        m.model_timestep_with(LST, vis[form])
+        m.close()
+    assert torch.linalg.norm(vis["tensor"] - vis["direct"]) < 1e-6 * torch.linalg.norm(vis["direct"])
 
 
 def test_chosen_form_shapelets_beyond_the_staged_window(oracle):
