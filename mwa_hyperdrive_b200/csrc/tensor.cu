@@ -67,8 +67,9 @@
 // and Y from the table and write all planes.  Planes are in the
 // K-major no-swizzle core-matrix layout (one warp store = one 128-byte core
 // matrix).  One thread issues the MMAs of a stage (plane pairs x {Xr, Xi},
-// N = 128 = [Re | Im] of the 64 columns) into 4 TMEM accumulators (one per
-// class, 128 columns each = all 512 columns).  The epilogue reads TMEM with
+// N = 128 = [Re | Im] of the 64 columns, or 256 for two Y digits whose classes
+// are neighbours) into 4 TMEM accumulators (one per class, 128 columns each =
+// all 512 columns).  The epilogue reads TMEM with
 // tcgen05.ld, combines the classes in FP64 and stores each of its baselines'
 // values once into a planar scratch [XX, XY, YX, YY][channel][baseline] (XY
 // of p < q as XY, of p > q as YX = conj); a coalesced pass then adds the four
@@ -76,10 +77,10 @@
 // once.
 //
 // MODE 1 is bound by shared memory's data path (the producers' loads and
-// stores and, level with them, the tensor core's operand reads: 20 products of
-// 8 KB a stage); tensor cores 0.46 busy.  One timestep of 2000 points, 17
+// stores and, level with them, the tensor core's operand reads, 128 KB a
+// stage); tensor cores 0.46 busy.  One timestep of 2000 points, 17
 // unique tiles, 128 tiles x 192 channels: 2.95 ms with the phasors (FP64
-// phases) and B S formed by each of a channel's six jobs for each row, 1.73 so,
+// phases) and B S formed by each of a channel's six jobs for each row, 1.71 so,
 // 0.2 of it the table; the table in chunks that stay in L2 (96 MB) 1.98.
 //
 // Every mbarrier wait is bounded by the global timer; on a timeout the CTA
@@ -131,13 +132,15 @@ struct Cfg<1> {
 // the FP32 phasors come from a table written once per (channel, stage).
 template <>
 struct Cfg<2> {
-    static constexpr int XDIG = 3, YDIG = 4, NSTAGE = 4, CPS = 32;
+    static constexpr int XDIG = 3, YDIG = 4, NSTAGE = 3, CPS = 32;
     static constexpr int KPASS = 16384;  // 3 products x 2 x 2^14 x KPASS < 2^31
     static constexpr int THREADS = NPT + 64;  // producers + the MMA warp + the copy warp
 };
 // Table of one (channel, stage): the A planes of each row block ([re, im]
 // x 3 digits in the shared-memory layout, 24 KB), then the FP32 phasors
-// (cos, sin) of each column block of 64 tiles (rows of 32 components).
+// (cos, sin) of each column block of 64 tiles, in the order in which the
+// producer warps read them: [8 tiles][16 components][first or second pair of
+// 4][tile][quad], 512 contiguous bytes a read.
 constexpr int PL_BYTES = 2 * 3 * XT_BYTES;
 constexpr int PH_ROW = KC * 8;
 constexpr int PH_BYTES = NH * PH_ROW;
@@ -152,8 +155,8 @@ constexpr int G1_ROW = 16 * 16;
 __host__ __device__ inline size_t ph1_bytes(int ntiles) { return (size_t)(ntiles + 8) / 8 * PH1_GROUP; }
 template <int MODE>
 struct Lay {
-    static constexpr int Y_OFF = 2 * Cfg<MODE>::XDIG * XT_BYTES;                     // X: [re, im][digits]
-    static constexpr int STAGE_BYTES = Y_OFF + 3 * Cfg<MODE>::YDIG * YT_BYTES;       // Y: [im, re, -im][digits]
+    static constexpr int Y_OFF = 2 * Cfg<MODE>::XDIG * XT_BYTES;                // X: [re, im][digits]
+    static constexpr int STAGE_BYTES = Y_OFF + 4 * Cfg<MODE>::YDIG * YT_BYTES;  // Y: [digits][re, -im], [digits][im, re]
     static constexpr int SMEM_BYTES = Cfg<MODE>::NSTAGE * STAGE_BYTES + 1024;
 };
 static_assert(Lay<2>::SMEM_BYTES <= 220 * 1024, "MODE 2 stages exceed shared memory");
@@ -203,8 +206,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 
 // kind::i8 instruction descriptor: s32 D (bits 4-5 = 2), A and B signed
 // (bits 7 and 10 = 1), K-major, N at bit 17 (>> 3), M at bit 24 (>> 4).
-__host__ __device__ constexpr uint32_t idesc_s8() {
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(NT >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_s8(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(NT >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
@@ -281,14 +284,25 @@ template <int MODE>
 __device__ __forceinline__ uint32_t x_tile(int part, int digit) {
     return (uint32_t)((part * Cfg<MODE>::XDIG + digit) * XT_BYTES);
 }
-// Y tiles of one digit lie in the order [Yi | Yr | -Yi] (64 rows each), so
-// that [Yr; -Yi] (from the Yr tile) and [Yi; Yr] (from the Yi tile) are
-// 128-row B operands: Xr [Yr; -Yi]^T + Xi [Yi; Yr]^T = [Re | Im] of X Y^H.
-// part: 0 = Yr, 1 = Yi, 2 = -Yi
+// Two stacks of Y tiles (64 rows each): the digits' [Yr; -Yi], then the
+// digits' [Yi; Yr], so that digits j and j + 1 of a stack are one 256-row B
+// operand whose products are those of classes w and w + 1:
+// Xr [Yr; -Yi]^T + Xi [Yi; Yr]^T = [Re | Im] of X Y^H.  Storing Yr twice costs
+// a seventh (MODE 1) or a third (MODE 2) more stores and saves eight of twenty
+// or of eighteen reads of an X plane.  128 tiles x 384 channels x 4000 points:
+// 2.80 ms with a product per digit pair, 2.79 so with four stages, 2.70 with
+// three (beside which the next table's CTAs fit), 2.67 with the phasors in
+// read order.
+// slot: 0 Yr, 1 -Yi (stack 0); 2 Yi, 3 Yr (stack 1)
 template <int MODE>
-__device__ __forceinline__ uint32_t y_tile(int part, int digit) {
-    const int slot = part == 0 ? 1 : (part == 1 ? 0 : 2);
-    return (uint32_t)(Lay<MODE>::Y_OFF + (digit * 3 + slot) * YT_BYTES);
+__device__ __forceinline__ uint32_t y_tile(int slot, int digit) {
+    return (uint32_t)(Lay<MODE>::Y_OFF + ((slot >> 1) * Cfg<MODE>::YDIG + digit) * 2 * YT_BYTES + (slot & 1) * YT_BYTES);
+}
+// one word of a Y byte plane into its stacks; part: 0 Yr, 1 Yi, 2 -Yi
+template <int MODE>
+__device__ __forceinline__ void store_y(unsigned char* at, int part, int digit, uint32_t w) {
+    *reinterpret_cast<uint32_t*>(at + y_tile<MODE>(part == 0 ? 0 : (part == 1 ? 2 : 1), digit)) = w;
+    if (part == 0) *reinterpret_cast<uint32_t*>(at + y_tile<MODE>(3, digit)) = w;
 }
 // TMEM column of accumulator class w ([Re | Im], NB columns)
 __device__ __forceinline__ uint32_t acc_col(int w) { return (uint32_t)(w * NB); }
@@ -416,7 +430,7 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
             const int cl0 = kq * 16 + quad * 4;
             const uint32_t yo = chunk_off(r, kq) + quad * 4;
             const unsigned char* tch = P.table + (size_t)blockIdx.y * P.tab_chan;
-            const unsigned char* phq = tch + P.tab_ph_off + (size_t)cb * PH_BYTES + r * PH_ROW + cl0 * 8;
+            const unsigned char* phq = tch + P.tab_ph_off + (size_t)cb * PH_BYTES + (g * 2 + kq) * 1024 + (rl * 4 + quad) * 16;
             const float2* wq = reinterpret_cast<const float2*>(tch + P.tab_w_off) + (size_t)pol * nchunks * KC + cl0;
             // stage k's phasors and W sx of this thread's four components
             // (the copy warp prefetches the phasor blocks into L2; past the
@@ -425,7 +439,7 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                 if (k < nchunks) {
                     const float4* q = reinterpret_cast<const float4*>(phq + (size_t)k * P.tab_block);
                     x = __ldg(q);
-                    y = __ldg(q + 1);
+                    y = __ldg(q + 32);
                     const float4* wv = reinterpret_cast<const float4*>(wq + (size_t)k * KC);
                     u = __ldg(wv);
                     v = __ldg(wv + 1);
@@ -472,9 +486,7 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                     byte_planes4(yv[part], pl);
                     // bytes 0-2 excess-128 lower digits, byte 3 the signed top digit
 #pragma unroll
-                    for (int b = 0; b < 4; b++)
-                        *reinterpret_cast<uint32_t*>(sb + y_tile<MODE>(part, 3 - b) + yo) =
-                            b < 3 ? pl[b] ^ 0x80808080u : pl[b];
+                    for (int b = 0; b < 4; b++) store_y<MODE>(sb + yo, part, 3 - b, b < 3 ? pl[b] ^ 0x80808080u : pl[b]);
                 }
                 fence_proxy_async_smem();  // make the generic-proxy stores visible to the tensor core
                 __syncwarp();
@@ -593,9 +605,7 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                 byte_planes4(part == 0 ? yr : (part == 1 ? yi : yn), pl);
                 // as x: bytes 0-2 excess-128, byte 3 signed
 #pragma unroll
-                for (int b = 0; b < 4; b++)
-                    *reinterpret_cast<uint32_t*>(sb + y_tile<MODE>(part, 3 - b) + yo) =
-                        b < 3 ? pl[b] ^ 0x80808080u : pl[b];
+                for (int b = 0; b < 4; b++) store_y<MODE>(sb + yo, part, 3 - b, b < 3 ? pl[b] ^ 0x80808080u : pl[b]);
             }
         };
         auto producer_loop = [&](auto skip_c) {
@@ -634,7 +644,7 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
         // ------------------------------------------------ MMA issuer (one thread)
         if (lane == 0) {
             const uint32_t sbase = smem_u32(smem);
-            const uint32_t id = idesc_s8();
+            const uint32_t id = idesc_s8(NB), id2 = idesc_s8(2 * NB);
             // MODE 1: the channel's first job brings the table's stages into L2
             // PF_STAGES ahead of the producers of all its jobs
             const unsigned char* tch = P.table + (size_t)blockIdx.y * P.tab_chan;
@@ -655,23 +665,21 @@ __global__ void __launch_bounds__(Cfg<MODE>::THREADS, 1) gram_i8_kernel(const __
                 tc_fence_after();
                 // straight-line issue: one base descriptor per stage plus
                 // compile-time tile offsets (in 16-byte units, the
-                // descriptor's address field); the first product of each
-                // class in the launch's first stage overwrites its accumulator
+                // descriptor's address field); X digit i meets Y digits j and
+                // j + 1 in one product of 256 columns where both are kept;
+                // the first stage's products with Xr's top digit overwrite
+                // the accumulators of every class
                 const uint64_t d0 = smem_desc(sbase + st * L::STAGE_BYTES);
                 const uint32_t acc0 = k > 0 ? 1u : 0u;
 #pragma unroll
                 for (int i = 0; i < C::XDIG; i++)
 #pragma unroll
-                    for (int j = 0; j < C::YDIG; j++) {
-                        const int cls = i + j;
-                        if (cls > 3) continue;
-                        const bool first = i == (cls - (C::YDIG - 1) > 0 ? cls - (C::YDIG - 1) : 0);
-                        // [Re | Im] += Xr [Yr; -Yi]^T + Xi [Yi; Yr]^T
-                        mma_i8(tmem + acc_col(cls), d0 + (x_tile<MODE>(0, i) >> 4), d0 + (y_tile<MODE>(0, j) >> 4),
-                               id, first ? acc0 : 1u);
-                        mma_i8(tmem + acc_col(cls), d0 + (x_tile<MODE>(1, i) >> 4), d0 + (y_tile<MODE>(1, j) >> 4),
-                               id, 1u);
-                    }
+                    for (int part = 0; part < 2; part++)
+#pragma unroll
+                        for (int j = 0; j <= 3 - i; j += 2)
+                            mma_i8(tmem + acc_col(i + j), d0 + (x_tile<MODE>(part, i) >> 4),
+                                   d0 + (y_tile<MODE>(2 * part, j) >> 4), j < 3 - i ? id2 : id,
+                                   i == 0 && part == 0 ? acc0 : 1u);
                 mma_commit(&empty_bar[st]);  // stage free once these MMAs have read it
             }
             mma_commit(&done_bar);
@@ -906,7 +914,7 @@ __global__ void __launch_bounds__(TT) phasor_table_kernel(const __grid_constant_
 #pragma unroll
         for (int i = t; i < NH * (PH_ROW / 16); i += TT) {
             const int rr = i / (PH_ROW / 16), uu = i % (PH_ROW / 16);
-            *reinterpret_cast<float4*>(pdst + (size_t)rr * PH_ROW + uu * 16) =
+            *reinterpret_cast<float4*>(pdst + (size_t)((rr >> 3) * 2 + (uu >> 3)) * 1024 + (uu & 1) * 512 + ((rr & 7) * 4 + ((uu >> 1) & 3)) * 16) =
                 *reinterpret_cast<const float4*>(phs + rr * TROW + uu * 16);
         }
     }
