@@ -20,9 +20,9 @@
 // sweep and tables) and, level with it, shared-memory reads (96 bytes a lane
 // and component of the four pairs, 128 bytes a clock).  128 tiles x 384
 // channels x 1000 points: 13.2 ms with a thread per baseline, 4.3 with the
-// library's sincospi, 4.0 so; 1 x 2 pairs a thread 4.3, 4 x 2 at half the
-// warps 4.8.  Every value is FP64,
-// tile positions are taken from the array's centroid (so a tile's phase is no
+// library's sincospi, 4.0 with this kernel's polynomials (1 x 2 pairs a thread
+// 4.3, 4 x 2 at half the warps 4.8), 3.7 with a diagonal block's two half-full
+// quarters summed as one.  Every value is FP64, tile positions are taken from the array's centroid (so a tile's phase is no
 // larger than its baselines'), and sums run over the components in order.
 // The drop-in calls keep the per-baseline kernel (predict.cu): their UVWs
 // are the caller's and need not be tile differences.
@@ -119,7 +119,7 @@ __device__ __forceinline__ cplx shapelet_env(const double* __restrict__ cm, doub
 // else in FP64 (error's p99.9 3.4e-7 with FP32 phasors and left operands,
 // 2.6e-7 so).  128 tiles x 192 channels x 250 Gaussians, 17 unique tiles: 2.37
 // ms with a thread per baseline (phasors and records of 17 tiles gathered from
-// shared memory per term), 1.95 so, the FP64 pipe 0.61 busy.
+// shared memory per term), 1.84 so, the FP64 pipe 0.61 busy.
 template <int TYPE, bool TILE, bool OUT64, bool FAST>
 __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
     constexpr int CH = Shape<TYPE, TILE>::CH;
@@ -159,16 +159,20 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
     // beams need both M and N)
     const bool same = !TILE && pb == qb;
 
-    // pairs of this thread: rows tr + 16 i, columns tc + 16 j.  want[h][j] is
-    // uniform over the CTA: false where no pair of that 16 x 16 quarter is a
-    // baseline.
-    const int tr = pb * TB + (tid >> 4), tc = qb * TB + (tid & 15);
+    // pairs of this thread: rows tr + 16 i, columns tc + 16 j.
+    // want[i][j] is uniform over the CTA: false where no pair of that 16 x 16
+    // quarter is a baseline.  A diagonal block's two diagonal quarters hold
+    // half as many each: they are one quarter's work, quarter (0, 0), whose
+    // threads below the diagonal take the mirrored pair of quarter (1, 1).
+    const int tr = tid >> 4, tc = tid & 15;
     bool want[2][2];
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int j = 0; j < 2; j++)
-            want[i][j] = pb * TB + 16 * i < p.ntiles && qb * TB + 16 * j < p.ntiles && !(pb == qb && i > j);
+            want[i][j] = pb * TB + 16 * i < p.ntiles && qb * TB + 16 * j < p.ntiles && !(pb == qb && i == 1);
+    const bool mirror = pb == qb && tr > tc;
+    const int r00 = mirror ? 16 + tc : tr, c00 = mirror ? 16 + tr : tc;
     const bool full = want[0][0] && want[0][1] && want[1][0] && want[1][1];
 
     const int nchunks = (p.nc + CH - 1) / CH;
@@ -264,11 +268,12 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
             for (int c = 0; c < n; c++) {
 #pragma unroll
                 for (int i = 0; i < RI; i++) {
-                    const int rp = (tid >> 4) + 16 * i;
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
-                        if (!decltype(all)::value && !want[i][j]) continue;
-                        const int cq = TB + (tid & 15) + 16 * j;
+                        constexpr bool ALL = decltype(all)::value;
+                        if (!ALL && !want[i][j]) continue;
+                        const int rp = !ALL && i + j == 0 ? r00 : tr + 16 * i;
+                        const int cq = TB + (!ALL && i + j == 0 ? c00 : tc + 16 * j);
                         cplx env = {1.0, 0.0};
                         if (TYPE) {
                             const double2 kp = s_k[TYPE ? c : 0][TYPE ? rp : 0], kq = s_k[TYPE ? c : 0][TYPE ? cq : 0];
@@ -339,8 +344,8 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
     for (int i = 0; i < RI; i++)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const int tp = tr + 16 * i, tq = tc + 16 * j;
-            if (tp >= tq || tq >= p.ntiles) continue;
+            const int tp = pb * TB + (i + j == 0 ? r00 : tr + 16 * i), tq = qb * TB + (i + j == 0 ? c00 : tc + 16 * j);
+            if (!want[i][j] || tp >= tq || tq >= p.ntiles) continue;
             const cplx(&m)[4] = acc[i][j];
             J2 r;
             if (TILE)

@@ -592,7 +592,7 @@ static cudaError_t launch_fast_shapelet(const DirectParams& p, cudaStream_t s) {
 // Four channels share the gathered basis records: 2 channels x 16 components
 // a chunk 5.4 ms, 4 x 8 4.6 ms, bit-identical (17 unique tiles, one timestep,
 // 128 tiles, 384 channels).  The tile-factored FP64 form (pairs.cu), which
-// evaluates the basis per pair and channel, takes 1.80 ms where this one takes
+// evaluates the basis per pair and channel, takes 1.8 ms where this one takes
 // 1.07 (50 shapelets, 128 tiles, 192 channels).
 constexpr int FT_FCH = 4;      // channels per thread
 constexpr int FT_CH = 8;       // components per staged chunk
@@ -826,8 +826,8 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
            (!tile_beam || (ty != 0 && p.n_uniq_tile > 0 && p.n_uniq_tile <= FT_MAX_NU && !p.unflagged_map));
     if (fast && ty == 2 && p.sdense && !p.sbfp) return cudaErrorInvalidValue;
     // UVWs that are tile differences: the FP64 form factored by tile (128
-    // tiles x 384 channels: 1000 points 13.2 -> 4.0 ms, 120 Gaussians 2.35 ->
-    // 1.32 ms, 24 shapelets 4.52 -> 1.40 ms).  Shapelets with an order of SDN
+    // tiles x 384 channels: 1000 points 13.2 -> 3.7 ms, 120 Gaussians 2.35 ->
+    // 1.22 ms, 24 shapelets 4.52 -> 1.29 ms).  Shapelets with an order of SDN
     // or more keep the per-baseline kernel, which reads the basis table per
     // coefficient.
     if (!fast && p.xyzs && (ty != 2 || p.sdense64)) return launch_pairs(ty, tile_beam, out64, p, s);
