@@ -163,11 +163,15 @@ __global__ void trace_kernel(const JonesF32* __restrict__ resid, const float* __
 
 // A sweep's block of tile pairs: rows 32 pb .., columns 32 qb .. (blocks on
 // or above the diagonal); 256 threads of 2 x 2 pairs, rows and columns 16
-// apart.
+// apart.  On the diagonal a thread has two pairs, (row 0, col 0) and (row 1,
+// col 1): one of the two half-full diagonal quarters' (below the diagonal of
+// the first, the pair (31 - row, 31 - column) of the other) and one of the full
+// quarter's.  Four pairs there as well: apply 1.18 ms, two 1.00.
 constexpr int TB = 32, NTH = 256;
 struct PairBlock {
-    int pb, qb, rp, cq;  // this thread's first row and column slot (columns after the TB rows)
-    int bl[4];           // baselines of the pairs (row 0 col 0, row 0 col 1, ..), -1 where none
+    int pb, qb;
+    int r[2], c[2];  // this thread's row and column slots (columns after the TB rows)
+    int bl[4];       // baselines of the pairs (row 0 col 0, row 0 col 1, ..), -1 where none
 };
 __device__ __forceinline__ PairBlock pair_block(int blk, int ntiles) {
     PairBlock B;
@@ -176,12 +180,16 @@ __device__ __forceinline__ PairBlock pair_block(int blk, int ntiles) {
         baseline_to_tiles(blk, nblk, B.pb, B.qb);
     else
         B.pb = B.qb = blk - noff;
-    B.rp = threadIdx.x >> 4;
-    B.cq = TB + (threadIdx.x & 15);
+    const int a = threadIdx.x >> 4, b = threadIdx.x & 15;
+    const bool diag = B.pb == B.qb, mirror = diag && a > b;
+    B.r[0] = mirror ? 31 - a : a;
+    B.c[0] = TB + (mirror ? 31 - b : b);
+    B.r[1] = diag ? a : a + 16;
+    B.c[1] = TB + b + 16;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int p = B.pb * TB + B.rp + 16 * (i >> 1), q = B.qb * TB + B.cq - TB + 16 * (i & 1);
-        B.bl[i] = p < q && q < ntiles ? baseline_index(p, q, ntiles) : -1;
+        const int p = B.pb * TB + B.r[i >> 1], q = (B.qb - 1) * TB + B.c[i & 1];
+        B.bl[i] = p < q && q < ntiles && !(diag && (i == 1 || i == 2)) ? baseline_index(p, q, ntiles) : -1;
     }
     return B;
 }
@@ -225,7 +233,7 @@ __device__ __forceinline__ JF load_jf(const JonesF32& j) {
     return JF{{make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)}};
 }
 
-// The accumulate sweep: traces of D_s and Mr_s of G sources (from blockIdx.z
+// The accumulate sweep: traces of D_s and Mr_s of G sources (from blockIdx.x
 // G) at the block's pairs and one low-resolution channel.  The tables of
 // NSAMP samples are copied while the previous ones are used; a sample and
 // source cost a pair two packed products for the two phasors and seven
@@ -234,13 +242,14 @@ __device__ __forceinline__ JF load_jf(const JonesF32& j) {
 // Bound: issue slots (about 60 % busy at 16 warps an SM, the residual's loads
 // read one sample ahead).  30 sources, 8 timesteps x 384 channels x 8128
 // baselines: 3.5 ms with all four correlations and a thread per baseline and
-// source, 1.16 ms so.
+// source, 1.16 ms with the groups of sources as the grid's slowest index, 1.13
+// as its fastest (a group finds the residual in L2).
 constexpr int NSAMP = 4;
 template <bool POINTS, int G>
 __global__ void __launch_bounds__(NTH, 2) accumulate_kernel(const SweepArgs A) {
     __shared__ alignas(16) float4 s_tab[2][NSAMP][G][2 * TB];
-    const PairBlock B = pair_block(blockIdx.x, A.ntiles);
-    const int flo = blockIdx.y, nlo = A.nf / A.favg, s0 = blockIdx.z * G;
+    const PairBlock B = pair_block(blockIdx.y, A.ntiles);
+    const int flo = blockIdx.z, nlo = A.nf / A.favg, s0 = blockIdx.x * G;
     const int ng = min(G, A.nsrc - s0), nsamp = A.nt * A.favg;
     const size_t nvis = (size_t)A.nt * A.nf * A.nbl, ntf = (size_t)A.nt * A.nf;
     // samples in order: timestep, then channel of the group; tf = t nf + f
@@ -321,9 +330,8 @@ __global__ void __launch_bounds__(NTH, 2) accumulate_kernel(const SweepArgs A) {
                     gm *= m.x + m.y;
                 }
                 const float4(&tab)[2 * TB] = s_tab[buf][k][j];
-                const float4 p[2] = {tab[B.rp], tab[B.rp + 16]}, q[2] = {tab[B.cq], tab[B.cq + 16]};
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
+                const float4 p[2] = {tab[B.r[0]], tab[B.r[1]]}, q[2] = {tab[B.c[0]], tab[B.c[1]]};
+                auto pair = [&](int i) {
                     uint64_t re2, im2;
                     pair_phasors(p[i >> 1], q[i & 1], re2, im2);
                     const float2 re = unpack2(re2), im = unpack2(im2);  // rotation, ionosphere
@@ -340,7 +348,10 @@ __global__ void __launch_bounds__(NTH, 2) accumulate_kernel(const SweepArgs A) {
                         sm[i][j].x = fmaf(cm.x, re.y, fmaf(-cm.y, im.y, sm[i][j].x));
                         sm[i][j].y = fmaf(cm.x, im.y, fmaf(cm.y, re.y, sm[i][j].y));
                     }
-                }
+                };
+                pair(0);
+                pair(3);
+                if (B.pb != B.qb) pair(1), pair(2);
             }
         }
         __syncthreads();
@@ -368,7 +379,7 @@ __global__ void __launch_bounds__(NTH, 2) accumulate_kernel(const SweepArgs A) {
 // and b z give XY = P + i Q, YX = P - i Q.  The tables of SCHUNK sources are
 // copied while the previous ones are used, across rows.
 // Bound: issue slots and, below them, the residual's two passes over memory
-// (0.3 ms).  The same problem: 2.97 ms with a thread per baseline, 1.18 ms so.
+// (0.3 ms).  The same problem: 2.97 ms with a thread per baseline, 1.00 ms so.
 constexpr int SCHUNK = 16, TFS = 8;
 template <bool POINTS>
 __global__ void __launch_bounds__(NTH, 2) apply_kernel(const SweepArgs A, bool next) {
@@ -418,15 +429,14 @@ __global__ void __launch_bounds__(NTH, 2) apply_kernel(const SweepArgs A, bool n
             const float4 gn = s_g[st & 1][j];
             if (gn.z != 0.f) continue;  // its constants did not change
             const float4(&tab)[2 * TB] = s_tab[st & 1][j];
-            const float4 p[2] = {tab[B.rp], tab[B.rp + 16]}, q[2] = {tab[B.cq], tab[B.cq + 16]};
+            const float4 p[2] = {tab[B.r[0]], tab[B.r[1]]}, q[2] = {tab[B.c[0]], tab[B.c[1]]};
             const uint64_t gg = pack2(gn.x, gn.y);
             uint64_t wm[4];
             if (POINTS) {
                 const float4 m = s_m[st & 1][j];
                 wm[0] = dup2(m.x), wm[1] = dup2(m.y), wm[2] = dup2(m.z), wm[3] = dup2(m.w);
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
+            auto pair = [&](int i) {
                 uint64_t re2, im2;
                 pair_phasors(p[i >> 1], q[i & 1], re2, im2);
                 const float2 re = unpack2(mul2(re2, gg)), im = unpack2(mul2(im2, gg));
@@ -443,7 +453,10 @@ __global__ void __launch_bounds__(NTH, 2) apply_kernel(const SweepArgs A, bool n
                         acc[i][e] = pack2(o.x + c.x, o.y + c.y);
                     }
                 }
-            }
+            };
+            pair(0);
+            pair(3);
+            if (B.pb != B.qb) pair(1), pair(2);
         }
         __syncthreads();
         if (chunk != nch - 1) continue;
@@ -478,7 +491,7 @@ struct Tuning {
 
 template <bool POINTS, int G>
 void launch_acc(const SweepArgs& A, cudaStream_t s) {
-    const dim3 grid(pair_blocks(A.ntiles), A.nf / A.favg, (A.nsrc + G - 1) / G);
+    const dim3 grid((A.nsrc + G - 1) / G, pair_blocks(A.ntiles), A.nf / A.favg);
     accumulate_kernel<POINTS, G><<<grid, NTH, 0, s>>>(A);
     count_launches(1);
 }
