@@ -593,7 +593,7 @@ static cudaError_t launch_fast_shapelet(const DirectParams& p, cudaStream_t s) {
 // a chunk 5.4 ms, 4 x 8 4.6 ms, bit-identical (17 unique tiles, one timestep,
 // 128 tiles, 384 channels).  The tile-factored FP64 form (pairs.cu), which
 // evaluates the basis per pair and channel, takes 1.8 ms where this one takes
-// 1.07 (50 shapelets, 128 tiles, 192 channels).
+// 0.98 (50 shapelets, 128 tiles, 192 channels).
 constexpr int FT_FCH = 4;      // channels per thread
 constexpr int FT_CH = 8;       // components per staged chunk
 constexpr int FT_RECS = FT_FCH * FT_CH;
@@ -601,8 +601,10 @@ constexpr int FT_MAX_NU = 32;  // unique tiles (more: the FP64 per-tile kernel)
 
 inline size_t fast_tile_smem_bytes(int nu) { return (size_t)FT_RECS * nu * 6 * sizeof(float4); }
 
-template <bool OUT64>
-__global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) {
+// MINB: CTAs an SM holds.  Two (128 registers, a few spilled) hide the gathers'
+// latency; one keeps all in registers.
+template <bool OUT64, int MINB>
+__global__ void __launch_bounds__(DT, MINB) fast_tile_kernel(const DirectParams p) {
     constexpr int FCH = FT_FCH;
     constexpr int CH = FT_CH;
     __shared__ alignas(128) double4 s_lmn[2][CH];
@@ -744,24 +746,36 @@ __global__ void __launch_bounds__(DT, 1) fast_tile_kernel(const DirectParams p) 
     }
 }
 
-template <bool OUT64>
-static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
+template <bool OUT64, int MINB>
+static cudaError_t launch_fast_tile(const DirectParams& p, dim3 grid, int dev, cudaStream_t s) {
     const size_t smem = fast_tile_smem_bytes(p.n_uniq_tile);
     // the opt-in above 48 KB of dynamic shared memory, once per device
     static std::atomic<bool> attr[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr[dev].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(fast_tile_kernel<OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)fast_tile_smem_bytes(FT_MAX_NU));
+        const cudaError_t e = cudaFuncSetAttribute(fast_tile_kernel<OUT64, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)fast_tile_smem_bytes(FT_MAX_NU));
         if (e != cudaSuccess) return e;
         attr[dev].store(true, std::memory_order_relaxed);
     }
-    const dim3 grid((p.nbl + DT - 1) / DT, (p.nf + FT_FCH - 1) / FT_FCH);
-    fast_tile_kernel<OUT64><<<grid, DT, smem, s>>>(p);
+    fast_tile_kernel<OUT64, MINB><<<grid, DT, smem, s>>>(p);
     return cudaSuccess;
+}
+
+// Two CTAs an SM where there are more CTAs than SMs and the records leave the
+// L1 cache room (50 shapelets, 128 tiles x 192 channels: 17 unique tiles 1.23
+// -> 1.08 ms with host work, 26 1.29 -> 1.19, 32 1.26 -> 1.28); else one (32
+// CTAs, 40 tiles x 32 channels x 20 shapelets: 123 us against 130).
+constexpr int FT_TWO_NU = 28;
+template <bool OUT64>
+static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    const dim3 grid((p.nbl + DT - 1) / DT, (p.nf + FT_FCH - 1) / FT_FCH);
+    if (p.n_uniq_tile <= FT_TWO_NU && (long long)grid.x * grid.y > sms) return launch_fast_tile<OUT64, 2>(p, grid, dev, s);
+    return launch_fast_tile<OUT64, 1>(p, grid, dev, s);
 }
 
 template <int TYPE>

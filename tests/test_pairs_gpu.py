@@ -99,6 +99,22 @@ def test_chosen_form_per_tile(oracle, kind, ntiles, n):
         assert np.linalg.norm(got - ref) < 1e-6 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("nuniq", [28, 29])
+def test_shapelets_per_tile_either_side_of_the_rule(nuniq):
+    """More CTAs than an SM each: two share one up to 28 unique tiles."""
+    ntiles, nf = 128, 48
+    obs = synth.Obs(synth.tiles_in_disk(ntiles, 750.0, 4), 167e6 + np.arange(nf) * 40e3, PC, np.array([LST]))
+    sky = sl.SkyModelArrays.from_components(components("shapelets", 9, 11))
+    gains = np.random.default_rng(9).uniform(0.5, 1.0, (nuniq, 2, 16))[np.arange(ntiles) % nuniq]
+    vis = {}
+    for form in ("direct", "tensor"):
+        m = SkyModeller(sky, obs.tile_xyzs, obs.freqs, PC, obs.latitude, form=form, beam="per_tile", dipole_gains=gains)
+        vis[form] = torch.zeros((nf, obs.num_baselines, 8), dtype=torch.float64, device="cuda")
+        m.model_timestep_with(LST, vis[form])
+        m.close()
+    assert torch.linalg.norm(vis["tensor"] - vis["direct"]) < 1e-6 * torch.linalg.norm(vis["direct"])
+
+
 def test_points_per_tile_in_chunks_of_channels():
     """More components than a pass takes and a table that exceeds its cap, so
     that channels go through it in turn, against the FP64 form."""
