@@ -720,9 +720,8 @@ int Modeller::model_channels(double lst, void* d_vis, bool out64, int f0, int nf
                                                 tensor_sync());
             if (rc) return rc;
         } else {
-            // the chosen (tensor) form keeps Gaussians and shapelets in the
-            // direct kernel, in its FP32 form with a shared beam (FP64 with
-            // per-tile beams)
+            // Gaussians and shapelets: the chosen (tensor) form's own kernels,
+            // or the FP64 form's
             DirectParams p = direct_params(ty, vis);
             set_tile_geometry(p, lst);
             p.nf = nfc;

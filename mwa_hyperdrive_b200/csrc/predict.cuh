@@ -121,9 +121,8 @@ struct TensorBeam {
     int n_uniq_freq;
 };
 
-// A second stream and its events, with which the tensor predict of a shared
-// beam writes the next chunk's table while the Gram kernel of the current
-// chunk runs (two tables in the workspace).  One per caller: not shared
+// A second stream and its events, with which the tensor predict writes the
+// next chunk's table while the Gram kernel of the current chunk runs (two tables in the workspace).  One per caller: not shared
 // between concurrent calls.
 struct TensorSync {
     cudaStream_t ts = nullptr;
