@@ -99,18 +99,20 @@ cudaError_t launch_pairs(int ty, bool tile_beam, bool out64, const DirectParams&
 // per tile with FP64 products); p.xyzs and p.gk set.
 cudaError_t launch_fast_gauss(bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s);
 
-// Launch the direct kernel for component type ty (0 point, 1 Gaussian,
-// 2 shapelet).  tile_beam selects per-tile beam Jones; out64 an FP64 output;
-// fast the FP32 form (errors ~1e-7 of the visibility; shared beam only).
+// Predict component type ty (0 point, 1 Gaussian, 2 shapelet) with the kernel
+// that its geometry and beam allow.  tile_beam selects per-tile beam Jones;
+// out64 an FP64 output; fast the chosen form's Gaussians and shapelets (errors
+// ~1e-7 of the visibility).
 cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams& p, cudaStream_t s,
                           bool fast = false);
+
+// components of a TensorBeam::beam32 row (pairs are read in one aligned load)
+__host__ __device__ inline size_t beam32_row(int nc) { return ((size_t)nc + 1) & ~(size_t)1; }
 
 // Per-tile beams for the tensor-core predict: beam [n_uniq_tile]
 // [n_uniq_freq][nc] (the reference's layout), the unique row of every tile
 // (any unflagged-tile map already applied) and the unique column of every
 // channel of the launch.
-// components of a TensorBeam::beam32 row (pairs are read in one aligned load)
-__host__ __device__ inline size_t beam32_row(int nc) { return ((size_t)nc + 1) & ~(size_t)1; }
 struct TensorBeam {
     const JonesF64* beam;
     const float4* beam32;  // its rows in FP32 (the producers' reads), or NULL: [unique tile][unique
