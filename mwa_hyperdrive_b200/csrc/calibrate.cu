@@ -37,6 +37,7 @@
 // relative); all arithmetic is FP64.
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -973,20 +974,32 @@ static size_t smem_bytes(int n, int form) {
     return smem_base_bytes(n, form) + (r ? 16 + r * RING_SLOT : 0);
 }
 
+// The iteration kernel's opt-in to the dynamic shared memory that any tile
+// count needs, once per device: calls on several threads have tile counts of
+// their own, and an attribute set for one would have another's launch refused.
 template <int FORM>
-static int launch_mitchcal_form(const CalParams& P, int nblocks, cudaStream_t s) {
-    const size_t sm = smem_bytes(P.ntiles, FORM);
+static int opt_in_smem() {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    HDC_CUDA_RET_INT(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return HDC_OK;
+    size_t most = 0;
+    for (int n = 2; n <= CT; n++) most = std::max(most, smem_bytes(n, FORM));
     HDC_CUDA_RET_INT(
-        cudaFuncSetAttribute(mitchcal_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    mitchcal_kernel<FORM><<<nblocks, cal_threads(FORM), sm, s>>>(P);
-    count_launches(1);
-    HDC_CUDA_RET_INT(cudaGetLastError());
+        cudaFuncSetAttribute(mitchcal_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return HDC_OK;
 }
 
-// Launch without setting the shared-memory attribute (inside a stream
-// capture, after prepare_mitchcal has set it).
-static void launch_mitchcal_captured(const CalParams& P, int form, int nblocks, cudaStream_t s) {
+static int prepare_mitchcal(int form) {
+    if (form == HDC_CAL_COLLAPSED) return opt_in_smem<1>();
+    if (form == HDC_CAL_COLLAPSED_F32) return opt_in_smem<2>();
+    return opt_in_smem<0>();
+}
+
+// Launch the iterations of nblocks chanblocks; prepare_mitchcal has run (before
+// a stream capture, if one is under way).
+static int launch_mitchcal(const CalParams& P, int form, int nblocks, cudaStream_t s) {
     const size_t sm = smem_bytes(P.ntiles, form);
     if (form == HDC_CAL_COLLAPSED)
         mitchcal_kernel<1><<<nblocks, cal_threads(1), sm, s>>>(P);
@@ -995,16 +1008,7 @@ static void launch_mitchcal_captured(const CalParams& P, int form, int nblocks, 
     else
         mitchcal_kernel<0><<<nblocks, cal_threads(0), sm, s>>>(P);
     count_launches(1);
-}
-
-static int prepare_mitchcal(int ntiles, int form) {
-    const int sm = (int)smem_bytes(ntiles, form);
-    if (form == HDC_CAL_COLLAPSED)
-        HDC_CUDA_RET_INT(cudaFuncSetAttribute(mitchcal_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    else if (form == HDC_CAL_COLLAPSED_F32)
-        HDC_CUDA_RET_INT(cudaFuncSetAttribute(mitchcal_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    else
-        HDC_CUDA_RET_INT(cudaFuncSetAttribute(mitchcal_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    HDC_CUDA_RET_INT(cudaGetLastError());
     return HDC_OK;
 }
 
@@ -1013,13 +1017,15 @@ __global__ void identity_kernel(JonesF64* dj, size_t n) {
     if (i < n) dj[i] = JonesF64{1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0};
 }
 
-static void launch_collapse(const CalParams& P, int form, void* cov, int nblocks, cudaStream_t s) {
+static int launch_collapse(const CalParams& P, int form, void* cov, int nblocks, cudaStream_t s) {
     const dim3 grid(2 * P.nblk, nblocks);
     if (form == HDC_CAL_COLLAPSED)
         collapse_kernel<double><<<grid, BLK / 2, 0, s>>>(P, static_cast<double*>(cov));
     else
         collapse_kernel<float><<<grid, BLK / 2, 0, s>>>(P, static_cast<float*>(cov));
     count_launches(1);
+    HDC_CUDA_RET_INT(cudaGetLastError());
+    return HDC_OK;
 }
 
 // A non-blocking stream per device on which the multi-timeblock graph is
@@ -1073,25 +1079,25 @@ struct PlainCov {
     }
     PlainCov(const PlainCov&) = delete;
     PlainCov& operator=(const PlainCov&) = delete;
-    // the group launches of nblocks chanblocks (P.chan_list's, or all)
-    void launch(CalParams P, int nblocks, cudaStream_t st) const {
+    // the iterations of nblocks chanblocks (P.chan_list's, or all) of `form`:
+    // in groups over the scratch where this holds some
+    int launch(CalParams P, int form, int nblocks, cudaStream_t st) const {
+        if (!group) return launch_mitchcal(P, form, nblocks, st);
         P.cov = p;
         P.cov_by_block = 1;
         P.nring = 0;
         for (int c = 0; c < nblocks; c += group) {
             const int n = std::min(group, nblocks - c);
             P.ch0 = c;
-            launch_collapse(P, HDC_CAL_COLLAPSED, p, n, st);
-            launch_mitchcal_captured(P, HDC_CAL_COLLAPSED, n, st);
+            int rc = launch_collapse(P, HDC_CAL_COLLAPSED, p, n, st);
+            if (!rc) rc = launch_mitchcal(P, HDC_CAL_COLLAPSED, n, st);
+            if (rc) return rc;
         }
+        return HDC_OK;
     }
+    // what launch() needs before it (and before a stream capture)
+    int prepare(int form) const { return prepare_mitchcal(group ? HDC_CAL_COLLAPSED : form); }
 };
-
-static int launch_mitchcal(const CalParams& P, int form, int nblocks, cudaStream_t s) {
-    if (form == HDC_CAL_COLLAPSED) return launch_mitchcal_form<1>(P, nblocks, s);
-    if (form == HDC_CAL_COLLAPSED_F32) return launch_mitchcal_form<2>(P, nblocks, s);
-    return launch_mitchcal_form<0>(P, nblocks, s);
-}
 
 // Grow-only per-device buffer for the collapsed covariances.
 static std::mutex g_cov_mu;
@@ -1149,17 +1155,16 @@ static int retry_failed(CalParams P, int form, const PlainCov& pcov, std::vector
             for (int c = 0; c < P.nchan; c++)
                 if (!res[c].converged) list.push_back(c);
             if (!pairs.empty()) {
-                cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, s);
+                HDC_CUDA_RET_INT(
+                    cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, s));
                 retry_seed_kernel<<<(P.ntiles + 127) / 128, 128, 0, s>>>(P.di_jones, P.nchan, P.ntiles, d_pairs,
                                                                         (int)pairs.size());
                 count_launches(1);
+                HDC_CUDA_RET_INT(cudaGetLastError());
             }
-            cudaMemcpyAsync(d_list, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, s);
+            HDC_CUDA_RET_INT(cudaMemcpyAsync(d_list, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, s));
             P.chan_list = d_list;
-            if (pcov.group)
-                pcov.launch(P, (int)list.size(), s);
-            else
-                rc = launch_mitchcal(P, form, (int)list.size(), s);
+            rc = pcov.launch(P, form, (int)list.size(), s);
             if (rc) return rc;
             if (cudaMemcpyAsync(res.data(), P.results, sizeof(HdcCalResult) * P.nchan, cudaMemcpyDeviceToHost,
                                 s) != cudaSuccess ||
@@ -1247,11 +1252,10 @@ static int calibrate_timeblock_impl(const JonesF32* d_data_tfb, const JonesF32* 
             return HDC_ERR_ALLOC;
         }
         P.cov = cov;
-        launch_collapse(P, form, cov, num_chanblocks, s);
-        if (cudaGetLastError() != cudaSuccess) {
+        rc = launch_collapse(P, form, cov, num_chanblocks, s);
+        if (rc) {
             cleanup();
-            set_error("hdc_calibrate_timeblock: collapse launch failed");
-            return HDC_ERR_CUDA;
+            return rc;
         }
     }
     int nblocks = num_chanblocks;
@@ -1276,16 +1280,8 @@ static int calibrate_timeblock_impl(const JonesF32* d_data_tfb, const JonesF32* 
         nblocks = num_listed;
     }
     const PlainCov pcov(form, nblocks, P.nblk, s);
-    if (pcov.group) {
-        rc = prepare_mitchcal(ntiles, HDC_CAL_COLLAPSED);
-        if (!rc) pcov.launch(P, nblocks, s);
-        if (!rc && cudaPeekAtLastError() != cudaSuccess) {
-            set_error("hdc_calibrate_timeblock: %s", cudaGetErrorString(cudaGetLastError()));
-            rc = HDC_ERR_CUDA;
-        }
-    } else {
-        rc = launch_mitchcal(P, form, nblocks, s);
-    }
+    rc = pcov.prepare(form);
+    if (!rc) rc = pcov.launch(P, form, nblocks, s);
     if (rc) {
         cleanup();
         return rc;
@@ -1409,8 +1405,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         }
     }
     const PlainCov pcov(form, num_chanblocks, nblk, s);
-    int rc = prepare_mitchcal(ntiles, form);
-    if (!rc && pcov.group) rc = prepare_mitchcal(ntiles, HDC_CAL_COLLAPSED);
+    int rc = pcov.prepare(form);
     cudaStream_t cs = capture_stream();
     if (rc || !cs) {
         cleanup();
@@ -1441,19 +1436,18 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
     };
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        for (int k = 0; k < num_timeblocks; k++) {
+        for (int k = 0; k < num_timeblocks && !rc; k++) {
             const CalParams P = params(k);
             identity_kernel<<<(unsigned)((nsol + 255) / 256), 256, 0, cs>>>(P.di_jones, nsol);
             count_launches(1);
-            if (form != HDC_CAL_PLAIN) launch_collapse(P, form, cov, num_chanblocks, cs);
-            if (pcov.group)
-                pcov.launch(P, num_chanblocks, cs);
-            else
-                launch_mitchcal_captured(P, form, num_chanblocks, cs);
+            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov, num_chanblocks, cs);
+            if (!rc) rc = pcov.launch(P, form, num_chanblocks, cs);
         }
-        const cudaError_t le = cudaGetLastError();
         e = cudaStreamEndCapture(cs, &graph);
-        if (e == cudaSuccess) e = le;
+        if (rc) {
+            cleanup();
+            return rc;
+        }
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (e == cudaSuccess) e = cudaGraphLaunch(exec, s);
@@ -1478,8 +1472,8 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         for (auto& r : rk) conv += r.converged;
         if (conv > 0 && conv != num_chanblocks) {
             const CalParams P = params(k);
-            if (form != HDC_CAL_PLAIN) launch_collapse(P, form, cov, num_chanblocks, s);  // this timeblock's covariances
-            rc = retry_failed(P, form, pcov, rk, d_list, d_pairs, s);
+            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov, num_chanblocks, s);  // this timeblock's covariances
+            if (!rc) rc = retry_failed(P, form, pcov, rk, d_list, d_pairs, s);
             if (rc) {
                 cleanup();
                 return rc;
