@@ -1029,12 +1029,12 @@ static int launch_collapse(const CalParams& P, int form, void* cov, int nblocks,
 }
 
 // A non-blocking stream per device on which the multi-timeblock graph is
-// captured (capture is not possible on the legacy default stream).
+// captured (capture is not possible on the legacy default stream); a caller
+// holds g_cs_mu from capture_stream() to the end of its capture.
 static std::mutex g_cs_mu;
 static cudaStream_t g_cs[16] = {nullptr};
 
 static cudaStream_t capture_stream() {
-    std::lock_guard<std::mutex> lk(g_cs_mu);
     int d = 0;
     if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 16) return nullptr;
     if (!g_cs[d] && cudaStreamCreateWithFlags(&g_cs[d], cudaStreamNonBlocking) != cudaSuccess) {
@@ -1406,6 +1406,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
     }
     const PlainCov pcov(form, num_chanblocks, nblk, s);
     int rc = pcov.prepare(form);
+    std::unique_lock<std::mutex> capturing(g_cs_mu);
     cudaStream_t cs = capture_stream();
     if (rc || !cs) {
         cleanup();
@@ -1444,6 +1445,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
             if (!rc) rc = pcov.launch(P, form, num_chanblocks, cs);
         }
         e = cudaStreamEndCapture(cs, &graph);
+        capturing.unlock();
         if (rc) {
             cleanup();
             return rc;

@@ -1,6 +1,7 @@
 """Calibrations of arrays of different sizes on several host threads: the
 kernel's shared-memory opt-in is one per device, so a small array's call must
-not have a large one's retry launch refused (csrc/calibrate.cu, opt_in_smem)."""
+not have a large one's retry launch refused (csrc/calibrate.cu, opt_in_smem),
+and the stream on which calls capture their graphs is one per device too."""
 
 import threading
 
@@ -75,3 +76,19 @@ def test_retry_beside_smaller_arrays():
     for dj, c in beside(large, [problem(n, 1, 3) for n in (5, 9, 17)], solve, 40):
         assert c == counts
         np.testing.assert_array_equal(dj, want)
+
+
+def solve_timeblocks(p, stream):
+    data, model, _ = p
+    out, results = cal.calibrate_timeblocks(data, model, [(t, t + 1) for t in range(data.shape[0])], 24, 1e-8, 1e-4,
+                                            stream=stream)
+    return out, [[(r.num_iterations, r.converged) for r in tb] for tb in results]
+
+
+def test_graphs_beside_each_other():
+    large = problem(60, 3, 5)
+    torch.cuda.synchronize()
+    want, counts = solve_timeblocks(large, torch.cuda.Stream())
+    for out, c in beside(large, [problem(n, 2, 3) for n in (5, 9, 17)], solve_timeblocks, 60):
+        assert c == counts
+        np.testing.assert_array_equal(out, want)
