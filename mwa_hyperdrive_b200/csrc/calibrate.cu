@@ -1099,30 +1099,42 @@ struct PlainCov {
     int prepare(int form) const { return prepare_mitchcal(group ? HDC_CAL_COLLAPSED : form); }
 };
 
-// Grow-only per-device buffer for the collapsed covariances.
-static std::mutex g_cov_mu;
+// The collapsed forms' covariances: a grow-only buffer per device, which a call
+// has to itself until it returns (calls of other threads, on other streams,
+// wait for it).
+static std::mutex g_cov_mu[16];
 static void* g_cov[16] = {nullptr};
 static size_t g_cov_size[16] = {0};
 
-static void* covariance_buffer(size_t bytes) {
-    std::lock_guard<std::mutex> lk(g_cov_mu);
-    int d = 0;
-    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 16) return nullptr;
-    if (g_cov_size[d] < bytes) {
-        if (g_cov[d]) {
-            cudaDeviceSynchronize();  // queued work may still read the old buffer
+struct Covariances {
+    std::unique_lock<std::mutex> lock;
+    void* p = nullptr;
+    cudaStream_t s = nullptr;
+    bool alloc(size_t bytes, cudaStream_t st) {
+        int d = 0;
+        if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 16) return false;
+        lock = std::unique_lock<std::mutex>(g_cov_mu[d]);
+        if (g_cov_size[d] < bytes) {
             cudaFree(g_cov[d]);
             g_cov[d] = nullptr;
             g_cov_size[d] = 0;
+            if (cudaMalloc(&g_cov[d], bytes) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            g_cov_size[d] = bytes;
         }
-        if (cudaMalloc(&g_cov[d], bytes) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        g_cov_size[d] = bytes;
+        p = g_cov[d];
+        s = st;
+        return true;
     }
-    return g_cov[d];
-}
+    ~Covariances() {
+        if (p) cudaStreamSynchronize(s);  // nothing of this call reads it any more (a call that failed may not have waited)
+    }
+    Covariances() = default;
+    Covariances(const Covariances&) = delete;
+    Covariances& operator=(const Covariances&) = delete;
+};
 
 // Retry failed chanblocks from interpolated neighbours (mod.rs:468-614):
 // res holds the first pass's results (read back); P.results/P.di_jones point
@@ -1243,16 +1255,16 @@ static int calibrate_timeblock_impl(const JonesF32* d_data_tfb, const JonesF32* 
     P.nblk = cov_blocks(ntiles);
     P.nring = ring_depth(ntiles, form);
     P.err = device_error_word();
+    Covariances cov;
     if (form != HDC_CAL_PLAIN) {
         const size_t elem = form == HDC_CAL_COLLAPSED ? sizeof(double) : sizeof(float);
-        void* cov = covariance_buffer(elem * NCOV * BLK * (size_t)num_chanblocks * P.nblk);
-        if (!cov) {
+        if (!cov.alloc(elem * NCOV * BLK * (size_t)num_chanblocks * P.nblk, s)) {
             cleanup();
             set_error("hdc_calibrate_timeblock: covariance allocation failed");
             return HDC_ERR_ALLOC;
         }
-        P.cov = cov;
-        rc = launch_collapse(P, form, cov, num_chanblocks, s);
+        P.cov = cov.p;
+        rc = launch_collapse(P, form, cov.p, num_chanblocks, s);
         if (rc) {
             cleanup();
             return rc;
@@ -1392,13 +1404,12 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         set_error("hdc_calibrate_timeblocks: device allocation failed");
         return HDC_ERR_ALLOC;
     }
-    void* cov = nullptr;
+    Covariances cov;
     const int nblk = cov_blocks(ntiles), nring = ring_depth(ntiles, form);
     int* errw = device_error_word();
     if (form != HDC_CAL_PLAIN) {
         const size_t elem = form == HDC_CAL_COLLAPSED ? sizeof(double) : sizeof(float);
-        cov = covariance_buffer(elem * NCOV * BLK * (size_t)num_chanblocks * nblk);
-        if (!cov) {
+        if (!cov.alloc(elem * NCOV * BLK * (size_t)num_chanblocks * nblk, s)) {
             cleanup();
             set_error("hdc_calibrate_timeblocks: covariance allocation failed");
             return HDC_ERR_ALLOC;
@@ -1429,7 +1440,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         P.min_thr = min_threshold;
         P.pols = pols;
         P.results = d_res + (size_t)k * num_chanblocks;
-        P.cov = cov;
+        P.cov = cov.p;
         P.nblk = nblk;
         P.nring = nring;
         P.err = errw;
@@ -1441,7 +1452,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
             const CalParams P = params(k);
             identity_kernel<<<(unsigned)((nsol + 255) / 256), 256, 0, cs>>>(P.di_jones, nsol);
             count_launches(1);
-            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov, num_chanblocks, cs);
+            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov.p, num_chanblocks, cs);
             if (!rc) rc = pcov.launch(P, form, num_chanblocks, cs);
         }
         e = cudaStreamEndCapture(cs, &graph);
@@ -1474,7 +1485,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         for (auto& r : rk) conv += r.converged;
         if (conv > 0 && conv != num_chanblocks) {
             const CalParams P = params(k);
-            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov, num_chanblocks, s);  // this timeblock's covariances
+            if (form != HDC_CAL_PLAIN) rc = launch_collapse(P, form, cov.p, num_chanblocks, s);  // this timeblock's covariances
             if (!rc) rc = retry_failed(P, form, pcov, rk, d_list, d_pairs, s);
             if (rc) {
                 cleanup();

@@ -1,7 +1,8 @@
 """Calibrations of arrays of different sizes on several host threads: the
 kernel's shared-memory opt-in is one per device, so a small array's call must
 not have a large one's retry launch refused (csrc/calibrate.cu, opt_in_smem),
-and the stream on which calls capture their graphs is one per device too."""
+and the stream on which calls capture their graphs and the collapsed forms'
+covariances are one per device too."""
 
 import threading
 
@@ -31,11 +32,11 @@ def problem(ntiles, nt, nch):
     return torch.from_numpy(data).cuda(), torch.from_numpy(model).cuda(), start
 
 
-def solve(p, stream):
+def solve(p, stream, form="plain"):
     data, model, start = p
     with torch.cuda.stream(stream):
         dj = start.clone()
-        res = cal.calibrate_timeblock(data, model, dj, (0, data.shape[0]), 40, 1e-8, 1e-4, stream=stream)
+        res = cal.calibrate_timeblock(data, model, dj, (0, data.shape[0]), 40, 1e-8, 1e-4, form=form, stream=stream)
     stream.synchronize()
     return dj.cpu().numpy(), [(r.num_iterations, r.converged) for r in res]
 
@@ -92,3 +93,17 @@ def test_graphs_beside_each_other():
     for out, c in beside(large, [problem(n, 2, 3) for n in (5, 9, 17)], solve_timeblocks, 60):
         assert c == counts
         np.testing.assert_array_equal(out, want)
+
+
+# the last size needs more covariances than the buffer holds
+@pytest.mark.parametrize("form", ["collapsed", "collapsed_f32"])
+def test_covariances_beside_each_other(form):
+    def run(p, stream):
+        return solve(p, stream, form)
+
+    large = problem(100, 2, 5)
+    torch.cuda.synchronize()
+    want, counts = run(large, torch.cuda.Stream())
+    for dj, c in beside(large, [problem(n, 1, 3) for n in (5, 40, 256)], run, 40):
+        assert c == counts
+        np.testing.assert_array_equal(dj, want)
