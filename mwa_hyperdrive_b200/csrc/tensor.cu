@@ -1047,24 +1047,25 @@ __global__ void combine_model_kernel(const void* planes, JonesF32* vis, const Jo
 // The MODE 1 scales: maxb[unique frequency], the largest |entry| of the beam
 // Jones over unique tiles and components there (channels share it; by channel
 // through row_map where there are fewer channels), and maxs[channel], that of
-// S.  Bound by reading them; blocks (x, y < nrow) take slices of the beam and
-// blocks (x, nrow + f) of S, and the slices meet in an integer maximum, which
+// S.  Bound by reading them; blocks (x < nrow, y) take slices of the beam and
+// blocks (nrow + f, y) of S, and the slices meet in an integer maximum, which
 // orders non-negative doubles (NaN entries are passed over, as fmax does).
 // The squares are compared; moduli whose squares leave FP64's range are taken
 // with hypot.  17 unique tiles x 2000 components, 192 channels of 13 unique
-// frequencies: 165 us with a block per channel, 18 us so.
+// frequencies: 165 us with a block per channel, 18 us so.  grid (nrow + nf,
+// BB_SPLIT): rows and channels together may be more than a grid's y extent.
 constexpr int BB_SPLIT = 16;
 __global__ void __launch_bounds__(256) beam_bounds_kernel(const JonesF64* beam, int n_uniq_tile, int n_uniq_freq,
                                                           const int* row_map, int nrow, const JonesF64* S, int nc,
                                                           int c0, int cn, double* maxb, double* maxs) {
-    const bool of_s = (int)blockIdx.y >= nrow;
-    const int row = of_s ? blockIdx.y - nrow : blockIdx.y;
+    const bool of_s = (int)blockIdx.x >= nrow;
+    const int row = of_s ? blockIdx.x - nrow : blockIdx.x;
     const int uf = of_s || !row_map ? row : row_map[row];
     const int n = (of_s ? 1 : n_uniq_tile) * cn;
     double m2 = 0.0;
     bool odd = false;  // a modulus whose square is not a normal number
     auto entries = [&](auto&& each) {
-        for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += BB_SPLIT * 256) {
+        for (int i = blockIdx.y * 256 + threadIdx.x; i < n; i += BB_SPLIT * 256) {
             const int u = i / cn, c = i - u * cn;
             const JonesF64* j = of_s ? S + (size_t)row * nc + c0 + c : beam + ((size_t)u * n_uniq_freq + uf) * nc + c0 + c;
             const double2* e = reinterpret_cast<const double2*>(j);
@@ -1313,7 +1314,7 @@ int launch_tensor_points(int nf, int nbl, int ntiles, int nc, const double* d_fr
         if (tile_beam) {
             HDC_CUDA_RET_INT(cudaMemsetAsync(bounds, 0, sizeof(double) * 2 * nf, s));
             const int nrow = std::min(beam->n_uniq_freq, nf);
-            tc::beam_bounds_kernel<<<dim3(tc::BB_SPLIT, nrow + nf), 256, 0, s>>>(
+            tc::beam_bounds_kernel<<<dim3(nrow + nf, tc::BB_SPLIT), 256, 0, s>>>(
                 beam->beam, beam->n_uniq_tile, beam->n_uniq_freq, P.by_channel ? beam->freq_map : nullptr, nrow, d_W, nc,
                 c0, P.cn, bounds, bounds + nf);
             count_launches(1);
