@@ -522,7 +522,7 @@ typedef struct HdcCalResult {
     int num_failed;
 } HdcCalResult;
 
-#define HDC_CAL_PLAIN 0         /* stream data and model every iteration */
+#define HDC_CAL_PLAIN 0         /* the reference's sums in FP64, over covariances of the call's own scratch */
 #define HDC_CAL_COLLAPSED 1     /* sum the timeblock's timesteps once into per-baseline covariances (FP64) */
 #define HDC_CAL_COLLAPSED_F32 2 /* the same with covariances stored in FP32 (half the bytes per iteration) */
 
@@ -534,7 +534,11 @@ typedef struct HdcCalResult {
  * [timeblock_start, timeblock_end).  d_di_jones is this timeblock's
  * [tile][chanblock] slice of the solutions (model -> data, not inverted): the
  * initial guesses in, the solutions out (NaN where failed).  h_results gets
- * one entry per chanblock.  Up to 256 tiles. */
+ * one entry per chanblock.  Up to 256 tiles.  The plain form takes up to 1 GiB
+ * of device memory for the call (covariances of a group of chanblocks), or
+ * none where that cannot be had (it then streams data and model each
+ * iteration).  Such scratch comes from a pool per device, which keeps up to 1
+ * GiB of it mapped between calls. */
 int hdc_calibrate_timeblock(const JonesF32 *d_data_tfb, const JonesF32 *d_model_tfb, int num_timesteps,
                             int timeblock_start, int timeblock_end, int num_chanblocks, int num_baselines,
                             JonesF64 *d_di_jones, int max_iterations, double stop_threshold, double min_threshold,

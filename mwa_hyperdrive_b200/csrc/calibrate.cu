@@ -1118,7 +1118,7 @@ struct Covariances {
             cudaFree(g_cov[d]);
             g_cov[d] = nullptr;
             g_cov_size[d] = 0;
-            if (cudaMalloc(&g_cov[d], bytes) != cudaSuccess) {
+            if (device_malloc(&g_cov[d], bytes) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
             }

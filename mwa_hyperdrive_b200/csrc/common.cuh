@@ -337,8 +337,15 @@ const char* cuda_msg(cudaError_t e);
 // have no workspace argument).  Returns NULL on allocation failure.
 void* device_scratch(size_t bytes);
 // Stream-ordered allocation from the library's own pool on the current device
-// (freed blocks stay mapped for reuse); release with cudaFreeAsync.
+// (up to 1 GiB of freed blocks stays mapped for reuse); release with
+// cudaFreeAsync.
 cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t s);
+// Bytes that the pool holds and no allocation uses.
+size_t pool_idle_bytes();
+// Give the pool's idle blocks back to the device (synchronises).
+void pool_trim();
+// cudaMalloc, again with the pool's idle blocks given back where memory is short.
+cudaError_t device_malloc(void** p, size_t bytes);
 // Device word for kernel error flags (per device, zero-initialised).
 int* device_error_word();
 // Read and clear the device error word (synchronises the stream).

@@ -280,7 +280,7 @@ template <class T>
 static cudaError_t dalloc(T** p, size_t n) {
     *p = nullptr;
     if (n == 0) return cudaSuccess;
-    return cudaMalloc((void**)p, sizeof(T) * n);
+    return device_malloc((void**)p, sizeof(T) * n);
 }
 template <class T>
 static void dfree(T*& p) {
@@ -1241,7 +1241,7 @@ extern "C" int hdc_modeller_model_timestep_with_host(HdcModeller* hm, double lst
         if (m->d_host_vis) cudaFree(m->d_host_vis);
         m->d_host_vis = nullptr;
         m->host_vis_bytes = 0;
-        HDC_CUDA_RET_INT(cudaMalloc(&m->d_host_vis, bytes));
+        HDC_CUDA_RET_INT(hdc::device_malloc((void**)&m->d_host_vis, bytes));
         m->host_vis_bytes = bytes;
     }
     if (m->form == HDC_PREDICT_TENSOR && !m->tile_beams() && m->t[0].nc > 0 &&
@@ -1250,7 +1250,7 @@ extern "C" int hdc_modeller_model_timestep_with_host(HdcModeller* hm, double lst
             if (m->d_host_model) cudaFree(m->d_host_model);
             m->d_host_model = nullptr;
             m->host_model_bytes = 0;
-            HDC_CUDA_RET_INT(cudaMalloc(&m->d_host_model, bytes));
+            HDC_CUDA_RET_INT(hdc::device_malloc((void**)&m->d_host_model, bytes));
             m->host_model_bytes = bytes;
         }
         return m->host_call_drained(m->model_host_points_last(lst, h_vis, h_uvws, s));

@@ -17,7 +17,7 @@ struct DevBuf {
         return pool_malloc_async(&p, bytes, st);
     }
     // large one-off buffers stay outside the pool, which keeps what it holds
-    cudaError_t alloc_plain(size_t bytes) { return cudaMalloc(&p, bytes); }
+    cudaError_t alloc_plain(size_t bytes) { return device_malloc(&p, bytes); }
     ~DevBuf() {
         if (p) pooled ? cudaFreeAsync(p, s) : cudaFree(p);
     }

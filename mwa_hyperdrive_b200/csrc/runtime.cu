@@ -48,6 +48,7 @@ __global__ void fma_probe_kernel(T seed, int iters, T* sink) {
 namespace {
 constexpr int MAX_DEV = 64;
 std::mutex g_mu;
+std::mutex g_scratch_mu;
 void* g_scratch[MAX_DEV] = {};
 size_t g_scratch_size[MAX_DEV] = {};
 int* g_errword[MAX_DEV] = {};
@@ -64,6 +65,15 @@ int cur_dev() {
 }
 }  // namespace
 
+// Freed blocks of up to this many bytes stay mapped, so that the next call
+// reuses them without a new physical mapping; what the pool holds beyond them
+// goes back at the next synchronisation, all of it when device_malloc runs
+// short.  Mapping anew costs about 13 ms a GiB: a plain calibration (384
+// chanblocks, 128 tiles, 0.7 GiB of covariances) takes 5.7 ms so, 15 with 256
+// MiB kept and 18 with nothing; the batched peel (30 sources, 0.7 GiB) 6.3, 11.3
+// and 14.3 ms.
+constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
+
 cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t s) {
     cudaMemPool_t pool = nullptr;
     {
@@ -77,10 +87,7 @@ cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t s) {
             props.location.id = d;
             cudaError_t e = cudaMemPoolCreate(&g_pool[d], &props);
             if (e != cudaSuccess) return e;
-            // keep freed blocks mapped: the next call reuses them without a
-            // new physical mapping (the default pool returns them at every
-            // synchronisation)
-            uint64_t keep = UINT64_MAX;
+            uint64_t keep = POOL_KEEP;
             e = cudaMemPoolSetAttribute(g_pool[d], cudaMemPoolAttrReleaseThreshold, &keep);
             if (e != cudaSuccess) return e;
         }
@@ -89,8 +96,38 @@ cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t s) {
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
-void* device_scratch(size_t bytes) {
+static cudaMemPool_t current_pool() {
     std::lock_guard<std::mutex> lk(g_mu);
+    const int d = cur_dev();
+    return d < 0 ? nullptr : g_pool[d];
+}
+
+size_t pool_idle_bytes() {
+    cudaMemPool_t pool = current_pool();
+    uint64_t reserved = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return 0;
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+void pool_trim() {
+    cudaMemPool_t pool = current_pool();
+    if (!pool) return;
+    cudaDeviceSynchronize();  // blocks freed on streams are idle once their work is done
+    cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !current_pool()) return e;
+    cudaGetLastError();
+    pool_trim();
+    return cudaMalloc(p, bytes);
+}
+
+void* device_scratch(size_t bytes) {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
     int d = cur_dev();
     if (d < 0) return nullptr;
     if (bytes == 0) bytes = 256;
@@ -103,7 +140,7 @@ void* device_scratch(size_t bytes) {
             g_scratch_size[d] = 0;
         }
         size_t want = bytes + bytes / 4;
-        if (cudaMalloc(&g_scratch[d], want) != cudaSuccess) {
+        if (device_malloc(&g_scratch[d], want) != cudaSuccess) {
             cudaGetLastError();
             set_error("device scratch allocation of %zu bytes failed", want);
             return nullptr;

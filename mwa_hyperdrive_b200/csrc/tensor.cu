@@ -1440,11 +1440,11 @@ void* Modeller::tensor_workspace(bool out64, size_t& bytes) {
         tc->ws = nullptr;
         tc->ws_bytes = 0;
         tc->ws_short = false;
-        if (cudaMalloc(&tc->ws, need) != cudaSuccess) {
+        if (device_malloc(&tc->ws, need) != cudaSuccess) {
             cudaGetLastError();
             tc->ws_short = true;
             need = least;
-            if (cudaMalloc(&tc->ws, need) != cudaSuccess) {
+            if (device_malloc(&tc->ws, need) != cudaSuccess) {
                 cudaGetLastError();
                 tc->ws = nullptr;
                 set_error("tensor predict workspace of %zu bytes: allocation failed", need);
