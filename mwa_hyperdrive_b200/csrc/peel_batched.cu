@@ -552,8 +552,9 @@ using namespace hdc;
     do {                                                                               \
         cudaError_t e_ = (call);                                                       \
         if (e_ != cudaSuccess) {                                                       \
+            cudaGetLastError();                                                        \
             set_error("hdc_peel_timeblock_batched: %s: %s", #call, cudaGetErrorString(e_)); \
-            return HDC_ERR_CUDA;                                                       \
+            return e_ == cudaErrorMemoryAllocation ? HDC_ERR_ALLOC : HDC_ERR_CUDA;     \
         }                                                                              \
     } while (0)
 
@@ -598,12 +599,21 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     // (with a beam shared by all tiles, or none: per-tile beams make a
     // point's model depend on the baseline)
     const bool points = peel_point_sources(h_sources, h_source_positions, ns, params->beam_kind);
+    const size_t need = points ? sizeof(float4) * (size_t)ns * nt * nf : sizeof(JonesF32) * nvis * (size_t)ns;
+    const size_t ntab = (size_t)ns * nt * nf * num_tiles;  // per-tile phasor tables
+    // one sub-batch's apply table at a time
+    const int batch = params->batch_size > 0 ? std::min(params->batch_size, ns) : ns;
+    // the call's larger buffers: models, phasor tables, traces and
+    // low-resolution sums, UVWs (what the pool holds idle serves them too)
+    const size_t buffers = need + sizeof(float4) * (ntab + (size_t)batch * nt * nf * num_tiles) + sizeof(float2) * nvis +
+                           sizeof(float2) * 2 * (size_t)batch * nlo * nbl + iono_partials_bytes(batch, nbl) +
+                           sizeof(UVW) * ((size_t)ns * nbl + (points ? 0 : (size_t)ns * nt * nbl));
     size_t free_b = 0, total_b = 0;
     PB_CK(cudaMemGetInfo(&free_b, &total_b));
-    const size_t need = points ? sizeof(float4) * (size_t)ns * nt * nf : sizeof(JonesF32) * nvis * (size_t)ns;
-    if (need + (size_t)(1u << 30) > free_b) {
-        set_error("hdc_peel_timeblock_batched: the %d source models need %zu MB of device memory, %zu MB free", ns,
-                  need >> 20, free_b >> 20);
+    free_b += pool_idle_bytes();
+    if (std::max(buffers, need + (size_t)(1u << 30)) > free_b) {
+        set_error("hdc_peel_timeblock_batched: %d sources need %zu MB of device memory (models %zu MB), %zu MB free", ns,
+                  buffers >> 20, need >> 20, free_b >> 20);
         return HDC_ERR_ALLOC;
     }
     DevBuf b_tuvw, b_radec, b_acc, b_app, b_wtr;
@@ -615,12 +625,9 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
     PB_CK(b_avg_lmst.alloc(sizeof(double), s));
     PB_CK(b_xyz.alloc(sizeof(XYZ) * xyz_t.size(), s));
     if (!points) PB_CK(b_uv_src.alloc(sizeof(UVW) * (size_t)ns * nt * nbl, s));
-    const size_t ntab = (size_t)ns * nt * nf * num_tiles;  // per-tile phasor tables
     PB_CK(b_tuvw.alloc(sizeof(UVW) * (size_t)(ns + 1) * nt * num_tiles, s));
     PB_CK(b_radec.alloc(sizeof(double2) * (ns + 1), s));
     PB_CK(b_acc.alloc(sizeof(float4) * ntab, s));
-    // one sub-batch's apply table at a time
-    const int batch = params->batch_size > 0 ? std::min(params->batch_size, ns) : ns;
     PB_CK(b_app.alloc(sizeof(float4) * (size_t)batch * nt * nf * num_tiles, s));
     PB_CK(b_wtr.alloc(sizeof(float2) * nvis, s));
     PB_CK(b_uv_lo.alloc(sizeof(UVW) * (size_t)ns * nbl, s));

@@ -43,3 +43,15 @@ def test_scratch_beyond_the_bound_is_given_back():
     run_peel(400, 128, 192, 4)
     kept = before - free_bytes()
     assert kept <= (1 << 30) + (32 << 20), kept
+
+
+def test_a_peel_that_cannot_fit_is_refused_before_it_allocates():
+    """40000 sources' phasor tables are 2 x 126 GB; their models 1 GB."""
+    from mwa_hyperdrive_b200._lib import HdcError
+
+    tiles, channels, timesteps, sources = 128, 384, 4, 40000
+    assert torch.cuda.mem_get_info()[1] < 2 * 16 * sources * timesteps * channels * tiles
+    before = free_bytes()
+    with pytest.raises(HdcError, match=r"status 3.*device memory"):  # HDC_ERR_ALLOC
+        run_peel(sources, tiles, channels, timesteps)
+    assert before - free_bytes() <= 32 << 20
