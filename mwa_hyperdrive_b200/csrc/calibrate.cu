@@ -422,14 +422,22 @@ __device__ __forceinline__ void group_sync(int grp) {
         asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory");
 }
 
-// Threads per CTA of the iteration kernel: the covariance forms run two
-// groups of 256 (one per parity of the block's storage index), in FP32 on one
-// shared ring.
-__host__ __device__ constexpr int cal_threads(int form) { return form == HDC_CAL_PLAIN ? CT : 2 * CT; }
+// Groups of 256 threads per CTA of the iteration kernel: the covariance forms
+// run two (one per parity of the block's storage index), in FP32 on one shared
+// ring.  FP64 covariances of at most ONE_GROUP_TILES tiles take one, and two
+// such CTAs share an SM: those arrays have three columns of blocks or fewer for
+// the groups to share out, and their covariances lie in L2.  30 iterations, one
+// group against two, us: 17 tiles x 8 chanblocks 414 / 443, x 500 1093 / 1429; 32
+// tiles x 300 965 / 1257; 40 tiles x 100 674 / 699, x 500 2220 / 2158; 48 tiles x
+// 100 692 / 712, x 500 2333 / 2247; 64 tiles x 100 1181 / 1022.
+constexpr int ONE_GROUP_TILES = 48;
+static int cal_groups(int form, int ntiles) {
+    return form == HDC_CAL_PLAIN || (form == HDC_CAL_COLLAPSED && ntiles <= ONE_GROUP_TILES) ? 1 : 2;
+}
 
-template <int FORM>
-__global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalParams P) {
-    constexpr int NTH = cal_threads(FORM);
+template <int FORM, int NG>
+__global__ void __launch_bounds__(NG * CT) mitchcal_kernel(const CalParams P) {
+    constexpr int NTH = NG * CT;
     extern __shared__ double smem[];
     const int n = P.ntiles;
     J2* G = reinterpret_cast<J2*>(smem);          // current gains
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
     // covariance forms: the second group's own accumulators, added into
     // top/bot once both groups have swept the blocks
     J2* top1 = reinterpret_cast<J2*>(colbuf + 16 * 16 * 12);
-    Herm* bot1 = reinterpret_cast<Herm*>(top1 + (FORM != 0 ? n : 0));
+    Herm* bot1 = reinterpret_cast<Herm*>(top1 + (NG == 2 ? n : 0));
 
     // (FP32 covariances are those of all chanblocks, in one launch)
     const int item = (FORM == 2 ? 0 : P.ch0) + (int)blockIdx.x;
@@ -469,7 +477,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
     __shared__ uint32_t ring_cnt[4];  // copies issued per slot
     __shared__ uint32_t ring_tag[4], ring_rel[4];
     const bool use_ring = FORM == 2 && P.nring > 0;
-    float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(bot1 + (FORM != 0 ? n : 0)) + 15) & ~(uintptr_t)15);
+    float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(bot1 + (NG == 2 ? n : 0)) + 15) & ~(uintptr_t)15);
     uint32_t jseq = 0;  // covariance blocks consumed so far (all threads alike)
     bool abort_loop = false;
 
@@ -504,7 +512,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
         for (int i = tid; i < n; i += NTH) {
             top[i] = jzero();
             bot[i] = Herm{0.0, 0.0, {0.0, 0.0}};
-            if (FORM != 0) {
+            if (NG == 2) {
                 top1[i] = jzero();
                 bot1[i] = Herm{0.0, 0.0, {0.0, 0.0}};
             }
@@ -582,7 +590,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
             // no atomics.  FP32 covariances arrive through the shared-memory
             // ring (bulk copies issued nring blocks ahead); FP64 ones are
             // loaded directly.
-            // Two groups of 256 threads run: group g takes the
+            // With two groups of 256 threads group g takes the
             // blocks of odd or even storage index (18 each for 128 tiles),
             // so the two groups consume alternate ring slots, and sums into
             // its own accumulators (group 1: top1/bot1, added to top/bot
@@ -591,7 +599,6 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
             // meet only at the end of the sweep.  Within a column block the
             // warps do not meet: a row of the block belongs to one warp in
             // every block, so each accumulator entry has one writer.
-            constexpr int NG = NTH / BLK;
             const int grp = tid / BLK, gt = tid % BLK;
             const int bi = gt >> 4, bj = gt & 15;
             const int nb = (n + 15) / 16;
@@ -629,7 +636,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
                         // the group's next block on its way to L2 (without it
                         // the iterations are bound by these loads' latency:
                         // 4.7 instead of 3.9 ms, 100 chanblocks of 113 tiles)
-                        if (FORM == 1 && gt == 0)
+                        if (FORM == 1 && NG == 2 && gt == 0)
                             prefetch_l2(static_cast<const double*>(P.cov) + ((size_t)cov_ch * P.nblk + (blk + NG) % P.nblk) * NCOV * BLK,
                                         NCOV * BLK * sizeof(double));
                         if (p < q && q < n) {
@@ -702,7 +709,7 @@ __global__ void __launch_bounds__(cal_threads(FORM)) mitchcal_kernel(const CalPa
             // both groups' sweeps done: fold group 1's sums into top/bot
             if (__syncthreads_or(gabort)) {
                 abort_loop = true;
-            } else {
+            } else if (NG == 2) {
                 for (int i = tid; i < n; i += NTH) {
                     top[i] = top[i] + top1[i];
                     bot[i].a += bot1[i].a;
@@ -977,7 +984,7 @@ static size_t smem_bytes(int n, int form) {
 // The iteration kernel's opt-in to the dynamic shared memory that any tile
 // count needs, once per device: calls on several threads have tile counts of
 // their own, and an attribute set for one would have another's launch refused.
-template <int FORM>
+template <int FORM, int NG>
 static int opt_in_smem() {
     static std::atomic<bool> done[64];
     int dev = 0;
@@ -986,27 +993,30 @@ static int opt_in_smem() {
     size_t most = 0;
     for (int n = 2; n <= CT; n++) most = std::max(most, smem_bytes(n, FORM));
     HDC_CUDA_RET_INT(
-        cudaFuncSetAttribute(mitchcal_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        cudaFuncSetAttribute(mitchcal_kernel<FORM, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return HDC_OK;
 }
 
-static int prepare_mitchcal(int form) {
-    if (form == HDC_CAL_COLLAPSED) return opt_in_smem<1>();
-    if (form == HDC_CAL_COLLAPSED_F32) return opt_in_smem<2>();
-    return opt_in_smem<0>();
+static int prepare_mitchcal(int form, int ntiles) {
+    if (form == HDC_CAL_COLLAPSED) return cal_groups(form, ntiles) == 1 ? opt_in_smem<1, 1>() : opt_in_smem<1, 2>();
+    if (form == HDC_CAL_COLLAPSED_F32) return opt_in_smem<2, 2>();
+    return opt_in_smem<0, 1>();
 }
 
 // Launch the iterations of nblocks chanblocks; prepare_mitchcal has run (before
 // a stream capture, if one is under way).
 static int launch_mitchcal(const CalParams& P, int form, int nblocks, cudaStream_t s) {
     const size_t sm = smem_bytes(P.ntiles, form);
-    if (form == HDC_CAL_COLLAPSED)
-        mitchcal_kernel<1><<<nblocks, cal_threads(1), sm, s>>>(P);
+    const int ng = cal_groups(form, P.ntiles);
+    if (form == HDC_CAL_COLLAPSED && ng == 1)
+        mitchcal_kernel<1, 1><<<nblocks, ng * CT, sm, s>>>(P);
+    else if (form == HDC_CAL_COLLAPSED)
+        mitchcal_kernel<1, 2><<<nblocks, ng * CT, sm, s>>>(P);
     else if (form == HDC_CAL_COLLAPSED_F32)
-        mitchcal_kernel<2><<<nblocks, cal_threads(2), sm, s>>>(P);
+        mitchcal_kernel<2, 2><<<nblocks, ng * CT, sm, s>>>(P);
     else
-        mitchcal_kernel<0><<<nblocks, cal_threads(0), sm, s>>>(P);
+        mitchcal_kernel<0, 1><<<nblocks, ng * CT, sm, s>>>(P);
     count_launches(1);
     HDC_CUDA_RET_INT(cudaGetLastError());
     return HDC_OK;
@@ -1096,7 +1106,7 @@ struct PlainCov {
         return HDC_OK;
     }
     // what launch() needs before it (and before a stream capture)
-    int prepare(int form) const { return prepare_mitchcal(group ? HDC_CAL_COLLAPSED : form); }
+    int prepare(int form, int ntiles) const { return prepare_mitchcal(group ? HDC_CAL_COLLAPSED : form, ntiles); }
 };
 
 // The collapsed forms' covariances: a grow-only buffer per device, which a call
@@ -1292,7 +1302,7 @@ static int calibrate_timeblock_impl(const JonesF32* d_data_tfb, const JonesF32* 
         nblocks = num_listed;
     }
     const PlainCov pcov(form, nblocks, P.nblk, s);
-    rc = pcov.prepare(form);
+    rc = pcov.prepare(form, ntiles);
     if (!rc) rc = pcov.launch(P, form, nblocks, s);
     if (rc) {
         cleanup();
@@ -1416,7 +1426,7 @@ extern "C" int hdc_calibrate_timeblocks(const JonesF32* d_data_tfb, const JonesF
         }
     }
     const PlainCov pcov(form, num_chanblocks, nblk, s);
-    int rc = pcov.prepare(form);
+    int rc = pcov.prepare(form, ntiles);
     std::unique_lock<std::mutex> capturing(g_cs_mu);
     cudaStream_t cs = capture_stream();
     if (rc || !cs) {
