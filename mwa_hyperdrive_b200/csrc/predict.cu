@@ -195,8 +195,11 @@ __device__ __forceinline__ void shapelet_dense(const DirectParams& p, const floa
     }
 }
 
-template <int TYPE, bool TILE_BEAM, bool OUT64>
-__global__ void __launch_bounds__(DT) direct_kernel(const DirectParams p) {
+// MINB: CTAs an SM holds (0: what the registers give).  The points' sum over
+// components is bound by the FP64 pipe, a few components by the latency of a
+// CTA's copies and visibilities, which only more CTAs hide.
+template <int TYPE, bool TILE_BEAM, bool OUT64, int MINB>
+__global__ void __launch_bounds__(DT, MINB) direct_kernel(const DirectParams p) {
     __shared__ alignas(128) double4 s_lmn[2][CH];
     __shared__ alignas(128) JonesF64 s_flux[2][CH];
     __shared__ alignas(128) double4 s_gp[2][CH];
@@ -778,26 +781,43 @@ static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
     return launch_fast_tile<OUT64, 1>(p, grid, dev, s);
 }
 
+// Points under a shared beam: 64 registers (four CTAs an SM), 48 for up to
+// FEW_POINTS of them (five, a few registers spilled in the loop).  128 tiles x
+// 384 channels, us at three CTAs / four / five: 1 point 86 / 75 / 66, 2 90 / 79 /
+// 73, 8 128 / 124 / 125, 64 703 / 694 / 729, 400 4275 / 4222 / 4434.
+constexpr int FEW_POINTS = 4;
+template <int TYPE, bool TILE_BEAM, bool OUT64>
+static void launch_direct_kernel(const DirectParams& p, cudaStream_t s) {
+    const dim3 grid((p.nbl + DT - 1) / DT, p.nf);
+    if constexpr (TYPE == 0 && !TILE_BEAM) {
+        if (p.nc <= FEW_POINTS)
+            direct_kernel<TYPE, TILE_BEAM, OUT64, 5><<<grid, DT, 0, s>>>(p);
+        else
+            direct_kernel<TYPE, TILE_BEAM, OUT64, 4><<<grid, DT, 0, s>>>(p);
+    } else {
+        direct_kernel<TYPE, TILE_BEAM, OUT64, 0><<<grid, DT, 0, s>>>(p);
+    }
+}
+
 template <int TYPE>
 static cudaError_t launch_t(bool tile_beam, bool out64, bool fast, const DirectParams& p, cudaStream_t s) {
-    dim3 grid((p.nbl + DT - 1) / DT, p.nf);
     if (tile_beam && fast && TYPE == 2) {
         const cudaError_t e = out64 ? launch_fast_tile<true>(p, s) : launch_fast_tile<false>(p, s);
         if (e != cudaSuccess) return e;
     } else if (tile_beam) {
         if (out64)
-            direct_kernel<TYPE, true, true><<<grid, DT, 0, s>>>(p);
+            launch_direct_kernel<TYPE, true, true>(p, s);
         else
-            direct_kernel<TYPE, true, false><<<grid, DT, 0, s>>>(p);
+            launch_direct_kernel<TYPE, true, false>(p, s);
     } else if (fast && TYPE == 2) {
         const cudaError_t e = p.sdense ? (out64 ? launch_fast_shapelet<true, true>(p, s) : launch_fast_shapelet<true, false>(p, s))
                                        : (out64 ? launch_fast_shapelet<false, true>(p, s) : launch_fast_shapelet<false, false>(p, s));
         if (e != cudaSuccess) return e;
     } else {
         if (out64)
-            direct_kernel<TYPE, false, true><<<grid, DT, 0, s>>>(p);
+            launch_direct_kernel<TYPE, false, true>(p, s);
         else
-            direct_kernel<TYPE, false, false><<<grid, DT, 0, s>>>(p);
+            launch_direct_kernel<TYPE, false, false>(p, s);
     }
     count_launches(1);
     return cudaGetLastError();
