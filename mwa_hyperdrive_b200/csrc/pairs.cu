@@ -3,12 +3,13 @@
 // A native modeller's baseline UVW is a tile difference (uvw_pq = uvw_p -
 // uvw_q), so the phasor of a term factors: exp(2 pi i t_pq) = A_p conj(A_q)
 // with A_p = exp(2 pi i (u_p l + v_p m + w_p (n - 1))), and an envelope's
-// coordinates are differences of per-tile ones.  A CTA takes a 32 x 32 block
-// of tile pairs of one channel (blocks on or above the diagonal) and, per
-// staged chunk of components, forms in shared memory the 64 tiles' phasors
-// (and Gaussian or shapelet coordinates); its 256 threads then take 2 x 2
-// pairs each, so one FP64 sincos serves 16 baselines and a pair costs a
-// complex product (4 operations) instead of a sincos.
+// coordinates are differences of per-tile ones.  A CTA takes a block of tile
+// pairs of one channel (on or above the diagonal) and, per staged chunk of
+// components, forms in shared memory its tiles' phasors (and Gaussian or
+// shapelet coordinates); its 256 threads then take the pairs, so one FP64
+// sincos serves 16 baselines (32 x 32 pairs, 2 x 2 a thread) or 8 (16 x 16, one
+// a thread) and a pair costs a complex product (4 operations) instead of a
+// sincos.  whole_tiles says which blocks.
 //
 // Shared beam (or none): W = B S B^H is Hermitian, so with W_xy = a + i b the
 // four correlations come from the sums of w_xx z, w_yy z, a z and b z (8
@@ -36,9 +37,133 @@
 namespace hdc {
 namespace pairs {
 
-constexpr int TB = 32;     // tiles per block side
-constexpr int NTH = 256;   // 16 x 16 threads of 2 x 2 pairs
-constexpr int RI = 2;      // rows per thread, two columns (all 16 apart)
+constexpr int NTH = 256;  // threads of a CTA, 16 x 16
+constexpr int GRP = 32;   // table slots a CTA of single pairs has (rows, then columns)
+
+// The tile pairs of a CTA (us per call, 65 tiles x 128 channels x 200, with a
+// thread per baseline and its own phasors / in 32 x 32 blocks only / so: FP64
+// Gaussians 389 / 404 / 268, the chosen form's 127 / 197 / 139, with per-tile
+// beams 379 / 587 / 400).  H 2: a block of 32 x 32 pairs of groups of 32 tiles,
+// on or above the diagonal; a thread takes 2 x 2 of them, 16 apart.  (The last
+// group may reach past the array: its places there repeat the last tile.)  H 1: at
+// most 256 pairs, one a thread: blocks of 16 x 16 of whole groups of 16 (a
+// diagonal block's 120 pairs counted), and strips of the last tiles, fewer than
+// 16, with as many others as fit the table slots (their pairs counted too).  Pairs
+// that are counted fill the first warps, and the others have nothing to do.
+template <int H>
+struct Block {
+    int p0, q0;    // first row tile, first column tile
+    int rs;        // row slots of the tables; the columns' follow
+    int count;     // its pairs (H 1)
+    int r, c;      // this thread's pair, its first with H 2, as table slots
+    bool diag;     // the column tiles are the row tiles
+    // blk: of num_blocks(); first: the tiles below it have their pairs with one
+    // another in the other launch
+    __device__ __forceinline__ Block(int blk, int ntiles, int first) {
+        const int tid = threadIdx.x;
+        r = tid >> 4, c = tid & 15;
+        if (H == 2) {
+            const int n = first / 32, noff = n * (n - 1) / 2;
+            // blocks off the diagonal first, then the cheaper diagonal ones
+            int pb, qb;
+            if (blk < noff)
+                baseline_to_tiles(blk, n, pb, qb);
+            else
+                pb = qb = blk - noff;
+            p0 = 32 * pb, q0 = 32 * qb, rs = 32, count = NTH;
+            diag = pb == qb;
+        } else {
+            const int n = ntiles / 16, n0 = first / 16, noff = (n * (n - 1) - n0 * (n0 - 1)) / 2;
+            int k = tid;
+            rs = 16;
+            diag = false;
+            if (blk < noff) {
+                const int x = blk + n0 * (n0 - 1) / 2;
+                int qb = (int)((1.f + sqrtf(8.f * x + 1.f)) * 0.5f);
+                while (qb * (qb - 1) / 2 > x) qb--;
+                while (qb * (qb + 1) / 2 <= x) qb++;
+                p0 = 16 * (x - qb * (qb - 1) / 2), q0 = 16 * qb;
+                count = NTH;
+            } else if (blk < noff + n - n0) {
+                p0 = q0 = 16 * (n0 + blk - noff);
+                count = 120;
+                diag = true;
+                baseline_to_tiles(k < count ? k : 0, 16, r, c);
+            } else {
+                q0 = 16 * n;
+                const int nc = ntiles - q0;
+                rs = GRP - nc;
+                p0 = rs * (blk - noff - (n - n0));
+                const int nr = min(rs, ntiles - p0), rect = min(max(q0 - p0, 0), nr);  // rows of other tiles
+                const int i0 = max(p0 - q0, 0), i1 = p0 + nr - q0;                       // of the strip's own
+                auto start = [&](int i) { return i * (2 * nc - i - 1) / 2; };
+                count = rect * nc + (i1 > i0 ? start(i1) - start(i0) : 0);
+                if (k >= count) k = 0;
+                if (k < rect * nc) {
+                    r = k / nc, c = k - r * nc;
+                } else if (count > 0) {
+                    baseline_to_tiles(k - rect * nc + start(i0), nc, r, c);
+                    r += q0 - p0;
+                } else {
+                    r = c = 0;
+                }
+            }
+        }
+        c += rs;
+    }
+    // this thread has a pair (H 1)
+    __device__ __forceinline__ bool mine() const { return (int)threadIdx.x < count; }
+    // the tile of a table slot
+    __device__ __forceinline__ int tile(int slot, int ntiles) const {
+        const int t = slot < rs ? p0 + slot : q0 + slot - rs;
+        return H == 2 ? min(t, ntiles - 1) : t;
+    }
+    // the visibility of a pair of table slots in channel f, or -1 (on or below
+    // the diagonal, or past the array)
+    __device__ __forceinline__ long long vis_index(const DirectParams& p, int f, int row, int col) const {
+        const int tp = p0 + row, tq = q0 + col - rs;
+        return tp < tq && tq < p.ntiles ? (long long)f * p.nbl + baseline_index(tp, tq, p.ntiles) : -1;
+    }
+};
+
+// its blocks
+static int num_blocks(int h, int ntiles, int first) {
+    if (h == 2) return first / 32 * (first / 32 + 1) / 2;
+    const int n = ntiles / 16, n0 = first / 16, rest = ntiles % 16;
+    return (n * (n - 1) - n0 * (n0 - 1)) / 2 + n - n0 + (rest ? (ntiles + GRP - rest - 1) / (GRP - rest) : 0);
+}
+
+// vis[at[i]] += value(i) where at[i] is not negative.  Every load comes before
+// the first store, so that the thread waits for them once (128 tiles x 384
+// channels, one component: 92 us, a pair after another, 76 so).
+template <bool OUT64, int N, class F>
+__device__ __forceinline__ void add_pairs(void* vis, const long long (&at)[N], F&& value) {
+    using V = typename std::conditional<OUT64, double2, float4>::type;
+    constexpr int NV = OUT64 ? 4 : 2;
+    V x[N][NV];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int e = 0; e < NV; e++)
+            if (at[i] >= 0) x[i][e] = reinterpret_cast<const V*>(vis)[at[i] * NV + e];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        if (at[i] < 0) continue;
+        const J2 d = value(i);
+        const cplx c[4] = {d.a, d.b, d.c, d.d};
+#pragma unroll
+        for (int e = 0; e < NV; e++) {
+            V y = x[i][e];
+            if constexpr (OUT64) {
+                y.x += c[e].re, y.y += c[e].im;
+            } else {
+                y.x += (float)c[2 * e].re, y.y += (float)c[2 * e].im;
+                y.z += (float)c[2 * e + 1].re, y.w += (float)c[2 * e + 1].im;
+            }
+            reinterpret_cast<V*>(vis)[at[i] * NV + e] = y;
+        }
+    }
+}
 
 // Tile's UVW from the array's centroid in wavelengths (ool = frequency / c).
 __device__ __forceinline__ void tile_uvw(const DirectParams& p, int tile, double ool, double& u, double& v, double& w) {
@@ -121,33 +246,33 @@ __device__ __forceinline__ cplx shapelet_env(const double* __restrict__ cm, doub
 // 2.6e-7 so).  128 tiles x 192 channels x 250 Gaussians, 17 unique tiles: 2.37
 // ms with a thread per baseline (phasors and records of 17 tiles gathered from
 // shared memory per term), 1.84 so, the FP64 pipe 0.61 busy.
-template <int TYPE, bool TILE, bool OUT64, bool FAST>
-__global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
-    constexpr int CH = Shape<TYPE, TILE>::CH;
+// H 1: three or, with per-tile beams, four CTAs an SM (65 tiles x 256 channels x
+// 200 Gaussians: 881 us at three, 826 at four; points under a shared beam are
+// slower by a tenth at four where the SMs are not full).
+template <int TYPE, bool TILE, bool OUT64, bool FAST, int H>
+__global__ void __launch_bounds__(NTH, H == 2 ? 2 : (TILE && TYPE != 2 ? 4 : 3)) pair_kernel(const DirectParams p, int first) {
+    constexpr int CH = Shape<TYPE, TILE>::CH, SLOTS = H == 2 ? 64 : GRP;
     __shared__ alignas(128) double4 s_lmn[2][CH];
     __shared__ alignas(128) JonesF64 s_flux[2][CH];
     __shared__ alignas(128) double4 s_gp[TYPE ? 2 : 1][TYPE ? CH : 1];
-    // shared beam: the phasors of the 32 row tiles, then the 32 column tiles;
+    // shared beam: the phasors of the row tiles, then the column tiles;
     // per-tile beams: M_p and N_q entries (xx, xy, yx, yy)
-    __shared__ alignas(16) double2 s_a[TILE ? 4 : 1][CH][2 * TB];
-    __shared__ alignas(16) double2 s_k[TYPE ? CH : 1][TYPE ? 2 * TB : 1];  // envelope coordinates
+    __shared__ alignas(16) double2 s_a[TILE ? 4 : 1][CH][SLOTS];
+    __shared__ alignas(16) double2 s_k[TYPE ? CH : 1][TYPE ? SLOTS : 1];  // envelope coordinates
     __shared__ alignas(16) double4 s_w[TILE ? 1 : CH];                    // xx, yy, Re xy, Im xy
     __shared__ double s_dense[TYPE == 2 ? CH * SDN * SDN : 1];
     __shared__ alignas(8) uint64_t bar[2];
 
-    const int tid = threadIdx.x, f = blockIdx.y;
-    const int nblk = (p.ntiles + TB - 1) / TB, noff = nblk * (nblk - 1) / 2;
-    // blocks off the diagonal first, then the cheaper diagonal ones
-    int pb, qb;
-    if ((int)blockIdx.x < noff)
-        baseline_to_tiles(blockIdx.x, nblk, pb, qb);
-    else
-        pb = qb = blockIdx.x - noff;
+    // H 1: the channels are the faster index, so that CTAs of one cost are
+    // spread over the SMs
+    const int tid = threadIdx.x, f = H == 2 ? blockIdx.y : blockIdx.x % p.nf;
+    const Block<H> B(H == 2 ? blockIdx.x : blockIdx.x / p.nf, p.ntiles, first);
+    if (H == 1 && B.count == 0) return;
+    const bool any = H == 2 || __any_sync(0xffffffffu, B.mine());
 
     // this thread's tile of the chunk tables: its UVW in wavelengths and, for
     // per-tile beams, its row of the beam table
-    const int slot = tid & (2 * TB - 1);
-    const int tile = slot < TB ? pb * TB + slot : qb * TB + slot - TB;
+    const int slot = tid & (SLOTS - 1), tile = B.tile(slot, p.ntiles);
     const double freq = p.freqs[f], ool = freq / VEL_C;
     double u = 0.0, v = 0.0, w = 0.0;
     const JonesF64* brow = nullptr;
@@ -158,23 +283,13 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
 
     // a diagonal block's column tiles are its row tiles: formed once (per-tile
     // beams need both M and N)
-    const bool same = !TILE && pb == qb;
+    const bool same = !TILE && B.diag;
 
-    // pairs of this thread: rows tr + 16 i, columns tc + 16 j.
-    // want[i][j] is uniform over the CTA: false where no pair of that 16 x 16
-    // quarter is a baseline.  A diagonal block's two diagonal quarters hold
-    // half as many each: they are one quarter's work, quarter (0, 0), whose
-    // threads below the diagonal take the mirrored pair of quarter (1, 1).
-    const int tr = tid >> 4, tc = tid & 15;
-    bool want[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-            want[i][j] = pb * TB + 16 * i < p.ntiles && qb * TB + 16 * j < p.ntiles && !(pb == qb && i == 1);
-    const bool mirror = pb == qb && tr > tc;
-    const int r00 = mirror ? 16 + tc : tr, c00 = mirror ? 16 + tr : tc;
-    const bool full = want[0][0] && want[0][1] && want[1][0] && want[1][1];
+    // H 2, a diagonal block: its two diagonal quarters hold half as many pairs
+    // each and are one quarter's work, pair 0, of which the threads below the
+    // diagonal take the mirrored pair of the second; pair 1 is the full quarter's
+    const bool mirror = H == 2 && B.diag && B.r > B.c - 32;
+    const int r00 = mirror ? 16 + B.c - 32 : B.r, c00 = mirror ? 48 + B.r : B.c;
 
     const int nchunks = (p.nc + CH - 1) / CH;
     if (tid == 0) {
@@ -202,13 +317,11 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
 
     // shared beam: sums of w_xx z, w_yy z, Re(w_xy) z, Im(w_xy) z; per-tile
     // beams: the four correlations
-    cplx acc[RI][2][4];
+    cplx acc[H * H][4];
 #pragma unroll
-    for (int i = 0; i < RI; i++)
+    for (int i = 0; i < H * H; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[i][j][e] = cplx{0.0, 0.0};
+        for (int e = 0; e < 4; e++) acc[i][e] = cplx{0.0, 0.0};
 
     bool aborted = false;
     for (int k = 0; k < nchunks; k++) {
@@ -217,17 +330,17 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
         const int c0 = k * CH, n = ok ? min(CH, p.nc - c0) : 0;
 
         // ---- the chunk's per-tile tables ----
-        if (!same || slot < TB) {
-            for (int c = tid / (2 * TB); c < n; c += NTH / (2 * TB)) {
+        if (tile < p.ntiles && (!same || slot < SLOTS / 2)) {
+            for (int c = tid / SLOTS; c < n; c += NTH / SLOTS) {
                 const double4 lmn = s_lmn[st][c];
                 const cplx a = phasor_quarter_f64(4.0 * (u * lmn.x + v * lmn.y + w * lmn.z));
                 if (!TILE) {
                     const double2 x = make_double2(a.re, a.im);
                     s_a[0][c][slot] = x;
-                    if (same) s_a[0][c][slot + TB] = x;
+                    if (same) s_a[0][c][slot + SLOTS / 2] = x;
                 } else {
-                    J2 b = brow ? ldg_j(brow + c0 + c) : jzero();
-                    if (slot < TB) b = b * load_j(s_flux[st][c]);
+                    J2 b = ldg_j(brow + c0 + c);
+                    if (slot < B.rs) b = b * load_j(s_flux[st][c]);
                     b = b * a;
                     s_a[0][c][slot] = make_double2(b.a.re, b.a.im);
                     s_a[TILE ? 1 : 0][c][slot] = make_double2(b.b.re, b.b.im);
@@ -241,13 +354,12 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
                         x = FAST ? make_double2(u * g.x + v * g.y, u * g.z + v * g.w)
                                  : make_double2(u * g.z + v * g.w, u * g.w - v * g.z);
                     } else {
-                        double2 q = make_double2(0.0, 0.0);
-                        if (tile < p.ntiles) q = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + tile);
+                        const double2 q = __ldg(p.suv_tile + (size_t)(c0 + c) * p.ntiles + tile);
                         const double su = q.x * ool, sv = q.y * ool;
                         x = make_double2((su * g.z + sv * g.w) * g.x, (su * g.w - sv * g.z) * g.y);
                     }
                     s_k[TYPE ? c : 0][TYPE ? slot : 0] = x;
-                    if (same) s_k[TYPE ? c : 0][TYPE ? slot + TB : 0] = x;
+                    if (same) s_k[TYPE ? c : 0][TYPE ? slot + SLOTS / 2 : 0] = x;
                 }
             }
         }
@@ -265,73 +377,69 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
         }
 
         // ---- the pairs ----
-        auto sweep = [&](auto all) {
-            for (int c = 0; c < n; c++) {
-#pragma unroll
-                for (int i = 0; i < RI; i++) {
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        constexpr bool ALL = decltype(all)::value;
-                        if (!ALL && !want[i][j]) continue;
-                        const int rp = !ALL && i + j == 0 ? r00 : tr + 16 * i;
-                        const int cq = TB + (!ALL && i + j == 0 ? c00 : tc + 16 * j);
-                        cplx env = {1.0, 0.0};
-                        if (TYPE) {
-                            const double2 kp = s_k[TYPE ? c : 0][TYPE ? rp : 0], kq = s_k[TYPE ? c : 0][TYPE ? cq : 0];
-                            const double dx = kp.x - kq.x, dy = kp.y - kq.y;
-                            if (TYPE == 1 && FAST) {
-                                env.re = (double)exp2_neg((float)fma(dx, dx, dy * dy));
-                            } else if (TYPE == 1) {
-                                const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
-                                env.re = exp(g.x * (dx * dx) + g.y * (dy * dy));
-                            } else {
-                                env = shapelet_env(s_dense + (TYPE == 2 ? c * SDN * SDN : 0), dx, dy);
-                            }
-                        }
-                        cplx(&m)[4] = acc[i][j];
-                        if (!TILE) {
-                            const double2 ap = s_a[0][c][rp], aq = s_a[0][c][cq];
-                            cplx z = {fma(ap.x, aq.x, ap.y * aq.y), fma(ap.y, aq.x, -(ap.x * aq.y))};
-                            if (TYPE == 1) z = z * env.re;
-                            if (TYPE == 2) z = z * env;
-                            const double4 wv = s_w[TILE ? 0 : c];
-                            const double we[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                m[e].re = fma(we[e], z.re, m[e].re);
-                                m[e].im = fma(we[e], z.im, m[e].im);
-                            }
-                        } else {
-                            cplx M[4], N[4];
-#pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                const double2 a = s_a[TILE ? e : 0][c][rp], b = s_a[TILE ? e : 0][c][cq];
-                                M[e] = cplx{a.x, a.y};
-                                N[e] = cplx{b.x, b.y};
-                                if (TYPE == 1) M[e] = M[e] * env.re;
-                                if (TYPE == 2) M[e] = M[e] * env;
-                            }
-#pragma unroll
-                            for (int a = 0; a < 2; a++)
-#pragma unroll
-                                for (int b = 0; b < 2; b++)
-#pragma unroll
-                                    for (int y = 0; y < 2; y++) {
-                                        // M^{ay} conj(N^{by})
-                                        const cplx x = M[2 * a + y], q = N[2 * b + y];
-                                        cplx& o = m[2 * a + b];
-                                        o.re = fma(x.re, q.re, fma(x.im, q.im, o.re));
-                                        o.im = fma(x.im, q.re, fma(-x.re, q.im, o.im));
-                                    }
-                        }
-                    }
+        auto term = [&](int c, int i, int rp, int cq) {
+            cplx env = {1.0, 0.0};
+            if (TYPE) {
+                const double2 kp = s_k[TYPE ? c : 0][TYPE ? rp : 0], kq = s_k[TYPE ? c : 0][TYPE ? cq : 0];
+                const double dx = kp.x - kq.x, dy = kp.y - kq.y;
+                if (TYPE == 1 && FAST) {
+                    env.re = (double)exp2_neg((float)fma(dx, dx, dy * dy));
+                } else if (TYPE == 1) {
+                    const double4 g = s_gp[TYPE ? st : 0][TYPE ? c : 0];
+                    env.re = exp(g.x * (dx * dx) + g.y * (dy * dy));
+                } else {
+                    env = shapelet_env(s_dense + (TYPE == 2 ? c * SDN * SDN : 0), dx, dy);
                 }
             }
+            cplx(&m)[4] = acc[i];
+            if (!TILE) {
+                const double2 ap = s_a[0][c][rp], aq = s_a[0][c][cq];
+                cplx z = {fma(ap.x, aq.x, ap.y * aq.y), fma(ap.y, aq.x, -(ap.x * aq.y))};
+                if (TYPE == 1) z = z * env.re;
+                if (TYPE == 2) z = z * env;
+                const double4 wv = s_w[TILE ? 0 : c];
+                const double we[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    m[e].re = fma(we[e], z.re, m[e].re);
+                    m[e].im = fma(we[e], z.im, m[e].im);
+                }
+            } else {
+                cplx M[4], N[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const double2 a = s_a[TILE ? e : 0][c][rp], b = s_a[TILE ? e : 0][c][cq];
+                    M[e] = cplx{a.x, a.y};
+                    N[e] = cplx{b.x, b.y};
+                    if (TYPE == 1) M[e] = M[e] * env.re;
+                    if (TYPE == 2) M[e] = M[e] * env;
+                }
+#pragma unroll
+                for (int a = 0; a < 2; a++)
+#pragma unroll
+                    for (int b = 0; b < 2; b++)
+#pragma unroll
+                        for (int y = 0; y < 2; y++) {
+                            // M^{ay} conj(N^{by})
+                            const cplx x = M[2 * a + y], q = N[2 * b + y];
+                            cplx& o = m[2 * a + b];
+                            o.re = fma(x.re, q.re, fma(x.im, q.im, o.re));
+                            o.im = fma(x.im, q.re, fma(-x.re, q.im, o.im));
+                        }
+            }
         };
-        if (full)
-            sweep(std::true_type{});
-        else
-            sweep(std::false_type{});
+        if (H == 1) {
+            for (int c = 0; c < n && any; c++) term(c, 0, B.r, B.c);
+        } else if (!B.diag) {
+            for (int c = 0; c < n; c++)
+#pragma unroll
+                for (int i = 0; i < H * H; i++) term(c, i, B.r + 16 * (i / H), B.c + 16 * (i % H));
+        } else {
+            for (int c = 0; c < n; c++) {
+                term(c, 0, r00, c00);
+                term(c, H - 1, B.r, B.c + 16);
+            }
+        }
         __syncthreads();
         if (tid == 0 && k + 2 < nchunks) {
             fence_proxy_async_smem();
@@ -340,33 +448,71 @@ __global__ void __launch_bounds__(NTH, 2) pair_kernel(const DirectParams p) {
         }
     }
 
-    if (aborted) return;
+    if (aborted || (H == 1 && !B.mine())) return;
+    long long at[H * H];
 #pragma unroll
-    for (int i = 0; i < RI; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int tp = pb * TB + (i + j == 0 ? r00 : tr + 16 * i), tq = qb * TB + (i + j == 0 ? c00 : tc + 16 * j);
-            if (!want[i][j] || tp >= tq || tq >= p.ntiles) continue;
-            const cplx(&m)[4] = acc[i][j];
-            J2 r;
-            if (TILE)
-                r = J2{m[0], m[1], m[2], m[3]};
-            else
-                r = J2{m[0], cplx{m[2].re - m[3].im, m[2].im + m[3].re}, cplx{m[2].re + m[3].im, m[2].im - m[3].re}, m[1]};
-            add_vis<OUT64>(p.vis, (size_t)f * p.nbl + baseline_index(tp, tq, p.ntiles), r);
-        }
+    for (int i = 0; i < H * H; i++) {
+        const int rp = H == 2 && i == 0 ? r00 : B.r + 16 * (i / H), cq = H == 2 && i == 0 ? c00 : B.c + 16 * (i % H);
+        at[i] = H == 2 && B.diag && i > 1 ? -1 : B.vis_index(p, f, rp, cq);
+    }
+    add_pairs<OUT64>(p.vis, at, [&](int i) {
+        const cplx(&m)[4] = acc[i];
+        if (TILE) return J2{m[0], m[1], m[2], m[3]};
+        return J2{m[0], cplx{m[2].re - m[3].im, m[2].im + m[3].re}, cplx{m[2].re + m[3].im, m[2].im - m[3].re}, m[1]};
+    });
+}
+
+// The tiles (a multiple of 32, or past the array) whose pairs with one another
+// go in blocks of 32 x 32; 0: none.  Those blocks reuse what they read from
+// shared memory, but a CTA's work is four times as much and waves of them must
+// fill the SMs: two (four for FP64 Gaussians, whose exponentials are bound by
+// the FP64 pipe either way).  60 components, us in 32 x 32 / 16 x 16 blocks, 128
+// tiles:
+//                          24 channels  64       128        384
+//   points                 39 / 39      66 / 74  104 / 123  259 / 324
+//   Gaussians              75 / 68      141 / 141  242 / 258  645 / 716
+//   Gaussians, chosen form 41 / 41      71 / 78  115 / 140  300 / 370
+//   same, per-tile beams   128 / 119    224 / 222  359 / 381  932 / 1037
+// A last group of fewer than 23 tiles goes in strips of the other launch, which
+// pays from three waves on (111 tiles x 128 channels, points: 100 / 103, the
+// chosen form's Gaussians 118 / 116; x 192 154 / 165); one of 23 or more is
+// padded (123 tiles x 128 channels, points: 105 padded, 121 with strips).
+// Shapelets evaluate their basis per pair and take 16 x 16 blocks at any size
+// (128 tiles x 384 channels x 20: 1097 / 1010 us).
+static int whole_tiles(const DirectParams& p, int type, bool f64) {
+    if (type == 2) return 0;
+    const int n = (p.ntiles + 9) / 32;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int waves = type == 1 && f64 ? 4 : (32 * n < p.ntiles ? 3 : 2);  // of two CTAs an SM
+    return (long long)n * (n + 1) / 2 * p.nf >= 2LL * waves * sms ? 32 * n : 0;
+}
+
+template <int H>
+static dim3 block_grid(const DirectParams& p, int first) {
+    const int n = num_blocks(H, p.ntiles, first);
+    return H == 2 ? dim3(n, p.nf) : dim3(n * p.nf);
+}
+
+template <int TYPE, bool TILE, bool FAST, int H>
+cudaError_t launch_h(bool out64, const DirectParams& p, int first, cudaStream_t s) {
+    const dim3 grid = block_grid<H>(p, first);
+    if (out64)
+        pair_kernel<TYPE, TILE, true, FAST, H><<<grid, NTH, 0, s>>>(p, first);
+    else
+        pair_kernel<TYPE, TILE, false, FAST, H><<<grid, NTH, 0, s>>>(p, first);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 template <int TYPE, bool TILE, bool FAST = false>
 cudaError_t launch_t(bool out64, const DirectParams& p, cudaStream_t s) {
-    const int nblk = (p.ntiles + TB - 1) / TB;
-    const dim3 grid(nblk * (nblk + 1) / 2, p.nf);
-    if (out64)
-        pair_kernel<TYPE, TILE, true, FAST><<<grid, NTH, 0, s>>>(p);
-    else
-        pair_kernel<TYPE, TILE, false, FAST><<<grid, NTH, 0, s>>>(p);
-    count_launches(1);
-    return cudaGetLastError();
+    const int first = whole_tiles(p, TYPE, !FAST);
+    if constexpr (TYPE != 2) {
+        const cudaError_t e = first ? launch_h<TYPE, TILE, FAST, 2>(out64, p, first, s) : cudaSuccess;
+        if (e != cudaSuccess) return e;
+    }
+    return first < p.ntiles ? launch_h<TYPE, TILE, FAST, 1>(out64, p, first, s) : cudaSuccess;
 }
 
 }  // namespace pairs
@@ -415,40 +561,35 @@ __device__ __forceinline__ float coarse(double x) {
     return fabsf(f) < 16384.f ? __fsub_rn(__fadd_rn(f, M), M) : f;
 }
 
+template <int H>
 struct FastSmem {
+    static constexpr int SLOTS = H == 2 ? 64 : GRP;
     double4 lmn[2][FCHUNK];
     JonesF64 flux[2][FCHUNK];
     double4 gp[2][FCHUNK];     // K = (u gp.x + v gp.y, u gp.z + v gp.w): the exponent is -|K_p - K_q|^2
-    float2 a[FCHUNK][2 * TB];  // phasors of the row tiles, then the column tiles
-    float4 k[FCHUNK][2 * TB];  // envelope coordinates (hx, hy, lx, ly), negated for column tiles
-    float4 w[FCHUNK];          // xx, yy, Re xy, Im xy
-    double2 sum[2 * RI][4][NTH];  // [pair][sum][thread]
+    float2 a[FCHUNK][SLOTS];  // phasors of the row tiles, then the column tiles
+    float4 k[FCHUNK][SLOTS];  // envelope coordinates (hx, hy, lx, ly), negated for column tiles
+    float4 w[FCHUNK];         // xx, yy, Re xy, Im xy
+    double2 sum[H * H][4][NTH];  // [pair][sum][thread]
     uint64_t bar[2];
 };
 
-template <bool OUT64>
-__global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p) {
+template <bool OUT64, int H>
+__global__ void __launch_bounds__(NTH, H == 2 ? 2 : 4) fast_gauss_kernel(const DirectParams p, int first) {
+    constexpr int SLOTS = FastSmem<H>::SLOTS;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    FastSmem& S = *reinterpret_cast<FastSmem*>(smem_raw);
-    const int tid = threadIdx.x, f = blockIdx.y;
-    const int nblk = (p.ntiles + TB - 1) / TB, noff = nblk * (nblk - 1) / 2;
-    int pb, qb;
-    if ((int)blockIdx.x < noff)
-        baseline_to_tiles(blockIdx.x, nblk, pb, qb);
-    else
-        pb = qb = blockIdx.x - noff;
+    FastSmem<H>& S = *reinterpret_cast<FastSmem<H>*>(smem_raw);
+    const int tid = threadIdx.x, f = H == 2 ? blockIdx.y : blockIdx.x % p.nf;
+    const Block<H> B(H == 2 ? blockIdx.x : blockIdx.x / p.nf, p.ntiles, first);
+    if (H == 1 && B.count == 0) return;
+    // warps without a pair have nothing to sum
+    const bool any = H == 2 || __any_sync(0xffffffffu, B.mine());
 
-    const int slot = tid & (2 * TB - 1);
-    const int tile = slot < TB ? pb * TB + slot : qb * TB + slot - TB;
+    const int slot = tid & (SLOTS - 1), tile = B.tile(slot, p.ntiles);
     const double freq = p.freqs[f], ool = freq / VEL_C;
     double u = 0.0, v = 0.0, w = 0.0;  // wavelengths
     if (tile < p.ntiles) tile_uvw(p, tile, ool, u, v, w);
-
-    const bool same = pb == qb;  // the column tiles are the row tiles
-    const int tr = pb * TB + (tid >> 4), tc = qb * TB + (tid & 15);
-    const int rp = tid >> 4, cq = TB + (tid & 15);
-    // warps whose pairs are all past the array have nothing to sum
-    const bool any = __any_sync(0xffffffffu, tr < p.ntiles && tc < p.ntiles);
+    const int rp = B.r, cq = B.c;
 
     const int nchunks = (p.nc + FCHUNK - 1) / FCHUNK;
     if (tid == 0) {
@@ -474,9 +615,9 @@ __global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p
     }
     const uint64_t limit = p.wait_ns ? p.wait_ns : 2000000000ull;
 
-    uint64_t acc[2 * RI][4];  // [pair] (re, im) of the sums of w_xx z, w_yy z, Re(w_xy) z, Im(w_xy) z
+    uint64_t acc[H * H][4];  // [pair] (re, im) of the sums of w_xx z, w_yy z, Re(w_xy) z, Im(w_xy) z
 #pragma unroll
-    for (int i = 0; i < 2 * RI; i++)
+    for (int i = 0; i < H * H; i++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[i][e] = 0;
 
@@ -490,8 +631,8 @@ __global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p
             const JonesF64 q = S.flux[st][tid];
             S.w[tid] = make_float4((float)q.j00_re, (float)q.j11_re, (float)q.j01_re, (float)q.j01_im);
         }
-        if (!same || slot < TB) {
-            for (int c = tid / (2 * TB); c < n; c += NTH / (2 * TB)) {
+        if (tile < p.ntiles && (!B.diag || slot < SLOTS / 2)) {
+            for (int c = tid / SLOTS; c < n; c += NTH / SLOTS) {
                 const double4 lmn = S.lmn[st][c], sc = S.gp[st][c];
                 float sn, cs;
                 phasor_quarter_f32(4.0 * (u * lmn.x + v * lmn.y + w * lmn.z), sn, cs);
@@ -500,10 +641,10 @@ __global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p
                 const float4 x = make_float4(hx, hy, (float)(xx.x - (double)hx), (float)(xx.y - (double)hy));
                 const float4 nx = make_float4(-x.x, -x.y, -x.z, -x.w);
                 S.a[c][slot] = make_float2(cs, sn);
-                S.k[c][slot] = slot < TB ? x : nx;
-                if (same) {
-                    S.a[c][slot + TB] = make_float2(cs, sn);
-                    S.k[c][slot + TB] = nx;
+                S.k[c][slot] = slot < B.rs ? x : nx;
+                if (B.diag) {
+                    S.a[c][slot + SLOTS / 2] = make_float2(cs, sn);
+                    S.k[c][slot + SLOTS / 2] = nx;
                 }
             }
         }
@@ -514,60 +655,62 @@ __global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p
             break;
         }
 
-        // in stages over the thread's four pairs, so that their chains (loads,
-        // exponent, exponential) overlap; a pair that is no baseline (past the
-        // array, or below the diagonal in a quarter on it) is summed like the
-        // others and not stored
+        // in stages over the thread's pairs, so that their chains (loads,
+        // exponent, exponential) overlap; a pair that is no baseline (H 2: below
+        // the diagonal in a quarter on it; H 1: past the count in a warp that
+        // holds some) is summed like the others and not stored
         auto sweep = [&](auto diag) {
             constexpr bool DIAG = decltype(diag)::value;  // the lower left quarter holds no baseline
             for (int c = 0; c < n; c++) {
                 const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(S.k[c]);
-                const ulonglong2 kq[2] = {kr[cq], kr[cq + 16]};
-                float e[2 * RI];
+                ulonglong2 kq[H];
 #pragma unroll
-                for (int i = 0; i < RI; i++) {
+                for (int j = 0; j < H; j++) kq[j] = kr[cq + 16 * j];
+                float e[H * H];
+#pragma unroll
+                for (int i = 0; i < H; i++) {
                     const ulonglong2 kp = kr[rp + 16 * i];
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
+                    for (int j = 0; j < H; j++) {
                         if (DIAG && i > j) continue;
                         // dh^2 + dl (2 dh + dl): dh exact, one rounding
                         const uint64_t dh = add2(kp.x, kq[j].x), dl = add2(kp.y, kq[j].y);
                         const float2 q = unpack2(fma2(dh, dh, mul2(dl, fma2(two, dh, dl))));
-                        e[2 * i + j] = q.x + q.y;
+                        e[H * i + j] = q.x + q.y;
                     }
                 }
                 const float4 wv = S.w[c];
                 const uint64_t w[4] = {dup2(wv.x), dup2(wv.y), dup2(wv.z), dup2(wv.w)};
-                uint64_t qx[2], qy[2];
+                uint64_t qx[H], qy[H];
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
+                for (int j = 0; j < H; j++) {
                     const float2 aq = S.a[c][cq + 16 * j];
                     qx[j] = dup2(aq.x);
                     qy[j] = dup2(aq.y);
                 }
 #pragma unroll
-                for (int i = 0; i < RI; i++) {
+                for (int i = 0; i < H; i++) {
                     const float2 ap = S.a[c][rp + 16 * i];
                     const uint64_t px = pack2(ap.x, ap.y), py = pack2(ap.y, -ap.x);
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
+                    for (int j = 0; j < H; j++) {
                         if (DIAG && i > j) continue;
-                        uint64_t(&m)[4] = acc[2 * i + j];
-                        const uint64_t z = mul2(fma2(py, qy[j], mul2(px, qx[j])), dup2(exp2_neg(e[2 * i + j])));
+                        uint64_t(&m)[4] = acc[H * i + j];
+                        const uint64_t z = mul2(fma2(py, qy[j], mul2(px, qx[j])), dup2(exp2_neg(e[H * i + j])));
 #pragma unroll
                         for (int x = 0; x < 4; x++) m[x] = fma2(w[x], z, m[x]);
                     }
                 }
             }
         };
-        if (any && same)
+        if (H == 2 && B.diag)
             sweep(std::true_type{});
         else if (any)
             sweep(std::false_type{});
         if (k % SUM == SUM - 1 || k == nchunks - 1) {
             const bool first = k < SUM;
 #pragma unroll
-            for (int i = 0; i < 2 * RI; i++)
+            for (int i = 0; i < H * H; i++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const float2 a = unpack2(acc[i][e]);
@@ -586,19 +729,18 @@ __global__ void __launch_bounds__(NTH, 2) fast_gauss_kernel(const DirectParams p
         }
     }
 
-    if (aborted) return;
+    if (aborted || (H == 1 && !B.mine())) return;
+    long long at[H * H];
 #pragma unroll
-    for (int i = 0; i < 2 * RI; i++) {
-        const int tp = tr + 16 * (i >> 1), tq = tc + 16 * (i & 1);
-        if (tp >= tq || tq >= p.ntiles) continue;
+    for (int i = 0; i < H * H; i++) at[i] = B.vis_index(p, f, rp + 16 * (i / H), cq + 16 * (i % H));
+    add_pairs<OUT64>(p.vis, at, [&](int i) {
         const double2 xx = S.sum[i][0][tid], yy = S.sum[i][1][tid], a = S.sum[i][2][tid], b = S.sum[i][3][tid];
-        add_vis<OUT64>(p.vis, (size_t)f * p.nbl + baseline_index(tp, tq, p.ntiles),
-                       J2{{xx.x, xx.y}, {a.x - b.y, a.y + b.x}, {a.x + b.y, a.y - b.x}, {yy.x, yy.y}});
-    }
+        return J2{{xx.x, xx.y}, {a.x - b.y, a.y + b.x}, {a.x + b.y, a.y - b.x}, {yy.x, yy.y}};
+    });
 }
 
-template <bool OUT64>
-cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
+template <bool OUT64, int H>
+cudaError_t launch_fast_gauss(const DirectParams& p, int first, cudaStream_t s) {
     // the opt-in above 48 KB of dynamic shared memory, once per device
     static std::atomic<bool> attr[64];
     int dev = 0;
@@ -606,15 +748,21 @@ cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr[dev].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(fast_gauss_kernel<OUT64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(FastSmem));
+        e = cudaFuncSetAttribute(fast_gauss_kernel<OUT64, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(FastSmem<H>));
         if (e != cudaSuccess) return e;
         attr[dev].store(true, std::memory_order_relaxed);
     }
-    const int nblk = (p.ntiles + TB - 1) / TB;
-    fast_gauss_kernel<OUT64><<<dim3(nblk * (nblk + 1) / 2, p.nf), NTH, sizeof(FastSmem), s>>>(p);
+    fast_gauss_kernel<OUT64, H><<<block_grid<H>(p, first), NTH, sizeof(FastSmem<H>), s>>>(p, first);
     count_launches(1);
     return cudaGetLastError();
+}
+
+template <bool OUT64>
+cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
+    const int first = whole_tiles(p, 1, false);
+    const cudaError_t e = first ? launch_fast_gauss<OUT64, 2>(p, first, s) : cudaSuccess;
+    return e != cudaSuccess || first >= p.ntiles ? e : launch_fast_gauss<OUT64, 1>(p, first, s);
 }
 
 }  // namespace pairs
