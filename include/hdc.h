@@ -500,6 +500,12 @@ const char *hdc_kernel_error_string(int word);
  * launch only; the library stays usable. */
 int hdc_test_stall_next_predict(unsigned long long wait_ns);
 
+/* Shortage-of-memory testing (no counterpart in the reference): on the calling
+ * thread, device scratch that a call can do without or with less of (the plain
+ * calibration's covariances, the tensor predict's table of per-tile beams) is
+ * treated as unavailable beyond `bytes`; 0 lifts the limit. */
+int hdc_test_limit_scratch(unsigned long long bytes);
+
 /* Per-kernel-class device time of a modeller's last calls, measured with
  * CUDA events on the launching stream when profiling is enabled.
  * out_ms[0..3] = points, Gaussians, shapelets, geometry/beam prep [ms],

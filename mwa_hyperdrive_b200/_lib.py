@@ -173,6 +173,7 @@ SIGNATURES = {
     "hdc_kernel_launches": (ctypes.c_longlong, []),
     "hdc_kernel_error_string": (c_char_p, [c_int]),
     "hdc_test_stall_next_predict": (c_int, [ctypes.c_ulonglong]),
+    "hdc_test_limit_scratch": (c_int, [ctypes.c_ulonglong]),
     "get_gpu_device_info": (c_char_p, [c_int, c_char_p, ctypes.POINTER(c_int), ctypes.POINTER(c_int),
                                        ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(c_int), ctypes.POINTER(c_int)]),
     "hdc_modeller_set_profiling": (c_int, [c_void_p, c_int]),

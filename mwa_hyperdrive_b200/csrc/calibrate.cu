@@ -1072,7 +1072,7 @@ struct PlainCov {
     PlainCov(int form, int nchan, int nblk, cudaStream_t st) : s(st) {
         if (form != HDC_CAL_PLAIN || nchan < 1) return;
         const size_t each = sizeof(double) * NCOV * BLK * (size_t)nblk;
-        int g = (int)std::min<size_t>(COV_CAP / each, (size_t)nchan), dev = 0, nsm = 0;
+        int g = (int)std::min<size_t>(std::min(COV_CAP, scratch_limit()) / each, (size_t)nchan), dev = 0, nsm = 0;
         if (g < nchan && cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && g > nsm)
             g -= g % nsm;

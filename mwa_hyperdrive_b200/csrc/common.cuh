@@ -346,6 +346,9 @@ size_t pool_idle_bytes();
 void pool_trim();
 // cudaMalloc, again with the pool's idle blocks given back where memory is short.
 cudaError_t device_malloc(void** p, size_t bytes);
+// Scratch above this many bytes that a call can do without is treated as
+// unavailable on this thread (hdc_test_limit_scratch; SIZE_MAX otherwise).
+size_t scratch_limit();
 // Device word for kernel error flags (per device, zero-initialised).
 int* device_error_word();
 // Read and clear the device error word (synchronises the stream).

@@ -1304,7 +1304,7 @@ extern "C" const char* model_points_tc(const Points* comps, const Addresses* a, 
     size_t off_ws = align256(off_map + sizeof(int) * (size_t)ntiles);
     const int nu = tile_beam ? n_uniq_tile : 0;
     size_t ws_bytes = tensor_workspace_bytes(nf, nbl, ntiles, nc, nu, false, false, false);
-    char* ws = (char*)device_scratch(align256(off_ws + ws_bytes));
+    char* ws = ws_bytes <= scratch_limit() ? (char*)device_scratch(align256(off_ws + ws_bytes)) : nullptr;
     if (!ws && tile_beam) {
         ws_bytes = tensor_workspace_bytes(nf, nbl, ntiles, nc, nu, false, false, true);
         ws = (char*)device_scratch(align256(off_ws + ws_bytes));

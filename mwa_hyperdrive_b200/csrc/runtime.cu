@@ -118,6 +118,9 @@ void pool_trim() {
     cudaMemPoolTrimTo(pool, 0);
 }
 
+static thread_local size_t g_scratch_limit = SIZE_MAX;
+size_t scratch_limit() { return g_scratch_limit; }
+
 cudaError_t device_malloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation || !current_pool()) return e;
@@ -290,6 +293,11 @@ const float4* device_shapelet_basis_pairs() {
 }
 
 }  // namespace hdc
+
+extern "C" int hdc_test_limit_scratch(unsigned long long bytes) {
+    hdc::g_scratch_limit = bytes ? (size_t)bytes : SIZE_MAX;
+    return HDC_OK;
+}
 
 extern "C" const char* hdc_last_error(void) { return hdc::g_err; }
 

@@ -1440,7 +1440,7 @@ void* Modeller::tensor_workspace(bool out64, size_t& bytes) {
         tc->ws = nullptr;
         tc->ws_bytes = 0;
         tc->ws_short = false;
-        if (device_malloc(&tc->ws, need) != cudaSuccess) {
+        if (need > scratch_limit() || device_malloc(&tc->ws, need) != cudaSuccess) {
             cudaGetLastError();
             tc->ws_short = true;
             need = least;

@@ -319,6 +319,7 @@ extern "C" {
     pub fn hdc_kernel_launches() -> c_longlong;
     pub fn hdc_kernel_error_string(word: c_int) -> *const c_char;
     pub fn hdc_test_stall_next_predict(wait_ns: c_ulonglong) -> c_int;
+    pub fn hdc_test_limit_scratch(bytes: c_ulonglong) -> c_int;
     pub fn hdc_modeller_set_profiling(m: *mut HdcModeller, enable: c_int) -> c_int;
     pub fn hdc_modeller_profile(m: *mut HdcModeller, out_ms: *mut f64, reset: c_int) -> c_int;
     pub fn hdc_probe_fp64_gflops(out_gflops: *mut f64) -> c_int;
