@@ -471,7 +471,8 @@ __device__ __forceinline__ float2 rotated(float re, float im, cplx r) {
 // Bound: the residual's and weights' one pass over memory, then FP64
 // arithmetic (two phasors a sample).  4 timesteps x 192 channels x 8128
 // baselines: 68 us for what took 680 us in seven launches.
-template <bool POINT>
+// VEC: the residual is 16-byte aligned (any alignment of float is taken).
+template <bool POINT, bool VEC>
 __global__ void __launch_bounds__(PT) seq_accumulate_kernel(const SeqArgs A, float2* __restrict__ d_lo,
                                                             float2* __restrict__ m_lo) {
     constexpr int BINS = 64, SPLIT = PT / BINS;
@@ -495,8 +496,16 @@ __global__ void __launch_bounds__(PT) seq_accumulate_kernel(const SeqArgs A, flo
                 tcur = t;
             }
             const size_t tf = (size_t)t * A.nf + f, i = tf * A.nbl + bl;
-            const float4 ra = __ldg(reinterpret_cast<const float4*>(A.resid + i));
-            const float4 rb = __ldg(reinterpret_cast<const float4*>(A.resid + i) + 1);
+            float2 xx, yy;  // the residual's
+            if (VEC) {
+                const float4 ra = __ldg(reinterpret_cast<const float4*>(A.resid + i));
+                const float4 rb = __ldg(reinterpret_cast<const float4*>(A.resid + i) + 1);
+                xx = make_float2(ra.x, ra.y), yy = make_float2(rb.z, rb.w);
+            } else {
+                const JonesF32* r = A.resid + i;
+                xx = make_float2(__ldg(&r->j00_re), __ldg(&r->j00_im));
+                yy = make_float2(__ldg(&r->j11_re), __ldg(&r->j11_im));
+            }
             const double wt = (double)__ldg(A.w + i), lam = __ldg(A.lam + f);
             float2 mx, my;
             if (POINT) {
@@ -510,7 +519,7 @@ __global__ void __launch_bounds__(PT) seq_accumulate_kernel(const SeqArgs A, flo
             const float2 io = iono_factor(c, to, lam);
             const cplx rot = phasor_turns(-dw / lam);
             mx = mul_rn(mx, io), my = mul_rn(my, io);
-            const float2 rx = rotated(ra.x, ra.y, rot), ry = rotated(rb.z, rb.w, rot);
+            const float2 rx = rotated(xx.x, xx.y, rot), ry = rotated(yy.x, yy.y, rot);
             v[0] = fma(wt, (double)__fadd_rn(rx.x, mx.x) + (double)__fadd_rn(ry.x, my.x), v[0]);
             v[1] = fma(wt, (double)__fadd_rn(rx.y, mx.y) + (double)__fadd_rn(ry.y, my.y), v[1]);
             v[2] = fma(wt, (double)mx.x + (double)my.x, v[2]);
@@ -570,10 +579,13 @@ __global__ void __launch_bounds__(PT) seq_update_kernel(const SeqArgs A) {
 
 cudaError_t seq_accumulate(const SeqArgs& A, float2* d_lo, float2* m_lo, cudaStream_t s) {
     const unsigned grid = (unsigned)(((size_t)(A.nf / A.favg) * A.nbl + 63) / 64);
+    const bool vec = (reinterpret_cast<uintptr_t>(A.resid) & 15) == 0;
     if (A.model)
-        seq_accumulate_kernel<false><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
+        vec ? seq_accumulate_kernel<false, true><<<grid, PT, 0, s>>>(A, d_lo, m_lo)
+            : seq_accumulate_kernel<false, false><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
     else
-        seq_accumulate_kernel<true><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
+        vec ? seq_accumulate_kernel<true, true><<<grid, PT, 0, s>>>(A, d_lo, m_lo)
+            : seq_accumulate_kernel<true, false><<<grid, PT, 0, s>>>(A, d_lo, m_lo);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -577,6 +577,10 @@ extern "C" int hdc_peel_timeblock_batched(JonesF32* d_resid_tfb, const float* d_
                   favg);
         return HDC_ERR_ARG;
     }
+    if (reinterpret_cast<uintptr_t>(d_resid_tfb) & 15) {
+        set_error("hdc_peel_timeblock_batched: the residual's address is not a multiple of 16 bytes");
+        return HDC_ERR_ARG;
+    }
     if (num_sources == 0) return HDC_OK;
     const int nt = num_timesteps, nf = num_freqs, nbl = num_tiles * (num_tiles - 1) / 2, nlo = nf / favg;
     const int ns = num_sources;
