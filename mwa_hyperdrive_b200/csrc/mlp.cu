@@ -237,10 +237,11 @@ struct Net {
     size_t nparams = 0;
     std::vector<size_t> w_off, b_off;
     // activations for training (acts[0] is unused: layer 0 reads the caller's
-    // input) and the gradient's parts per batch split
+    // input), and the gradient's parts per batch split
     std::vector<float*> acts, deltas;
-    float* d_part = nullptr;
     int cap_batch = 0;
+    float* d_part = nullptr;
+    int cap_splits = 0;
     double* d_loss = nullptr;
     long long step = 0;
 
@@ -254,8 +255,6 @@ struct Net {
     void free_acts() {
         for (float* p : acts) cudaFree(p);
         for (float* p : deltas) cudaFree(p);
-        cudaFree(d_part);
-        d_part = nullptr;
         acts.clear();
         deltas.clear();
         cap_batch = 0;
@@ -264,7 +263,7 @@ struct Net {
     int ensure(int batch) {
         if (batch <= cap_batch) return HDC_OK;
         free_acts();
-        bool ok = cudaMalloc(&d_part, sizeof(float) * nparams * splits(batch)) == cudaSuccess;
+        bool ok = true;
         for (int l = 0; l <= layers(); l++) {
             float *a = nullptr, *d = nullptr;
             if (l > 0) {
@@ -284,8 +283,26 @@ struct Net {
         return HDC_OK;
     }
 
+    // the gradient's parts, which a network that only predicts does without
+    int ensure_parts(int batch) {
+        const int n = splits(batch);
+        if (n <= cap_splits) return HDC_OK;
+        cudaFree(d_part);
+        d_part = nullptr;
+        cap_splits = 0;
+        if (cudaMalloc(&d_part, sizeof(float) * nparams * n) != cudaSuccess) {
+            cudaGetLastError();
+            d_part = nullptr;
+            set_error("mlp: gradient allocation failed");
+            return HDC_ERR_ALLOC;
+        }
+        cap_splits = n;
+        return HDC_OK;
+    }
+
     ~Net() {
         free_acts();
+        cudaFree(d_part);
         cudaFree(d_params);
         cudaFree(d_grads);
         cudaFree(d_m);
@@ -317,6 +334,8 @@ struct Net {
     int backward(const float* d_x, const float* d_target, int batch, double* h_loss, cudaStream_t s) {
         const int L = layers();
         const int n = batch * dims[L];
+        const int rc = ensure_parts(batch);
+        if (rc) return rc;
         HDC_CUDA_RET_INT(cudaMemsetAsync(d_loss, 0, sizeof(double), s));
         mse_grad_kernel<<<(n + 255) / 256, 256, 0, s>>>(acts[L], d_target, deltas[L], n, 1.f / (float)n, d_loss);
         count_launches(1);
