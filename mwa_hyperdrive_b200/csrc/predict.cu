@@ -785,18 +785,23 @@ static cudaError_t launch_fast_tile(const DirectParams& p, cudaStream_t s) {
 // FEW_POINTS of them (five, a few registers spilled in the loop).  128 tiles x
 // 384 channels, us at three CTAs / four / five: 1 point 86 / 75 / 66, 2 90 / 79 /
 // 73, 8 128 / 124 / 125, 64 703 / 694 / 729, 400 4275 / 4222 / 4434.
+// Per-tile beams: two CTAs, with the registers to load a component's two beams
+// ahead of its phasor (three for up to FEW_POINTS points).  128 tiles x 64
+// channels, 16 unique tiles, us at three (80 registers, some spilled) / two: 3
+// points 49 / 56, 120 points 1201 / 1113, 120 Gaussians 1164 / 1135, 120 shapelets
+// 2647 / 2276.
 constexpr int FEW_POINTS = 4;
 template <int TYPE, bool TILE_BEAM, bool OUT64>
 static void launch_direct_kernel(const DirectParams& p, cudaStream_t s) {
     const dim3 grid((p.nbl + DT - 1) / DT, p.nf);
-    if constexpr (TYPE == 0 && !TILE_BEAM) {
-        if (p.nc <= FEW_POINTS)
-            direct_kernel<TYPE, TILE_BEAM, OUT64, 5><<<grid, DT, 0, s>>>(p);
-        else
-            direct_kernel<TYPE, TILE_BEAM, OUT64, 4><<<grid, DT, 0, s>>>(p);
-    } else {
-        direct_kernel<TYPE, TILE_BEAM, OUT64, 0><<<grid, DT, 0, s>>>(p);
+    constexpr int MINB = TILE_BEAM ? 2 : (TYPE == 0 ? 4 : 0), FEW = TILE_BEAM ? 3 : 5;
+    if constexpr (TYPE == 0) {
+        if (p.nc <= FEW_POINTS) {
+            direct_kernel<TYPE, TILE_BEAM, OUT64, FEW><<<grid, DT, 0, s>>>(p);
+            return;
+        }
     }
+    direct_kernel<TYPE, TILE_BEAM, OUT64, MINB><<<grid, DT, 0, s>>>(p);
 }
 
 template <int TYPE>
