@@ -464,28 +464,36 @@ __global__ void __launch_bounds__(NTH, H == 2 ? 2 : (TILE && TYPE != 2 ? 4 : 3))
 
 // The tiles (a multiple of 32, or past the array) whose pairs with one another
 // go in blocks of 32 x 32; 0: none.  Those blocks reuse what they read from
-// shared memory, but a CTA's work is four times as much and waves of them must
-// fill the SMs: two (four for FP64 Gaussians, whose exponentials are bound by
-// the FP64 pipe either way).  60 components, us in 32 x 32 / 16 x 16 blocks, 128
-// tiles:
-//                          24 channels  64       128        384
-//   points                 39 / 39      66 / 74  104 / 123  259 / 324
+// shared memory, but a CTA's work is four times as much, so that they need
+// enough of them for each SM: twice as many for FP64 Gaussians, whose
+// exponentials are bound by the FP64 pipe either way, fewer for the points.  60
+// components, us in 32 x 32 / 16 x 16 blocks, 128 tiles:
+//                          24 channels  64         128        384
+//   points                 39 / 39      66 / 74    104 / 123  259 / 324
 //   Gaussians              75 / 68      141 / 141  242 / 258  645 / 716
-//   Gaussians, chosen form 41 / 41      71 / 78  115 / 140  300 / 370
+//   Gaussians, chosen form 41 / 41      71 / 78    115 / 140  300 / 370
 //   same, per-tile beams   128 / 119    224 / 222  359 / 381  932 / 1037
-// A last group of fewer than 23 tiles goes in strips of the other launch, which
-// pays from three waves on (111 tiles x 128 channels, points: 100 / 103, the
-// chosen form's Gaussians 118 / 116; x 192 154 / 165); one of 23 or more is
-// padded (123 tiles x 128 channels, points: 105 padded, 121 with strips).
+// (2534 points, 151 tiles x 28 channels: 1241 / 1388.)  A last group of fewer
+// than 23 tiles goes in strips of the other launch, which pays later (111 tiles
+// x 128 channels, points: 100 / 103, Gaussians of the chosen form 118 / 116, with
+// per-tile beams 350 / 330); one of 23 or more is padded (123 tiles x 128
+// channels, points: 105 padded, 121 with strips).
 // Shapelets evaluate their basis per pair and take 16 x 16 blocks at any size
 // (128 tiles x 384 channels x 20: 1097 / 1010 us).
-static int whole_tiles(const DirectParams& p, int type, bool f64) {
+static int whole_tiles(const DirectParams& p, int type, bool tile_beam, bool fast) {
     if (type == 2) return 0;
     const int n = (p.ntiles + 9) / 32;
+    const bool strips = 32 * n < p.ntiles;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int waves = type == 1 && f64 ? 4 : (32 * n < p.ntiles ? 3 : 2);  // of two CTAs an SM
-    return (long long)n * (n + 1) / 2 * p.nf >= 2LL * waves * sms ? 32 * n : 0;
+    double ctas;  // blocks of 32 x 32 per SM from which they pay
+    if (type == 1 && !fast)
+        ctas = 8.0;
+    else if (tile_beam)
+        ctas = strips ? 6.0 : 4.0;
+    else
+        ctas = type == 0 && !strips ? 2.5 : 4.0;
+    return 0.5 * n * (n + 1) * p.nf >= ctas * sms ? 32 * n : 0;
 }
 
 template <int H>
@@ -507,7 +515,7 @@ cudaError_t launch_h(bool out64, const DirectParams& p, int first, cudaStream_t 
 
 template <int TYPE, bool TILE, bool FAST = false>
 cudaError_t launch_t(bool out64, const DirectParams& p, cudaStream_t s) {
-    const int first = whole_tiles(p, TYPE, !FAST);
+    const int first = whole_tiles(p, TYPE, TILE, FAST);
     if constexpr (TYPE != 2) {
         const cudaError_t e = first ? launch_h<TYPE, TILE, FAST, 2>(out64, p, first, s) : cudaSuccess;
         if (e != cudaSuccess) return e;
@@ -760,7 +768,7 @@ cudaError_t launch_fast_gauss(const DirectParams& p, int first, cudaStream_t s) 
 
 template <bool OUT64>
 cudaError_t launch_fast_gauss(const DirectParams& p, cudaStream_t s) {
-    const int first = whole_tiles(p, 1, false);
+    const int first = whole_tiles(p, 1, false, true);
     const cudaError_t e = first ? launch_fast_gauss<OUT64, 2>(p, first, s) : cudaSuccess;
     return e != cudaSuccess || first >= p.ntiles ? e : launch_fast_gauss<OUT64, 1>(p, first, s);
 }
