@@ -329,13 +329,11 @@ struct Net {
         return HDC_OK;
     }
 
-    // gradients of the mean squared error into d_grads after forward() of the
-    // same d_x; loss (sum of squares / n) to *loss
+    // gradients of the mean squared error into d_grads after ensure_parts() and
+    // forward() of the same d_x; loss (sum of squares / n) to *loss
     int backward(const float* d_x, const float* d_target, int batch, double* h_loss, cudaStream_t s) {
         const int L = layers();
         const int n = batch * dims[L];
-        const int rc = ensure_parts(batch);
-        if (rc) return rc;
         HDC_CUDA_RET_INT(cudaMemsetAsync(d_loss, 0, sizeof(double), s));
         mse_grad_kernel<<<(n + 255) / 256, 256, 0, s>>>(acts[L], d_target, deltas[L], n, 1.f / (float)n, d_loss);
         count_launches(1);
@@ -471,7 +469,9 @@ extern "C" int hdc_mlp_gradients(HdcMlp* hm, const float* d_x, const float* d_ta
                                  double* h_loss, hdcStream_t stream) {
     Net* n = reinterpret_cast<Net*>(hm);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = n->forward(d_x, batch, nullptr, s);
+    int rc = n->ensure_parts(batch);
+    if (rc) return rc;
+    rc = n->forward(d_x, batch, nullptr, s);
     if (rc) return rc;
     rc = n->backward(d_x, d_target, batch, h_loss, s);
     if (rc) return rc;
@@ -486,7 +486,9 @@ extern "C" int hdc_mlp_train_step(HdcMlp* hm, const float* d_x, const float* d_t
                                   double* h_loss, hdcStream_t stream) {
     Net* n = reinterpret_cast<Net*>(hm);
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = n->forward(d_x, batch, nullptr, s);
+    int rc = n->ensure_parts(batch);
+    if (rc) return rc;
+    rc = n->forward(d_x, batch, nullptr, s);
     if (rc) return rc;
     rc = n->backward(d_x, d_target, batch, h_loss, s);
     if (rc) return rc;
