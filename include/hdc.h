@@ -357,7 +357,7 @@ int hdc_source_brightness(const HdcSkyModel *sky, const int *h_comp_source, int 
                           double source_dist_cutoff_rad, double min_elevation_rad, double *h_brightness);
 
 /* Precision form of the point-source predict. */
-#define HDC_PREDICT_DIRECT 0     /* FP64 direct per-baseline kernel (the plain form) */
+#define HDC_PREDICT_DIRECT 0     /* the plain form: every value in FP64 */
 #define HDC_PREDICT_TENSOR 1     /* factored tcgen05 contraction (points only) */
 
 /* Polarisations (context/mod.rs:26): 0 XX_XY_YX_YY, 1 XX, 2 YY, 3 XX_YY,

@@ -1061,9 +1061,12 @@ static cudaStream_t capture_stream() {
 // needs no atomics.  Two timeblocks of 5 timesteps, 100 chanblocks of 113
 // tiles: 11.7 -> 3.9 ms; one timestep 4.6 -> 3.1 ms; 24 chanblocks, 8
 // timesteps 8.0 -> 2.0 ms.  The covariances live in call-scoped scratch of at
-// most COV_CAP bytes, group after group of chanblocks (whole waves of the SMs
-// where it holds one); where it cannot be had the data and model are streamed
-// each iteration.
+// most COV_CAP bytes, group after group of chanblocks: whole waves of the SMs
+// where it holds one.  From about 190 tiles a chanblock's covariances are so
+// large that a group leaves SMs idle (256 tiles: groups of 80), and still takes
+// less than the streaming kernel on all of them: 148 chanblocks, one timestep,
+// 256 tiles 17.9 -> 12.2 ms, 200 tiles 11.1 -> 9.3.  Where the scratch for a
+// whole group cannot be had the data and model are streamed each iteration.
 constexpr size_t COV_CAP = (size_t)1 << 30;
 struct PlainCov {
     void* p = nullptr;

@@ -242,8 +242,7 @@ constexpr double QMAGIC = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds t
 // rint(z) and r = z - q are exact; sin and cos of (pi/2) r on |r| <= 1/2 from
 // polynomials in r^2 (interpolated at Chebyshev nodes by
 // mwa_hyperdrive_b200/phasor_poly.py, within an ulp); the quadrant q mod 4
-// swaps and signs them.  18 FP64 operations, where sincospi takes about 40
-// and twice the integer ones.
+// swaps and signs them.  18 FP64 operations.
 constexpr double QS0 = 1.57079632679489656e+00, QS1 = -6.45964097506244284e-01, QS2 = 7.96926262460435075e-02,
                  QS3 = -4.68175413235088697e-03, QS4 = 1.60441150826272252e-04, QS5 = -3.59864367056375883e-06,
                  QS6 = 5.63397775242345925e-08;

@@ -23,11 +23,12 @@
 // channels x 1000 points: 13.2 ms with a thread per baseline, 4.3 with the
 // library's sincospi, 4.0 with this kernel's polynomials (1 x 2 pairs a thread
 // 4.3, 4 x 2 at half the warps 4.8), 3.7 with a diagonal block's two half-full
-// quarters summed as one.  Every value is FP64, tile positions are taken from
-// the array's centroid (so a tile's phase is no larger than its baselines'),
-// and sums run over the components in order.
+// quarters summed as one, 3.5 with those blocks last.  Every value is FP64,
+// tile positions are taken from the array's centroid (so a tile's phase is no
+// larger than its baselines'), and sums run over the components in order.
 // The drop-in calls keep the per-baseline kernel (predict.cu): their UVWs
-// are the caller's and need not be tile differences.
+// are the caller's and need not be tile differences.  So do one or two
+// components, which do not pay for the tables (launch_direct).
 
 #include <atomic>
 #include <type_traits>

@@ -19,7 +19,7 @@
 //      source and <.> the weighted mean over the timeblock and each channel
 //      group (the reference's rotate, add_model and vis_average_tfb);
 //   2. all sources' iono_loop fits in one launch per iteration
-//      (iono_loop_batched_on, the reference's arithmetic);
+//      (iono_traces_kernel over iono_fit, the reference's arithmetic);
 //   3. apply sweep: R += sum_s conj(rot_s) M_s (iono_s(old) - iono_s(new))
 //      (the reference's subtract_iono, rotated back).
 // Every phase on a baseline is a difference of per-tile phases (uvw_pq =

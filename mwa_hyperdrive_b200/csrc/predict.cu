@@ -7,9 +7,10 @@
 // parameters) are streamed through shared memory in chunks by the TMA engine
 // (cp.async.bulk) with a two-stage mbarrier pipeline; every thread reads them
 // as broadcasts.  The phase 2 pi (u l + v m + w (n - 1)) is formed in turns
-// and range-reduced exactly in FP64 (t - rint(t)) before sincospi; the
-// accumulation is FP64 and the visibility is updated once per type, as the
-// reference does (model/cpu.rs:341-348, gpu/model.cu:171).
+// and range-reduced exactly in FP64, its sine and cosine are polynomials
+// (phasor_quarter_f64); the accumulation is FP64 and the visibility is updated
+// once per type, as the reference does (model/cpu.rs:341-348,
+// gpu/model.cu:171).
 
 #include <atomic>
 #include <climits>
@@ -865,8 +866,8 @@ cudaError_t launch_direct(int ty, bool tile_beam, bool out64, const DirectParams
            (!tile_beam || (ty != 0 && p.n_uniq_tile > 0 && p.n_uniq_tile <= FT_MAX_NU && !p.unflagged_map));
     if (fast && ty == 2 && p.sdense && !p.sbfp) return cudaErrorInvalidValue;
     // UVWs that are tile differences: the FP64 form factored by tile (128
-    // tiles x 384 channels: 1000 points 13.2 -> 3.7 ms, 120 Gaussians 2.35 ->
-    // 1.22 ms, 24 shapelets 4.52 -> 1.29 ms).  Shapelets with an order of SDN
+    // tiles x 384 channels: 1000 points 13.2 -> 3.5 ms, 120 Gaussians 2.35 ->
+    // 1.22 ms, 24 shapelets 4.52 -> 1.21 ms).  Shapelets with an order of SDN
     // or more keep the per-baseline kernel, which reads the basis table per
     // coefficient.
     // One or two points or Gaussians under a shared beam do not pay for per-tile

@@ -31,10 +31,12 @@ struct DirectParams {
     // shapelets
     const double* sbf;  // [SBF_N][SBF_L]
     const float* sbf32; // the same table in FP32 (chosen form), or NULL
-    // chosen form, orders below SDN: the table as FP32 (value, next - value)
-    // pairs, position-major [SBF_L][SDN / 2] float4, and per component a dense SDN x SDN coefficient
-    // matrix [nc][n1][n2] with the sign of i^(n1+n2) folded in; NULL when
-    // some coefficient's order is SDN or more
+    // chosen form, orders below SDN: the table in FP32, position-major
+    // [SBF_L][SDN / 2] float4, each (v, v', d, d') of two neighbouring orders
+    // with v the value at the position and d the next position's less v; and
+    // per component a dense SDN x SDN coefficient matrix [nc][n1][n2] with the
+    // sign of i^(n1+n2) folded in; NULL when some coefficient's order is SDN or
+    // more
     const float4* sbfp;
     const float* sdense;
     const ShapeletCoeff* coeffs;
