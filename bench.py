@@ -1022,8 +1022,8 @@ def guarded(fn, args):
 # timestep) once from DRAM.
 NCU_TRAFFIC_SOURCE = "ncu launch list of this bench command (launch-list summary of the predict kernels)"
 NCU_DRAM_BYTES_PER_LAUNCH = {
-    ("points", "tensor"): 2927e6, ("gaussians", "tensor"): 156.0e6, ("shapelets", "tensor"): 164.5e6,
-    ("points", "direct"): 268.0e6, ("gaussians", "direct"): 152.0e6, ("shapelets", "direct"): 142.0e6,
+    ("points", "tensor"): 2931.8e6, ("gaussians", "tensor"): 152.1e6, ("shapelets", "tensor"): 141.5e6,
+    ("points", "direct"): 260.1e6, ("gaussians", "direct"): 153.3e6, ("shapelets", "direct"): 145.1e6,
 }
 
 
@@ -1145,7 +1145,6 @@ def gpu_arm(args, rank, world, local_rank):
     npts = int(np.sum(sky.comp_type == 0))
     nga = int(np.sum(sky.comp_type == 1))
     nsh = int(np.sum(sky.comp_type == 2))
-    ncoef = int(np.sum(sky.coeff_count))
     launches_per_step = nt
     g64, g32 = ctypes.c_double(), ctypes.c_double()
     _lib.check(L.hdc_probe_fp64_gflops(ctypes.byref(g64)), "fp64 probe")
@@ -1163,11 +1162,16 @@ def gpu_arm(args, rank, world, local_rank):
                      "peak": peaks.get("bf16_tflops", 1590.0),
                      "peak_source": "MEASURED_PEAKS.json bf16 burst" if peaks else "fallback 1590 TFLOP/s"}
         else:
-            # algorithmic FLOPs per visibility-component: phase 5 + Jones x phasor 24 + accumulate 8;
-            # Gaussians +10 (envelope); shapelets +12 per coefficient
-            fl_per = {0: 37.0, 1: 47.0, 2: 37.0 + 12.0 * ncoef / max(nsh, 1)}[k]
-            flops = fl_per * nbl * nf * ncomp
+            # the operations that the kernels execute per visibility and component in the stated precision (a
+            # fused multiply-add is 2; exponentials, conversions and index work not counted).  FP64, by tile
+            # pairs: phasor product 6 + sums 16; Gaussians +9 (coordinates, exponent, envelope); shapelets +200
+            # (two bases of 48, 6 x 6 contraction 96, coordinates and envelope 8); of a tile's phasor and
+            # coordinates, 37 to 47, one in 16 (blocks of 32 x 32 pairs) or 8 (16 x 16, shapelets).  FP32: Gaussians
+            # exponent 15 + phasor and envelope 8 + sums 16 + a sixteenth of a phasor's 16; shapelets bases 24 +
+            # contraction 82 + phasor and envelope 22 + sums 16
             fast = form == "tensor"
+            fl_per = {1: 40.0, 2: 144.0}[k] if fast else {0: 22 + 37 / 16, 1: 31 + 43 / 16, 2: 222 + 47 / 8}[k]
+            flops = fl_per * nbl * nf * ncomp
             entry = {"bound": "fp32" if fast else "fp64",
                      "kernel": (f"{'fast_gauss' if k == 1 else 'fast_shapelet'}_kernel ({names[k]}, FP32 form)" if fast
                                 else f"pair_kernel ({names[k]}, FP64)"),
@@ -1177,9 +1181,9 @@ def gpu_arm(args, rank, world, local_rank):
         entry.update({"achieved": flops / t_launch / 1e12, "unit": "TFLOP/s", "traffic": traffic,
                       "traffic_source": NCU_TRAFFIC_SOURCE if traffic else None, "ms_per_step": per_step_ms[k]})
         if k == 0 and form == "tensor":
-            # what the tensor pipe executes: 18 kind::i8 MMAs of 128 x 128 x 32 per 32-component stage of each
-            # (channel, polarisation, column block) CTA, against 8190 int8 MAC/clk/SM (a probe of back-to-back
-            # kind::i8 MMAs) at this run's median SM clock
+            # what the tensor pipe executes: 18 plane products of 128 x 128 x 32 (issued as 10 kind::i8 MMAs, most
+            # of 256 columns) per 32-component stage of each (channel, polarisation, column block) CTA, against
+            # 8190 int8 MAC/clk/SM (a probe of back-to-back kind::i8 MMAs) at this run's median SM clock
             macs = nf * 6 * ((npts + 31) // 32) * 18 * 128 * 128 * 32
             n_sm = torch.cuda.get_device_properties(0).multi_processor_count
             mhz = (clk or {}).get("sm_mhz") or 1965.0
@@ -1196,7 +1200,7 @@ def gpu_arm(args, rank, world, local_rank):
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_chosen, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f64" if form == "direct" else "f64 phases, s8 digit planes with exact s32 accumulation (points); f32 terms with f64 arguments and chunk sums (Gaussians, shapelets)",
+            "vs_baseline": None, "dtype": "f64" if form == "direct" else "f64 phases, s8 digit planes with exact s32 accumulation (points); f32 terms of f64 phases and coordinates (a Gaussian's held as two f32) with f64 chunk sums (Gaussians, shapelets)",
             "data": "synthetic (seeded)", "config": config_dict(obs, sky, form),
             "plain": {"form": "direct", "value": work * world / (ms_plain * 1e-3), "ms_per_step": ms_plain},
             "e2e": None if e2e_s is None else {"value": work * world / e2e_s, "unit": UNIT,
